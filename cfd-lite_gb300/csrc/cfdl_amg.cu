@@ -778,6 +778,7 @@ __global__ void __launch_bounds__(kTile) k_apc_init(const CaseDev *__restrict__ 
     const Tile t = tiles[blockIdx.x];
     const CaseDev &C = cases[t.c];
     SolveScalars *S = C.sc;
+    const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     if (S->halted) return;
     double v[2] = {0, 0};
     FOR_CELLS(t) {
@@ -785,10 +786,8 @@ __global__ void __launch_bounds__(kTile) k_apc_init(const CaseDev *__restrict__ 
         C.kr[i] = r; C.phic[i] = 0.0;
         v[0] += r * r; v[1] += C.b[i] * C.b[i];
     }
-    block_reduce<2>(v, &partials[(size_t)blockIdx.x * kNPart]);
-    if (last_tile_of_case(&C.counters[CNT_A0], cnt[t.c])) {
-        __shared__ double s[2];
-        sum_partials<2>(partials, cfirst[t.c], cnt[t.c], s);
+    __shared__ double s[2];
+    if (case_sums<2>(v, &C.counters[CNT_A0], partials, tile0, ntiles, s)) {
         if (threadIdx.x == 0) {
             const int cap = C.solve_mode == 0 ? C.nit : C.tight_maxit;
             S->r0norm_p = S->rnorm_p = sqrt(s[0]);
@@ -808,15 +807,14 @@ __global__ void __launch_bounds__(kTile) k_apc_rz(const CaseDev *__restrict__ ca
     const Tile t = tiles[blockIdx.x];
     const CaseDev &C = cases[t.c];
     SolveScalars *S = C.sc;
+    const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     if (!S->active_p) return;
     // one row per step in FP64: the paired form (cg_rz_rows) measured slower
     // here (21.4 against 18.8 us a launch at 128^3)
     double v[1] = {0.0};
     FOR_CELLS(t) v[0] += C.kr[i] * C.ks[i];
-    block_reduce<1>(v, &partials[(size_t)blockIdx.x * kNPart]);
-    if (last_tile_of_case(&C.counters[CNT_A1], cnt[t.c])) {
-        __shared__ double s[1];
-        sum_partials<1>(partials, cfirst[t.c], cnt[t.c], s);
+    __shared__ double s[1];
+    if (case_sums<1>(v, &C.counters[CNT_A1], partials, tile0, ntiles, s)) {
         if (threadIdx.x == 0) {
             S->beta_p = S->iters_p == 0 || S->rz == 0.0 ? 0.0 : s[0] / S->rz;
             S->rz = s[0];
@@ -842,12 +840,11 @@ __global__ void __launch_bounds__(kTile) k_apc_q(const CaseDev *__restrict__ cas
     const Tile t = tiles[blockIdx.x];
     const CaseDev &C = cases[t.c];
     SolveScalars *S = C.sc;
+    const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     if (!S->active_p) return;
     double v[1] = {cg_aq_rows<double, false>(level<double>(C, 0), C.kp, C.kv, t)};
-    block_reduce<1>(v, &partials[(size_t)blockIdx.x * kNPart]);
-    if (last_tile_of_case(&C.counters[CNT_A2], cnt[t.c])) {
-        __shared__ double s[1];
-        sum_partials<1>(partials, cfirst[t.c], cnt[t.c], s);
+    __shared__ double s[1];
+    if (case_sums<1>(v, &C.counters[CNT_A2], partials, tile0, ntiles, s)) {
         if (threadIdx.x == 0) {
             if (!(s[0] > 0.0) || !isfinite(s[0])) {
                 // runs only while ||r|| is above the tolerance, where p.Ap > 0 for the SPD system
@@ -866,6 +863,7 @@ __global__ void __launch_bounds__(kTile) k_apc_x(const CaseDev *__restrict__ cas
     const Tile t = tiles[blockIdx.x];
     const CaseDev &C = cases[t.c];
     SolveScalars *S = C.sc;
+    const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     if (!S->active_p) return;
     // one row per step in FP64: the paired form (cg_x_rows, 48 registers
     // against 32) measured slower here (31.9 against 28.5 us a launch)
@@ -877,10 +875,8 @@ __global__ void __launch_bounds__(kTile) k_apc_x(const CaseDev *__restrict__ cas
         C.kr[i] = r;
         v[0] += r * r;
     }
-    block_reduce<1>(v, &partials[(size_t)blockIdx.x * kNPart]);
-    if (last_tile_of_case(&C.counters[CNT_A3], cnt[t.c])) {
-        __shared__ double s[1];
-        sum_partials<1>(partials, cfirst[t.c], cnt[t.c], s);
+    __shared__ double s[1];
+    if (case_sums<1>(v, &C.counters[CNT_A3], partials, tile0, ntiles, s)) {
         if (threadIdx.x == 0) {
             const int cap = C.solve_mode == 0 ? C.nit : C.tight_maxit;
             const double rn = sqrt(s[0]);
@@ -1284,6 +1280,7 @@ __global__ void __launch_bounds__(kTile) k_mx_init(const CaseDev *__restrict__ c
     const Tile t = tiles[blockIdx.x];
     const CaseDev &C = cases[t.c];
     SolveScalars *S = C.sc;
+    const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     if (S->halted) return;
     double v[2] = {0, 0};
     FOR_CELLS(t) {
@@ -1291,10 +1288,8 @@ __global__ void __launch_bounds__(kTile) k_mx_init(const CaseDev *__restrict__ c
         C.kr[i] = r; C.phic[i] = 0.0;
         v[0] += r * r; v[1] += C.b[i] * C.b[i];
     }
-    block_reduce<2>(v, &partials[(size_t)blockIdx.x * kNPart]);
-    if (last_tile_of_case(&C.counters[CNT_A0], cnt[t.c])) {
-        __shared__ double s[2];
-        sum_partials<2>(partials, cfirst[t.c], cnt[t.c], s);
+    __shared__ double s[2];
+    if (case_sums<2>(v, &C.counters[CNT_A0], partials, tile0, ntiles, s)) {
         if (threadIdx.x == 0) {
             S->r0norm_p = S->rnorm_p = sqrt(s[0]);
             S->mass_imbalance = sqrt(s[1]);
@@ -1313,6 +1308,7 @@ __global__ void __launch_bounds__(kTile) k_mx_start(const CaseDev *__restrict__ 
     const Tile t = tiles[blockIdx.x];
     const CaseDev &C = cases[t.c];
     SolveScalars *S = C.sc;
+    const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     if (!S->active_p) return;
     float v[1] = {0.f};
     FOR_CELLS(t) {
@@ -1320,10 +1316,8 @@ __global__ void __launch_bounds__(kTile) k_mx_start(const CaseDev *__restrict__ 
         C.fr[i] = r; C.fx[i] = 0.f;
         v[0] += r * r;
     }
-    block_reduce<1, float>(v, &partials[(size_t)blockIdx.x * kNPart]);
-    if (last_tile_of_case(&C.counters[CNT_A1], cnt[t.c])) {
-        __shared__ float s[1];
-        sum_partials<1, float>(partials, cfirst[t.c], cnt[t.c], s);
+    __shared__ float s[1];
+    if (case_sums<1>(v, &C.counters[CNT_A1], partials, tile0, ntiles, s)) {
         if (threadIdx.x == 0) {
             const float rn = sqrtf(s[0]);
             // inner tolerance: the reference's drop in mode 0; when tight, half the
@@ -1355,12 +1349,11 @@ __global__ void __launch_bounds__(kTile) k_mx_rz(const CaseDev *__restrict__ cas
     const Tile t = tiles[blockIdx.x];
     const CaseDev &C = cases[t.c];
     SolveScalars *S = C.sc;
+    const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     if (!S->active32) return;
     float v[1] = {cg_rz_rows<float>(C.fr, C.fz, t)};
-    block_reduce<1, float>(v, &partials[(size_t)blockIdx.x * kNPart]);
-    if (last_tile_of_case(&C.counters[CNT_A2], cnt[t.c])) {
-        __shared__ float s[1];
-        sum_partials<1, float>(partials, cfirst[t.c], cnt[t.c], s);
+    __shared__ float s[1];
+    if (case_sums<1>(v, &C.counters[CNT_A2], partials, tile0, ntiles, s)) {
         if (threadIdx.x == 0) {
             S->beta32 = S->iters32 == 0 || S->rz32 == 0.f ? 0.f : s[0] / S->rz32;
             S->rz32 = s[0];
@@ -1385,12 +1378,11 @@ __global__ void __launch_bounds__(kTile) k_mx_q(const CaseDev *__restrict__ case
     const Tile t = tiles[blockIdx.x];
     const CaseDev &C = cases[t.c];
     SolveScalars *S = C.sc;
+    const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     if (!S->active32) return;
     float v[1] = {cg_aq_rows<float, k16>(level<float>(C, 0), C.fp, C.fq, t)};
-    block_reduce<1, float>(v, &partials[(size_t)blockIdx.x * kNPart]);
-    if (last_tile_of_case(&C.counters[CNT_A3], cnt[t.c])) {
-        __shared__ float s[1];
-        sum_partials<1, float>(partials, cfirst[t.c], cnt[t.c], s);
+    __shared__ float s[1];
+    if (case_sums<1>(v, &C.counters[CNT_A3], partials, tile0, ntiles, s)) {
         if (threadIdx.x == 0) {
             if (!(s[0] > 0.f) || !isfinite(s[0])) S->active32 = 0;
             else S->alpha32 = S->rz32 / s[0];
@@ -1404,12 +1396,11 @@ __global__ void __launch_bounds__(kTile) k_mx_x(const CaseDev *__restrict__ case
     const Tile t = tiles[blockIdx.x];
     const CaseDev &C = cases[t.c];
     SolveScalars *S = C.sc;
+    const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     if (!S->active32) return;
     float v[1] = {cg_x_rows<float>(C.fx, C.fp, C.fr, C.fq, S->alpha32, t)};
-    block_reduce<1, float>(v, &partials[(size_t)blockIdx.x * kNPart]);
-    if (last_tile_of_case(&C.counters[CNT_A4], cnt[t.c])) {
-        __shared__ float s[1];
-        sum_partials<1, float>(partials, cfirst[t.c], cnt[t.c], s);
+    __shared__ float s[1];
+    if (case_sums<1>(v, &C.counters[CNT_A4], partials, tile0, ntiles, s)) {
         if (threadIdx.x == 0) {
             const float rn = sqrtf(s[0]);
             S->rnorm32 = rn;
@@ -1436,6 +1427,7 @@ __global__ void __launch_bounds__(kTile) k_mx_res(const CaseDev *__restrict__ ca
     const Tile t = tiles[blockIdx.x];
     const CaseDev &C = cases[t.c];
     SolveScalars *S = C.sc;
+    const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     if (!S->active_p) return;
     // two rows per step, both rows' loads before either store
     double v[1] = {0};
@@ -1448,10 +1440,8 @@ __global__ void __launch_bounds__(kTile) k_mx_res(const CaseDev *__restrict__ ca
         if (ok0) { C.kr[i0] = r0; v[0] += r0 * r0; }
         if (ok1) { C.kr[i1] = r1; v[0] += r1 * r1; }
     }
-    block_reduce<1>(v, &partials[(size_t)blockIdx.x * kNPart]);
-    if (last_tile_of_case(&C.counters[CNT_M0], cnt[t.c])) {
-        __shared__ double s[1];
-        sum_partials<1>(partials, cfirst[t.c], cnt[t.c], s);
+    __shared__ double s[1];
+    if (case_sums<1>(v, &C.counters[CNT_M0], partials, tile0, ntiles, s)) {
         if (threadIdx.x == 0) {
             const double rn = sqrt(s[0]);
             S->rnorm_p = rn;

@@ -10,12 +10,60 @@ namespace cfdl {
 // and its writes are visible (a no-op when launched the ordinary way).
 #define CFDL_PDL_WAIT() asm volatile("griddepcontrol.wait;" ::: "memory")
 
-// Deterministic block reduction of K doubles (kTile threads): a fixed
-// shuffle tree per warp, then warp partials summed in warp order by one
-// thread.  The result lands in out[0..K-1].
-template <int K, class T = double>
-__device__ __forceinline__ void block_reduce(T (&v)[K], T *out) {
-    __shared__ T sm[K][kTile / 32];
+// Deterministic sums over the kTile threads of a block: K sums of v land in
+// shared out[0..K-1] (valid after the caller's next barrier).  The order is a
+// fixed tree over each warp's 32 values (lane l with l+16, then l+8, ...),
+// then the warps' sums in warp order.
+//
+// FP64: through shared memory.  GB300 issues 2 FP64 thread-instructions per SM
+// per clock, so a warp's FP64 add costs 16 clocks whatever its lanes hold: a
+// shuffle tree in every warp spends 48 warp-adds per value (8 warps x 5
+// steps, then the warps), more than the rows' own arithmetic when a thread has
+// few rows.  Here each thread stores its K values and warp k alone forms the
+// eight warps' trees of value k with every lane busy -- 4 adds for the first
+// step of all eight trees, 2, 1, 1 and 1 for the next -- and adds the eight
+// sums in order: 17 warp-adds, the same sums in the same order.
+template <int K>
+__device__ __forceinline__ void block_sums(double (&v)[K], double *out) {
+    constexpr int kWarps = kTile / 32;
+    static_assert(kWarps == 8, "the packing below is for eight warps");
+    __shared__ double sm[K][kTile];
+#pragma unroll
+    for (int k = 0; k < K; k++) sm[k][threadIdx.x] = v[k];
+    __syncthreads();
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const bool b8 = (lane & 8) != 0, b4 = (lane & 4) != 0;
+    for (int k = wid; k < K; k += kWarps) {
+        // x[j]: lane l & 15 of tree w = 2 j + (lane >> 4) after its first step
+        double x[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int at = (2 * j + (lane >> 4)) * 32 + (lane & 15);
+            x[j] = sm[k][at] + sm[k][at + 16];
+        }
+        // second step: lanes with bit 8 clear take trees j, the others j + 1
+        double y[2];
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const double own = b8 ? x[2 * j + 1] : x[2 * j], other = b8 ? x[2 * j] : x[2 * j + 1];
+            y[j] = own + __shfl_xor_sync(0xffffffffu, other, 8);
+        }
+        double z = (b4 ? y[1] : y[0]) + __shfl_xor_sync(0xffffffffu, b4 ? y[0] : y[1], 4);
+        z += __shfl_xor_sync(0xffffffffu, z, 2);
+        z += __shfl_xor_sync(0xffffffffu, z, 1);
+        // the sum of warp w = 2 j + h, j = (bit 8) + 2 (bit 4), is in lane 16 h + 8 (j & 1) + 4 (j >> 1)
+        double s = 0.0;
+#pragma unroll
+        for (int w = 0; w < kWarps; w++)
+            s += __shfl_sync(0xffffffffu, z, 16 * (w & 1) + 8 * ((w >> 1) & 1) + 4 * (w >> 2));
+        if (lane == 0) out[k] = s;
+    }
+}
+// FP32: a fixed shuffle tree per warp, then the warps' sums in warp order
+// (FP32 adds are cheap here; the order is part of the FP32 forms' results).
+template <int K>
+__device__ __forceinline__ void block_sums(float (&v)[K], float *out) {
+    __shared__ float sm[K][kTile / 32];
 #pragma unroll
     for (int k = 0; k < K; k++)
 #pragma unroll
@@ -26,62 +74,63 @@ __device__ __forceinline__ void block_reduce(T (&v)[K], T *out) {
         for (int k = 0; k < K; k++) sm[k][wid] = v[k];
     __syncthreads();
     if (threadIdx.x < K) {
-        T s = 0;
+        float s = 0;
         for (int w = 0; w < kTile / 32; w++) s += sm[threadIdx.x][w];
         out[threadIdx.x] = s;
     }
-    __syncthreads();
 }
 
-// Sum the K partials of tiles [first, first+n) in tile order (whole block),
-// result broadcast in shared memory res[0..K-1].
-template <int K, class T = double>
-__device__ __forceinline__ void sum_partials(const T *partials, int first, int n, T *res) {
-    T v[K];
-#pragma unroll
-    for (int k = 0; k < K; k++) v[k] = 0;
-    // thread-strided in a fixed order with four independent accumulators (so
-    // the loads overlap instead of forming one dependent chain), then the
-    // fixed tree
-    T a1[K], a2[K], a3[K];
-#pragma unroll
-    for (int k = 0; k < K; k++) a1[k] = a2[k] = a3[k] = 0;
-    int i = threadIdx.x;
-    for (; i + 3 * kTile < n; i += 4 * kTile)
-#pragma unroll
-        for (int k = 0; k < K; k++) {
-            v[k] += __ldcg(&partials[(size_t)(first + i) * kNPart + k]);
-            a1[k] += __ldcg(&partials[(size_t)(first + i + kTile) * kNPart + k]);
-            a2[k] += __ldcg(&partials[(size_t)(first + i + 2 * kTile) * kNPart + k]);
-            a3[k] += __ldcg(&partials[(size_t)(first + i + 3 * kTile) * kNPart + k]);
-        }
-    for (; i < n; i += kTile)
-#pragma unroll
-        for (int k = 0; k < K; k++) v[k] += __ldcg(&partials[(size_t)(first + i) * kNPart + k]);
-#pragma unroll
-    for (int k = 0; k < K; k++) v[k] = (v[k] + a1[k]) + (a2[k] + a3[k]);
-    __shared__ T tmp[K];
-    block_reduce<K, T>(v, tmp);
-    if (threadIdx.x < K) res[threadIdx.x] = tmp[threadIdx.x];
-    __syncthreads();
-}
-
-// "Last tile of the case finalises": every tile of case c publishes its
-// partials, then increments the case counter; the tile that brings it to
-// ntiles sums all partials (in tile order, so the result does not depend on
-// which tile came last) and resets the counter.
-__device__ __forceinline__ bool last_tile_of_case(int *counter, int ntiles) {
+// The K sums of v over all tiles of a case, in shared s[0..K-1] of the case's
+// last tile to finish; returns true (to the whole block) in that tile only.
+// tile0, ntiles: the case's tiles in the launch's work list; the case's
+// partials are K planes of ntiles values from partials[tile0 * kNPart].
+// Every tile publishes its partials and then raises the case's counter; the
+// tile that brings it to ntiles sums all partials in tile order, so the
+// result does not depend on which tile came last, and clears the counter.
+// One thread writes the partials, fences and raises the counter: the fence
+// then waits for those few stores only, not for the block's vector stores,
+// which are read by later kernels alone.
+template <int K, class T>
+__device__ __forceinline__ bool case_sums(T (&v)[K], int *counter, T *partials, int tile0, int ntiles, T *s) {
     __shared__ int is_last;
-    __threadfence();
+    T *part = partials + (size_t)tile0 * kNPart;
+    const int tile = (int)blockIdx.x - tile0;
+    block_sums<K>(v, s);
     __syncthreads();
     if (threadIdx.x == 0) {
-        int prev = atomicAdd(counter, 1);
-        is_last = (prev == ntiles - 1);
-        if (is_last) *counter = 0;
+#pragma unroll
+        for (int k = 0; k < K; k++) __stcg(&part[(size_t)k * ntiles + tile], s[k]);
+        __threadfence();
+        const bool last = atomicAdd(counter, 1) == ntiles - 1;
+        if (last) { *counter = 0; __threadfence(); }
+        is_last = last;
     }
     __syncthreads();
-    if (is_last) __threadfence();
-    return is_last != 0;
+    if (!is_last) return false;
+    // thread-strided in a fixed order with four independent accumulators (so
+    // the loads overlap instead of forming one dependent chain), then the
+    // block sum
+    T a1[K], a2[K], a3[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) v[k] = a1[k] = a2[k] = a3[k] = 0;
+    int i = threadIdx.x;
+    for (; i + 3 * kTile < ntiles; i += 4 * kTile)
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            const T *p = part + (size_t)k * ntiles + i;
+            v[k] += __ldcg(p);
+            a1[k] += __ldcg(p + kTile);
+            a2[k] += __ldcg(p + 2 * kTile);
+            a3[k] += __ldcg(p + 3 * kTile);
+        }
+    for (; i < ntiles; i += kTile)
+#pragma unroll
+        for (int k = 0; k < K; k++) v[k] += __ldcg(&part[(size_t)k * ntiles + i]);
+#pragma unroll
+    for (int k = 0; k < K; k++) v[k] = (v[k] + a1[k]) + (a2[k] + a3[k]);
+    block_sums<K>(v, s);
+    __syncthreads();
+    return true;
 }
 
 __device__ __forceinline__ int face_of(int fc) { return fc >= 0 ? fc : ~fc; }

@@ -49,17 +49,11 @@ __device__ __forceinline__ double csr_amul(NoAllocScratch *S, int ne, int nh, co
     return s;
 }
 
-__device__ __forceinline__ bool na_last(NoAllocScratch *S, int which, int ntiles) {
-    return last_tile_of_case(&S->counter[which], ntiles);
-}
-
 __global__ void __launch_bounds__(kTile) k_na_mean(NoAllocScratch *S, int ne, const double *b) {
     const int i = blockIdx.x * kTile + threadIdx.x;
     double v[1] = {i < ne ? b[i] : 0.0};
-    block_reduce<1>(v, &S->partials[(size_t)blockIdx.x * kNPart]);
-    if (na_last(S, 0, gridDim.x)) {
-        __shared__ double s[1];
-        sum_partials<1>(S->partials, 0, gridDim.x, s);
+    __shared__ double s[1];
+    if (case_sums<1>(v, &S->counter[0], S->partials, 0, (int)gridDim.x, s)) {
         if (threadIdx.x == 0) S->mean = s[0] / ne;
     }
 }
@@ -73,10 +67,8 @@ __global__ void __launch_bounds__(kTile) k_na_init(NoAllocScratch *S, int ne, co
         S->r[i] = r; S->z[i] = z; S->p[i] = z; x[i] = 0.0;
         v[0] = r * r; v[1] = r * z;
     }
-    block_reduce<2>(v, &S->partials[(size_t)blockIdx.x * kNPart]);
-    if (na_last(S, 1, gridDim.x)) {
-        __shared__ double s[2];
-        sum_partials<2>(S->partials, 0, gridDim.x, s);
+    __shared__ double s[2];
+    if (case_sums<2>(v, &S->counter[1], S->partials, 0, (int)gridDim.x, s)) {
         if (threadIdx.x == 0) {
             S->r0 = S->rnorm = sqrt(s[0]);
             S->rz = s[1];
@@ -100,10 +92,8 @@ __global__ void __launch_bounds__(kTile) k_na_q(NoAllocScratch *S, int ne, int n
         S->q[i] = q;
         v[0] = S->p[i] * q;
     }
-    block_reduce<1>(v, &S->partials[(size_t)blockIdx.x * kNPart]);
-    if (na_last(S, 2, gridDim.x)) {
-        __shared__ double s[1];
-        sum_partials<1>(S->partials, 0, gridDim.x, s);
+    __shared__ double s[1];
+    if (case_sums<1>(v, &S->counter[2], S->partials, 0, (int)gridDim.x, s)) {
         if (threadIdx.x == 0) {
             // only runs while ||r|| is above the tolerance, where an SPD system has p.Ap > 0
             if (S->bad) S->active = 0;
@@ -125,10 +115,8 @@ __global__ void __launch_bounds__(kTile) k_na_x(NoAllocScratch *S, int ne, const
         S->r[i] = r; S->z[i] = z;
         v[0] = r * r; v[1] = r * z;
     }
-    block_reduce<2>(v, &S->partials[(size_t)blockIdx.x * kNPart]);
-    if (na_last(S, 3, gridDim.x)) {
-        __shared__ double s[2];
-        sum_partials<2>(S->partials, 0, gridDim.x, s);
+    __shared__ double s[2];
+    if (case_sums<2>(v, &S->counter[3], S->partials, 0, (int)gridDim.x, s)) {
         if (threadIdx.x == 0) {
             S->rnorm = sqrt(s[0]);
             S->iters += 1;

@@ -42,15 +42,14 @@ __global__ void __launch_bounds__(kTile) k_run_end(const CaseDev *__restrict__ c
     const Tile t = tiles[blockIdx.x];
     const CaseDev &C = cases[t.c];
     SolveScalars *S = C.sc;
+    const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     if (S->halted) return;
     // several faces per thread (wide tiles), then one block tree: the FP64
     // reduction tree is paid once per kTile*kFaceVec faces
     double v[1] = {0.0};
     FOR_CELLS(t) v[0] += fabs(C.mip[i]);
-    block_reduce<1>(v, &partials[(size_t)blockIdx.x * kNPart]);
-    if (last_tile_of_case(&C.counters[CNT_RUN], cnt[t.c])) {
-        __shared__ double s[1];
-        sum_partials<1>(partials, cfirst[t.c], cnt[t.c], s);
+    __shared__ double s[1];
+    if (case_sums<1>(v, &C.counters[CNT_RUN], partials, tile0, ntiles, s)) {
         if (threadIdx.x == 0) {
             S->mip_abs = s[0];
             S->mass_ratio = s[0] > 0.0 ? S->mass_imbalance / s[0] : S->mass_imbalance;

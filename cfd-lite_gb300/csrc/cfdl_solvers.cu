@@ -114,27 +114,25 @@ __global__ void __launch_bounds__(kTile, 3) k_mom_init(const CaseDev *__restrict
                                                     const int *__restrict__ cfirst, const int *__restrict__ cnt, double *partials) {
     CFDL_PDL_WAIT();
     TILE_HEAD
+    const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     double v[6] = {0, 0, 0, 0, 0, 0};
     const bool m32 = C.precision >= 2;
     if (C.W == 6) { FOR_CELLS(t) mom_init_row<6>(C, i, ne, v, m32); }
     else if (C.W == 4) { FOR_CELLS(t) mom_init_row<4>(C, i, ne, v, m32); }
     else { FOR_CELLS(t) mom_init_row<kMaxW>(C, i, ne, v, m32); }
-    block_reduce<6>(v, &partials[(size_t)blockIdx.x * kNPart]);
-    if (last_tile_of_case(&C.counters[CNT_M1], cnt[t.c])) {
-        __shared__ double s[6];
-        sum_partials<6>(partials, cfirst[t.c], cnt[t.c], s);
-        if (threadIdx.x == 0) {
+    __shared__ double s[6];
+    if (case_sums<6>(v, &C.counters[CNT_M1], partials, tile0, ntiles, s)) {
+        const int q = threadIdx.x;          // one thread per component
+        if (q < 3) {
             const int cap = C.solve_mode == 0 ? C.nit : C.tight_maxit;
-            for (int q = 0; q < 3; q++) {
-                S->bnorm[q] = sqrt(s[q]);
-                S->r0norm[q] = S->rnorm[q] = sqrt(s[3 + q]);
-                S->rho[q] = s[3 + q];
-                S->alpha[q] = 1.0; S->omega[q] = 1.0; S->beta[q] = 0.0; S->half[q] = 0;
-                S->iters[q] = 0; S->status[q] = 0;
-                S->tol[q] = C.solve_mode == 0 ? C.rtol_u * S->r0norm[q] : C.tight_rtol * S->bnorm[q];
-                S->active[q] = (S->r0norm[q] > S->tol[q]) && cap > 0;
-                if (!isfinite(S->r0norm[q]) || !isfinite(S->bnorm[q])) { S->active[q] = 0; S->status[q] = CFDL_ERR_NONFINITE; }
-            }
+            S->bnorm[q] = sqrt(s[q]);
+            S->r0norm[q] = S->rnorm[q] = sqrt(s[3 + q]);
+            S->rho[q] = s[3 + q];
+            S->alpha[q] = 1.0; S->omega[q] = 1.0; S->beta[q] = 0.0; S->half[q] = 0;
+            S->iters[q] = 0; S->status[q] = 0;
+            S->tol[q] = C.solve_mode == 0 ? C.rtol_u * S->r0norm[q] : C.tight_rtol * S->bnorm[q];
+            S->active[q] = (S->r0norm[q] > S->tol[q]) && cap > 0;
+            if (!isfinite(S->r0norm[q]) || !isfinite(S->bnorm[q])) { S->active[q] = 0; S->status[q] = CFDL_ERR_NONFINITE; }
         }
     }
 }
@@ -219,6 +217,7 @@ __global__ void __launch_bounds__(kTile, 4) k_mom_v(const CaseDev *__restrict__ 
                                                  const int *__restrict__ cfirst, const int *__restrict__ cnt, T *partials) {
     CFDL_PDL_WAIT();
     TILE_HEAD
+    const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     KLanes *L = lanes<NC>(S);
     if (!lanes_active<NC>(L)) return;
     const MomVec<T> M = mom_vec<T, NC>(C);
@@ -238,18 +237,15 @@ __global__ void __launch_bounds__(kTile, 4) k_mom_v(const CaseDev *__restrict__ 
             v[q] += rh[q] * y[q];
         }
     }
-    block_reduce<NC, T>(v, &partials[(size_t)blockIdx.x * kNPart]);
-    if (last_tile_of_case(&C.counters[CNT_M2], cnt[t.c])) {
-        __shared__ T s[NC];
-        sum_partials<NC, T>(partials, cfirst[t.c], cnt[t.c], s);
-        if (threadIdx.x == 0)
-            for (int q = 0; q < NC; q++) {
-                if (!L->active[q]) continue;
-                const double sq = (double)s[q];
-                const double a = L->rho[q] / sq;
-                if (sq == 0.0 || !isfinite(a)) { L->active[q] = 0; L->status[q] = isfinite(a) || sq == 0.0 ? L->status[q] : CFDL_ERR_NONFINITE; continue; }
-                L->alpha[q] = a;
-            }
+    __shared__ T s[NC];
+    if (case_sums<NC>(v, &C.counters[CNT_M2], partials, tile0, ntiles, s)) {
+        if (threadIdx.x < NC && L->active[threadIdx.x]) {   // one thread per component
+            const int q = threadIdx.x;
+            const double sq = (double)s[q];
+            const double a = L->rho[q] / sq;
+            if (sq == 0.0 || !isfinite(a)) { L->active[q] = 0; L->status[q] = isfinite(a) || sq == 0.0 ? L->status[q] : CFDL_ERR_NONFINITE; }
+            else L->alpha[q] = a;
+        }
     }
 }
 
@@ -259,6 +255,7 @@ __global__ void __launch_bounds__(kTile) k_mom_s(const CaseDev *__restrict__ cas
                                                  const int *__restrict__ cfirst, const int *__restrict__ cnt, T *partials) {
     CFDL_PDL_WAIT();
     TILE_HEAD
+    const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     KLanes *L = lanes<NC>(S);
     if (!lanes_active<NC>(L)) return;
     const MomVec<T> M = mom_vec<T, NC>(C);
@@ -299,15 +296,10 @@ __global__ void __launch_bounds__(kTile) k_mom_s(const CaseDev *__restrict__ cas
             }
         }
     }
-    block_reduce<NC, T>(v, &partials[(size_t)blockIdx.x * kNPart]);
-    if (last_tile_of_case(&C.counters[CNT_M3], cnt[t.c])) {
-        __shared__ T s[NC];
-        sum_partials<NC, T>(partials, cfirst[t.c], cnt[t.c], s);
-        if (threadIdx.x == 0)
-            for (int q = 0; q < NC; q++) {
-                if (!L->active[q]) continue;
-                L->half[q] = sqrt((double)s[q]) <= L->tol[q];
-            }
+    __shared__ T s[NC];
+    if (case_sums<NC>(v, &C.counters[CNT_M3], partials, tile0, ntiles, s)) {
+        const int q = threadIdx.x;
+        if (q < NC && L->active[q]) L->half[q] = sqrt((double)s[q]) <= L->tol[q];
     }
 }
 
@@ -317,6 +309,7 @@ __global__ void __launch_bounds__(kTile, 4) k_mom_t(const CaseDev *__restrict__ 
                                                  const int *__restrict__ cfirst, const int *__restrict__ cnt, T *partials) {
     CFDL_PDL_WAIT();
     TILE_HEAD
+    const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     KLanes *L = lanes<NC>(S);
     if (!lanes_active<NC>(L)) return;
     const MomVec<T> M = mom_vec<T, NC>(C);
@@ -338,16 +331,13 @@ __global__ void __launch_bounds__(kTile, 4) k_mom_t(const CaseDev *__restrict__ 
             v[NC + q] += y[q] * y[q];
         }
     }
-    block_reduce<2 * NC, T>(v, &partials[(size_t)blockIdx.x * kNPart]);
-    if (last_tile_of_case(&C.counters[CNT_M4], cnt[t.c])) {
-        __shared__ T s[2 * NC];
-        sum_partials<2 * NC, T>(partials, cfirst[t.c], cnt[t.c], s);
-        if (threadIdx.x == 0)
-            for (int q = 0; q < NC; q++) {
-                if (!L->active[q]) continue;
-                const double ts = (double)s[q], tt = (double)s[NC + q];
-                L->omega[q] = L->half[q] ? 0.0 : (tt > 0.0 ? ts / tt : 0.0);
-            }
+    __shared__ T s[2 * NC];
+    if (case_sums<2 * NC>(v, &C.counters[CNT_M4], partials, tile0, ntiles, s)) {
+        const int q = threadIdx.x;
+        if (q < NC && L->active[q]) {
+            const double ts = (double)s[q], tt = (double)s[NC + q];
+            L->omega[q] = L->half[q] ? 0.0 : (tt > 0.0 ? ts / tt : 0.0);
+        }
     }
 }
 
@@ -357,6 +347,7 @@ __global__ void __launch_bounds__(kTile, 4) k_mom_x(const CaseDev *__restrict__ 
                                                  const int *__restrict__ cfirst, const int *__restrict__ cnt, T *partials) {
     CFDL_PDL_WAIT();
     TILE_HEAD
+    const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     KLanes *L = lanes<NC>(S);
     if (!lanes_active<NC>(L)) return;
     const MomVec<T> M = mom_vec<T, NC>(C);
@@ -388,26 +379,22 @@ __global__ void __launch_bounds__(kTile, 4) k_mom_x(const CaseDev *__restrict__ 
             v[NC + q] += rh[q] * r;
         }
     }
-    block_reduce<2 * NC, T>(v, &partials[(size_t)blockIdx.x * kNPart]);
-    if (last_tile_of_case(&C.counters[CNT_M5], cnt[t.c])) {
-        __shared__ T s[2 * NC];
-        sum_partials<2 * NC, T>(partials, cfirst[t.c], cnt[t.c], s);
-        if (threadIdx.x == 0) {
+    __shared__ T s[2 * NC];
+    if (case_sums<2 * NC>(v, &C.counters[CNT_M5], partials, tile0, ntiles, s)) {
+        const int q = threadIdx.x;
+        if (q < NC && L->active[q]) {
             const int cap = C.solve_mode == 0 ? C.nit : C.tight_maxit;
-            for (int q = 0; q < NC; q++) {
-                if (!L->active[q]) continue;
-                const double rn = sqrt((double)s[q]), rho_new = (double)s[NC + q];
-                L->rnorm[q] = rn;
-                L->iters[q] += 1;
-                const double om = L->omega[q];
-                L->beta[q] = (om != 0.0 && L->rho[q] != 0.0) ? (rho_new / L->rho[q]) * (L->alpha[q] / om) : 0.0;
-                L->rho[q] = rho_new;
-                int act = rn > L->tol[q];
-                if (!isfinite(rn)) { act = 0; L->status[q] = CFDL_ERR_NONFINITE; }
-                else if (act && (om == 0.0 || rho_new == 0.0)) act = 0;           // breakdown: stop here
-                else if (act && L->iters[q] >= cap) { act = 0; if (C.solve_mode == 1) L->status[q] = CFDL_ERR_ITER_CAP; }
-                L->active[q] = act;
-            }
+            const double rn = sqrt((double)s[q]), rho_new = (double)s[NC + q];
+            L->rnorm[q] = rn;
+            L->iters[q] += 1;
+            const double om = L->omega[q];
+            L->beta[q] = (om != 0.0 && L->rho[q] != 0.0) ? (rho_new / L->rho[q]) * (L->alpha[q] / om) : 0.0;
+            L->rho[q] = rho_new;
+            int act = rn > L->tol[q];
+            if (!isfinite(rn)) { act = 0; L->status[q] = CFDL_ERR_NONFINITE; }
+            else if (act && (om == 0.0 || rho_new == 0.0)) act = 0;           // breakdown: stop here
+            else if (act && L->iters[q] >= cap) { act = 0; if (C.solve_mode == 1) L->status[q] = CFDL_ERR_ITER_CAP; }
+            L->active[q] = act;
         }
     }
 }
@@ -452,6 +439,7 @@ __global__ void __launch_bounds__(kTile, 3) k_en_init(const CaseDev *__restrict_
                                                    const int *__restrict__ cfirst, const int *__restrict__ cnt, double *partials) {
     CFDL_PDL_WAIT();
     TILE_HEAD
+    const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     double v[2] = {0, 0};
     const bool m32 = C.precision >= 2;
     if (C.ee) {
@@ -459,10 +447,8 @@ __global__ void __launch_bounds__(kTile, 3) k_en_init(const CaseDev *__restrict_
         else if (C.W == 4) { FOR_CELLS(t) en_init_row<4>(C, i, ne, v, m32); }
         else { FOR_CELLS(t) en_init_row<kMaxW>(C, i, ne, v, m32); }
     }
-    block_reduce<2>(v, &partials[(size_t)blockIdx.x * kNPart]);
-    if (last_tile_of_case(&C.counters[CNT_M1], cnt[t.c])) {
-        __shared__ double s[2];
-        sum_partials<2>(partials, cfirst[t.c], cnt[t.c], s);
+    __shared__ double s[2];
+    if (case_sums<2>(v, &C.counters[CNT_M1], partials, tile0, ntiles, s)) {
         if (threadIdx.x == 0) {
             KLanes *L = &S->en;
             const int cap = C.solve_mode == 0 ? C.nit : C.tight_maxit;
@@ -506,12 +492,11 @@ __global__ void __launch_bounds__(kTile) k_pc_mean(const CaseDev *__restrict__ c
                                                    const int *__restrict__ cfirst, const int *__restrict__ cnt, double *partials) {
     CFDL_PDL_WAIT();
     TILE_HEAD
+    const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     double v[1] = {0.0};
     FOR_CELLS(t) v[0] += C.b[i];
-    block_reduce<1>(v, &partials[(size_t)blockIdx.x * kNPart]);
-    if (last_tile_of_case(&C.counters[CNT_P0], cnt[t.c])) {
-        __shared__ double s[1];
-        sum_partials<1>(partials, cfirst[t.c], cnt[t.c], s);
+    __shared__ double s[1];
+    if (case_sums<1>(v, &C.counters[CNT_P0], partials, tile0, ntiles, s)) {
         if (threadIdx.x == 0) S->mean_b = s[0] / ne;
     }
 }
@@ -521,16 +506,15 @@ __global__ void __launch_bounds__(kTile) k_pc_init(const CaseDev *__restrict__ c
                                                    const int *__restrict__ cfirst, const int *__restrict__ cnt, double *partials) {
     CFDL_PDL_WAIT();
     TILE_HEAD
+    const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     double v[3] = {0, 0, 0};
     FOR_CELLS(t) {
         const double r = C.b[i] - S->mean_b, z = r / C.ap_p[i];
         C.kr[i] = r; C.ks[i] = z; C.kp[i] = z; C.phic[i] = 0.0;
         v[0] += r * r; v[1] += r * z; v[2] += C.b[i] * C.b[i];
     }
-    block_reduce<3>(v, &partials[(size_t)blockIdx.x * kNPart]);
-    if (last_tile_of_case(&C.counters[CNT_P1], cnt[t.c])) {
-        __shared__ double s[3];
-        sum_partials<3>(partials, cfirst[t.c], cnt[t.c], s);
+    __shared__ double s[3];
+    if (case_sums<3>(v, &C.counters[CNT_P1], partials, tile0, ntiles, s)) {
         if (threadIdx.x == 0) {
             const int cap = C.solve_mode == 0 ? C.nit : C.tight_maxit;
             S->r0norm_p = S->rnorm_p = sqrt(s[0]);
@@ -549,6 +533,7 @@ __global__ void __launch_bounds__(kTile) k_pc_q(const CaseDev *__restrict__ case
                                                 const int *__restrict__ cfirst, const int *__restrict__ cnt, double *partials) {
     CFDL_PDL_WAIT();
     TILE_HEAD
+    const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     if (!S->active_p) return;
     double v[1] = {0};
     FOR_CELLS(t) {
@@ -556,10 +541,8 @@ __global__ void __launch_bounds__(kTile) k_pc_q(const CaseDev *__restrict__ case
         C.kv[i] = q;
         v[0] += C.kp[i] * q;
     }
-    block_reduce<1>(v, &partials[(size_t)blockIdx.x * kNPart]);
-    if (last_tile_of_case(&C.counters[CNT_P2], cnt[t.c])) {
-        __shared__ double s[1];
-        sum_partials<1>(partials, cfirst[t.c], cnt[t.c], s);
+    __shared__ double s[1];
+    if (case_sums<1>(v, &C.counters[CNT_P2], partials, tile0, ntiles, s)) {
         if (threadIdx.x == 0) {
             if (!(s[0] > 0.0) || !isfinite(s[0])) {
                 // runs only while ||r|| is above the tolerance, where p.Ap > 0 for the SPD system
@@ -576,6 +559,7 @@ __global__ void __launch_bounds__(kTile) k_pc_x(const CaseDev *__restrict__ case
                                                 const int *__restrict__ cfirst, const int *__restrict__ cnt, double *partials) {
     CFDL_PDL_WAIT();
     TILE_HEAD
+    const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     if (!S->active_p) return;
     double v[2] = {0, 0};
     FOR_CELLS(t) {
@@ -585,10 +569,8 @@ __global__ void __launch_bounds__(kTile) k_pc_x(const CaseDev *__restrict__ case
         C.kr[i] = r; C.ks[i] = z;
         v[0] += r * r; v[1] += r * z;
     }
-    block_reduce<2>(v, &partials[(size_t)blockIdx.x * kNPart]);
-    if (last_tile_of_case(&C.counters[CNT_P3], cnt[t.c])) {
-        __shared__ double s[2];
-        sum_partials<2>(partials, cfirst[t.c], cnt[t.c], s);
+    __shared__ double s[2];
+    if (case_sums<2>(v, &C.counters[CNT_P3], partials, tile0, ntiles, s)) {
         if (threadIdx.x == 0) {
             const int cap = C.solve_mode == 0 ? C.nit : C.tight_maxit;
             const double rn = sqrt(s[0]);
