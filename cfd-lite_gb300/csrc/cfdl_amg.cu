@@ -22,6 +22,7 @@
 #include "cfdl_device.cuh"
 #include "cfdl_par.h"
 #include <algorithm>
+#include <cooperative_groups.h>
 #include <new>
 
 namespace cfdl {
@@ -47,7 +48,6 @@ constexpr double kOverCorrect = 3.0;   // scaling of the prolongated coarse corr
 constexpr int kG = 8;                  // lanes per row on the small coarse levels
 constexpr int kGroupedRows = 65536;    // levels below this many rows (per case) run grouped
 constexpr int kTailRows = 2048;        // a case's levels at or below this many rows run in its V-cycle tail
-constexpr int kTailThreads = 1024;     // threads of the tail's one CTA per case
 enum { CNT_A0 = 9, CNT_A1, CNT_A2, CNT_A3, CNT_A4, CNT_A5 };
 
 template <class T> struct LP {
@@ -571,78 +571,211 @@ __global__ void __launch_bounds__(kTile) k_amg_gal(const CaseDev *__restrict__ c
 
 // ------------------------------------------------- the V-cycle's tail
 // The small coarse levels of a case, from its tail level (the first level of
-// at most kTailRows rows) down to the coarsest and back, in one CTA: the
-// steps of k_v_jac0 / k_v_jac / k_v_resid / k_v_restrict, the coarsest solve
-// and k_v_lift / k_v_jac, one row per thread per pass, with a block
-// barrier between steps.  Each step is a few microseconds of dependent loads
-// from L2; launched one by one, every step costs a kernel launch instead.
-// The CTA waits only at __syncthreads, on its own threads.
+// at most kTailRows rows) down to the coarsest and back, on one cluster of
+// kTailCtas CTAs: the steps of k_v_jac0 / k_v_jac / k_v_resid / k_v_restrict,
+// the coarsest solve and k_v_lift / k_v_jac, one row per thread, each row's
+// sum in its slot order.  A step is a fraction of a microsecond of arithmetic
+// behind a chain of dependent loads of about 0.35 us each from L2, so the
+// chain is what is cut: everything a step needs is staged in shared memory
+// first, all of it in flight together (cp.async), and every CTA keeps a whole
+// copy of the vectors that the next step gathers from, written by a row's
+// owner into all CTAs' shared memory before the cluster barrier (0.6 us).
+// Levels small enough are done whole by every CTA for itself, behind block
+// barriers; more rows would cost more than the barrier, FP64 ones sooner (16
+// clocks of the SM's FP64 pipe per warp and slot).
+// Measured per V-cycle (events around the launch) against one CTA of 1024
+// threads reading everything from L2 at every step: 128^3 cavity (levels of
+// 662 and 37 rows) 43.5 -> 22.0 us FP64, 25.7 -> 15.0 FP32; 24^3 (1685, 105,
+// 8 rows) 36.9 -> 20.0 FP32; 41^3 prisms (1263, 70, 6) 69 -> 30 FP64; twelve
+// uneven cases 79 -> 30 FP64.
+constexpr int kTailCtas = 8;                               // portable cluster size
+constexpr int kTailBlock = kTailRows / kTailCtas;          // one row of the largest level per thread
+constexpr int kTailMaxSmem = 200 * 1024;
+static_assert(kTailBlock == 256, "a level done whole has at most this many rows");
+template <class T> constexpr int tail_whole() { return sizeof(T) == 8 ? 128 : 256; }
+
+// 4 or 8 bytes from global to shared memory, asynchronously
+__device__ __forceinline__ void stage(float *s, const float *g) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(s)), "l"(g));
+}
+__device__ __forceinline__ void stage(int *s, const int *g) { stage((float *)s, (const float *)g); }
+__device__ __forceinline__ void stage(double *s, const double *g) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(s)), "l"(g));
+}
+
 template <class T>
-__global__ void __launch_bounds__(kTailThreads) k_v_tail(const CaseDev *__restrict__ cases, int ncases) {
+__global__ void __launch_bounds__(kTailBlock) k_v_tail(const CaseDev *__restrict__ cases, int ncases) {
     CFDL_PDL_WAIT();
-    const int c = blockIdx.x;
-    if (c >= ncases) return;
+    namespace cg = cooperative_groups;
+    extern __shared__ __align__(16) unsigned char tail_mem[];
+    __shared__ TailPlan Q;
+    const int c = (int)blockIdx.x / kTailCtas, rank = (int)blockIdx.x % kTailCtas, tid = (int)threadIdx.x;
+    if (c >= ncases) return;                               // the whole cluster
     const CaseDev &C = cases[c];
-    if (C.precond != 1 || (sizeof(T) == 8 ? !pactive(C) : !mactive(C))) return;
-    const int L = C.nlev, lt = C.amg_tail, nt = (int)blockDim.x;
-    for (int l = lt; l < L; l++) {
-        const LP<T> P = level<T>(C, l);
-        for (int i = threadIdx.x; i < P.n; i += nt) P.t[i] = P.rd[i] * P.r[i];
-        __syncthreads();
-        for (int i = threadIdx.x; i < P.n; i += nt) P.z[i] = jacobi_step<T>(P.t[i], P.r[i], P.rd[i], offsum<T>(P, P.t, i));
-        __syncthreads();
-        for (int i = threadIdx.x; i < P.n; i += nt) P.t[i] = P.r[i] - amul_coarse<T>(P, P.z, i);
-        __syncthreads();
-        const AmgLevelDev &Lc = C.lev[l];                  // level l + 1
-        T *rc = sizeof(T) == 8 ? (T *)Lc.r : (T *)Lc.r32;
-        for (int I = threadIdx.x; I < Lc.n; I += nt) rc[I] = restrict_row<T>(Lc, P.t, I);
-        __syncthreads();
-    }
-    {   // coarsest: z_L = Minv r_L
-        const LP<T> P = level<T>(C, L);
-        const T *Mi = sizeof(T) == 8 ? (const T *)C.cinv : (const T *)C.cinv32;
-        const int n = P.n;
-        for (int i = threadIdx.x; i < n; i += nt) {
-            T sum = 0;
-            for (int j = 0; j < n; j++) sum += Mi[i * n + j] * P.r[j];
-            P.z[i] = sum;
-        }
-        __syncthreads();
-    }
-    const T sc = (T)kOverCorrect;
-    constexpr int kCh = coarse_chunk<T>();
-    for (int l = L - 1; l >= lt; l--) {
-        const LP<T> P = level<T>(C, l);
-        const AmgLevelDev &Lc = C.lev[l];
-        const T *zc = sizeof(T) == 8 ? (const T *)Lc.z : (const T *)Lc.z32;
-        for (int i = threadIdx.x; i < P.n; i += nt) {
-            const T xi = P.z[i] + sc * zc[Lc.agg[i]];
-            // the neighbours' lifted values, kCh slots per step with
-            // each step's loads issued together, summed in slot order
-            T off = 0;
-            const int len = row_len(P, i);
-            for (int k0 = 0; k0 < len; k0 += kCh) {
-                int jj[kCh], ag[kCh];
-                bool ok[kCh];
-                T ak[kCh], zj[kCh];
-#pragma unroll
-                for (int u = 0; u < kCh; u++) jj[u] = k0 + u < len ? P.nb[(k0 + u) * P.n + i] : -1;
-#pragma unroll
-                for (int u = 0; u < kCh; u++) {
-                    ok[u] = (unsigned)jj[u] < (unsigned)P.n;
-                    ak[u] = ok[u] ? P.a[(k0 + u) * P.n + i] : (T)0;
-                    zj[u] = ok[u] ? P.z[jj[u]] : (T)0;
-                    ag[u] = ok[u] ? Lc.agg[jj[u]] : 0;
-                }
-#pragma unroll
-                for (int u = 0; u < kCh; u++)
-                    if (ok[u]) off += ak[u] * (zj[u] + sc * zc[ag[u]]);
+    const long long *plan = (const long long *)(sizeof(T) == 8 ? C.tail64 : C.tail32);
+    if (C.precond != 1 || (sizeof(T) == 8 ? !pactive(C) : !mactive(C))) return;   // the whole cluster
+    cg::cluster_group cluster = cg::this_cluster();
+    auto started = cluster.barrier_arrive();               // waited for before the first write to another CTA
+    static_assert(sizeof(TailPlan) % 8 == 0, "copied by 8-byte words");
+    for (int j = tid; j < (int)(sizeof(TailPlan) / 8); j += kTailBlock) ((long long *)&Q)[j] = plan[j];
+    __syncthreads();
+    auto vec = [&](int off) { return (T *)(tail_mem + off); };
+    auto idx = [&](int off) { return (int *)(tail_mem + off); };
+    const int nl = Q.nl, nc = Q.nc;
+    for (int l = 0; l < nl; l++) {
+        const TailLevel &v = Q.lv[l];
+        const int i = (v.whole ? 0 : rank * v.R) + tid;
+        if (tid < v.R && i < v.n) {
+            const T *a = (const T *)v.a + i;
+            const int *nb = v.nb + i;
+            for (int k = 0; k < v.S; k++) {
+                stage(vec(v.sa) + k * v.R + tid, a + (size_t)k * v.n);
+                stage(idx(v.snb) + k * v.R + tid, nb + (size_t)k * v.n);
             }
-            P.t[i] = jacobi_step<T, 1>(xi, P.r[i], P.rd[i], off);
+            stage(vec(v.srd) + tid, (const T *)v.rd + i);
+            stage(vec(v.sdg) + tid, (const T *)v.dg + i);
+            stage(idx(v.slen) + tid, v.len + i);
+            if (l == 0) stage(vec(v.sr) + tid, (const T *)Q.r + i);
         }
+        for (int j = tid; j < v.n; j += kTailBlock) {
+            stage(idx(v.sagg) + j, v.agg + j);
+            stage(idx(v.smem_) + j, v.mem + j);
+        }
+        const int n1 = l + 1 < nl ? Q.lv[l + 1].n : nc;
+        for (int j = tid; j <= n1; j += kTailBlock) stage(idx(v.smptr) + j, v.mptr + j);
+    }
+    for (int e = tid; e < nc * nc; e += kTailBlock)        // transposed: a thread sums a row of it
+        stage(vec(Q.sminv) + (e % nc) * nc + e / nc, (const T *)Q.minv + e);
+    if (nl == 0)
+        for (int e = tid; e < nc; e += kTailBlock) stage(vec(Q.sr) + e, (const T *)Q.r + e);
+    // t = w D^-1 r of the whole tail level, by every CTA for itself
+    auto t_down = [&](int l) { return Q.lv[l].whole ? Q.w[l & 1] : Q.t[l & 1]; };
+    auto t_up = [&](int l) { return Q.lv[l].whole ? Q.w[(l + 1) & 1] : Q.t[(l + 1) & 1]; };
+    if (nl > 0) {
+        T *t = vec(t_down(0));
+        const T *r = (const T *)Q.r, *rd = (const T *)Q.lv[0].rd;
+        constexpr int kPer = kTailRows / kTailBlock;
+        T rv[kPer], dv[kPer];
+#pragma unroll
+        for (int u = 0; u < kPer; u++) {
+            const int j = tid + u * kTailBlock;
+            rv[u] = j < Q.lv[0].n ? r[j] : (T)0;
+            dv[u] = j < Q.lv[0].n ? rd[j] : (T)0;
+        }
+#pragma unroll
+        for (int u = 0; u < kPer; u++) {
+            const int j = tid + u * kTailBlock;
+            if (j < Q.lv[0].n) t[j] = dv[u] * rv[u];
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    // one value of a level's vector, into every CTA's copy (a level done whole: into this one's)
+    auto put = [&](const TailLevel &v, int off, int i, T x) {
+        T *p = vec(off) + i;
+        if (v.whole) { *p = x; return; }
+#pragma unroll
+        for (int k = 0; k < kTailCtas; k++) *cluster.map_shared_rank(p, k) = x;
+    };
+    auto sync = [&](const TailLevel &v) {
+        if (v.whole) __syncthreads();
+        else cluster.sync();
+    };
+    // s +- the sum of a_ij x(j) over the couplings of this thread's row i of a level, slots in order
+    auto row_sum = [&](const TailLevel &v, int i, int len, T s, auto x, bool minus) {
+        const int R = v.R, m = min(len, v.S);
+        const T *sa = vec(v.sa) + tid;
+        const int *sn = idx(v.snb) + tid;
+        if (minus) {
+#pragma unroll 4
+            for (int k = 0; k < m; k++) s -= sa[k * R] * x(sn[k * R]);
+        } else {
+#pragma unroll 4
+            for (int k = 0; k < m; k++) s += sa[k * R] * x(sn[k * R]);
+        }
+        for (int k = m; k < len; k++) {                    // slots that were not staged
+            const T ak = ((const T *)v.a)[(size_t)k * v.n + i], xk = x(v.nb[(size_t)k * v.n + i]);
+            if (minus) s -= ak * xk;
+            else s += ak * xk;
+        }
+        return s;
+    };
+    // the residual of a level summed over the members of aggregate i, in member order
+    auto restrict_to = [&](int l, int i) {
+        const TailLevel &v = Q.lv[l];
+        const T *tf = vec(t_down(l));
+        const int *mm = idx(v.smem_), m0 = idx(v.smptr)[i], m1 = idx(v.smptr)[i + 1];
+        T r = 0;
+#pragma unroll 4
+        for (int m = m0; m < m1; m++) r += tf[mm[m]];
+        return r;
+    };
+    cluster.barrier_wait(std::move(started));
+    for (int l = 0; l < nl; l++) {
+        const TailLevel &v = Q.lv[l];
+        const int i = (v.whole ? 0 : rank * v.R) + tid, tb = t_down(l);
+        const bool mine = tid < v.R && i < v.n;
+        const T rd = mine ? vec(v.srd)[tid] : (T)0;
+        const int len = mine ? idx(v.slen)[tid] : 0;
+        T r = 0;
+        if (l == 0) {
+            if (mine) r = vec(v.sr)[tid];
+        } else {
+            if (mine) {
+                r = restrict_to(l - 1, i);
+                vec(v.sr)[tid] = r;
+                put(v, tb, i, rd * r);
+            }
+            sync(v);
+        }
+        const T *tc = vec(tb), *zc = vec(v.sz);
+        T z = 0;
+        if (mine) {
+            z = jacobi_step<T>(tc[i], r, rd, row_sum(v, i, len, (T)0, [&](int j) { return tc[j]; }, false));
+            put(v, v.sz, i, z);
+        }
+        sync(v);
+        if (mine) put(v, tb, i, r - row_sum(v, i, len, vec(v.sdg)[tid] * z, [&](int j) { return zc[j]; }, true));
+        sync(v);
+    }
+    // coarsest, by every CTA for itself: z_L = Minv r_L
+    if (nl > 0) {
+        for (int i = tid; i < nc; i += kTailBlock) vec(Q.sr)[i] = restrict_to(nl - 1, i);
         __syncthreads();
-        for (int i = threadIdx.x; i < P.n; i += nt) P.z[i] = jacobi_step<T>(P.t[i], P.r[i], P.rd[i], offsum<T>(P, P.t, i));
-        __syncthreads();
+    }
+    for (int i = tid; i < nc; i += kTailBlock) {
+        const T *Mi = vec(Q.sminv) + i, *r = vec(Q.sr);
+        T sum = 0;
+#pragma unroll 8
+        for (int j = 0; j < nc; j++) sum += Mi[j * nc] * r[j];
+        vec(Q.sz)[i] = sum;
+        if (nl == 0 && rank == 0) ((T *)Q.z)[i] = sum;
+    }
+    __syncthreads();
+    const T sc = (T)kOverCorrect;
+    for (int l = nl - 1; l >= 0; l--) {
+        // t goes to the other buffer than on the way down: a slower CTA may
+        // still be summing the last residual of that
+        const TailLevel &v = Q.lv[l];
+        const int i = (v.whole ? 0 : rank * v.R) + tid, tb = t_up(l);
+        const bool mine = tid < v.R && i < v.n;
+        const int len = mine ? idx(v.slen)[tid] : 0;
+        const T *zl = vec(v.sz), *zc = vec(l + 1 < nl ? Q.lv[l + 1].sz : Q.sz), *tc = vec(tb);
+        const int *ag = idx(v.sagg);
+        const T r = mine ? vec(v.sr)[tid] : (T)0, rd = mine ? vec(v.srd)[tid] : (T)0;
+        T tv = 0;
+        if (mine) {
+            const T xi = zl[i] + sc * zc[ag[i]];
+            tv = jacobi_step<T, 1>(xi, r, rd, row_sum(v, i, len, (T)0, [&](int j) { return zl[j] + sc * zc[ag[j]]; }, false));
+            put(v, tb, i, tv);
+        }
+        sync(v);
+        if (mine) {
+            const T z = jacobi_step<T>(tv, r, rd, row_sum(v, i, len, (T)0, [&](int j) { return tc[j]; }, false));
+            if (l > 0) put(v, v.sz, i, z);
+            else if (!v.whole || rank == 0) ((T *)Q.z)[i] = z;
+        }
+        if (l > 0) sync(v);
     }
 }
 
@@ -982,6 +1115,67 @@ int prepare_case_amg(CasePrep *p) {
     return CFDL_OK;
 }
 
+// The plan of a case's tail for one precision, uploaded once (its hierarchy
+// does not change).
+template <class T> static int build_tail_plan(HostCase *hc, const AmgLevelDev *lev, const TailPlan **out, int *smem) {
+    const CaseDev &d = hc->dev;
+    const int lt = d.amg_tail, nl = d.nlev - lt;
+    constexpr int sz = (int)sizeof(T);
+    TailPlan plan{}, *P = &plan;
+    int at = 0;
+    auto take = [&](long bytes) { const int o = at; at += (int)((bytes + 15) & ~15L); return o; };
+    auto rows = [&](int l) { return l == 0 ? hc->ne : lev[l - 1].n; };
+    P->nl = nl;
+    P->nc = d.ncoarse;
+    P->sz = take((long)P->nc * sz);
+    P->sr = take((long)P->nc * sz);
+    P->sminv = take((long)P->nc * P->nc * sz);
+    P->minv = sz == 8 ? (const void *)d.cinv : (const void *)d.cinv32;
+    if (lt == 0) {                                         // no coarse level: the mesh level is solved directly
+        P->r = sz == 8 ? (const void *)d.kr : (const void *)d.fr;
+        P->z = sz == 8 ? (void *)d.ks : (void *)d.fz;
+    } else {
+        P->r = sz == 8 ? (const void *)lev[lt - 1].r : (const void *)lev[lt - 1].r32;
+        P->z = sz == 8 ? (void *)lev[lt - 1].z : (void *)lev[lt - 1].z32;
+    }
+    for (int b = 0; b < 2; b++) {
+        P->t[b] = take(nl > 0 ? (long)rows(lt) * sz : 0);
+        P->w[b] = take((long)tail_whole<T>() * sz);
+    }
+    for (int l = 0; l < nl; l++) {
+        const AmgLevelDev &A = lev[lt + l - 1], &B = lev[lt + l];   // level lt + l and the one below
+        TailLevel &v = P->lv[l];
+        v.n = A.n;
+        v.whole = v.n <= tail_whole<T>();
+        v.R = v.whole ? v.n : (v.n + kTailCtas - 1) / kTailCtas;
+        v.a = sz == 8 ? (const void *)A.a : (const void *)A.a32;
+        v.rd = sz == 8 ? (const void *)A.rd : (const void *)A.rd32;
+        v.dg = sz == 8 ? (const void *)A.dg : (const void *)A.dg32;
+        v.nb = A.nb; v.len = A.len;
+        v.agg = B.agg; v.mem = B.mem; v.mptr = B.mem_ptr;
+        v.srd = take((long)v.R * sz); v.sdg = take((long)v.R * sz); v.sr = take((long)v.R * sz);
+        v.slen = take(4L * v.R);
+        v.sz = take((long)v.n * sz);
+        v.sagg = take(4L * v.n); v.smem_ = take(4L * v.n); v.smptr = take(4L * (B.n + 1));
+    }
+    for (int l = nl - 1; l >= 0; l--) {                    // the small levels first: the tail level takes what is left
+        TailLevel &v = P->lv[l];
+        const int room = kTailMaxSmem - at - 32, per = v.R * (sz + 4);
+        v.S = std::min(lev[lt + l - 1].W, room > 0 ? room / per : 0);
+        v.sa = take((long)v.R * v.S * sz);
+        v.snb = take(4L * v.R * v.S);
+    }
+    P->total = at;
+    if (at > kTailMaxSmem) return CFDL_ERR_MESH;           // cannot happen (see TailPlan)
+    TailPlan *dp = nullptr;
+    int st = dzeros(hc, &dp, 1);
+    if (st) return st;
+    if ((st = cuda_status(cudaMemcpy(dp, P, sizeof(TailPlan), cudaMemcpyHostToDevice)))) return st;
+    *out = dp;
+    *smem = at;
+    return CFDL_OK;
+}
+
 // Upload a host-built hierarchy into the case, which takes ownership of it.
 int upload_case_amg(HostCase *hc, AmgHierarchy *H) {
     CaseDev &d = hc->dev;
@@ -1034,6 +1228,17 @@ int upload_case_amg(HostCase *hc, AmgHierarchy *H) {
     d.nlev = nlev;
     d.ncoarse = ncoarse;
     d.lev = dlev;
+    // the tail level: the first coarse level of at most kTailRows rows (the
+    // coarsest always qualifies); a case without coarse levels solves its mesh
+    // level directly (tail level 0)
+    d.amg_tail = 0;
+    for (int l = 1; l <= nlev; l++)
+        if (H->levels[l - 1].n <= kTailRows) { d.amg_tail = l; break; }
+    const TailPlan *tp = nullptr;
+    if ((st = build_tail_plan<double>(hc, devl.data(), &tp, &hc->tail_smem64))) return st;
+    d.tail64 = tp;
+    if ((st = build_tail_plan<float>(hc, devl.data(), &tp, &hc->tail_smem32))) return st;
+    d.tail32 = tp;
     return CFDL_OK;
 }
 
@@ -1066,15 +1271,6 @@ int ensure_amg(cfdl_ctx *ctx) {
     ctx->amg_restr.assign(lmax + 1, WorkList());
     ctx->amg_grestr.assign(lmax + 1, WorkList());
     ctx->amg_grouped.assign(lmax + 1, 0);
-    // each case's tail level: its first coarse level of at most kTailRows rows
-    // (the coarsest always qualifies); a case without coarse levels solves its
-    // mesh level directly (tail level 0)
-    for (HostCase *hc : ctx->cases) {
-        int lt = 0;
-        for (int l = 1; l <= hc->dev.nlev; l++)
-            if (hc->amg->levels[l - 1].n <= kTailRows) { lt = l; break; }
-        hc->dev.amg_tail = lt;
-    }
     for (int l = 0; l <= lmax; l++) {
         std::vector<int> cells, smooth, restr;
         for (HostCase *hc : ctx->cases) {
@@ -1123,6 +1319,33 @@ int ensure_amg(cfdl_ctx *ctx) {
         if (p_) prof_end(ctx);                                                                       \
         ctx->launches++;                                                                             \
     } while (0)
+
+// The V-cycle's tail: one cluster of kTailCtas CTAs per case
+template <class T> static void launch_tail(cfdl_ctx *ctx) {
+    const int nc = (int)ctx->cases.size();
+    if (nc == 0) return;
+    int smem = 0;                       // the largest plan of the cases
+    for (const HostCase *hc : ctx->cases) smem = std::max(smem, sizeof(T) == 8 ? hc->tail_smem64 : hc->tail_smem32);
+    const bool p_ = ctx->prof && prof_wants(ctx, "k_v_tail");
+    if (p_) prof_begin(ctx, "k_v_tail");
+    cudaFuncSetAttribute(k_v_tail<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailMaxSmem);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(nc * kTailCtas));
+    cfg.blockDim = dim3((unsigned)kTailBlock);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kTailCtas;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = ctx->pdl ? 2 : 1;
+    cudaLaunchKernelEx(&cfg, k_v_tail<T>, (const CaseDev *)ctx->d_cases, nc);
+    if (p_) prof_end(ctx);
+    ctx->launches++;
+}
 
 // Coarse operators of every level and the coarsest inverse.
 static void amg_setup_operators(cfdl_ctx *ctx) {
@@ -1192,8 +1415,8 @@ template <class T> static void vcycle(cfdl_ctx *ctx) {
         if (G > 1) { GROUPED(l ? "k_v_restrict_c" : "k_v_restrict_f", k_vg_restrict, ctx->amg_grestr[l + 1], 0, l + 1) }
         else ALAUNCH(l ? "k_v_restrict_c" : "k_v_restrict_f", k_v_restrict<T>, ctx->amg_restr[l + 1], l + 1);
     }
-    // each case's small levels and its coarsest solve, one CTA per case
-    CLAUNCH("k_v_tail", k_v_tail<T>, kTailThreads);
+    // each case's small levels and its coarsest solve, one cluster per case
+    launch_tail<T>(ctx);
     for (int l = L - 1; l >= 0; l--) {
         const int G = ctx->amg_grouped[l];
         if (G > 1) {

@@ -40,4 +40,28 @@ struct AmgLevelDev {
     float *a32, *dg32, *rd32, *r32, *z32, *t32; // FP32 copies (mixed-precision form)
 };
 
+// Plan of a case's tail for one precision, built on the host when the
+// hierarchy is: the levels counted from the tail level, their arrays, and the
+// places (bytes from the start of the dynamic shared memory) they are staged
+// at.  S slots of each row are staged: all of them unless memory runs out; the
+// tail level's last slots are then read from global memory.  The rest is
+// bounded: aggregation at least halves a level but for isolated cells, of
+// which a usable hierarchy has at most kAmgCoarsest, so the levels hold fewer
+// than 5000 rows in all and everything but the slots takes under 190 KB.
+struct TailLevel {
+    int n, R, S, whole;                                    // rows, rows per CTA, staged slots, done whole
+    int sa, snb, srd, sdg, slen, sr;                       // the CTA's own rows
+    int sz, sagg, smem_, smptr;                            // the whole level
+    const void *a, *rd, *dg;
+    const int *nb, *len, *agg, *mem, *mptr;
+};
+struct TailPlan {
+    int nl, nc;                                            // smoothed levels; rows of the coarsest
+    int t[2], w[2], sz, sr, sminv, total;
+    const void *r, *minv;                                  // the tail level's r, the coarsest inverse
+    void *z;                                               // the tail level's z
+    TailLevel lv[kAmgMaxLevels];
+};
+
+
 }  // namespace cfdl

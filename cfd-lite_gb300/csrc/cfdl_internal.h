@@ -82,6 +82,7 @@ enum FaceProp {
 
 struct AmgLevelDev;
 struct AmgHierarchy;
+struct TailPlan;
 
 // BiCGStab scalars, one lane per right-hand side
 struct KLanes {
@@ -150,7 +151,8 @@ struct CaseDev {
     // 1/ap of the operator being solved (momentum, then pressure), AMG levels, coarsest inverse
     double *rap;
     int nlev, ncoarse;                    // coarse levels; cells of the coarsest level
-    int amg_tail;                         // first level the one-CTA V-cycle tail runs (k_v_tail)
+    int amg_tail;                         // first level the V-cycle's tail runs (k_v_tail)
+    const struct TailPlan *tail64, *tail32;   // the tail's levels and shared-memory plan, FP64 and FP32
     const AmgLevelDev *lev;               // [nlev] device array
     // [W][ne] the mesh level's interior neighbours as 16-bit offsets j - i
     // (kNb16None: no interior neighbour) for the mixed pressure solve's FP32
@@ -195,6 +197,7 @@ struct HostCase {
     CaseDev dev{};                   // host mirror of the device struct
     AmgHierarchy *amg = nullptr;     // host hierarchy, built on first AMG use
     std::vector<void *> amg_allocs;  // device allocations of the hierarchy
+    int tail_smem64 = 0, tail_smem32 = 0;   // shared memory of the V-cycle's tail (TailPlan), FP64 and FP32
     int id = 0;                      // stable case id within its context
     bool props_dirty = true;         // fprop must be recomputed (rho or mu changed)
     size_t bytes = 0;                // device bytes held (mesh, fields, solver, hierarchy)
