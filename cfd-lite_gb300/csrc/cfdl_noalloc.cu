@@ -9,8 +9,21 @@
 // partials, scalars) in one file-scope __device__ array of fixed size.
 //
 // Algorithm: the Jacobi-preconditioned CG of the context path (set_a_0 then
-// CG from zero on the zero-mean right-hand side), one thread per cell over
-// the CSR rows, deterministic tile reductions.
+// CG from zero on the zero-mean right-hand side), the whole solve in one
+// cooperative launch.  At up to 131072 rows an iteration's arithmetic is
+// 1-4 us and the rest of it latency.  As three launches (A p with its dot
+// product; x, r, z with theirs; p) with a host poll every few iterations it
+// took 24 us an iteration at 729 rows, 28 at 64000 and 33 at 125000.  Here a
+// thread owns a row: its coefficients, x, r, z and p stay in registers, and an
+// iteration is two all-reduces with one exchange of z and p through L2 between
+// them: 7.0, 13.5 and 15.8 us.  About one CTA per SM, so that every SM's FP64
+// pipe (2 instructions per clock) takes an equal share.
+//
+// An all-reduce is barrier and sum in one: each CTA publishes its partials as
+// 8-byte words that carry 32 bits of the value and the step's number, and
+// every CTA polls all of them and sums them in CTA order (deterministic, the
+// same in all CTAs).  The polls are bounded: a CTA that gives up sets its
+// failure and leaves, and so do the others after it.
 #include "cfdl_internal.h"
 #include "cfdl_device.cuh"
 #include <cstddef>
@@ -19,119 +32,242 @@ namespace cfdl {
 namespace {
 
 constexpr int kNaMaxCells = 131072;                 // CFDL_NOALLOC_MAX_CELLS
-constexpr int kNaMaxTiles = kNaMaxCells / kTile;
+constexpr int kNaMaxCtas = 512;                     // CTAs of a solve (their partials' slots)
+constexpr int kNaMinBlock = 128, kNaMaxBlock = 1024;
+constexpr int kNaW = 6;                             // couplings of a row kept in registers
+constexpr int kNaVals = 3;                          // values of the widest all-reduce
+constexpr int kNaPolls = 1 << 22;                   // about a second
 
 struct NoAllocScratch {
-    double r[kNaMaxCells], z[kNaMaxCells], p[kNaMaxCells], q[kNaMaxCells];
-    double partials[kNaMaxTiles * kNPart];
-    double mean, rz, alpha, beta, rnorm, r0, tol;
-    int counter[4];
-    int active, iters, bad;
-    int fail;           // why CG stopped early: 0 it did not, 1 a non-finite value, 2 p.Ap <= 0
+    double z[kNaMaxCells], p[kNaMaxCells];          // what neighbouring rows read
+    ulonglong2 slot[2][kNaVals][kNaMaxCtas];        // partials of two consecutive all-reduces
+    // how CG ended
+    double rnorm, tol;
+    int iters, bad;
+    int fail;           // why CG stopped early: 0 it did not, 1 a non-finite value, 2 p.Ap <= 0, 3 a wait ran out
 };
 
 // Shared by every call on a device and kept between calls.
 static __device__ __align__(256) NoAllocScratch g_na_scratch;
 
-// Row i of the pressure operator from the caller's CSR arrays.  Indices are
-// checked against ne and nh; a bad one is recorded and its access skipped.
-__device__ __forceinline__ double csr_amul(NoAllocScratch *S, int ne, int nh, const int *ef1, const int *idx,
-                                           const double *ap, const double *anb, const double *x, int i) {
-    double s = ap[i] * x[i];
-    int h0 = idx[i] - 1, h1 = idx[i + 1] - 1;
-    if (h0 < 0 || h1 > nh || h0 > h1) { S->bad = 1; return s; }
-    for (int h = h0; h < h1; h++) {
-        const int enb = (int)((unsigned)ef1[h] >> 5), lf = ef1[h] & 31;
-        if (!lf) continue;
-        if (enb < 1 || enb > ne) { S->bad = 1; continue; }
-        s -= anb[h] * x[enb - 1];
+// The scalars of CG, one copy per CTA (every CTA forms the same ones).
+struct NaScalars {
+    double mean, rz, alpha, beta, rr, tol2;    // rr = ||r||^2, stopped at tol2
+    int iters, bad, fail, active;
+};
+template <int NT> struct NaShared {
+    double sm[kNaVals][NT], res[kNaVals];
+    NaScalars c;
+};
+
+// Sums v over all CTAs; thread 0 of each then runs fin(sums), which updates
+// the block's scalars: one thread, because an FP64 division or square root is
+// 600 clocks of latency for one warp but 2500 when sixteen warps repeat it.
+// False when a wait ran out.  step counts the all-reduces from 1.  With
+// exchange, what the block wrote to global memory before is visible to every
+// CTA after.
+template <int K, int NT, class F>
+__device__ __forceinline__ bool na_all_sum(NoAllocScratch *S, NaShared<NT> &B, const double (&v)[K], unsigned step,
+                                           bool exchange, F fin) {
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nt = blockDim.x, n = gridDim.x;
+    ulonglong2(*slot)[kNaMaxCtas] = S->slot[step & 1];
+#pragma unroll
+    for (int k = 0; k < K; k++) B.sm[k][tid] = v[k];
+    __syncthreads();
+    const unsigned long long tag = (unsigned long long)step << 32;
+    if (wid < K) {                                  // a warp per value (blocks have at least four)
+        constexpr int kPer = NT / 32;
+        double a[kPer];
+#pragma unroll
+        for (int u = 0; u < kPer; u++) a[u] = u * 32 < nt ? B.sm[wid][u * 32 + lane] : 0.0;
+#pragma unroll
+        for (int o = kPer / 2; o > 0; o >>= 1)
+#pragma unroll
+            for (int u = 0; u < o; u++) a[u] += a[u + o];
+        double s = a[0];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+        if (lane == 0) {
+            if (exchange) __threadfence();          // the block's writes, ordered before by the barrier
+            const unsigned long long b = (unsigned long long)__double_as_longlong(s);
+            ulonglong2 *w = &slot[wid][blockIdx.x];
+            asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(&w->x), "l"(tag | (b >> 32)) : "memory");
+            asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(&w->y), "l"(tag | (b & 0xffffffffull)) : "memory");
+        }
     }
-    return s;
+    __syncthreads();                                // sm is read; it takes the CTAs' partials next
+    bool ok = true;
+#pragma unroll
+    for (int k = 0; k < K; k++)
+        for (int cta = tid; cta < n; cta += nt) {
+            const ulonglong2 *w = &slot[k][cta];
+            unsigned long long x = 0, y = 0;
+            int it = 0;
+            do {
+                asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(x) : "l"(&w->x) : "memory");
+                asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(y) : "l"(&w->y) : "memory");
+            } while (((x >> 32) != step || (y >> 32) != step) && ++it < kNaPolls);
+            ok = ok && it < kNaPolls;
+            if (cta < NT) B.sm[k][cta] = __longlong_as_double((long long)(x << 32 | (y & 0xffffffffull)));
+        }
+    if (exchange) __threadfence();
+    ok = __syncthreads_and(ok);
+    if (!ok) return false;
+    if (wid < K) {
+        double s0 = 0.0, s1 = 0.0;
+        for (int i = lane; i < n; i += 64) {
+            s0 += B.sm[wid][i];
+            if (i + 32 < n) s1 += B.sm[wid][i + 32];
+        }
+        s0 += s1;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+        if (lane == 0) B.res[wid] = s0;
+    }
+    if (K > 1) __syncthreads();
+    if (tid == 0) fin(B.res);
+    __syncthreads();
+    return true;
 }
 
-__global__ void __launch_bounds__(kTile) k_na_mean(NoAllocScratch *S, int ne, const double *b) {
-    const int i = blockIdx.x * kTile + threadIdx.x;
-    double v[1] = {i < ne ? b[i] : 0.0};
-    __shared__ double s[1];
-    if (case_sums<1>(v, &S->counter[0], S->partials, 0, (int)gridDim.x, s)) {
-        if (threadIdx.x == 0) S->mean = s[0] / ne;
+// The solve.  Thread t of the grid owns rows t, t + T, ... (T threads; R rows
+// at most).  Indices are checked against ne and nh; a bad one is recorded and
+// its access skipped.  NT: the largest block (1024 threads have 64 registers
+// each, and spill; 512 have 128).
+template <int R, int NT>
+__global__ void __launch_bounds__(NT) k_na_solve(NoAllocScratch *S, int ne, int nh, const int *ef1, const int *idx,
+                                                 const double *ap, const double *anb, const double *b, double *phic,
+                                                 double rtol, int maxit) {
+    const int T = (int)(gridDim.x * blockDim.x), t0 = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    __shared__ NaShared<NT> B;
+    NaScalars &c = B.c;
+    unsigned step = 0;
+    double x[R], r[R], z[R], p[R], q[R], d[R], rd[R], a[R][kNaW];
+    int j[R][kNaW], h0[R], h1[R];
+    double s1[1] = {0.0}, s2[2], s3[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int u = 0; u < R; u++) {
+        const int i = t0 + u * T;
+        x[u] = r[u] = z[u] = p[u] = q[u] = 0.0;
+        d[u] = rd[u] = 1.0;
+        h0[u] = h1[u] = 0;
+#pragma unroll
+        for (int k = 0; k < kNaW; k++) { a[u][k] = 0.0; j[u][k] = -1; }
+        if (i >= ne) continue;
+        r[u] = b[i];
+        s1[0] += r[u];
+        d[u] = ap[i];
+        rd[u] = 1.0 / d[u];
+        h0[u] = idx[i] - 1;
+        h1[u] = idx[i + 1] - 1;
+        if (h0[u] < 0 || h1[u] > nh || h0[u] > h1[u]) { s3[2] = 1.0; h0[u] = h1[u] = 0; }
+        for (int h = h0[u]; h < h1[u]; h++) {
+            const int enb = (int)((unsigned)ef1[h] >> 5), lf = ef1[h] & 31;
+            if (lf && (enb < 1 || enb > ne)) s3[2] = 1.0;
+        }
+#pragma unroll
+        for (int k = 0; k < kNaW; k++) {
+            const int h = h0[u] + k;
+            if (h >= h1[u]) continue;
+            const int enb = (int)((unsigned)ef1[h] >> 5), lf = ef1[h] & 31;
+            if (lf && enb >= 1 && enb <= ne) { j[u][k] = enb - 1; a[u][k] = anb[h]; }
+        }
     }
-}
-
-__global__ void __launch_bounds__(kTile) k_na_init(NoAllocScratch *S, int ne, const double *ap, const double *b,
-                                                  double *x, double rtol, int maxit) {
-    const int i = blockIdx.x * kTile + threadIdx.x;
-    double v[2] = {0, 0};
-    if (i < ne) {
-        const double r = b[i] - S->mean, z = r / ap[i];
-        S->r[i] = r; S->z[i] = z; S->p[i] = z; x[i] = 0.0;
-        v[0] = r * r; v[1] = r * z;
+    auto give_up = [&]() { S->fail = 3; };
+    if (!na_all_sum<1>(S, B, s1, ++step, false, [&](const double *s) { c.mean = s[0] / ne; })) { give_up(); return; }
+#pragma unroll
+    for (int u = 0; u < R; u++) {
+        const int i = t0 + u * T;
+        if (i >= ne) continue;
+        r[u] -= c.mean;
+        z[u] = r[u] * rd[u];
+        __stcg(&S->z[i], z[u]);
+        s3[0] += r[u] * r[u];
+        s3[1] += r[u] * z[u];
     }
-    __shared__ double s[2];
-    if (case_sums<2>(v, &S->counter[1], S->partials, 0, (int)gridDim.x, s)) {
-        if (threadIdx.x == 0) {
-            S->r0 = S->rnorm = sqrt(s[0]);
-            S->rz = s[1];
-            S->tol = rtol * S->r0;
-            S->iters = 0;
-            S->bad = 0;
+    if (!na_all_sum<3>(S, B, s3, ++step, true, [&](const double *s) {
+            c.rz = s[1];
+            c.rr = s[0];
+            c.tol2 = rtol * rtol * s[0];
+            c.beta = 0.0;
+            c.iters = c.bad = 0;
             // a zero or non-finite diagonal entry makes z = r/ap, and so (r, z), non-finite
-            S->fail = isfinite(S->r0) && isfinite(S->rz) ? 0 : 1;
-            S->active = S->r0 > S->tol && maxit > 0 && !S->fail;
+            c.fail = isfinite(c.rr) && isfinite(c.rz) ? 0 : 1;
+            c.active = c.rr > c.tol2 && maxit > 0 && !c.fail;
+            if (c.active && s[2] > 0.0) { c.bad = 1; c.active = 0; }
+        })) { give_up(); return; }
+    bool first = true;
+    while (c.active) {
+        // p = z + beta p, formed for the row and its neighbours (their p is not
+        // written yet); q = A p
+        const double beta = c.beta;
+        s1[0] = 0.0;
+#pragma unroll
+        for (int u = 0; u < R; u++) {
+            const int i = t0 + u * T;
+            if (i >= ne) continue;
+            double zn[kNaW], pn[kNaW];
+#pragma unroll
+            for (int k = 0; k < kNaW; k++) {
+                const bool in = j[u][k] >= 0;
+                zn[k] = in ? __ldcg(&S->z[j[u][k]]) : 0.0;
+                pn[k] = in && !first ? __ldcg(&S->p[j[u][k]]) : 0.0;
+            }
+            p[u] = z[u] + beta * p[u];
+            // two sums of three slots: half the dependent chain
+            double s = d[u] * p[u], s4 = 0.0;
+#pragma unroll
+            for (int k = 0; k < kNaW; k += 2) {
+                s -= a[u][k] * (zn[k] + beta * pn[k]);
+                s4 += a[u][k + 1] * (zn[k + 1] + beta * pn[k + 1]);
+            }
+            s -= s4;
+            for (int h = h0[u] + kNaW; h < h1[u]; h++) {    // rows of more couplings
+                const int enb = (int)((unsigned)ef1[h] >> 5), lf = ef1[h] & 31;
+                if (lf) s -= anb[h] * (__ldcg(&S->z[enb - 1]) + (first ? 0.0 : beta * __ldcg(&S->p[enb - 1])));
+            }
+            q[u] = s;
+            s1[0] += p[u] * s;
         }
-    }
-}
-
-__global__ void __launch_bounds__(kTile) k_na_q(NoAllocScratch *S, int ne, int nh, const int *ef1, const int *idx,
-                                               const double *ap, const double *anb) {
-    if (!S->active) return;
-    const int i = blockIdx.x * kTile + threadIdx.x;
-    double v[1] = {0};
-    if (i < ne) {
-        const double q = csr_amul(S, ne, nh, ef1, idx, ap, anb, S->p, i);
-        S->q[i] = q;
-        v[0] = S->p[i] * q;
-    }
-    __shared__ double s[1];
-    if (case_sums<1>(v, &S->counter[2], S->partials, 0, (int)gridDim.x, s)) {
-        if (threadIdx.x == 0) {
-            // only runs while ||r|| is above the tolerance, where an SPD system has p.Ap > 0
-            if (S->bad) S->active = 0;
-            else if (!isfinite(s[0])) { S->active = 0; S->fail = 1; }
-            else if (!(s[0] > 0.0)) { S->active = 0; S->fail = 2; }
-            else S->alpha = S->rz / s[0];
+        first = false;
+        if (!na_all_sum<1>(S, B, s1, ++step, false, [&](const double *s) {
+                // only runs while ||r|| is above the tolerance, where an SPD system has p.Ap > 0
+                if (!isfinite(s[0])) { c.fail = 1; c.active = 0; }
+                else if (!(s[0] > 0.0)) { c.fail = 2; c.active = 0; }
+                else c.alpha = c.rz / s[0];
+            })) { give_up(); return; }
+        if (!c.active) break;
+        const double alpha = c.alpha;
+        s2[0] = s2[1] = 0.0;
+#pragma unroll
+        for (int u = 0; u < R; u++) {
+            const int i = t0 + u * T;
+            if (i >= ne) continue;
+            x[u] += alpha * p[u];
+            r[u] -= alpha * q[u];
+            z[u] = r[u] * rd[u];
+            __stcg(&S->z[i], z[u]);
+            __stcg(&S->p[i], p[u]);
+            s2[0] += r[u] * r[u];
+            s2[1] += r[u] * z[u];
         }
+        if (!na_all_sum<2>(S, B, s2, ++step, true, [&](const double *s) {
+                c.rr = s[0];
+                c.iters += 1;
+                c.beta = c.rz != 0.0 ? s[1] / c.rz : 0.0;
+                c.rz = s[1];
+                if (!isfinite(c.rr) || !isfinite(c.rz)) c.fail = 1;
+                c.active = c.rr > c.tol2 && c.iters < maxit && !c.fail;
+            })) { give_up(); return; }
     }
-}
-
-__global__ void __launch_bounds__(kTile) k_na_x(NoAllocScratch *S, int ne, const double *ap, double *x, int maxit) {
-    if (!S->active) return;
-    const int i = blockIdx.x * kTile + threadIdx.x;
-    double v[2] = {0, 0};
-    if (i < ne) {
-        const double a = S->alpha;
-        x[i] = x[i] + a * S->p[i];
-        const double r = S->r[i] - a * S->q[i], z = r / ap[i];
-        S->r[i] = r; S->z[i] = z;
-        v[0] = r * r; v[1] = r * z;
+#pragma unroll
+    for (int u = 0; u < R; u++)
+        if (t0 + u * T < ne) phic[t0 + u * T] = x[u];
+    if (t0 == 0) {
+        S->rnorm = sqrt(c.rr); S->tol = sqrt(c.tol2);
+        S->iters = c.iters; S->bad = c.bad;
+        if (c.fail) S->fail = c.fail;
     }
-    __shared__ double s[2];
-    if (case_sums<2>(v, &S->counter[3], S->partials, 0, (int)gridDim.x, s)) {
-        if (threadIdx.x == 0) {
-            S->rnorm = sqrt(s[0]);
-            S->iters += 1;
-            S->beta = S->rz != 0.0 ? s[1] / S->rz : 0.0;
-            S->rz = s[1];
-            if (!isfinite(S->rnorm) || !isfinite(S->rz)) S->fail = 1;
-            S->active = S->rnorm > S->tol && S->iters < maxit && !S->fail;
-        }
-    }
-}
-
-__global__ void __launch_bounds__(kTile) k_na_p(NoAllocScratch *S, int ne) {
-    if (!S->active) return;
-    const int i = blockIdx.x * kTile + threadIdx.x;
-    if (i < ne) S->p[i] = S->z[i] + S->beta * S->p[i];
 }
 
 // Device address of the scratch array on the current device.  The host-side
@@ -169,42 +305,45 @@ extern "C" int cfdl_solve_pc_noalloc(int ne, int nh, const int *ef2nb1, const in
     int st = na_scratch(&S);
     if (st) return st;
     const cudaStream_t s0 = 0;
-    const int grid = (ne + kTile - 1) / kTile;
-    // the last-tile counters must start at zero on every call
-    cudaError_t e = cudaMemsetAsync(S->counter, 0, sizeof(S->counter), s0);
+    // about one CTA per SM; a device of fewer SMs than the rows need at one row
+    // a thread takes eight
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return cuda_status(e);
-    k_na_mean<<<grid, kTile, 0, s0>>>(S, ne, b);
-    k_na_init<<<grid, kTile, 0, s0>>>(S, ne, ap, b, phic, rtol, maxit);
-    int it = 0, active = 1, chunk = 4;
-    while (it < maxit) {
-        for (int k = 0; k < chunk && it < maxit; k++, it++) {
-            k_na_q<<<grid, kTile, 0, s0>>>(S, ne, nh, ef2nb1, ef2nb_idx, ap, anb);
-            k_na_x<<<grid, kTile, 0, s0>>>(S, ne, ap, phic, maxit);
-            k_na_p<<<grid, kTile, 0, s0>>>(S, ne);
-        }
-        e = cudaMemcpyAsync(&active, &S->active, sizeof(int), cudaMemcpyDeviceToHost, s0);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s0);
-        if (e != cudaSuccess) return cuda_status(e);
-        if (!active) break;
-        chunk = chunk < 64 ? chunk * 2 : 64;
-    }
-    // iters, bad and fail are adjacent ints; rnorm and tol are read alone
-    int flags[3] = {0, 0, 0};
-    double rn = 0.0, tol = 0.0;
-    static_assert(offsetof(NoAllocScratch, bad) == offsetof(NoAllocScratch, iters) + sizeof(int) &&
-                  offsetof(NoAllocScratch, fail) == offsetof(NoAllocScratch, bad) + sizeof(int),
-                  "iters, bad, fail must be adjacent");
-    e = cudaMemcpyAsync(flags, &S->iters, sizeof(flags), cudaMemcpyDeviceToHost, s0);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&rn, &S->rnorm, sizeof(double), cudaMemcpyDeviceToHost, s0);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&tol, &S->tol, sizeof(double), cudaMemcpyDeviceToHost, s0);
+    if (sms > kNaMaxCtas) sms = kNaMaxCtas;
+    const int rows = (long long)sms * kNaMaxBlock >= ne ? 1 : 8;
+    const int threads = (ne + rows - 1) / rows;
+    int block = ((threads + sms - 1) / sms + 31) & ~31;
+    if (block < kNaMinBlock) block = kNaMinBlock;
+    if (block > kNaMaxBlock) return CFDL_ERR_CUDA;
+    const int grid = (threads + block - 1) / block;
+    // step numbers start over with every call: no slot may hold one
+    e = cudaMemsetAsync(S->slot, 0, sizeof(NoAllocScratch) - offsetof(NoAllocScratch, slot), s0);
+    if (e != cudaSuccess) return cuda_status(e);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.stream = s0;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;       // every CTA resident: they wait for one another
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelEx(&cfg, rows > 1 ? k_na_solve<8, 1024> : block > 512 ? k_na_solve<1, 1024> : k_na_solve<1, 512>, S, ne, nh, ef2nb1, ef2nb_idx, ap, anb, b, phic,
+                           rtol, maxit);
+    struct { double rnorm, tol; int iters, bad, fail; } end = {};
+    static_assert(offsetof(NoAllocScratch, fail) == offsetof(NoAllocScratch, rnorm) + 24, "the end record is copied whole");
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(&end, &S->rnorm, 28, cudaMemcpyDeviceToHost, s0);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s0);
     if (e != cudaSuccess) return cuda_status(e);
-    const int it_dev = flags[0], bad = flags[1], fail = flags[2];
-    if (iters) *iters = it_dev;
-    if (rnorm) *rnorm = rn;
-    if (bad) return CFDL_ERR_INVALID;
-    if (fail == 1 || !isfinite(rn)) return CFDL_ERR_NONFINITE;
-    if (fail == 2) return CFDL_ERR_BREAKDOWN;
-    if (rn > tol) return CFDL_ERR_ITER_CAP;       // stopped at maxit above the tolerance
+    if (end.fail == 3) return CFDL_ERR_CUDA;
+    if (iters) *iters = end.iters;
+    if (rnorm) *rnorm = end.rnorm;
+    if (end.bad) return CFDL_ERR_INVALID;
+    if (end.fail == 1 || !isfinite(end.rnorm)) return CFDL_ERR_NONFINITE;
+    if (end.fail == 2) return CFDL_ERR_BREAKDOWN;
+    if (end.rnorm > end.tol) return CFDL_ERR_ITER_CAP;       // stopped at maxit above the tolerance
     return CFDL_OK;
 }

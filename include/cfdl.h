@@ -311,7 +311,7 @@ int cfdl_probe_fp64(double *fma_per_s, double *ms);
  *   phic [ne]: output, the interior cells of the pressure correction.
  * It allocates nothing, on the device or the host: its Krylov vectors,
  * reduction partials and scalars live in one file-scope device array sized
- * for CFDL_NOALLOC_MAX_CELLS cells (about 4.2 MB), which every GPU that loads
+ * for CFDL_NOALLOC_MAX_CELLS cells (about 2.2 MB), which every GPU that loads
  * the library holds until the process exits.  Larger systems are rejected
  * with CFDL_ERR_TOO_LARGE.  Each call asks the runtime for that array's
  * device address with the device current (so a cudaDeviceReset between calls
