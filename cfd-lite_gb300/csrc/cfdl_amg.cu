@@ -57,18 +57,19 @@ template <class T> struct LP {
     T *r, *z, *t;
     const int *len;         // coarse levels: valid slots of each row, packed first (null on the mesh level)
     const short *nb16;      // mesh level: the neighbours as 16-bit offsets (CaseDev::nb16), or null
+    int ld;                 // stride of a's and nb16's planes on the FP32 mesh level (n elsewhere)
 };
 
 template <class T> __device__ __forceinline__ LP<T> level(const CaseDev &C, int l);
 template <> __device__ __forceinline__ LP<double> level<double>(const CaseDev &C, int l) {
-    if (l == 0) return {C.ne, C.W, C.hf_nb, C.anb_p, C.ap_p, C.rap_p, C.kr, C.ks, C.ksh, nullptr, C.nb16};
+    if (l == 0) return {C.ne, C.W, C.hf_nb, C.anb_p, C.ap_p, C.rap_p, C.kr, C.ks, C.ksh, nullptr, nullptr, C.ne};
     const AmgLevelDev &L = C.lev[l - 1];
-    return {L.n, L.W, L.nb, L.a, L.dg, L.rd, L.r, L.z, L.t, L.len, nullptr};
+    return {L.n, L.W, L.nb, L.a, L.dg, L.rd, L.r, L.z, L.t, L.len, nullptr, L.n};
 }
 template <> __device__ __forceinline__ LP<float> level<float>(const CaseDev &C, int l) {
-    if (l == 0) return {C.ne, C.W, C.hf_nb, C.fanb_p, C.fdiag_p, C.frap_p, C.fr, C.fz, C.ft, nullptr, C.nb16};
+    if (l == 0) return {C.ne, C.W, C.hf_nb, C.fanb_p, C.fdiag_p, C.frap_p, C.fr, C.fz, C.ft, nullptr, C.nb16, C.ld32};
     const AmgLevelDev &L = C.lev[l - 1];
-    return {L.n, L.W, L.nb, L.a32, L.dg32, L.rd32, L.r32, L.z32, L.t32, L.len, nullptr};
+    return {L.n, L.W, L.nb, L.a32, L.dg32, L.rd32, L.r32, L.z32, L.t32, L.len, nullptr, L.n};
 }
 
 // (A x)_i at a level; neighbours outside [0, n) (halos, padding) are skipped
@@ -87,19 +88,16 @@ template <class T> __device__ __forceinline__ T amul(const LP<T> &P, const T *x,
         if (const int i1 = i0 + kTile, ok0 = i0 < (t).last, ok1 = j_ + 1 < (t).pad && i1 < (t).last; \
             true)
 
-template <class T, bool k16> __device__ __forceinline__ T amul_mesh(const LP<T> &P, const T *x, int i);
-
-// CG's q = A p over a thread's rows of a wide tile, returning its share of
-// (p, q), two rows per step
-template <class T, bool k16>
-__device__ __forceinline__ T cg_aq_rows(const LP<T> &P, const T *p, T *q, const Tile &t) {
-    T v = 0;
+// CG's q = A p (FP64) over a thread's rows of a wide tile, returning its share
+// of (p, q), two rows per step
+__device__ __forceinline__ double cg_aq_rows(const LP<double> &P, const double *p, double *q, const Tile &t) {
+    double v = 0;
     FOR_ROW_PAIRS(t) {
-        T q0 = 0, q1 = 0, p0 = 0, p1 = 0;
-        // the int32 form keeps amul's guarded coefficient loads (measured
-        // faster in these multi-row tiles than the mesh sweeps' eager ones)
-        if (ok0) { q0 = k16 ? amul_mesh<T, true>(P, p, i0) : amul<T>(P, p, i0); p0 = p[i0]; }
-        if (ok1) { q1 = k16 ? amul_mesh<T, true>(P, p, i1) : amul<T>(P, p, i1); p1 = p[i1]; }
+        double q0 = 0, q1 = 0, p0 = 0, p1 = 0;
+        // amul's guarded coefficient loads measured faster in these multi-row
+        // tiles than the mesh sweeps' eager ones
+        if (ok0) { q0 = amul<double>(P, p, i0); p0 = p[i0]; }
+        if (ok1) { q1 = amul<double>(P, p, i1); p1 = p[i1]; }
         if (ok0) { q[i0] = q0; v += p0 * q0; }
         if (ok1) { q[i1] = q1; v += p1 * q1; }
     }
@@ -181,18 +179,12 @@ template <class T> __device__ __forceinline__ T amul_coarse(const LP<T> &P, cons
 // kGuard: the row has P.W <= W slots (the mesh level, W = kMaxW); slots past
 // P.W are not read.  kEager false: the coefficient load waits for the index
 // (the coarse levels' kernels, where that form measured faster).
-template <int W, class T, bool kGuard, bool kEager = true, bool k16 = false>
+template <int W, class T, bool kGuard, bool kEager = true>
 __device__ __forceinline__ void row_slots(const LP<T> &P, int i, int (&j)[W], T (&c)[W]) {
 #pragma unroll
     for (int k = 0; k < W; k++) {
         const bool in = !kGuard || k < P.W;
-        int jj;
-        if (k16) {      // the mesh level's 16-bit offsets: half the index bytes
-            const int d = in ? (int)P.nb16[k * P.n + i] : (int)kNb16None;
-            jj = d == (int)kNb16None ? -1 : i + d;
-        } else {
-            jj = in ? P.nb[k * P.n + i] : -1;
-        }
+        const int jj = in ? P.nb[k * P.n + i] : -1;
         const bool ok = (unsigned)jj < (unsigned)P.n;
         j[k] = ok ? jj : i;
         if (kEager) {
@@ -204,55 +196,124 @@ __device__ __forceinline__ void row_slots(const LP<T> &P, int i, int (&j)[W], T 
     }
 }
 
-// The vector a sweep reads: a stored one, or t = w D^-1 r formed on the fly
-// for the first pre-smoothing sweep (the product k_v_jac0 would store; the
-// same multiplication, so the same values)
-template <class T> struct VecIn {
-    const T *x;
-    __device__ __forceinline__ T operator()(int j) const { return x[j]; }
-};
-template <class T> struct VecRdR {
-    const T *rd, *r;
-    __device__ __forceinline__ T operator()(int j) const { return rd[j] * r[j]; }
-};
-
 // sum_j a_ij x_j over the row's couplings inside the level (the ELL values
 // are the off-diagonal magnitudes: A = D - offdiag)
-template <int W, class T, bool kGuard = false, bool kEager = true, bool k16 = false, class X>
-__device__ __forceinline__ T offsum_w(const LP<T> &P, const X &xv, int i) {
+template <int W, class T, bool kGuard = false, bool kEager = true>
+__device__ __forceinline__ T offsum_w(const LP<T> &P, const T *x, int i) {
     int j[W];
     T c[W];
-    row_slots<W, T, kGuard, kEager, k16>(P, i, j, c);
+    row_slots<W, T, kGuard, kEager>(P, i, j, c);
     T xj[W];
 #pragma unroll
-    for (int k = 0; k < W; k++) xj[k] = xv(j[k]);
+    for (int k = 0; k < W; k++) xj[k] = x[j[k]];
     T s = 0;
 #pragma unroll
     for (int k = 0; k < W; k++) s += c[k] * xj[k];
     return s;
 }
 
-// The mesh level (level 0): at most kMaxW slots a row, every width on the
+// The FP64 mesh level (level 0): at most kMaxW slots a row, every width on the
 // short fixed-width paths (no wide-row code in the kernels that use these)
-// k16: the level's neighbours are read from P.nb16 (every case of the launch has them)
-template <class T, bool k16, class X> __device__ __forceinline__ T offsum_mesh(const LP<T> &P, const X &x, int i) {
-    if (P.W == 6) return offsum_w<6, T, false, true, k16>(P, x, i);
-    if (P.W == 4) return offsum_w<4, T, false, true, k16>(P, x, i);
-    return offsum_w<kMaxW, T, true, true, k16>(P, x, i);
+__device__ __forceinline__ double offsum_mesh(const LP<double> &P, const double *x, int i) {
+    if (P.W == 6) return offsum_w<6, double, false>(P, x, i);
+    if (P.W == 4) return offsum_w<4, double, false>(P, x, i);
+    return offsum_w<kMaxW, double, true>(P, x, i);
 }
-template <int W, class T, bool kGuard = false, bool k16 = false> __device__ __forceinline__ T amul_w(const LP<T> &P, const T *x, int i) {
+template <int W, bool kGuard = false> __device__ __forceinline__ double amul_w(const LP<double> &P, const double *x, int i) {
     int j[W];
-    T c[W];
-    row_slots<W, T, kGuard, true, k16>(P, i, j, c);
-    T s = P.dg[i] * x[i];
+    double c[W];
+    row_slots<W, double, kGuard>(P, i, j, c);
+    double s = P.dg[i] * x[i];
 #pragma unroll
     for (int k = 0; k < W; k++) s -= c[k] * x[j[k]];
     return s;
 }
-template <class T, bool k16> __device__ __forceinline__ T amul_mesh(const LP<T> &P, const T *x, int i) {
-    if (P.W == 6) return amul_w<6, T, false, k16>(P, x, i);
-    if (P.W == 4) return amul_w<4, T, false, k16>(P, x, i);
-    return amul_w<kMaxW, T, true, k16>(P, x, i);
+__device__ __forceinline__ double amul_mesh(const LP<double> &P, const double *x, int i) {
+    if (P.W == 6) return amul_w<6>(P, x, i);
+    if (P.W == 4) return amul_w<4>(P, x, i);
+    return amul_w<kMaxW, true>(P, x, i);
+}
+
+// The FP32 mesh level takes its rows two at a time, i (even) and i + 1, with
+// 8-byte coefficient and 4-byte offset (k16; else 8-byte index) loads.  One row
+// per thread was bound by the load instructions, not by the bytes: at 128^3
+// two rows per thread move the same bytes in 18.7 instead of 24.7 us, and with
+// int32 indices in 23.1 instead of 27.1; the FP64 sweep is bound by its FP64
+// instructions and gains nothing.  Planes and vectors have an even length
+// (CaseDev::ld32); the padding row of an odd level has no couplings.
+template <int W, bool k16, bool kGuard>
+__device__ __forceinline__ void pair_slots(const LP<float> &P, int i, int (&j)[2][W], float (&c)[2][W]) {
+    const int n = P.n;
+#pragma unroll
+    for (int k = 0; k < W; k++) {
+        const bool in = !kGuard || k < P.W;
+        int j0 = -1, j1 = -1;
+        float2 a = make_float2(0.f, 0.f);
+        if (in) {
+            if (k16) {
+                const short2 d = *(const short2 *)&P.nb16[k * P.ld + i];
+                j0 = d.x == kNb16None ? -1 : i + d.x;
+                j1 = d.y == kNb16None ? -1 : i + 1 + d.y;
+            } else if ((n & 1) == 0) {
+                const int2 d = *(const int2 *)&P.nb[k * n + i];
+                j0 = d.x;
+                j1 = d.y;
+            } else {                                       // odd rows: the planes are not aligned to pairs
+                j0 = P.nb[k * n + i];
+                j1 = i + 1 < n ? P.nb[k * n + i + 1] : -1;
+            }
+            a = *(const float2 *)&P.a[k * P.ld + i];
+        }
+        const bool ok0 = (unsigned)j0 < (unsigned)n, ok1 = (unsigned)j1 < (unsigned)n;
+        j[0][k] = ok0 ? j0 : i;
+        j[1][k] = ok1 ? j1 : i + 1;
+        c[0][k] = ok0 ? a.x : 0.f;
+        c[1][k] = ok1 ? a.y : 0.f;
+    }
+}
+// the rows' off-diagonal sums of x (kRd: of rd[j] x[j], the product k_v_jac0
+// would store: the same multiplication, so the same values)
+template <int W, bool k16, bool kGuard, bool kRd>
+__device__ __forceinline__ float2 pair_offsum(const LP<float> &P, const float *x, int i) {
+    int j[2][W];
+    float c[2][W], v[2][W];
+    pair_slots<W, k16, kGuard>(P, i, j, c);
+#pragma unroll
+    for (int k = 0; k < W; k++)
+#pragma unroll
+        for (int u = 0; u < 2; u++) v[u][k] = kRd ? P.rd[j[u][k]] * x[j[u][k]] : x[j[u][k]];
+    float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < W; k++) { s.x += c[0][k] * v[0][k]; s.y += c[1][k] * v[1][k]; }
+    return s;
+}
+// the rows of A x
+template <int W, bool k16, bool kGuard>
+__device__ __forceinline__ float2 pair_amul(const LP<float> &P, const float *x, int i) {
+    int j[2][W];
+    float c[2][W], v[2][W];
+    pair_slots<W, k16, kGuard>(P, i, j, c);
+#pragma unroll
+    for (int k = 0; k < W; k++)
+#pragma unroll
+        for (int u = 0; u < 2; u++) v[u][k] = x[j[u][k]];
+    const float2 xi = *(const float2 *)&x[i], d = *(const float2 *)&P.dg[i];
+    // d x_i - c_0 x_0 - c_1 x_1 - ...; its roundings are spelled out, so they do
+    // not depend on which product the compiler would contract
+    float2 s = make_float2(__fmaf_rn(d.x, xi.x, -__fmul_rn(c[0][0], v[0][0])), __fmaf_rn(d.y, xi.y, -__fmul_rn(c[1][0], v[1][0])));
+#pragma unroll
+    for (int k = 1; k < W; k++) { s.x = __fmaf_rn(-c[0][k], v[0][k], s.x); s.y = __fmaf_rn(-c[1][k], v[1][k], s.y); }
+    return s;
+}
+template <bool k16, bool kRd = false> __device__ __forceinline__ float2 pair_offsum_mesh(const LP<float> &P, const float *x, int i) {
+    if (P.W == 6) return pair_offsum<6, k16, false, kRd>(P, x, i);
+    if (P.W == 4) return pair_offsum<4, k16, false, kRd>(P, x, i);
+    return pair_offsum<kMaxW, k16, true, kRd>(P, x, i);
+}
+template <bool k16> __device__ __forceinline__ float2 pair_amul_mesh(const LP<float> &P, const float *x, int i) {
+    if (P.W == 6) return pair_amul<6, k16, false>(P, x, i);
+    if (P.W == 4) return pair_amul<4, k16, false>(P, x, i);
+    return pair_amul<kMaxW, k16, true>(P, x, i);
 }
 // Valid slots of row i: a coarse row's couplings are packed in its first
 // len[i] slots (the rest is padding up to the level's widest row, W).
@@ -260,7 +321,7 @@ template <class T> __device__ __forceinline__ int row_len(const LP<T> &P, int i)
     return P.len ? P.len[i] : P.W;
 }
 
-template <class T, class X> __device__ __forceinline__ T offsum_x(const LP<T> &P, const X &x, int i) {
+template <class T> __device__ __forceinline__ T offsum(const LP<T> &P, const T *x, int i) {
     if (P.W == 6) return offsum_w<6, T, false, false>(P, x, i);
     if (P.W == 4) return offsum_w<4, T, false, false>(P, x, i);
     constexpr int kCh = coarse_chunk<T>();
@@ -277,22 +338,25 @@ template <class T, class X> __device__ __forceinline__ T offsum_x(const LP<T> &P
         for (int u = 0; u < kCh; u++) {
             const bool ok = (unsigned)jj[u] < (unsigned)P.n;
             c[u] = ok ? P.a[(k0 + u) * P.n + i] : (T)0;
-            xv[u] = x(ok ? jj[u] : i);
+            xv[u] = x[ok ? jj[u] : i];
         }
 #pragma unroll
         for (int u = 0; u < kCh; u++) s += c[u] * xv[u];
     }
     return s;
 }
-template <class T> __device__ __forceinline__ T offsum(const LP<T> &P, const T *x, int i) {
-    return offsum_x<T>(P, VecIn<T>{x}, i);
-}
-
 // damped Jacobi sweep from x: x + w D^-1 (r - A x) = (1 - w) x + (w/D)(r + offsum);
 // kSweep 1 with w = kOmega (wrd = rd as stored), 2 with w = kOmega2
 template <class T, int kSweep = 2> __device__ __forceinline__ T jacobi_step(T x, T r, T wrd, T off) {
     if (kSweep == 1) return (T)(1.0 - kOmega) * x + wrd * (r + off);
     return (T)(1.0 - kOmega2) * x + (wrd * (T)(kOmega2 / kOmega)) * (r + off);
+}
+
+// the same on the FP32 mesh level, its roundings spelled out (as pair_amul's)
+template <int kSweep> __device__ __forceinline__ float pair_jacobi(float x, float r, float wrd, float off) {
+    const float b = __fadd_rn(r, off);
+    if (kSweep == 1) return __fmaf_rn((float)(1.0 - kOmega), x, __fmul_rn(wrd, b));
+    return __fmaf_rn(__fmul_rn(wrd, (float)(kOmega2 / kOmega)), b, __fmul_rn((float)(1.0 - kOmega2), x));
 }
 
 __device__ __forceinline__ bool pactive(const CaseDev &C) { return C.sc->active_p != 0; }
@@ -328,7 +392,7 @@ __global__ void __launch_bounds__(kTile) k_amg_prep0(const CaseDev *__restrict__
         C.frap_p[i] = narrow_f32(rd);
 #pragma unroll
         for (int k = 0; k < kMaxW; k++)
-            if (k < C.W) C.fanb_p[k * C.ne + i] = narrow_f32(a[k]);
+            if (k < C.W) C.fanb_p[k * C.ld32 + i] = narrow_f32(a[k]);
     }
 }
 
@@ -414,53 +478,63 @@ __global__ void __launch_bounds__(kTile) k_v_jac0(const CaseDev *__restrict__ ca
     P.t[i] = P.rd[i] * P.r[i];
 }
 
-// z = t + w D^-1 (r - A t).  kMesh: launched on the mesh level only.
-// kToT: the sweep from z into t instead (the first post-smoothing sweep,
-// after k_v_lift has added the prolongated coarse correction to z).
-// kFromR: the first pre-smoothing sweep, from t = w D^-1 r formed on the fly
-// for the row and its neighbours instead of read from k_v_jac0's pass (the
-// same products, so the same z; one pass over the level fewer)
-template <class T, bool kMesh, bool kToT, bool kFromR = false, bool k16 = false>
-__device__ __forceinline__ void v_jac_row(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles, int l) {
+// z = t + w D^-1 (r - A t).  kToT: the sweep from z into t instead (the first
+// post-smoothing sweep, after k_v_lift has added the prolongated coarse
+// correction to z).
+template <class T, bool kToT = false>
+__global__ void __launch_bounds__(kTile) k_v_jac(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles, int l) {
+    CFDL_PDL_WAIT();
     const Tile tl = tiles[blockIdx.x];
     const CaseDev &C = cases[tl.c];
     if (sizeof(T) == 8 ? !pactive(C) : !mactive(C)) return;
     const int i = tl.first + (int)threadIdx.x;
     if (i >= tl.last) return;
     const LP<T> P = level<T>(C, l);
-    if (kFromR) {
-        const VecRdR<T> tv{P.rd, P.r};
-        const T ri = P.r[i], rdi = P.rd[i];
-        const T off = kMesh ? offsum_mesh<T, k16>(P, tv, i) : offsum_x<T>(P, tv, i);
-        P.z[i] = jacobi_step<T, 2>(rdi * ri, ri, rdi, off);
-        return;
-    }
     const T *x = kToT ? P.z : P.t;
     T *y = kToT ? P.t : P.z;
-    if (kMesh) {
-        const T off = offsum_mesh<T, k16>(P, VecIn<T>{x}, i);
-        y[i] = jacobi_step<T, kToT ? 1 : 2>(x[i], P.r[i], P.rd[i], off);
-    } else {
-        // the row's own values first: measured faster on the coarse levels
-        y[i] = jacobi_step<T, kToT ? 1 : 2>(x[i], P.r[i], P.rd[i], offsum<T>(P, x, i));
-    }
+    // the row's own values first: measured faster on the coarse levels
+    y[i] = jacobi_step<T, kToT ? 1 : 2>(x[i], P.r[i], P.rd[i], offsum<T>(P, x, i));
 }
-template <class T, bool kToT = false, bool kFromR = false>
-__global__ void __launch_bounds__(kTile) k_v_jac(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles, int l) {
+// The FP64 mesh-level sweeps (one row per thread, two dependent trips to
+// memory a row) are kernels of their own, so that their register cap, and with
+// it the resident warps and the loads in flight, is set apart from the coarse
+// levels' sweeps: 32 registers, 8 CTAs per SM (one 8-byte spill slot),
+// measured 2-4% faster at 128^3 than the 40 registers and 6 CTAs the compiler
+// picks unbounded; the coarse sweeps would spill 100+ bytes under the same cap.
+template <bool kToT>
+__global__ void __launch_bounds__(kTile, 8) k_v_jac_mesh(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles) {
     CFDL_PDL_WAIT();
-    v_jac_row<T, false, kToT, kFromR>(cases, tiles, l);
+    const Tile tl = tiles[blockIdx.x];
+    const CaseDev &C = cases[tl.c];
+    if (!pactive(C)) return;
+    const int i = tl.first + (int)threadIdx.x;
+    if (i >= tl.last) return;
+    const LP<double> P = level<double>(C, 0);
+    const double *x = kToT ? P.z : P.t;
+    double *y = kToT ? P.t : P.z;
+    const double off = offsum_mesh(P, x, i);
+    y[i] = jacobi_step<double, kToT ? 1 : 2>(x[i], P.r[i], P.rd[i], off);
 }
-// The mesh-level sweeps (one row per thread, two dependent trips to memory
-// a row) are kernels of their own, so that their register cap, and with it
-// the resident warps and the loads in flight, is set apart from the coarse
-// levels' sweeps: 32 registers, 8 CTAs per SM (the FP64 forms keep one
-// 8-byte spill slot), measured 2-4% faster at 128^3 than the 40 registers
-// and 6 CTAs the compiler picks unbounded; the coarse sweeps would spill
-// 100+ bytes under the same cap.
-template <class T, bool k16, bool kToT = false, bool kFromR = false>
-__global__ void __launch_bounds__(kTile, 8) k_v_jac_mesh(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles, int l) {
+// The FP32 mesh-level sweeps, two rows per thread (pair_slots).  kFromR: the
+// first pre-smoothing sweep, from t = w D^-1 r formed on the fly for the rows
+// and their neighbours instead of read from k_v_jac0's pass (the same
+// products, so the same z; one pass over the level fewer)
+template <bool k16, bool kToT, bool kFromR>
+__global__ void __launch_bounds__(kTile / 2, 16) k_v_jac_pair(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles) {
     CFDL_PDL_WAIT();
-    v_jac_row<T, true, kToT, kFromR, k16>(cases, tiles, l);
+    const Tile tl = tiles[blockIdx.x];
+    const CaseDev &C = cases[tl.c];
+    if (!mactive(C)) return;
+    const int i = tl.first + 2 * (int)threadIdx.x;
+    if (i >= tl.last) return;
+    const LP<float> P = level<float>(C, 0);
+    const float *x = kFromR ? P.r : kToT ? P.z : P.t;
+    float *y = kToT ? P.t : P.z;
+    const float2 off = pair_offsum_mesh<k16, kFromR>(P, x, i);
+    const float2 r = *(const float2 *)&P.r[i], rd = *(const float2 *)&P.rd[i];
+    const float2 xi = kFromR ? make_float2(rd.x * r.x, rd.y * r.y) : *(const float2 *)&x[i];
+    *(float2 *)&y[i] = make_float2(pair_jacobi<kToT ? 1 : 2>(xi.x, r.x, rd.x, off.x),
+                                   pair_jacobi<kToT ? 1 : 2>(xi.y, r.y, rd.y, off.y));
 }
 
 // z = z + s P z_{l+1}: the prolongated coarse correction, added in place.
@@ -481,27 +555,41 @@ __global__ void __launch_bounds__(kTile) k_v_lift(const CaseDev *__restrict__ ca
     P.z[i] = P.z[i] + (T)kOverCorrect * zc[L.agg[i]];
 }
 
-// t = r - A z (the smoothed residual, one thread per cell, coalesced)
-template <class T, bool kMesh, bool k16 = false>
-__device__ __forceinline__ void v_resid_row(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles, int l) {
+// t = r - A z (the smoothed residual)
+template <class T>
+__global__ void __launch_bounds__(kTile) k_v_resid(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles, int l) {
+    CFDL_PDL_WAIT();
     const Tile tl = tiles[blockIdx.x];
     const CaseDev &C = cases[tl.c];
     if (sizeof(T) == 8 ? !pactive(C) : !mactive(C)) return;
     const int i = tl.first + (int)threadIdx.x;
     if (i >= tl.last) return;
     const LP<T> P = level<T>(C, l);
-    P.t[i] = P.r[i] - (kMesh ? amul_mesh<T, k16>(P, P.z, i) : amul_coarse<T>(P, P.z, i));
+    P.t[i] = P.r[i] - amul_coarse<T>(P, P.z, i);
 }
-template <class T>
-__global__ void __launch_bounds__(kTile) k_v_resid(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles, int l) {
+// the mesh level's residual, as its sweeps: FP64 with their register cap, FP32
+// two rows per thread
+__global__ void __launch_bounds__(kTile, 8) k_v_resid_mesh(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles) {
     CFDL_PDL_WAIT();
-    v_resid_row<T, false>(cases, tiles, l);
+    const Tile tl = tiles[blockIdx.x];
+    const CaseDev &C = cases[tl.c];
+    if (!pactive(C)) return;
+    const int i = tl.first + (int)threadIdx.x;
+    if (i >= tl.last) return;
+    const LP<double> P = level<double>(C, 0);
+    P.t[i] = P.r[i] - amul_mesh(P, P.z, i);
 }
-// the mesh level's residual, with the mesh sweeps' register cap
-template <class T, bool k16>
-__global__ void __launch_bounds__(kTile, 8) k_v_resid_mesh(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles, int l) {
+template <bool k16>
+__global__ void __launch_bounds__(kTile / 2, 16) k_v_resid_pair(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles) {
     CFDL_PDL_WAIT();
-    v_resid_row<T, true, k16>(cases, tiles, l);
+    const Tile tl = tiles[blockIdx.x];
+    const CaseDev &C = cases[tl.c];
+    if (!mactive(C)) return;
+    const int i = tl.first + 2 * (int)threadIdx.x;
+    if (i >= tl.last) return;
+    const LP<float> P = level<float>(C, 0);
+    const float2 y = pair_amul_mesh<k16>(P, P.z, i), r = *(const float2 *)&P.r[i];
+    *(float2 *)&P.t[i] = make_float2(r.x - y.x, r.y - y.y);
 }
 
 // sum of t over the members of aggregate I of the level below L: four
@@ -975,7 +1063,7 @@ __global__ void __launch_bounds__(kTile) k_apc_q(const CaseDev *__restrict__ cas
     SolveScalars *S = C.sc;
     const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     if (!S->active_p) return;
-    double v[1] = {cg_aq_rows<double, false>(level<double>(C, 0), C.kp, C.kv, t)};
+    double v[1] = {cg_aq_rows(level<double>(C, 0), C.kp, C.kv, t)};
     __shared__ double s[1];
     if (case_sums<1>(v, &C.counters[CNT_A2], partials, tile0, ntiles, s)) {
         if (threadIdx.x == 0) {
@@ -1025,11 +1113,11 @@ __global__ void __launch_bounds__(kTile) k_apc_x(const CaseDev *__restrict__ cas
 
 // the mesh level's neighbour offsets for CaseDev::nb16; overflow is set when
 // an offset does not fit in 16 bits
-__global__ void k_nb16(const int *__restrict__ nb, short *__restrict__ out, int ne, int W, unsigned *overflow) {
+__global__ void k_nb16(const int *__restrict__ nb, short *__restrict__ out, int ne, int ld, int W, unsigned *overflow) {
     const size_t s = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if (s >= (size_t)W * ne) return;
-    const int i = (int)(s % (size_t)ne);
-    const int j = nb[s];
+    if (s >= (size_t)W * ld) return;
+    const int i = (int)(s % (size_t)ld), k = (int)(s / (size_t)ld);
+    const int j = i < ne ? nb[(size_t)k * ne + i] : -1;       // the padding row has no neighbours
     short v = kNb16None;
     if (j >= 0 && j < ne) {
         const int d = j - i;
@@ -1216,11 +1304,11 @@ int upload_case_amg(HostCase *hc, AmgHierarchy *H) {
     if ((st = dzeros(hc, &d.cinv, (size_t)ncoarse * ncoarse))) return st;
     if ((st = dzeros(hc, &d.cinv32, (size_t)ncoarse * ncoarse))) return st;
     if (hc->cfg.precision >= 1) {   // the FP32 mesh kernels' 16-bit neighbour offsets, used when every one fits
-        const size_t nslot = (size_t)hc->W * ne;
+        const size_t nslot = (size_t)hc->W * d.ld32;
         short *nb16 = nullptr;
         unsigned *flag = nullptr, over = 0;
         if ((st = dzeros(hc, &nb16, nslot)) || (st = dzeros(hc, &flag, 1))) return st;
-        k_nb16<<<(unsigned)((nslot + kTile - 1) / kTile), kTile>>>(d.hf_nb, nb16, ne, hc->W, flag);
+        k_nb16<<<(unsigned)((nslot + kTile - 1) / kTile), kTile>>>(d.hf_nb, nb16, ne, d.ld32, hc->W, flag);
         if ((st = cuda_status(cudaGetLastError()))) return st;
         if ((st = cuda_status(cudaMemcpy(&over, flag, sizeof(unsigned), cudaMemcpyDeviceToHost)))) return st;
         d.nb16 = over ? nullptr : nb16;
@@ -1298,12 +1386,13 @@ int ensure_amg(cfdl_ctx *ctx) {
     return upload_case_table(ctx);
 }
 
-#define ALAUNCH(name, kern, WL, ...)                                                                 \
+#define ALAUNCH(name, kern, WL, ...) ALAUNCH_N(name, kern, WL, kTile, ##__VA_ARGS__)
+#define ALAUNCH_N(name, kern, WL, threads, ...)                                                      \
     do {                                                                                             \
         if ((WL).ntiles > 0) {                                                                       \
             const bool p_ = ctx->prof && prof_wants(ctx, name);                                      \
             if (p_) prof_begin(ctx, name);                                                           \
-            launch_k(ctx->pdl, kern, (unsigned)(WL).ntiles, (unsigned)kTile, ctx->stream,                 \
+            launch_k(ctx->pdl, kern, (unsigned)(WL).ntiles, (unsigned)(threads), ctx->stream,             \
                      (const CaseDev *)ctx->d_cases, (const Tile *)(WL).d_tiles, ##__VA_ARGS__);          \
             if (p_) prof_end(ctx);                                                                   \
             ctx->launches++;                                                                         \
@@ -1371,15 +1460,21 @@ static void amg_setup_operators(cfdl_ctx *ctx) {
     default: break;                                                             \
     }
 
+// An FP32 mesh-level kernel, two rows per thread: with 16-bit neighbour offsets
+// when every case has them, else with the int32 indices
+#define MESH32(NAME, K, ...)                                                                              \
+    if (n16) ALAUNCH_N(NAME, (K<true, ##__VA_ARGS__>), ctx->amg_smooth[0], kTile / 2);                    \
+    else ALAUNCH_N(NAME, (K<false, ##__VA_ARGS__>), ctx->amg_smooth[0], kTile / 2);
+
 template <class T> static void vcycle(cfdl_ctx *ctx) {
     // Large levels run one thread per row (G = 1) or a few lanes per row
     // (the autotuned cgroup); small levels run 8 lanes per row, which
     // shortens each thread's chain of loads (amg_grouped[l] = G).
     const int L = ctx->amg_lmax;
     // the FP32 mesh-level kernels read 16-bit neighbour offsets when every
-    // case has them: 52 B a row instead of 64, 8% faster at 128^3; the FP64
-    // sweeps gained 3% for 12% fewer bytes (latency-bound) and keep int32
-    const bool n16 = sizeof(T) == 4 && ctx->amg_nb16;
+    // case has them: 52 B a row instead of 64, 19% faster at 128^3; the FP64
+    // sweeps are bound by their FP64 instructions and keep int32
+    const bool n16 = ctx->amg_nb16;
     for (int l = 0; l < L; l++) {
         int G = ctx->amg_grouped[l];
         if (G > 1) {
@@ -1391,21 +1486,13 @@ template <class T> static void vcycle(cfdl_ctx *ctx) {
             // pass (46.6 -> 33.2 us at 128^3).  The FP64 form keeps the two
             // passes: there the fused sweep measured slower (65.0 -> 74.7 us),
             // and so did the coarse levels' in both forms.
-            if (n16) {
-                ALAUNCH("k_v_jacr_f", (k_v_jac_mesh<T, true, false, true>), ctx->amg_smooth[l], l);
-                ALAUNCH("k_v_resid_f", (k_v_resid_mesh<T, true>), ctx->amg_smooth[l], l);
-            } else {
-                ALAUNCH("k_v_jacr_f", (k_v_jac_mesh<T, false, false, true>), ctx->amg_smooth[l], l);
-                ALAUNCH("k_v_resid_f", (k_v_resid_mesh<T, false>), ctx->amg_smooth[l], l);
-            }
+            MESH32("k_v_jacr_f", k_v_jac_pair, false, true)
+            MESH32("k_v_resid_f", k_v_resid_pair)
         } else {
             ALAUNCH(l ? "k_v_jac0_c" : "k_v_jac0_f", k_v_jac0<T>, ctx->amg_smooth[l], l);
-            if (l == 0 && n16) {
-                ALAUNCH("k_v_jac_f", (k_v_jac_mesh<T, true>), ctx->amg_smooth[l], l);
-                ALAUNCH("k_v_resid_f", (k_v_resid_mesh<T, true>), ctx->amg_smooth[l], l);
-            } else if (l == 0) {
-                ALAUNCH("k_v_jac_f", (k_v_jac_mesh<T, false>), ctx->amg_smooth[l], l);
-                ALAUNCH("k_v_resid_f", (k_v_resid_mesh<T, false>), ctx->amg_smooth[l], l);
+            if (l == 0) {
+                ALAUNCH("k_v_jac_f", k_v_jac_mesh<false>, ctx->amg_smooth[l]);
+                ALAUNCH("k_v_resid_f", k_v_resid_mesh, ctx->amg_smooth[l]);
             } else {
                 ALAUNCH("k_v_jac_c", (k_v_jac<T>), ctx->amg_smooth[l], l);
                 ALAUNCH("k_v_resid_c", (k_v_resid<T>), ctx->amg_smooth[l], l);
@@ -1425,12 +1512,12 @@ template <class T> static void vcycle(cfdl_ctx *ctx) {
         } else {
             // z += s P z_{l+1}; t = J(z); z = J(t)
             ALAUNCH(l ? "k_v_lift_c" : "k_v_lift_f", k_v_lift<T>, ctx->amg_smooth[l], l);
-            if (l == 0 && n16) {
-                ALAUNCH("k_v_jac_f", (k_v_jac_mesh<T, true, true>), ctx->amg_smooth[l], l);
-                ALAUNCH("k_v_jac_f", (k_v_jac_mesh<T, true>), ctx->amg_smooth[l], l);
+            if (l == 0 && sizeof(T) == 4) {
+                MESH32("k_v_jac_f", k_v_jac_pair, true, false)
+                MESH32("k_v_jac_f", k_v_jac_pair, false, false)
             } else if (l == 0) {
-                ALAUNCH("k_v_jac_f", (k_v_jac_mesh<T, false, true>), ctx->amg_smooth[l], l);
-                ALAUNCH("k_v_jac_f", (k_v_jac_mesh<T, false>), ctx->amg_smooth[l], l);
+                ALAUNCH("k_v_jac_f", k_v_jac_mesh<true>, ctx->amg_smooth[l]);
+                ALAUNCH("k_v_jac_f", k_v_jac_mesh<false>, ctx->amg_smooth[l]);
             } else {
                 ALAUNCH("k_v_jac_c", (k_v_jac<T, true>), ctx->amg_smooth[l], l);
                 ALAUNCH("k_v_jac_c", (k_v_jac<T>), ctx->amg_smooth[l], l);
@@ -1603,7 +1690,26 @@ __global__ void __launch_bounds__(kTile) k_mx_q(const CaseDev *__restrict__ case
     SolveScalars *S = C.sc;
     const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     if (!S->active32) return;
-    float v[1] = {cg_aq_rows<float, k16>(level<float>(C, 0), C.fp, C.fq, t)};
+    // rows in pairs (pair_slots); then (p, q), each thread its rows 256 apart in
+    // row order, which is the order of the FP32 sums
+    __shared__ __align__(8) float qs[2 * kTile];
+    const LP<float> P = level<float>(C, 0);
+    const float *p = C.fp;
+    const int tid = (int)threadIdx.x;
+    float v[1] = {0.f};
+    for (int c0 = t.first; c0 < t.last; c0 += 2 * kTile) {
+        const int i = c0 + 2 * tid, i0 = c0 + tid, i1 = i0 + kTile;
+        if (i < t.last) {
+            const float2 y = pair_amul_mesh<k16>(P, p, i);
+            *(float2 *)&C.fq[i] = y;
+            *(float2 *)&qs[2 * tid] = y;
+        }
+        const float p0 = i0 < t.last ? p[i0] : 0.f, p1 = i1 < t.last ? p[i1] : 0.f;
+        __syncthreads();
+        if (i0 < t.last) v[0] += p0 * qs[tid];
+        if (i1 < t.last) v[0] += p1 * qs[tid + kTile];
+        __syncthreads();
+    }
     __shared__ float s[1];
     if (case_sums<1>(v, &C.counters[CNT_A3], partials, tile0, ntiles, s)) {
         if (threadIdx.x == 0) {

@@ -646,7 +646,7 @@ int cfdl_case_info(const cfdl_ctx *ctx, int id, int *ne, size_t *device_bytes) {
 }
 
 size_t cfdl_case_bytes_estimate(int ne, int nf, int nbf, int W) {
-    const size_t c = (size_t)ne, f = (size_t)nf, b = (size_t)nbf, nc = c + b, w = (size_t)W;
+    const size_t c = (size_t)ne + 1, f = (size_t)nf, b = (size_t)nbf, nc = c + b, w = (size_t)W;   // + 1: planes padded to an even length
     size_t bytes = 0;
     bytes += 2 * w * c * 4 + 3 * w * c * 8;          // ELL connectivity, gradient stencil
     bytes += 2 * f * 4 + 16 * f * 8;                 // face tables, geometry planes

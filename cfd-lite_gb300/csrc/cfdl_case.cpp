@@ -152,6 +152,7 @@ int upload_all(HostCase *hc, const cfdl_config *cfg, const FillVec<int> &hf_nb, 
     CaseDev &d = hc->dev;
     const int ne = hc->ne, nf = hc->nf, nbf = hc->nbf, W = hc->W, nc = ne + nbf;
     d.ne = ne; d.nbf = nbf; d.nf = nf; d.W = W;
+    d.ld32 = (ne + 1) & ~1;
     int st;
     if ((st = upload(hc, (int **)&d.hf_nb, hf_nb))) return st;
     if ((st = upload(hc, (int **)&d.hf_fc, hf_fc))) return st;
@@ -176,9 +177,10 @@ int upload_all(HostCase *hc, const cfdl_config *cfg, const FillVec<int> &hf_nb, 
     if ((st = zeros(hc, &d.anb_p, (size_t)W * ne))) return st;
     if ((st = zeros(hc, &d.ap_p, (size_t)ne))) return st;
     if ((st = zeros(hc, &d.rap_p, (size_t)ne))) return st;
-    if ((st = zeros(hc, &d.fanb_p, (size_t)W * ne))) return st;
-    if ((st = zeros(hc, &d.fdiag_p, (size_t)ne))) return st;
-    if ((st = zeros(hc, &d.frap_p, (size_t)ne))) return st;
+    const size_t ld = d.ld32;            // even: the FP32 mesh-level kernels take rows in pairs
+    if ((st = zeros(hc, &d.fanb_p, W * ld))) return st;
+    if ((st = zeros(hc, &d.fdiag_p, ld))) return st;
+    if ((st = zeros(hc, &d.frap_p, ld))) return st;
     if ((st = zeros(hc, &d.fdiff, (size_t)nf))) return st;
     if ((st = zeros(hc, &d.fS, 3 * (size_t)nf))) return st;
     if ((st = zeros(hc, &d.hbc, 4 * (size_t)nbf))) return st;
@@ -186,7 +188,7 @@ int upload_all(HostCase *hc, const cfdl_config *cfg, const FillVec<int> &hf_nb, 
     double **kv[] = {&d.kr, &d.krh, &d.kp, &d.kph, &d.kv, &d.ks, &d.ksh, &d.kt};
     for (double **pp : kv) if ((st = zeros(hc, pp, 3 * (size_t)ne))) return st;
     float **fv[] = {&d.fr, &d.fz, &d.fp, &d.fq, &d.fx, &d.fdiag, &d.ft, &d.frap};
-    for (float **pp : fv) if ((st = zeros(hc, pp, (size_t)ne))) return st;
+    for (float **pp : fv) if ((st = zeros(hc, pp, ld))) return st;
     if ((st = zeros(hc, &d.fanb, (size_t)W * ne))) return st;
     if ((st = zeros(hc, &d.rap, (size_t)ne))) return st;
     if ((st = zeros(hc, &d.sc, 1))) return st;

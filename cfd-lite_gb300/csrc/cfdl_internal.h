@@ -112,6 +112,7 @@ struct SolveScalars : KLanes {
 
 struct CaseDev {
     int ne, nbf, nf, W;
+    int ld32;                             // ne rounded up to even: the stride of fanb_p's and nb16's planes
     // mesh
     const int *hf_nb, *hf_fc;
     const double *hf_G;
@@ -130,7 +131,7 @@ struct CaseDev {
     // ap/anb): it depends only on dc, so it and the multigrid set-up are built
     // beside the momentum solve; its 1/ap scaling and FP32 copies likewise
     double *ap_p, *anb_p, *rap_p;
-    float *fdiag_p, *fanb_p, *frap_p;
+    float *fdiag_p, *fanb_p, *frap_p;     // fanb_p [W][ld32]; the FP32 vectors have ld32 elements
     // face intermediates of the assemblies
     double *fdiff, *fS;                   // [nf] pressure face coefficient, [3][nf] explicit momentum face terms
     double *hbc;                          // [4][nbf] per halo: the wall diffusion added to ap and anb, and the
@@ -154,7 +155,7 @@ struct CaseDev {
     int amg_tail;                         // first level the V-cycle's tail runs (k_v_tail)
     const struct TailPlan *tail64, *tail32;   // the tail's levels and shared-memory plan, FP64 and FP32
     const AmgLevelDev *lev;               // [nlev] device array
-    // [W][ne] the mesh level's interior neighbours as 16-bit offsets j - i
+    // [W][ld32] the mesh level's interior neighbours as 16-bit offsets j - i
     // (kNb16None: no interior neighbour) for the mixed pressure solve's FP32
     // mesh-level kernels; null when an offset does not fit, or in FP64
     const short *nb16;
