@@ -196,17 +196,16 @@ __device__ __forceinline__ void row_slots(const LP<T> &P, int i, int (&j)[W], T 
     }
 }
 
-// sum_j a_ij x_j over the row's couplings inside the level (the ELL values
+// s + sum_j a_ij x_j over the row's couplings inside the level (the ELL values
 // are the off-diagonal magnitudes: A = D - offdiag)
 template <int W, class T, bool kGuard = false, bool kEager = true>
-__device__ __forceinline__ T offsum_w(const LP<T> &P, const T *x, int i) {
+__device__ __forceinline__ T offsum_w(const LP<T> &P, const T *x, int i, T s = 0) {
     int j[W];
     T c[W];
     row_slots<W, T, kGuard, kEager>(P, i, j, c);
     T xj[W];
 #pragma unroll
     for (int k = 0; k < W; k++) xj[k] = x[j[k]];
-    T s = 0;
 #pragma unroll
     for (int k = 0; k < W; k++) s += c[k] * xj[k];
     return s;
@@ -214,24 +213,10 @@ __device__ __forceinline__ T offsum_w(const LP<T> &P, const T *x, int i) {
 
 // The FP64 mesh level (level 0): at most kMaxW slots a row, every width on the
 // short fixed-width paths (no wide-row code in the kernels that use these)
-__device__ __forceinline__ double offsum_mesh(const LP<double> &P, const double *x, int i) {
-    if (P.W == 6) return offsum_w<6, double, false>(P, x, i);
-    if (P.W == 4) return offsum_w<4, double, false>(P, x, i);
-    return offsum_w<kMaxW, double, true>(P, x, i);
-}
-template <int W, bool kGuard = false> __device__ __forceinline__ double amul_w(const LP<double> &P, const double *x, int i) {
-    int j[W];
-    double c[W];
-    row_slots<W, double, kGuard>(P, i, j, c);
-    double s = P.dg[i] * x[i];
-#pragma unroll
-    for (int k = 0; k < W; k++) s -= c[k] * x[j[k]];
-    return s;
-}
-__device__ __forceinline__ double amul_mesh(const LP<double> &P, const double *x, int i) {
-    if (P.W == 6) return amul_w<6>(P, x, i);
-    if (P.W == 4) return amul_w<4>(P, x, i);
-    return amul_w<kMaxW, true>(P, x, i);
+__device__ __forceinline__ double offsum_mesh(const LP<double> &P, const double *x, int i, double s) {
+    if (P.W == 6) return offsum_w<6, double, false>(P, x, i, s);
+    if (P.W == 4) return offsum_w<4, double, false>(P, x, i, s);
+    return offsum_w<kMaxW, double, true>(P, x, i, s);
 }
 
 // The FP32 mesh level takes its rows two at a time, i (even) and i + 1, with
@@ -385,6 +370,7 @@ __global__ void __launch_bounds__(kTile) k_amg_prep0(const CaseDev *__restrict__
     for (int k = 0; k < kMaxW; k++) a[k] = mixed && k < C.W ? C.anb_p[k * C.ne + i] : 0.0;
     const double rd = kOmega / ap;
     C.rap_p[i] = rd;
+    if (!mixed) C.rap2_p[i] = rd * (kOmega2 / kOmega);
     if (mixed) {
         // the FP32 copies converted in the integer pipe (GB300 runs the hardware
         // conversions at its FP64 rate)
@@ -495,12 +481,12 @@ __global__ void __launch_bounds__(kTile) k_v_jac(const CaseDev *__restrict__ cas
     // the row's own values first: measured faster on the coarse levels
     y[i] = jacobi_step<T, kToT ? 1 : 2>(x[i], P.r[i], P.rd[i], offsum<T>(P, x, i));
 }
-// The FP64 mesh-level sweeps (one row per thread, two dependent trips to
-// memory a row) are kernels of their own, so that their register cap, and with
-// it the resident warps and the loads in flight, is set apart from the coarse
-// levels' sweeps: 32 registers, 8 CTAs per SM (one 8-byte spill slot),
-// measured 2-4% faster at 128^3 than the 40 registers and 6 CTAs the compiler
-// picks unbounded; the coarse sweeps would spill 100+ bytes under the same cap.
+// The FP64 mesh-level sweeps are bound by their FP64 instructions: 4.5 us each
+// per 2.1M rows, whatever the launch shape or the index width.  Eight per row
+// of six slots: the sum starts from r, and the second sweep's w2/D is a plane
+// of its own (rap2_p) instead of w/D times w2/w (ten, MEASURED_SWEEP).
+// 32 registers, 8 CTAs per SM: the coarse levels' sweeps would spill 100+
+// bytes under that cap, so these are kernels of their own.
 template <bool kToT>
 __global__ void __launch_bounds__(kTile, 8) k_v_jac_mesh(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles) {
     CFDL_PDL_WAIT();
@@ -510,10 +496,11 @@ __global__ void __launch_bounds__(kTile, 8) k_v_jac_mesh(const CaseDev *__restri
     const int i = tl.first + (int)threadIdx.x;
     if (i >= tl.last) return;
     const LP<double> P = level<double>(C, 0);
-    const double *x = kToT ? P.z : P.t;
+    const double *x = kToT ? P.z : P.t, *rd = kToT ? P.rd : C.rap2_p;
     double *y = kToT ? P.t : P.z;
-    const double off = offsum_mesh(P, x, i);
-    y[i] = jacobi_step<double, kToT ? 1 : 2>(x[i], P.r[i], P.rd[i], off);
+    constexpr double om = kToT ? 1.0 - kOmega : 1.0 - kOmega2;
+    const double s = offsum_mesh(P, x, i, P.r[i]);
+    y[i] = om * x[i] + rd[i] * s;
 }
 // The FP32 mesh-level sweeps, two rows per thread (pair_slots).  kFromR: the
 // first pre-smoothing sweep, from t = w D^-1 r formed on the fly for the rows
@@ -577,7 +564,7 @@ __global__ void __launch_bounds__(kTile, 8) k_v_resid_mesh(const CaseDev *__rest
     const int i = tl.first + (int)threadIdx.x;
     if (i >= tl.last) return;
     const LP<double> P = level<double>(C, 0);
-    P.t[i] = P.r[i] - amul_mesh(P, P.z, i);
+    P.t[i] = offsum_mesh(P, P.z, i, P.r[i] - P.dg[i] * P.z[i]);
 }
 template <bool k16>
 __global__ void __launch_bounds__(kTile / 2, 16) k_v_resid_pair(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles) {

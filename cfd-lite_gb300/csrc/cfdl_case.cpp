@@ -177,6 +177,7 @@ int upload_all(HostCase *hc, const cfdl_config *cfg, const FillVec<int> &hf_nb, 
     if ((st = zeros(hc, &d.anb_p, (size_t)W * ne))) return st;
     if ((st = zeros(hc, &d.ap_p, (size_t)ne))) return st;
     if ((st = zeros(hc, &d.rap_p, (size_t)ne))) return st;
+    if ((st = zeros(hc, &d.rap2_p, (size_t)ne))) return st;
     const size_t ld = d.ld32;            // even: the FP32 mesh-level kernels take rows in pairs
     if ((st = zeros(hc, &d.fanb_p, W * ld))) return st;
     if ((st = zeros(hc, &d.fdiag_p, ld))) return st;

@@ -130,7 +130,7 @@ struct CaseDev {
     // the pressure-correction matrix in its own storage (the reference shares
     // ap/anb): it depends only on dc, so it and the multigrid set-up are built
     // beside the momentum solve; its 1/ap scaling and FP32 copies likewise
-    double *ap_p, *anb_p, *rap_p;
+    double *ap_p, *anb_p, *rap_p, *rap2_p;   // rap_p, rap2_p: first and second sweep weight / ap (rap2_p: FP64 form)
     float *fdiag_p, *fanb_p, *frap_p;     // fanb_p [W][ld32]; the FP32 vectors have ld32 elements
     // face intermediates of the assemblies
     double *fdiff, *fS;                   // [nf] pressure face coefficient, [3][nf] explicit momentum face terms
