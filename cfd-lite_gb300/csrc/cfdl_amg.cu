@@ -484,9 +484,13 @@ __global__ void __launch_bounds__(kTile) k_v_jac(const CaseDev *__restrict__ cas
 // The FP64 mesh-level sweeps are bound by their FP64 instructions: 4.5 us each
 // per 2.1M rows, whatever the launch shape or the index width.  Eight per row
 // of six slots: the sum starts from r, and the second sweep's w2/D is a plane
-// of its own (rap2_p) instead of w/D times w2/w (ten, MEASURED_SWEEP).
+// of its own (rap2_p) instead of w/D times w2/w (ten: 45.7 us at 128^3; eight: 43.1).
 // 32 registers, 8 CTAs per SM: the coarse levels' sweeps would spill 100+
 // bytes under that cap, so these are kernels of their own.
+// The roundings of both launch shapes, spelled out: a case has the same result
+// alone and in a batch, whichever shape its launch takes.
+__device__ __forceinline__ double sweep64(double om, double x, double w, double s) { return __fma_rn(w, s, __dmul_rn(om, x)); }
+__device__ __forceinline__ double resid64(double r, double d, double z) { return __fma_rn(-d, z, r); }
 template <bool kToT>
 __global__ void __launch_bounds__(kTile, 8) k_v_jac_mesh(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles) {
     CFDL_PDL_WAIT();
@@ -499,8 +503,61 @@ __global__ void __launch_bounds__(kTile, 8) k_v_jac_mesh(const CaseDev *__restri
     const double *x = kToT ? P.z : P.t, *rd = kToT ? P.rd : C.rap2_p;
     double *y = kToT ? P.t : P.z;
     constexpr double om = kToT ? 1.0 - kOmega : 1.0 - kOmega2;
-    const double s = offsum_mesh(P, x, i, P.r[i]);
-    y[i] = om * x[i] + rd[i] * s;
+    y[i] = sweep64(om, x[i], rd[i], offsum_mesh(P, x, i, P.r[i]));
+}
+// The same two rows per thread, i (even) and i + 1, with 8-byte index and
+// 16-byte coefficient and vector loads where the case's row count is even (an
+// odd one's planes are not aligned to pairs: its rows go one after the other).
+// Used where the mesh fills the SMs more than once: 43.1 -> 40 us at 128^3; on
+// small meshes the longer thread is the latency (32^3: an outer iteration 3%
+// slower).
+template <int W, bool kGuard>
+__device__ __forceinline__ double2 pair_sum64(const LP<double> &P, const double *x, int i, double2 s) {
+    const int n = P.n;
+    int j[2][W];
+    double c[2][W], v[2][W];
+#pragma unroll
+    for (int k = 0; k < W; k++) {
+        const bool in = !kGuard || k < P.W;
+        int2 d = make_int2(-1, -1);
+        double2 a = make_double2(0.0, 0.0);
+        if (in) { d = *(const int2 *)&P.nb[k * n + i]; a = *(const double2 *)&P.a[k * n + i]; }
+        const bool ok0 = (unsigned)d.x < (unsigned)n, ok1 = (unsigned)d.y < (unsigned)n;
+        j[0][k] = ok0 ? d.x : i; j[1][k] = ok1 ? d.y : i + 1;
+        c[0][k] = ok0 ? a.x : 0.0; c[1][k] = ok1 ? a.y : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < W; k++) { v[0][k] = x[j[0][k]]; v[1][k] = x[j[1][k]]; }
+#pragma unroll
+    for (int k = 0; k < W; k++) { s.x = __fma_rn(c[0][k], v[0][k], s.x); s.y = __fma_rn(c[1][k], v[1][k], s.y); }
+    return s;
+}
+// s + the off-diagonal sums of rows i and i + 1 (both inside the level)
+__device__ __forceinline__ double2 pair_sum64_mesh(const LP<double> &P, const double *x, int i, double2 s) {
+    if (P.n & 1) return make_double2(offsum_mesh(P, x, i, s.x), offsum_mesh(P, x, i + 1, s.y));
+    if (P.W == 6) return pair_sum64<6, false>(P, x, i, s);
+    if (P.W == 4) return pair_sum64<4, false>(P, x, i, s);
+    return pair_sum64<kMaxW, true>(P, x, i, s);
+}
+template <bool kToT>
+__global__ void __launch_bounds__(kTile / 2, 16) k_v_jac_pair64(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles) {
+    CFDL_PDL_WAIT();
+    const Tile tl = tiles[blockIdx.x];
+    const CaseDev &C = cases[tl.c];
+    if (!pactive(C)) return;
+    const int i = tl.first + 2 * (int)threadIdx.x;
+    if (i >= tl.last) return;
+    const LP<double> P = level<double>(C, 0);
+    const double *x = kToT ? P.z : P.t, *rd = kToT ? P.rd : C.rap2_p;
+    double *y = kToT ? P.t : P.z;
+    constexpr double om = kToT ? 1.0 - kOmega : 1.0 - kOmega2;
+    if (i + 1 < P.n) {
+        const double2 s = pair_sum64_mesh(P, x, i, *(const double2 *)&P.r[i]);
+        const double2 xi = *(const double2 *)&x[i], w = *(const double2 *)&rd[i];
+        *(double2 *)&y[i] = make_double2(sweep64(om, xi.x, w.x, s.x), sweep64(om, xi.y, w.y, s.y));
+    } else {
+        y[i] = sweep64(om, x[i], rd[i], offsum_mesh(P, x, i, P.r[i]));
+    }
 }
 // The FP32 mesh-level sweeps, two rows per thread (pair_slots).  kFromR: the
 // first pre-smoothing sweep, from t = w D^-1 r formed on the fly for the rows
@@ -564,7 +621,22 @@ __global__ void __launch_bounds__(kTile, 8) k_v_resid_mesh(const CaseDev *__rest
     const int i = tl.first + (int)threadIdx.x;
     if (i >= tl.last) return;
     const LP<double> P = level<double>(C, 0);
-    P.t[i] = offsum_mesh(P, P.z, i, P.r[i] - P.dg[i] * P.z[i]);
+    P.t[i] = offsum_mesh(P, P.z, i, resid64(P.r[i], P.dg[i], P.z[i]));
+}
+__global__ void __launch_bounds__(kTile / 2, 16) k_v_resid_pair64(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles) {
+    CFDL_PDL_WAIT();
+    const Tile tl = tiles[blockIdx.x];
+    const CaseDev &C = cases[tl.c];
+    if (!pactive(C)) return;
+    const int i = tl.first + 2 * (int)threadIdx.x;
+    if (i >= tl.last) return;
+    const LP<double> P = level<double>(C, 0);
+    if (i + 1 < P.n) {
+        const double2 r = *(const double2 *)&P.r[i], d = *(const double2 *)&P.dg[i], z = *(const double2 *)&P.z[i];
+        *(double2 *)&P.t[i] = pair_sum64_mesh(P, P.z, i, make_double2(resid64(r.x, d.x, z.x), resid64(r.y, d.y, z.y)));
+    } else {
+        P.t[i] = offsum_mesh(P, P.z, i, resid64(P.r[i], P.dg[i], P.z[i]));
+    }
 }
 template <bool k16>
 __global__ void __launch_bounds__(kTile / 2, 16) k_v_resid_pair(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles) {
@@ -1453,6 +1525,13 @@ static void amg_setup_operators(cfdl_ctx *ctx) {
     if (n16) ALAUNCH_N(NAME, (K<true, ##__VA_ARGS__>), ctx->amg_smooth[0], kTile / 2);                    \
     else ALAUNCH_N(NAME, (K<false, ##__VA_ARGS__>), ctx->amg_smooth[0], kTile / 2);
 
+// An FP64 mesh-level kernel: two rows per thread where one row per thread would
+// fill the SMs (8 CTAs of kTile threads each) more than once.  Each row's
+// arithmetic is the same either way.
+#define MESH64(NAME, K1, K2)                                                                              \
+    if (ctx->amg_smooth[0].ntiles > 8 * 152) ALAUNCH_N(NAME, K2, ctx->amg_smooth[0], kTile / 2);          \
+    else ALAUNCH(NAME, K1, ctx->amg_smooth[0]);
+
 template <class T> static void vcycle(cfdl_ctx *ctx) {
     // Large levels run one thread per row (G = 1) or a few lanes per row
     // (the autotuned cgroup); small levels run 8 lanes per row, which
@@ -1478,8 +1557,8 @@ template <class T> static void vcycle(cfdl_ctx *ctx) {
         } else {
             ALAUNCH(l ? "k_v_jac0_c" : "k_v_jac0_f", k_v_jac0<T>, ctx->amg_smooth[l], l);
             if (l == 0) {
-                ALAUNCH("k_v_jac_f", k_v_jac_mesh<false>, ctx->amg_smooth[l]);
-                ALAUNCH("k_v_resid_f", k_v_resid_mesh, ctx->amg_smooth[l]);
+                MESH64("k_v_jac_f", k_v_jac_mesh<false>, k_v_jac_pair64<false>)
+                MESH64("k_v_resid_f", k_v_resid_mesh, k_v_resid_pair64)
             } else {
                 ALAUNCH("k_v_jac_c", (k_v_jac<T>), ctx->amg_smooth[l], l);
                 ALAUNCH("k_v_resid_c", (k_v_resid<T>), ctx->amg_smooth[l], l);
@@ -1503,8 +1582,8 @@ template <class T> static void vcycle(cfdl_ctx *ctx) {
                 MESH32("k_v_jac_f", k_v_jac_pair, true, false)
                 MESH32("k_v_jac_f", k_v_jac_pair, false, false)
             } else if (l == 0) {
-                ALAUNCH("k_v_jac_f", k_v_jac_mesh<true>, ctx->amg_smooth[l]);
-                ALAUNCH("k_v_jac_f", k_v_jac_mesh<false>, ctx->amg_smooth[l]);
+                MESH64("k_v_jac_f", k_v_jac_mesh<true>, k_v_jac_pair64<true>)
+                MESH64("k_v_jac_f", k_v_jac_mesh<false>, k_v_jac_pair64<false>)
             } else {
                 ALAUNCH("k_v_jac_c", (k_v_jac<T, true>), ctx->amg_smooth[l], l);
                 ALAUNCH("k_v_jac_c", (k_v_jac<T>), ctx->amg_smooth[l], l);
