@@ -283,7 +283,7 @@ static int append_uvwp(Builder &b, cudaGraph_t G, cudaGraphNode_t *prev, Pre pre
     if ((st = b.segment(G, prev, [&] {
              launch_adjust_pc(ctx);
              launch_grad(ctx, 3);
-             launch_update_uvwp(ctx);
+             launch_update_uvwp(ctx, true);
              post();
          }, &k)))
         return st;

@@ -134,6 +134,7 @@ struct CaseDev {
     float *fdiag_p, *fanb_p, *frap_p;     // fanb_p [W][ld32]; the FP32 vectors have ld32 elements
     // face intermediates of the assemblies
     double *fdiff, *fS;                   // [nf] pressure face coefficient, [3][nf] explicit momentum face terms
+    double *fmip;                         // [nf] rho_face area/(dr.n) dc_ip: update_uvwp's flux factor, left by k_coef_p_face
     double *hbc;                          // [4][nbf] per halo: the wall diffusion added to ap and anb, and the
                                           // three momentum sources of the BC loop (k_coef_uvw_halo)
     double *fprop;                        // [PR_N][nf] property planes
@@ -323,7 +324,7 @@ void launch_coef_p(cfdl_ctx *ctx);             // matrix and right-hand side
 void launch_coef_p_matrix(cfdl_ctx *ctx);      // face coefficients, ap_p/anb_p (needs dc only)
 void launch_coef_p_rhs(cfdl_ctx *ctx);         // b (needs the fluxes of calc_mip)
 void launch_adjust_pc(cfdl_ctx *ctx);
-void launch_update_uvwp(cfdl_ctx *ctx);
+void launch_update_uvwp(cfdl_ctx *ctx, bool fresh);
 void launch_update_time(cfdl_ctx *ctx);
 void launch_set_mip0(cfdl_ctx *ctx);
 

@@ -58,6 +58,12 @@ __global__ void __launch_bounds__(kTile) k_bc(const CaseDev *__restrict__ cases,
 // the neighbour takes them with the opposite sign.  Boundary faces: the wall
 // diffusion mu*area/ds of the BC loop (mod_uvwp.f90:257).
 // ---------------------------------------------------------------------------
+// Bound by the FP64 pipe (4.5 us per instruction and 2.1M faces).  kFast
+// (precision 0): interpolation as go + wt (gn - go) and each component's six
+// products as one chain, 36 FP64 instructions a face instead of 40
+// (445 -> 392 us at 128^3); the mixed forms keep the other order, on
+// which their FP32 roundings depend.
+template <bool kFast>
 __global__ void __launch_bounds__(kTile) k_coef_uvw_face(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles) {
     CFDL_PDL_WAIT();
     TILE_PROLOGUE(faces)
@@ -65,7 +71,7 @@ __global__ void __launch_bounds__(kTile) k_coef_uvw_face(const CaseDev *__restri
     const int nf = C.nf, o = C.f_own[i], n = C.f_nb[i];
     if (n >= C.ne) return;                  // boundary faces: only their (precomputed) diffusion
     const double *g = C.fgeo, *pr = C.fprop;
-    const double wt = g[FG_WT * nf + i], omw = 1.0 - wt;
+    const double wt = g[FG_WT * nf + i];
     const double A0 = pr[PR_MAX * nf + i], A1 = pr[PR_MAY * nf + i], A2 = pr[PR_MAZ * nf + i];
     const double E0 = pr[PR_MEX * nf + i], E1 = pr[PR_MEY * nf + i], E2 = pr[PR_MEZ * nf + i];
     double gi[3][3];   // gi[q][m]: component m of grad(u_q) at the face
@@ -73,15 +79,22 @@ __global__ void __launch_bounds__(kTile) k_coef_uvw_face(const CaseDev *__restri
 #pragma unroll
     for (int q = 0; q < 3; q++)
 #pragma unroll
-        for (int m = 0; m < 3; m++) gi[q][m] = omw * gq[q][3 * o + m] + wt * gq[q][3 * n + m];
+        for (int m = 0; m < 3; m++) {
+            const double go = gq[q][3 * o + m], gn = gq[q][3 * n + m];
+            if (kFast) gi[q][m] = go + wt * (gn - go);
+            else { const double omw = 1.0 - wt; gi[q][m] = omw * go + wt * gn; }
+        }
     // the two explicit face terms of component m, which the cell sums add to
     // the same right-hand side, stored as one value:
     //   sumss(m):   mu_ip (du/dx_m, dv/dx_m, dw/dx_m) . dr
     //   sumdefc(m): mu_ip grad(u_m) . (dr_p/ds_p - dr/ds)
     // (mu_ip is folded into the property planes)
 #pragma unroll
-    for (int m = 0; m < 3; m++)
-        C.fS[m * nf + i] = (gi[0][m] * A0 + gi[1][m] * A1 + gi[2][m] * A2) + (gi[m][0] * E0 + gi[m][1] * E1 + gi[m][2] * E2);
+    for (int m = 0; m < 3; m++) {
+        const double ss = gi[0][m] * A0 + gi[1][m] * A1 + gi[2][m] * A2;
+        if (kFast) C.fS[m * nf + i] = fma(gi[m][2], E2, fma(gi[m][1], E1, fma(gi[m][0], E0, ss)));
+        else C.fS[m * nf + i] = ss + (gi[m][0] * E0 + gi[m][1] * E1 + gi[m][2] * E2);
+    }
 }
 
 // Property planes of every face (recomputed when rho or mu change): the mesh
@@ -419,8 +432,14 @@ __global__ void k_check_conversions(int n, unsigned *bad) {
 
 // ---------------------------------------------------------------------------
 // calc_mip, mod_uvwp.f90:438-490.  One thread per face; boundary faces keep
-// the value their BC set.
+// the value their BC set.  Bound by the FP64 pipe.  kFast (precision 0): each
+// side's dot products first, then one interpolation, so a vector's three
+// components cost 8 FP64 instructions instead of 9 and 1 - wt is not formed:
+// 23 a face instead of 26 (262 -> 228 us at 128^3); the mixed forms
+// keep the order their FP32 roundings depend on.
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ double lerp64(double a, double b, double wt) { return a + wt * (b - a); }
+template <bool kFast>
 __global__ void __launch_bounds__(kTile) k_calc_mip(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles, int rc) {
     CFDL_PDL_WAIT();
     TILE_PROLOGUE(faces)
@@ -430,6 +449,23 @@ __global__ void __launch_bounds__(kTile) k_calc_mip(const CaseDev *__restrict__ 
     const double *g = C.fgeo;
     const double wt = g[FG_WT * nf + i], omw = 1.0 - wt;
     const double A0 = g[FG_AX * nf + i], A1 = g[FG_AY * nf + i], A2 = g[FG_AZ * nf + i];
+    if (kFast) {
+        const double rho = C.fprop[PR_RHO * nf + i];
+        double m = lerp64(C.u[o] * A0 + C.v[o] * A1 + C.w[o] * A2, C.u[n] * A0 + C.v[n] * A1 + C.w[n] * A2, wt) * rho;
+        if (rc) {
+            const double D0 = g[FG_DRX * nf + i], D1 = g[FG_DRY * nf + i], D2 = g[FG_DRZ * nf + i];
+            const double *go = C.gp + 3 * (size_t)o, *gn = C.gp + 3 * (size_t)n;
+            const double gd = lerp64(go[0] * D0 + go[1] * D1 + go[2] * D2, gn[0] * D0 + gn[1] * D1 + gn[2] * D2, wt);
+            const double dip = lerp64(C.d[o], C.d[n], wt);
+            m = m - dip * C.fprop[PR_RHOADN * nf + i] * ((C.p[n] - C.p[o]) - gd);
+            if (!C.steady) {   // the transient term carries 1/dt and vanishes when steady
+                const double ua = lerp64(C.u0[o] * A0 + C.v0[o] * A1 + C.w0[o] * A2, C.u0[n] * A0 + C.v0[n] * A1 + C.w0[n] * A2, wt);
+                m = m - rho * dip * C.rdt * (C.mip0[i] - ua * rho);
+            }
+        }
+        C.mip[i] = m;
+        return;
+    }
     const double vx = omw * C.u[o] + wt * C.u[n], vy = omw * C.v[o] + wt * C.v[n], vz = omw * C.w[o] + wt * C.w[n];
     const double rhoip = C.fprop[PR_RHO * nf + i];
     double mip = (vx * A0 + vy * A1 + vz * A2) * rhoip;
@@ -499,7 +535,9 @@ __global__ void __launch_bounds__(kTile) k_coef_p_face(const CaseDev *__restrict
     const int nf = C.nf, o = C.f_own[i], n = C.f_nb[i];
     if (n >= C.ne) { C.fdiff[i] = 0.0; return; }
     const double wt = C.fgeo[FG_WT * nf + i], omw = 1.0 - wt;
-    C.fdiff[i] = (omw * C.dc[o] + wt * C.dc[n]) * C.fprop[PR_RHOADN * nf + i];
+    const double dip = omw * C.dc[o] + wt * C.dc[n];
+    C.fdiff[i] = dip * C.fprop[PR_RHOADN * nf + i];
+    C.fmip[i] = C.fprop[PR_RHOMADN * nf + i] * dip;
 }
 
 // the matrix: anb = the face coefficient on interior slots (0 on walls,
@@ -632,6 +670,19 @@ __global__ void __launch_bounds__(kTile) k_update_faces(const CaseDev *__restric
     C.mip[i] = C.mip[i] - C.fprop[PR_RHOMADN * nf + i] * dip * (C.phic[n] - C.phic[o]);
 }
 
+// the same from the face factors k_coef_p_face left (solve_uvwp, where dc has
+// not changed since): two FP64 instructions a face instead of six and no
+// weight, plane or dc to read (76 -> 59 us at 128^3; the factor's
+// product and store take k_coef_p_face from 66 to 81 beside the momentum solve)
+__global__ void __launch_bounds__(kTile) k_update_faces_fresh(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles) {
+    CFDL_PDL_WAIT();
+    TILE_PROLOGUE(faces)
+    if (i >= t.last) return;
+    const int o = C.f_own[i], n = C.f_nb[i];
+    if (n >= C.ne) return;
+    C.mip[i] = C.mip[i] - C.fmip[i] * (C.phic[n] - C.phic[o]);
+}
+
 // update_time, mod_physics.f90:101-112
 __global__ void __launch_bounds__(kTile) k_update_time(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles) {
     CFDL_PDL_WAIT();
@@ -662,6 +713,7 @@ void ensure_face_props(cfdl_ctx *ctx) {
     CFDL_LAUNCH("k_face_props", k_face_props, faces);
     for (HostCase *hc : ctx->cases) hc->props_dirty = false;
 }
+static bool fp64_only(const cfdl_ctx *ctx) { return ctx->cases[0]->cfg.precision == 0; }
 static bool f32_assembly(const cfdl_ctx *ctx) { return ctx->cases[0]->cfg.precision == 3; }
 
 void ensure_g32(cfdl_ctx *ctx) {
@@ -682,7 +734,8 @@ void launch_coef_uvw(cfdl_ctx *ctx) {
         return;
     }
     CFDL_LAUNCH("k_coef_uvw_halo", k_coef_uvw_halo, halos);
-    CFDL_LAUNCH("k_coef_uvw_face", k_coef_uvw_face, faces);
+    if (fp64_only(ctx)) CFDL_LAUNCH("k_coef_uvw_face", k_coef_uvw_face<true>, faces);
+    else CFDL_LAUNCH("k_coef_uvw_face", k_coef_uvw_face<false>, faces);
     CFDL_LAUNCH("k_coef_uvw_cell", k_coef_uvw_cell<false>, cells);
 }
 void launch_grad(cfdl_ctx *ctx, int field) {
@@ -698,7 +751,8 @@ void launch_calc_mip(cfdl_ctx *ctx, int rc) {
         CFDL_LAUNCH("k_calc_mip", k_calc_mip_f32, faces, rc);
         return;
     }
-    CFDL_LAUNCH("k_calc_mip", k_calc_mip, faces, rc);
+    if (fp64_only(ctx)) CFDL_LAUNCH("k_calc_mip", k_calc_mip<true>, faces, rc);
+    else CFDL_LAUNCH("k_calc_mip", k_calc_mip<false>, faces, rc);
 }
 void launch_coef_p_matrix(cfdl_ctx *ctx) {
     ensure_face_props(ctx);
@@ -723,10 +777,12 @@ void launch_adjust_pc(cfdl_ctx *ctx) {
     ctx->launches++;
     CFDL_LAUNCH("k_adjust_pc", k_adjust_pc, cells);
 }
-void launch_update_uvwp(cfdl_ctx *ctx) {
+// fresh: calc_coef_p's face factors are of the present dc (solve_uvwp)
+void launch_update_uvwp(cfdl_ctx *ctx, bool fresh) {
     ensure_face_props(ctx);
     CFDL_LAUNCH("k_update_cells", k_update_cells, cells);
-    CFDL_LAUNCH("k_update_faces", k_update_faces, faces);
+    if (fresh) CFDL_LAUNCH("k_update_faces", k_update_faces_fresh, faces);
+    else CFDL_LAUNCH("k_update_faces", k_update_faces, faces);
 }
 void launch_update_time(cfdl_ctx *ctx) {
     CFDL_LAUNCH("k_update_time", k_update_time, cells);
