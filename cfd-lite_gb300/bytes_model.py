@@ -21,6 +21,8 @@ def kernel_bytes(name, ne, nf, nbf, W, ncomp_active=3):
         "k_coef_uvw_face": nfi * (8 + 56 + 24) + ne * 72,
         # momentum cell gather: ELL nb/fc, 5 face doubles, 13 cell doubles in, 6 out, anb ELL out
         "k_coef_uvw_cell": 2 * ell_i + nf * 40 + ne * (104 + 48) + ell_d + nbf * (24 + 4 + 32),
+        # the same with the start of the momentum solve (solve_uvwp): also r and rh of three components and 1/ap out
+        "k_coef_uvw_init": 2 * ell_i + nf * 40 + ne * (104 + 48 + 56) + ell_d + nbf * (24 + 4 + 32),
         "k_grad3": ell_i + 3 * ell_d + 24 * (ne + nbf) + 72 * ne,
         # precision 3: FP32 stencil, FP32 gradients out and the widened FP64 copies
         "k_grad3_f32": ell_i + 3 * 4 * W * ne + 24 * (ne + nbf) + 108 * ne,

@@ -147,10 +147,10 @@ int solve_uvwp_all(cfdl_ctx *ctx) {
     if (ctx->use_graph && !prof_active(ctx)) return solve_uvwp_graph(ctx);
     int st;
     if (ctx->cases[0]->cfg.precond == 1 && (st = ensure_amg(ctx))) return st;
-    launch_coef_uvw(ctx);
+    launch_coef_uvw_init(ctx);
     launch_coef_p_matrix(ctx);
     pressure_operators(ctx);
-    if ((st = solve_momentum(ctx))) return st;
+    if ((st = solve_momentum_started(ctx))) return st;
     launch_grad(ctx, 4);
     if (ctx->ev_mom) cudaEventRecord(ctx->ev_mom, ctx->stream);
     launch_calc_mip(ctx, 1);
@@ -263,6 +263,7 @@ int cfdl_ctx_destroy(cfdl_ctx *ctx) {
     for (WorkList *wl : wls) free_worklist(*wl);
     free_worklist(ctx->cellsv);
     free_worklist(ctx->cellse);
+    free_worklist(ctx->cellsr);
     free_worklist(ctx->facesv);
     for (auto &wl : ctx->amg_cells) free_worklist(wl);
     for (auto &wl : ctx->amg_smooth) free_worklist(wl);

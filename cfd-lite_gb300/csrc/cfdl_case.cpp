@@ -62,11 +62,24 @@ void free_worklist(WorkList &wl) {
 
 // Tile list over per-case entity counts (sizes[c] = 0 leaves case c out).
 int build_worklist(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &sizes, int tile) {
+    return build_worklist(ctx, wl, sizes, std::vector<int>(sizes.size(), tile));
+}
+
+// Rows per thread of an FP64 pass with a reduction: one while the case's tiles
+// then fit the chip at once (152 SMs, four CTAs each), as a small case is bound
+// by its chain of latencies and by the SMs it leaves idle; four on large ones,
+// where the block's reduction is paid once for them.  It goes by the case alone,
+// so a case's sums are the same alone and in a batch.
+static int rows_per_thread(int ne) { return ne <= 152 * 4 * kTile ? 1 : ne <= 2 * 152 * 4 * kTile ? 2 : 4; }
+
+// tiles: entities per tile of each case
+int build_worklist(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &sizes, const std::vector<int> &tiles) {
     free_worklist(wl);
     wl.h_tiles.clear(); wl.case_first.clear(); wl.case_ntiles.clear();
     for (size_t c = 0; c < sizes.size(); c++) {
         wl.case_first.push_back((int)wl.h_tiles.size());
         int cnt = 0;
+        const int tile = tiles[c];
         for (int s = 0; s < sizes[c]; s += tile, cnt++)
             wl.h_tiles.push_back({(int)c, s, std::min(sizes[c], s + tile), (tile + kTile - 1) / kTile});
         wl.case_ntiles.push_back(cnt);
@@ -97,6 +110,7 @@ void apply_config(HostCase *hc, const cfdl_config *cfg) {
     d.steady = std::isinf(cfg->dt) ? 1 : 0;
     d.rdt = d.steady ? 0.0 : 1.0 / cfg->dt;
     d.ralpha_u = 1.0 / cfg->alpha_u;
+    d.omalpha_u = 1.0 - cfg->alpha_u;
 }
 
 namespace {
@@ -447,6 +461,9 @@ int rebuild_worklists(cfdl_ctx *ctx) {
     if ((st = build_worklist(ctx, ctx->halos, nh))) return st;
     if ((st = build_worklist(ctx, ctx->cellsv, nc, kTile * ctx->vec))) return st;
     if ((st = build_worklist(ctx, ctx->cellse, nc, kTile * ctx->en_vec))) return st;
+    std::vector<int> tiles;
+    for (int ne : nc) tiles.push_back(kTile * rows_per_thread(ne));
+    if ((st = build_worklist(ctx, ctx->cellsr, nc, tiles))) return st;
     for (auto &wl : ctx->amg_cells) free_worklist(wl);
     for (auto &wl : ctx->amg_smooth) free_worklist(wl);
     for (auto &wl : ctx->amg_gcells) free_worklist(wl);

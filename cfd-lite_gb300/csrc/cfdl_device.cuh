@@ -133,6 +133,24 @@ __device__ __forceinline__ bool case_sums(T (&v)[K], int *counter, T *partials, 
     return true;
 }
 
+// Start of a case's momentum solve from s[0..2] = sum b'^2 and s[3..5] =
+// sum r^2 per component (the whole block calls it; one thread per component).
+constexpr int kCntMomInit = 0;           // its last-tile counter
+__device__ __forceinline__ void mom_start(const CaseDev &C, const double *s) {
+    const int q = threadIdx.x;
+    if (q >= 3) return;
+    SolveScalars *S = C.sc;
+    const int cap = C.solve_mode == 0 ? C.nit : C.tight_maxit;
+    S->bnorm[q] = sqrt(s[q]);
+    S->r0norm[q] = S->rnorm[q] = sqrt(s[3 + q]);
+    S->rho[q] = s[3 + q];
+    S->alpha[q] = 1.0; S->omega[q] = 1.0; S->beta[q] = 0.0; S->half[q] = 0;
+    S->iters[q] = 0; S->status[q] = 0;
+    S->tol[q] = C.solve_mode == 0 ? C.rtol_u * S->r0norm[q] : C.tight_rtol * S->bnorm[q];
+    S->active[q] = (S->r0norm[q] > S->tol[q]) && cap > 0;
+    if (!isfinite(S->r0norm[q]) || !isfinite(S->bnorm[q])) { S->active[q] = 0; S->status[q] = CFDL_ERR_NONFINITE; }
+}
+
 __device__ __forceinline__ int face_of(int fc) { return fc >= 0 ? fc : ~fc; }
 
 // Row i of an ELL operator, y_c = diag*x_c[i] - sum_k a[k][i]*x_c[nb[k][i]]

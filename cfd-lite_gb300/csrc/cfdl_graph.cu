@@ -17,7 +17,6 @@
 
 namespace cfdl {
 
-void mom_init(cfdl_ctx *ctx);
 void mom_iter(cfdl_ctx *ctx);
 void mom_finish(cfdl_ctx *ctx);
 void pcj_init(cfdl_ctx *ctx);
@@ -194,8 +193,7 @@ static int append_uvwp(Builder &b, cudaGraph_t G, cudaGraphNode_t *prev, Pre pre
     // momentum assembly and BiCGStab
     if ((st = b.segment(G, prev, [&] {
              pre();
-             launch_coef_uvw(ctx);
-             mom_init(ctx);
+             launch_coef_uvw_init(ctx);
              b.setone(hm);
          }, &k)))
         return st;

@@ -105,6 +105,7 @@ struct SolveScalars : KLanes {
     float rz32, tol32, alpha32, beta32, rnorm32;
     int active32, iters32;
     double mass_imbalance;
+    double big[3];            // sum of the squares of momentum right-hand sides beyond 2^400 (k_coef_uvw_init)
     // outer-iteration runs (cfdl_run.cu): per-case targets and progress
     int run_left, outer_done, ncoef, halted, time_due, converged;
     double conv_tol, mip_abs, mass_ratio;
@@ -172,7 +173,7 @@ struct CaseDev {
     double *eprop;                        // [EP_N][nf] energy property planes
     // parameters
     double dt, alpha_u, alpha_p, rtol_u, rtol_p, tight_rtol;
-    double rdt, ralpha_u;                 // 1/dt (0 when steady), 1/alpha_u
+    double rdt, ralpha_u, omalpha_u;      // 1/dt (0 when steady), 1/alpha_u, 1 - alpha_u
     int nit, solve_mode, tight_maxit, precision, precond;
     int steady;                           // dt = INFINITY: the transient terms vanish
 };
@@ -227,6 +228,7 @@ struct cfdl_ctx {
     cfdl::WorkList cells, faces, halos;
     cfdl::WorkList cellsv;               // wide tiles (kTile*vec cells) for the solver kernels
     int vec = cfdl::kVec;                // cells per thread in those tiles (autotuned)
+    cfdl::WorkList cellsr;               // tiles of the FP64 passes whose shape goes by the case's size (rows_per_thread)
     cfdl::WorkList cellse;               // tiles of the energy solve (kTile*en_vec cells)
     cfdl::WorkList facesv;               // wide face tiles (kTile*kFaceVec faces) for face reductions
     int en_vec = 1;                      // cells per thread in those tiles (autotuned with the energy equation)
@@ -318,6 +320,7 @@ void ensure_face_props(cfdl_ctx *ctx);   // recompute the property planes of cas
 void ensure_g32(cfdl_ctx *ctx);          // precision 3: rebuild stale FP32 gradients from gu, gv, gw
 int ensure_f32_assembly(HostCase *hc, cudaStream_t stream);   // precision 3 arrays (allocated once)
 void launch_coef_uvw(cfdl_ctx *ctx);
+void launch_coef_uvw_init(cfdl_ctx *ctx);      // with the start of the momentum solve
 void launch_grad(cfdl_ctx *ctx, int field);     // 0 u, 1 v, 2 w, 3 phic, 4 = u,v,w fused, 5 = energy t, phi
 void launch_calc_mip(cfdl_ctx *ctx, int rhie_chow);
 void launch_coef_p(cfdl_ctx *ctx);             // matrix and right-hand side
@@ -390,6 +393,7 @@ inline void launch_k(bool pdl, void (*k)(KArgs...), unsigned grid, unsigned bloc
 
 // solvers (cfdl_solvers.cu)
 int solve_momentum(cfdl_ctx *ctx);
+int solve_momentum_started(cfdl_ctx *ctx);      // after launch_coef_uvw_init
 int solve_pressure(cfdl_ctx *ctx);              // operators (multigrid / FP32 copies) + solve
 int solve_pressure_prepared(cfdl_ctx *ctx);     // the solve, operators already built
 void pressure_operators(cfdl_ctx *ctx);         // what the pressure solve needs of its matrix
@@ -399,6 +403,7 @@ int solve_pressure_amg(cfdl_ctx *ctx);
 int solve_pressure_mixed(cfdl_ctx *ctx);
 void free_worklist(WorkList &wl);
 int build_worklist(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &sizes, int tile = kTile);
+int build_worklist(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &sizes, const std::vector<int> &tiles);
 int read_stats(cfdl_ctx *ctx, int c, cfdl_stats *st);
 int poll_kind(cfdl_ctx *ctx, int kind, int *maxit);
 int poll_chunk(int done, int expected);

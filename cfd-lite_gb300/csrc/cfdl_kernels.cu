@@ -277,6 +277,209 @@ __global__ void __launch_bounds__(kTile) k_coef_uvw_cell(const CaseDev *__restri
     C.dc[i] = vol / (ap - asum);            // SIMPLEC: vol / (ap - sum anb)
 }
 
+// calc_coef_uvw, cell part, and the start of the momentum solve in one pass
+// (solve_uvwp; the single routines keep k_coef_uvw_cell and k_mom_init): the
+// row's coefficients, diagonal and right-hand sides go from registers into
+// b' = b + sum_bdry anb*phi_halo and r = b' - A phi, instead of through
+// memory.  Bound by the FP64 pipe, so what it saves above all are FP64
+// instructions: rows without a boundary slot (the whole warp's) start their
+// sums from the first slot and skip the boundary terms, and sum b'^2 is formed
+// in tight mode only (otherwise it is only asked whether it is finite, see
+// kBigExp).  FORM 0 (precision 0) also forms vol/ap, vol/(ap - sum anb) and
+// 1/ap from one reciprocal and chains its sums: 85 FP64 instructions a row for
+// the 113 of the two kernels.  FORM 1 (precision 1 and 2) and 3 (FP32 explicit
+// face terms) keep every rounding of the two kernels, spelled out where the
+// compiler could contract either of two products.  At four CTAs per SM it
+// spills, and is still faster than at three or two without (128^3, an outer
+// iteration: FP64 4.635 ms against 4.643 and 4.679, precision 3 2.996 against
+// 3.015 and 3.031).  The two
+// kernels took 543 us FP64 and 483 in precision 3, this one 440 and 456.
+constexpr int kBigExp = 1023 + 400;     // |b'| below 2^400: no sum of squares of fewer than 2^31 rows overflows
+__device__ __forceinline__ bool is_big(double x) { return ((int)((unsigned long long)__double_as_longlong(x) >> 52) & 0x7ff) >= kBigExp; }
+
+template <int FORM, int W, bool INNER>
+__device__ __forceinline__ void coef_init_row(const CaseDev &C, int i, const int (&nb)[W], const int (&fc)[W], double (&v)[6]) {
+    const int ne = C.ne, nf = C.nf, nbf = C.nbf;
+    const bool m32 = FORM == 3 || (FORM == 1 && C.precision >= 2), tight = FORM != 3 && C.solve_mode != 0;
+    const float *fS32 = (const float *)C.fS;
+    double a[W], ap = 0.0, sumf = 0.0, ss[3] = {0.0, 0.0, 0.0}, bap = 0.0, bs[3] = {0.0, 0.0, 0.0};
+    float fs[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+    for (int k = 0; k < W; k++) {
+        a[k] = 0.0;
+        if (INNER ? k >= C.W : nb[k] < 0) continue;
+        if (!INNER && nb[k] >= ne) {
+            const int q = nb[k] - ne;
+            const double dbc = C.hbc[q];
+            a[k] = dbc;
+            bap += dbc;
+#pragma unroll
+            for (int m = 0; m < 3; m++) bs[m] += C.hbc[(m + 1) * nbf + q];
+            continue;
+        }
+        const int f = face_of(fc[k]);
+        const double fl = flip_sign(C.mip[f], fc[k] >= 0);   // inward flux
+        const double ak = C.fprop[PR_FDIFF * nf + f] + positive_part(fl);
+        a[k] = ak;
+        const bool first = INNER && k == 0, ng = fc[k] < 0;
+        sumf = first ? fl : sumf + fl;
+        ap = first ? ak : ap + ak;
+#pragma unroll
+        for (int m = 0; m < 3; m++) {
+            if (FORM == 3) fs[m] += flip_sign_f(fS32[m * nf + f], ng);
+            else { const double s = flip_sign(C.fS[m * nf + f], ng); ss[m] = first ? s : ss[m] + s; }
+        }
+    }
+    if (FORM == 3)
+#pragma unroll
+        for (int m = 0; m < 3; m++) ss[m] = widen_f64(fs[m]);
+    double asum = ap;
+    const double vol = C.vol[i], phi[3] = {C.u[i], C.v[i], C.w[i]};
+    double b[3], ap0 = 0.0, old[3] = {0.0, 0.0, 0.0};
+    if (!C.steady) {                        // ap0 = rho*vol/dt
+        ap0 = C.rho[i] * vol * C.rdt;
+        ap = ap + ap0;
+        old[0] = C.u0[i]; old[1] = C.v0[i]; old[2] = C.w0[i];
+    }
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+        const double g = C.gp[3 * i + q];
+        if (FORM == 0) {
+            b[q] = __fma_rn(-vol, g, __fma_rn(sumf, phi[q], ss[q]));
+            if (!C.steady) b[q] = __fma_rn(ap0, old[q], b[q]);
+        } else {
+            const double s = C.steady ? __fma_rn(sumf, phi[q], -__dmul_rn(vol, g))
+                                      : __fma_rn(-vol, g, __fma_rn(sumf, phi[q], __dmul_rn(ap0, old[q])));
+            b[q] = __dadd_rn(s, ss[q]);
+        }
+    }
+    if (!INNER) {                           // the boundary-condition loop's additions
+        ap = ap + bap;
+        asum = C.steady ? ap : asum + bap;
+#pragma unroll
+        for (int q = 0; q < 3; q++) b[q] = b[q] + bs[q];
+    }
+    if (C.alpha_u != 1.0) {
+        const double apr = __dmul_rn(ap, C.ralpha_u), f1 = __dmul_rn(C.omalpha_u, apr);
+#pragma unroll
+        for (int q = 0; q < 3; q++) b[q] = __fma_rn(f1, phi[q], b[q]);
+        ap = apr;
+    }
+    C.ap[i] = ap;
+    C.bu[i] = b[0]; C.bv[i] = b[1]; C.bw[i] = b[2];
+#pragma unroll
+    for (int k = 0; k < W; k++)
+        if (k < C.W) C.anb[k * ne + i] = a[k];
+    const double ec = __dsub_rn(ap, asum);  // SIMPLEC: vol / (ap - sum anb)
+    const double pr = FORM == 0 ? ap * ec : 0.0;
+    const int pe = (int)((unsigned long long)__double_as_longlong(pr) >> 52);   // sign and exponent
+    if (FORM == 0 && pe > 64 && pe < 1983) {
+        // one reciprocal for the three quotients (pr positive, its inverse and
+        // the products far from the ends of the range)
+        const double inv = 1.0 / pr, rap = inv * ec;
+        C.rap[i] = rap;
+        C.d[i] = vol * rap;
+        C.dc[i] = vol * (inv * ap);
+    } else {
+        const double dd = vol / ap;
+        C.d[i] = dd;
+        if (FORM == 3) C.d32[i] = narrow_f32(dd);
+        C.dc[i] = vol / ec;
+        if (m32) {
+            const float fa = narrow_f32(ap);
+            C.fdiag[i] = fa;
+            C.frap[i] = 1.0f / fa;
+#pragma unroll
+            for (int k = 0; k < W; k++)
+                if (k < C.W) C.fanb[k * ne + i] = narrow_f32(a[k]);
+        } else {
+            C.rap[i] = 1.0 / ap;            // the Jacobi scaling of the FP64 solve
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+        const double *__restrict__ x = q == 0 ? C.u : q == 1 ? C.v : C.w;
+        double pv[W];
+#pragma unroll
+        for (int k = 0; k < W; k++) pv[k] = x[nb[k] >= 0 ? nb[k] : i];
+        double bb = b[q], r;
+        if (FORM == 0) {
+            if (!INNER)
+#pragma unroll
+                for (int k = 0; k < W; k++)
+                    if (nb[k] >= ne) bb = __fma_rn(a[k], pv[k], bb);
+            r = __fma_rn(-ap, phi[q], bb);
+#pragma unroll
+            for (int k = 0; k < W; k++)
+                if (INNER || (nb[k] >= 0 && nb[k] < ne)) r = __fma_rn(a[k], pv[k], r);
+        } else {
+            double s = __dmul_rn(ap, phi[q]);
+#pragma unroll
+            for (int k = 0; k < W; k++) {
+                if (!INNER && nb[k] >= ne) bb = __fma_rn(a[k], pv[k], bb);
+                else if (INNER || nb[k] >= 0) s = __fma_rn(-a[k], pv[k], s);
+            }
+            r = __dsub_rn(bb, s);
+        }
+        if (m32) {
+            // FP32 correction solve A d = r from d = 0 (first halves of kr, krh; d after kt's)
+            const float rf = narrow_f32(r);
+            ((float *)C.kr)[q * ne + i] = rf;
+            ((float *)C.krh)[q * ne + i] = rf;
+            ((float *)C.kt)[3 * (size_t)ne + q * ne + i] = 0.f;
+        } else {
+            C.kr[q * ne + i] = r;
+            C.krh[q * ne + i] = r;
+        }
+        v[3 + q] += r * r;
+        if (tight) v[q] += bb * bb;
+        else if (is_big(bb)) atomicAdd(&C.sc->big[q], bb * bb);   // never, but for a solution beyond all bounds
+    }
+}
+
+template <int FORM, int W>
+__device__ __forceinline__ void coef_init_rows(const CaseDev &C, const Tile &t, double (&v)[6]) {
+    const int ne = C.ne;
+    FOR_CELLS(t) {
+        int nb[W], fc[W];
+        bool inner = true;
+#pragma unroll
+        for (int k = 0; k < W; k++) {
+            nb[k] = k < C.W ? C.hf_nb[k * ne + i] : -1;
+            fc[k] = k < C.W ? C.hf_fc[k * ne + i] : 0;
+            inner = inner && (k >= C.W || (nb[k] >= 0 && nb[k] < ne));
+        }
+        if (__all_sync(__activemask(), inner)) coef_init_row<FORM, W, true>(C, i, nb, fc, v);
+        else coef_init_row<FORM, W, false>(C, i, nb, fc, v);
+    }
+}
+
+template <int FORM>
+__global__ void __launch_bounds__(kTile, 4) k_coef_uvw_init(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles,
+                                                            const int *__restrict__ cfirst, const int *__restrict__ cnt,
+                                                            double *partials) {
+    CFDL_PDL_WAIT();
+    const Tile t = tiles[blockIdx.x];
+    const CaseDev &C = cases[t.c];
+    if (C.sc->halted) return;
+    const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
+    double v[6] = {0, 0, 0, 0, 0, 0};
+    if (C.W == 6) coef_init_rows<FORM, 6>(C, t, v);
+    else if (C.W == 4) coef_init_rows<FORM, 4>(C, t, v);
+    else coef_init_rows<FORM, kMaxW>(C, t, v);
+    __shared__ double s[6];
+    if (FORM == 3 || C.solve_mode == 0) {
+        double r[3] = {v[3], v[4], v[5]};
+        if (case_sums<3>(r, &C.counters[kCntMomInit], partials, tile0, ntiles, s + 3)) {
+            if (threadIdx.x < 3) {
+                s[threadIdx.x] = C.sc->big[threadIdx.x];
+                C.sc->big[threadIdx.x] = 0.0;
+            }
+            mom_start(C, s);                // a thread reads its own component's sums
+        }
+    } else if (case_sums<6>(v, &C.counters[kCntMomInit], partials, tile0, ntiles, s)) mom_start(C, s);
+}
+
 // ---------------------------------------------------------------------------
 // calc_grad, mod_solver.f90:40-81, as the stencil sum grad = sum_k G_k dphi_k.
 // NF fields at once (u,v,w or the energy equation's t and phi share the
@@ -723,20 +926,27 @@ void ensure_g32(cfdl_ctx *ctx) {
     CFDL_LAUNCH("k_narrow_grad", k_narrow_grad, cells);
     for (HostCase *hc : ctx->cases) hc->g32_stale = false;
 }
-void launch_coef_uvw(cfdl_ctx *ctx) {
+static void launch_coef_uvw_faces(cfdl_ctx *ctx) {
     ensure_face_props(ctx);
     for (HostCase *hc : ctx->cases) hc->coef_is_pressure = false;
-    if (f32_assembly(ctx)) {
-        ensure_g32(ctx);
-        CFDL_LAUNCH("k_coef_uvw_halo", k_coef_uvw_halo, halos);
-        CFDL_LAUNCH("k_coef_uvw_face_f32", k_coef_uvw_face_f32, faces);
-        CFDL_LAUNCH("k_coef_uvw_cell", k_coef_uvw_cell<true>, cells);
-        return;
-    }
+    if (f32_assembly(ctx)) ensure_g32(ctx);
     CFDL_LAUNCH("k_coef_uvw_halo", k_coef_uvw_halo, halos);
-    if (fp64_only(ctx)) CFDL_LAUNCH("k_coef_uvw_face", k_coef_uvw_face<true>, faces);
+    if (f32_assembly(ctx)) CFDL_LAUNCH("k_coef_uvw_face_f32", k_coef_uvw_face_f32, faces);
+    else if (fp64_only(ctx)) CFDL_LAUNCH("k_coef_uvw_face", k_coef_uvw_face<true>, faces);
     else CFDL_LAUNCH("k_coef_uvw_face", k_coef_uvw_face<false>, faces);
-    CFDL_LAUNCH("k_coef_uvw_cell", k_coef_uvw_cell<false>, cells);
+}
+void launch_coef_uvw(cfdl_ctx *ctx) {
+    launch_coef_uvw_faces(ctx);
+    if (f32_assembly(ctx)) CFDL_LAUNCH("k_coef_uvw_cell", k_coef_uvw_cell<true>, cells);
+    else CFDL_LAUNCH("k_coef_uvw_cell", k_coef_uvw_cell<false>, cells);
+}
+// calc_coef_uvw and the start of the momentum solve (solve_uvwp)
+void launch_coef_uvw_init(cfdl_ctx *ctx) {
+    launch_coef_uvw_faces(ctx);
+    const WorkList &wl = ctx->cellsr;
+    if (f32_assembly(ctx)) CFDL_LAUNCH("k_coef_uvw_init", k_coef_uvw_init<3>, cellsr, wl.d_case_first, wl.d_case_ntiles, ctx->d_partials);
+    else if (fp64_only(ctx)) CFDL_LAUNCH("k_coef_uvw_init", k_coef_uvw_init<0>, cellsr, wl.d_case_first, wl.d_case_ntiles, ctx->d_partials);
+    else CFDL_LAUNCH("k_coef_uvw_init", k_coef_uvw_init<1>, cellsv, ctx->cellsv.d_case_first, ctx->cellsv.d_case_ntiles, ctx->d_partials);
 }
 void launch_grad(cfdl_ctx *ctx, int field) {
     if (field == 4 && f32_assembly(ctx)) CFDL_LAUNCH("k_grad3_f32", k_grad3_f32, cells);

@@ -26,7 +26,7 @@
 namespace cfdl {
 namespace {
 
-enum { CNT_M1 = 0, CNT_M2, CNT_M3, CNT_M4, CNT_M5, CNT_P0, CNT_P1, CNT_P2, CNT_P3 };
+enum { CNT_M1 = kCntMomInit, CNT_M2, CNT_M3, CNT_M4, CNT_M5, CNT_P0, CNT_P1, CNT_P2, CNT_P3 };
 
 __device__ __forceinline__ double *comp_field(const CaseDev &C, int q) { return q == 0 ? C.u : q == 1 ? C.v : C.w; }
 __device__ __forceinline__ const double *comp_rhs(const CaseDev &C, int q) { return q == 0 ? C.bu : q == 1 ? C.bv : C.bw; }
@@ -121,20 +121,7 @@ __global__ void __launch_bounds__(kTile, 3) k_mom_init(const CaseDev *__restrict
     else if (C.W == 4) { FOR_CELLS(t) mom_init_row<4>(C, i, ne, v, m32); }
     else { FOR_CELLS(t) mom_init_row<kMaxW>(C, i, ne, v, m32); }
     __shared__ double s[6];
-    if (case_sums<6>(v, &C.counters[CNT_M1], partials, tile0, ntiles, s)) {
-        const int q = threadIdx.x;          // one thread per component
-        if (q < 3) {
-            const int cap = C.solve_mode == 0 ? C.nit : C.tight_maxit;
-            S->bnorm[q] = sqrt(s[q]);
-            S->r0norm[q] = S->rnorm[q] = sqrt(s[3 + q]);
-            S->rho[q] = s[3 + q];
-            S->alpha[q] = 1.0; S->omega[q] = 1.0; S->beta[q] = 0.0; S->half[q] = 0;
-            S->iters[q] = 0; S->status[q] = 0;
-            S->tol[q] = C.solve_mode == 0 ? C.rtol_u * S->r0norm[q] : C.tight_rtol * S->bnorm[q];
-            S->active[q] = (S->r0norm[q] > S->tol[q]) && cap > 0;
-            if (!isfinite(S->r0norm[q]) || !isfinite(S->bnorm[q])) { S->active[q] = 0; S->status[q] = CFDL_ERR_NONFINITE; }
-        }
-    }
+    if (case_sums<6>(v, &C.counters[CNT_M1], partials, tile0, ntiles, s)) mom_start(C, s);
 }
 
 // The BiCGStab vectors and operator of a case's solve, [NC][ne] per vector.
@@ -646,7 +633,7 @@ static int max_cap(cfdl_ctx *ctx) {
     return cap;
 }
 
-void mom_init(cfdl_ctx *ctx) { CFDL_LAUNCH("k_mom_init", k_mom_init, cellsv, RED); }
+static void mom_init(cfdl_ctx *ctx) { CFDL_LAUNCH("k_mom_init", k_mom_init, cellsv, RED); }
 
 #define RED32 ctx->cellsv.d_case_first, ctx->cellsv.d_case_ntiles, (float *)ctx->d_partials
 
@@ -732,6 +719,11 @@ void pcj_iter(cfdl_ctx *ctx) {
 int solve_momentum(cfdl_ctx *ctx) {
     if (ctx->cells.ntiles == 0) return CFDL_OK;
     mom_init(ctx);
+    return solve_momentum_started(ctx);
+}
+
+int solve_momentum_started(cfdl_ctx *ctx) {
+    if (ctx->cells.ntiles == 0) return CFDL_OK;
     const int cap = max_cap(ctx);
     int it = 0, maxit = 0;
     while (it < cap) {

@@ -18,6 +18,8 @@ for them:
   k_coef_uvw_cell  70 per cell (6 per slot, the three right-hand sides, the
                    relaxation, the divisions of d and dc) and about 50 per
                    wall face (unit normal, tangential slip, wall terms)
+  k_coef_uvw_init  85 per cell in FP64: k_coef_uvw_cell with the start of the
+                   momentum solve (one reciprocal, no zero terms)
   k_grad<N>        4 per slot and field (a difference and three FMAs)
   k_mom_*          BiCGStab with three active right-hand sides
   k_v_* , k_apc_q  the pressure solve's mesh-level rows
@@ -34,6 +36,7 @@ def fp64_inst(name, ne, nf, nbf, W):
         "k_coef_uvw_face": 40 * nfi,
         "k_calc_mip": 21 * nfi,
         "k_coef_uvw_cell": 70 * ne + 50 * nbf,
+        "k_coef_uvw_init": (25 + 60 * w) * ne + 50 * nbf,
         "k_grad3": 12 * W * ne,
         "k_grad1": 4 * W * ne,
         "k_mom_init": 42.7 * w * ne,
