@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(kTile) k_amg_prep0(const CaseDev *__restrict__
     double a[kMaxW];
 #pragma unroll
     for (int k = 0; k < kMaxW; k++) a[k] = mixed && k < C.W ? C.anb_p[k * C.ne + i] : 0.0;
-    const double rd = kOmega / ap;
+    const double rd = div_rn(kOmega, ap);
     C.rap_p[i] = rd;
     if (!mixed) C.rap2_p[i] = rd * (kOmega2 / kOmega);
     if (mixed) {
@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(kInvThreads) k_amg_coarse_inv(const CaseDev *_
         const int t = (int)threadIdx.x;
         if (t < n) {
             const double p = M[k * n + k];
-            R[t] = (t == k ? 1.0 : M[k * n + t]) / p;     // the pivot row, scaled
+            R[t] = div_rn(t == k ? 1.0 : M[k * n + t], p);   // the pivot row, scaled
             Q[t] = M[t * n + k];                          // the pivot column, before the update
         }
         __syncthreads();
@@ -712,8 +712,9 @@ __global__ void __launch_bounds__(kTile) k_amg_gal(const CaseDev *__restrict__ c
         dsum += v;
     }
     L.dg[I] = dsum;
-    L.rd[I] = kOmega / dsum;
-    if (mixed) { L.dg32[I] = narrow_f32(dsum); L.rd32[I] = narrow_f32(kOmega / dsum); }
+    const double rd = div_rn(kOmega, dsum);
+    L.rd[I] = rd;
+    if (mixed) { L.dg32[I] = narrow_f32(dsum); L.rd32[I] = narrow_f32(rd); }
 }
 
 // ------------------------------------------------- the V-cycle's tail
@@ -1045,8 +1046,9 @@ __global__ void __launch_bounds__(kTile) k_amg_galg(const CaseDev *__restrict__ 
     dsum = group_sum<G>(dsum);
     if (ok && g == 0) {
         L.dg[i] = dsum;
-        L.rd[i] = kOmega / dsum;
-        if (mixed) { L.dg32[i] = narrow_f32(dsum); L.rd32[i] = narrow_f32(kOmega / dsum); }
+        const double rd = div_rn(kOmega, dsum);
+        L.rd[i] = rd;
+        if (mixed) { L.dg32[i] = narrow_f32(dsum); L.rd32[i] = narrow_f32(rd); }
     }
 }
 

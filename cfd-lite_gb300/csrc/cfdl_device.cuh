@@ -257,4 +257,28 @@ __device__ __forceinline__ double widen_f64(float f) {
     return __longlong_as_double((long long)(sign | (de << 52) | ((unsigned long long)m << 29)));
 }
 
+// b / a, correctly rounded, for a row's quotients.  The built-in FP64 division
+// is about 18 FP64 instructions, 4 us each per 2.1M rows on GB300; this is 7.
+// The reciprocal of a starts from the FP32 one (22 bits; FP32 and integer
+// instructions only) and takes two Newton steps, y += y (1 - a y), to within
+// a half ulp; the quotient q = b y is then corrected by its remainder,
+// q += y (b - a q), which rounds it correctly (Markstein, IBM J. Res. Dev. 34,
+// 1990).  Numbers near the ends of either format's range, zeros and
+// non-finite values take the division.
+__device__ __forceinline__ bool rcp_in_range(double a) {      // 2^-100 <= |a| < 2^101
+    const unsigned e = (unsigned)(__double2hiint(a) >> 20) & 0x7ffu;
+    return e - (1023u - 100u) <= 200u;
+}
+__device__ __forceinline__ double rcp_near(double a) {
+    const double y0 = widen_f64(__fdividef(1.0f, narrow_f32(a)));
+    const double y1 = __fma_rn(y0, __fma_rn(-a, y0, 1.0), y0);
+    return __fma_rn(y1, __fma_rn(-a, y1, 1.0), y1);
+}
+__device__ __forceinline__ double div_rn(double b, double a) {
+    const unsigned e = (unsigned)(__double2hiint(b) >> 20) & 0x7ffu;
+    if (!rcp_in_range(a) || e - (1023u - 500u) > 1000u) return b / a;
+    const double y = rcp_near(a), q = __dmul_rn(b, y);
+    return __fma_rn(__fma_rn(-a, q, b), y, q);
+}
+
 }  // namespace cfdl

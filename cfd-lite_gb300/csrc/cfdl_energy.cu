@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(kTile) k_en_cell(const CaseDev *__restrict__ c
 __global__ void __launch_bounds__(kTile) k_en_temp(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles) {
     CFDL_PDL_WAIT();
     EN_PROLOGUE
-    if (i < t.last) C.et[i] = C.ee[i] / C.ecp[i];
+    if (i < t.last) C.et[i] = div_rn(C.ee[i], C.ecp[i]);
 }
 
 // t = t_init, phi = cp*t, phi0 = phi over cells and halos (construct_energy,

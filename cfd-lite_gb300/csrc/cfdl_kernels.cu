@@ -179,8 +179,8 @@ __global__ void __launch_bounds__(kTile) k_coef_uvw_halo(const CaseDev *__restri
         if (kind == CFDL_BC_WALL) {
             const double ue = C.u[e], ve = C.v[e], we = C.w[e];
             const double area = C.fgeo[FG_AREA * nf + f];
-            const double n0 = C.fgeo[FG_AX * nf + f] / area, n1 = C.fgeo[FG_AY * nf + f] / area,
-                         n2 = C.fgeo[FG_AZ * nf + f] / area;
+            const double n0 = div_rn(C.fgeo[FG_AX * nf + f], area), n1 = div_rn(C.fgeo[FG_AY * nf + f], area),
+                         n2 = div_rn(C.fgeo[FG_AZ * nf + f], area);
             const double tn = ue * n0 + ve * n1 + we * n2;
             const double r0 = C.u[h] - (ue - tn * n0), r1 = C.v[h] - (ve - tn * n1), r2 = C.w[h] - (we - tn * n2);
             s0 = dbc * r0 - dbc * ue;
@@ -285,11 +285,11 @@ __global__ void __launch_bounds__(kTile) k_coef_uvw_cell(const CaseDev *__restri
 // instructions: rows without a boundary slot (the whole warp's) start their
 // sums from the first slot and skip the boundary terms, and sum b'^2 is formed
 // in tight mode only (otherwise it is only asked whether it is finite, see
-// kBigExp).  FORM 0 (precision 0) also forms vol/ap, vol/(ap - sum anb) and
-// 1/ap from one reciprocal and chains its sums: 85 FP64 instructions a row for
-// the 113 of the two kernels.  FORM 1 (precision 1 and 2) and 3 (FP32 explicit
-// face terms) keep every rounding of the two kernels, spelled out where the
-// compiler could contract either of two products.  At four CTAs per SM it
+// kBigExp).  FORM 0 (precision 0) also takes its quotients by reciprocals
+// (rcp_near) and chains its sums.  FORM 1 (precision 1 and 2) and 3 (FP32
+// explicit face terms) keep every rounding of the two kernels, spelled out
+// where the compiler could contract either of two products (div_rn rounds as
+// the division does).  At four CTAs per SM it
 // spills, and is still faster than at three or two without (128^3, an outer
 // iteration: FP64 4.635 ms against 4.643 and 4.679, precision 3 2.996 against
 // 3.015 and 3.031).  The two
@@ -371,20 +371,15 @@ __device__ __forceinline__ void coef_init_row(const CaseDev &C, int i, const int
     for (int k = 0; k < W; k++)
         if (k < C.W) C.anb[k * ne + i] = a[k];
     const double ec = __dsub_rn(ap, asum);  // SIMPLEC: vol / (ap - sum anb)
-    const double pr = FORM == 0 ? ap * ec : 0.0;
-    const int pe = (int)((unsigned long long)__double_as_longlong(pr) >> 52);   // sign and exponent
-    if (FORM == 0 && pe > 64 && pe < 1983) {
-        // one reciprocal for the three quotients (pr positive, its inverse and
-        // the products far from the ends of the range)
-        const double inv = 1.0 / pr, rap = inv * ec;
-        C.rap[i] = rap;
-        C.d[i] = vol * rap;
-        C.dc[i] = vol * (inv * ap);
+    if (FORM == 0) {
+        C.rap[i] = rcp_in_range(ap) ? rcp_near(ap) : 1.0 / ap;   // the Jacobi scaling of the solve
+        C.d[i] = div_rn(vol, ap);
+        C.dc[i] = rcp_in_range(ec) ? vol * rcp_near(ec) : vol / ec;
     } else {
-        const double dd = vol / ap;
+        const double dd = div_rn(vol, ap);
         C.d[i] = dd;
         if (FORM == 3) C.d32[i] = narrow_f32(dd);
-        C.dc[i] = vol / ec;
+        C.dc[i] = div_rn(vol, ec);
         if (m32) {
             const float fa = narrow_f32(ap);
             C.fdiag[i] = fa;
@@ -393,7 +388,7 @@ __device__ __forceinline__ void coef_init_row(const CaseDev &C, int i, const int
             for (int k = 0; k < W; k++)
                 if (k < C.W) C.fanb[k * ne + i] = narrow_f32(a[k]);
         } else {
-            C.rap[i] = 1.0 / ap;            // the Jacobi scaling of the FP64 solve
+            C.rap[i] = div_rn(1.0, ap);     // the Jacobi scaling of the FP64 solve
         }
     }
 #pragma unroll

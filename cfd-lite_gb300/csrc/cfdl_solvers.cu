@@ -78,7 +78,7 @@ __device__ __forceinline__ void mom_init_row(const CaseDev &C, int i, int ne, do
         for (int k = 0; k < W; k++)
             if (k < C.W) C.fanb[k * ne + i] = narrow_f32(a[k]);
     } else {
-        C.rap[i] = 1.0 / api;               // the Jacobi scaling of the whole FP64 solve, divided once
+        C.rap[i] = div_rn(1.0, api);        // the Jacobi scaling of the whole FP64 solve, divided once
     }
 #pragma unroll
     for (int q = 0; q < 3; q++) {
@@ -396,7 +396,7 @@ template <int W>
 __device__ __forceinline__ void en_init_row(const CaseDev &C, int i, int ne, double (&v)[2], bool m32) {
     const double api = C.ap[i];
     if (m32) { const float fa = narrow_f32(api); C.fdiag[i] = fa; C.frap[i] = 1.0f / fa; }
-    else C.rap[i] = 1.0 / api;
+    else C.rap[i] = div_rn(1.0, api);
     const double *__restrict__ phi = C.ee;
     double bb = C.b[i], s = api * phi[i];
 #pragma unroll
