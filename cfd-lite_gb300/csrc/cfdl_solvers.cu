@@ -160,6 +160,62 @@ template <int NC> __device__ __forceinline__ bool lanes_active(const KLanes *L) 
     return a != 0;
 }
 
+// The FP32 momentum solve keeps the two vectors whose neighbours are gathered,
+// ph and sh, with a row's three components together (float4), so a neighbour is
+// one 16-byte load instead of three: its SpMV was bound by the latency and the
+// number of its loads (A ph 67.7 -> 53 us at 128^3, A sh 63.2 -> 49).
+template <class T, int NC> constexpr bool kInter = sizeof(T) == 4 && NC == 3;
+
+// (A x)_i of the three components in FP32, x interleaved: d x_i - sum_k c_k x_k
+// in slot order.  Index and coefficient loads do not wait for one another.
+// k16: the neighbours as 16-bit offsets.  kGuard: rows of fewer than W slots.
+template <int W, bool k16, bool kGuard>
+__device__ __forceinline__ void row3_w(const CaseDev &C, const float4 *x, int i, float (&y)[3]) {
+    const int n = C.ne, ld = C.ld32;
+    int j[W];
+    float c[W];
+#pragma unroll
+    for (int k = 0; k < W; k++) {
+        const bool in = !kGuard || k < C.W;
+        int jj = -1;
+        if (in) {
+            if (k16) { const int d = C.nb16[k * ld + i]; jj = d == (int)kNb16None ? -1 : i + d; }
+            else jj = C.hf_nb[k * n + i];
+        }
+        const float a = in ? C.fanb[k * n + i] : 0.f;
+        const bool ok = (unsigned)jj < (unsigned)n;
+        j[k] = ok ? jj : i;
+        c[k] = ok ? a : 0.f;
+    }
+    const float d = C.fdiag[i];
+    const float4 xi = x[i];
+    float4 xk[W];
+#pragma unroll
+    for (int k = 0; k < W; k++) xk[k] = x[j[k]];
+    // the roundings spelled out: the first two products could be contracted
+    // either way
+    if (!kGuard) {
+        y[0] = __fmaf_rn(d, xi.x, -__fmul_rn(c[0], xk[0].x));
+        y[1] = __fmaf_rn(d, xi.y, -__fmul_rn(c[0], xk[0].y));
+        y[2] = __fmaf_rn(d, xi.z, -__fmul_rn(c[0], xk[0].z));
+    } else {
+        y[0] = __fmaf_rn(-c[0], xk[0].x, __fmul_rn(d, xi.x));
+        y[1] = __fmaf_rn(-c[0], xk[0].y, __fmul_rn(d, xi.y));
+        y[2] = __fmaf_rn(-c[0], xk[0].z, __fmul_rn(d, xi.z));
+    }
+#pragma unroll
+    for (int k = 1; k < W; k++) {
+        y[0] = __fmaf_rn(-c[k], xk[k].x, y[0]);
+        y[1] = __fmaf_rn(-c[k], xk[k].y, y[1]);
+        y[2] = __fmaf_rn(-c[k], xk[k].z, y[2]);
+    }
+}
+template <bool k16> __device__ __forceinline__ void row3(const CaseDev &C, const float4 *x, int i, float (&y)[3]) {
+    if (C.W == 6) row3_w<6, k16, false>(C, x, i, y);
+    else if (C.W == 4) row3_w<4, k16, false>(C, x, i, y);
+    else row3_w<kMaxW, k16, true>(C, x, i, y);
+}
+
 // p = r + beta (p - omega v); ph = p / ap
 template <class T, int NC>
 __global__ void __launch_bounds__(kTile) k_mom_p(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles) {
@@ -187,20 +243,24 @@ __global__ void __launch_bounds__(kTile) k_mom_p(const CaseDev *__restrict__ cas
             rr[q] = M.r[j];
             if (!first[q]) { pp[q] = M.p[j]; vv[q] = M.v[j]; }
         }
+        T ph[NC];
 #pragma unroll
         for (int q = 0; q < NC; q++) {
+            ph[q] = 0;
             if (!act[q]) continue;
             const int j = q * ne + i;
             const T pn = first[q] ? rr[q] : rr[q] + be[q] * (pp[q] - om[q] * vv[q]);
             M.p[j] = pn;
-            M.ph[j] = pn * rap;
+            ph[q] = pn * rap;
+            if (!kInter<T, NC>) M.ph[j] = ph[q];
         }
+        if (kInter<T, NC>) ((float4 *)M.ph)[i] = make_float4(ph[0], ph[1 % NC], ph[2 % NC], 0.f);
     }
 }
 
 // v = A ph; alpha = rho / (rh, v)
-template <class T, int NC>
-__global__ void __launch_bounds__(kTile, 4) k_mom_v(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles,
+template <class T, int NC, bool k16 = false>
+__global__ void __launch_bounds__(kTile, 5) k_mom_v(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles,
                                                  const int *__restrict__ cfirst, const int *__restrict__ cnt, T *partials) {
     CFDL_PDL_WAIT();
     TILE_HEAD
@@ -214,7 +274,8 @@ __global__ void __launch_bounds__(kTile, 4) k_mom_v(const CaseDev *__restrict__ 
     for (int q = 0; q < NC; q++) { v[q] = 0; act[q] = L->active[q]; }
     FOR_CELLS(t) {
         T y[NC], rh[NC];   // one pass over the row for the components
-        ell_row<NC, T>(C.hf_nb, M.a, M.ap[i], M.ph, ne, ne, C.W, i, y);
+        if constexpr (kInter<T, NC>) row3<k16>(C, (const float4 *)M.ph, i, y);
+        else ell_row<NC, T>(C.hf_nb, M.a, M.ap[i], M.ph, ne, ne, C.W, i, y);
 #pragma unroll
         for (int q = 0; q < NC; q++) rh[q] = act[q] ? M.rh[q * ne + i] : (T)0;   // loads before the stores
 #pragma unroll
@@ -262,15 +323,19 @@ __global__ void __launch_bounds__(kTile) k_mom_s(const CaseDev *__restrict__ cas
                 rr[q] = act[q] ? M.r[q * ne + i] : (T)0;
                 vv[q] = act[q] ? M.v[q * ne + i] : (T)0;
             }
+            T sh[NC];
 #pragma unroll
             for (int q = 0; q < NC; q++) {
+                sh[q] = 0;
                 if (!act[q]) continue;
                 const int j = q * ne + i;
                 const T sv = rr[q] - al[q] * vv[q];
                 M.s[j] = sv;
-                M.sh[j] = sv * rap;
+                sh[q] = sv * rap;
+                if (!kInter<T, NC>) M.sh[j] = sh[q];
                 v[q] += sv * sv;
             }
+            if (kInter<T, NC>) ((float4 *)M.sh)[i] = make_float4(sh[0], sh[1 % NC], sh[2 % NC], 0.f);
         } else {
 #pragma unroll
             for (int q = 0; q < NC; q++) {
@@ -291,8 +356,8 @@ __global__ void __launch_bounds__(kTile) k_mom_s(const CaseDev *__restrict__ cas
 }
 
 // t = A sh; omega = (t,s)/(t,t)
-template <class T, int NC>
-__global__ void __launch_bounds__(kTile, 4) k_mom_t(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles,
+template <class T, int NC, bool k16 = false>
+__global__ void __launch_bounds__(kTile, 5) k_mom_t(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles,
                                                  const int *__restrict__ cfirst, const int *__restrict__ cnt, T *partials) {
     CFDL_PDL_WAIT();
     TILE_HEAD
@@ -306,7 +371,8 @@ __global__ void __launch_bounds__(kTile, 4) k_mom_t(const CaseDev *__restrict__ 
     for (int q = 0; q < NC; q++) { v[q] = v[NC + q] = 0; act[q] = L->active[q] && !L->half[q]; }
     FOR_CELLS(t) {
         T y[NC], sv[NC];
-        ell_row<NC, T>(C.hf_nb, M.a, M.ap[i], M.sh, ne, ne, C.W, i, y);
+        if constexpr (kInter<T, NC>) row3<k16>(C, (const float4 *)M.sh, i, y);
+        else ell_row<NC, T>(C.hf_nb, M.a, M.ap[i], M.sh, ne, ne, C.W, i, y);
 #pragma unroll
         for (int q = 0; q < NC; q++) sv[q] = act[q] ? M.s[q * ne + i] : (T)0;   // loads before the stores
 #pragma unroll
@@ -344,6 +410,24 @@ __global__ void __launch_bounds__(kTile, 4) k_mom_x(const CaseDev *__restrict__ 
     for (int q = 0; q < NC; q++) {
         v[q] = v[NC + q] = 0; act[q] = L->active[q]; al[q] = (T)L->alpha[q]; om[q] = (T)L->omega[q];
     }
+    if (sizeof(T) == 8 && NC == 3) {
+        // FP64: one component's loads at a time; all eighteen together spilled
+        // 200 bytes under four CTAs per SM (128^3: an outer iteration 0.4%)
+        FOR_CELLS(t) {
+#pragma unroll
+            for (int q = 0; q < NC; q++) {
+                if (!act[q]) continue;
+                const int j = q * ne + i;
+                const T xv = M.x[q][i], ph = M.ph[j], sh = M.sh[j], sv = M.s[j], rh = M.rh[j];
+                const T tv = om[q] != (T)0 ? M.t[j] : (T)0;
+                M.x[q][i] = xv + al[q] * ph + om[q] * sh;
+                const T r = om[q] == (T)0 ? sv : sv - om[q] * tv;
+                M.r[j] = r;
+                v[q] += r * r;
+                v[NC + q] += rh * r;
+            }
+        }
+    } else
     FOR_CELLS(t) {
         // the row's loads, every component's, before its stores
         T xv[NC], ph[NC], sh[NC], sv[NC], tv[NC], rh[NC];
@@ -352,8 +436,14 @@ __global__ void __launch_bounds__(kTile, 4) k_mom_x(const CaseDev *__restrict__ 
             const int j = q * ne + i;
             xv[q] = ph[q] = sh[q] = sv[q] = tv[q] = rh[q] = 0;
             if (!act[q]) continue;
-            xv[q] = M.x[q][i]; ph[q] = M.ph[j]; sh[q] = M.sh[j]; sv[q] = M.s[j]; rh[q] = M.rh[j];
+            xv[q] = M.x[q][i]; sv[q] = M.s[j]; rh[q] = M.rh[j];
+            if (!kInter<T, NC>) { ph[q] = M.ph[j]; sh[q] = M.sh[j]; }
             if (om[q] != (T)0) tv[q] = M.t[j];
+        }
+        if constexpr (kInter<T, NC>) {
+            const float4 a = ((const float4 *)M.ph)[i], b = ((const float4 *)M.sh)[i];
+            ph[0] = a.x; ph[1] = a.y; ph[2] = a.z;
+            sh[0] = b.x; sh[1] = b.y; sh[2] = b.z;
         }
 #pragma unroll
         for (int q = 0; q < NC; q++) {
@@ -639,10 +729,14 @@ static void mom_init(cfdl_ctx *ctx) { CFDL_LAUNCH("k_mom_init", k_mom_init, cell
 
 void mom_iter(cfdl_ctx *ctx) {
     if (ctx->cases[0]->cfg.precision >= 2) {
+        bool n16 = ctx->amg_nb16;           // the 16-bit neighbour offsets, where every case has them
+        for (const HostCase *hc : ctx->cases) n16 = n16 && hc->dev.nb16;   // (one added since may not)
         CFDL_LAUNCH("k_mom_p", (k_mom_p<float, 3>), cellsv);
-        CFDL_LAUNCH("k_mom_v", (k_mom_v<float, 3>), cellsv, RED32);
+        if (n16) CFDL_LAUNCH("k_mom_v", (k_mom_v<float, 3, true>), cellsv, RED32);
+        else CFDL_LAUNCH("k_mom_v", (k_mom_v<float, 3, false>), cellsv, RED32);
         CFDL_LAUNCH("k_mom_s", (k_mom_s<float, 3>), cellsv, RED32);
-        CFDL_LAUNCH("k_mom_t", (k_mom_t<float, 3>), cellsv, RED32);
+        if (n16) CFDL_LAUNCH("k_mom_t", (k_mom_t<float, 3, true>), cellsv, RED32);
+        else CFDL_LAUNCH("k_mom_t", (k_mom_t<float, 3, false>), cellsv, RED32);
         CFDL_LAUNCH("k_mom_x", (k_mom_x<float, 3>), cellsv, RED32);
         return;
     }
