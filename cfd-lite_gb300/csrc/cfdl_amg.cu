@@ -383,70 +383,79 @@ __global__ void __launch_bounds__(kTile) k_amg_prep0(const CaseDev *__restrict__
 }
 
 // Dense inverse of A_L + c 11^T at each case's coarsest level (one CTA per
-// case, Gauss-Jordan in shared memory; the matrix is SPD, no pivoting).  Per
-// pivot k, the first n threads scale the pivot row into R (R[k] = 1/p, one
-// division per column: FP64 division is a long instruction sequence on a
-// single SM's FP64 pipe) and save the pivot column into Q; after a barrier
-// every thread updates its own entries (up to four: n <= 64, so
-// n^2 <= 4 * kInvThreads) from M, Q and R alone, so the update is in place;
-// a second barrier ends the pivot.
-constexpr int kInvThreads = 1024;
+// case, Gauss-Jordan; the matrix is SPD, no pivoting).  Each thread holds its
+// entries in registers; per pivot k their owners publish the pivot row and
+// column, the first n threads scale the row (R[k] = 1/p, one division per
+// column), and every thread updates its own entries from Q and R.  The FP64
+// pipe sets the pace: n^2/32 warp instructions of 16 clocks per pivot, behind
+// two barriers and a quotient; 256, 512 and 1024 threads measure the same.
+// With the matrix in shared memory the 37-row inverse of the 128^3 cavity
+// took 77 us and the 8-row one of the 24^3 cavity 17; this takes 55 and 11.7.
+// The same with a branch per kind of entry took 101.
+constexpr int kInvThreads = 256;
 __global__ void __launch_bounds__(kInvThreads) k_amg_coarse_inv(const CaseDev *__restrict__ cases, int ncases) {
     CFDL_PDL_WAIT();
     const int c = blockIdx.x;
     if (c >= ncases) return;
     const CaseDev &C = cases[c];
     if (C.precond != 1 || C.sc->halted) return;
-    __shared__ double M[kAmgCoarsest * kAmgCoarsest];
-    __shared__ double R[kAmgCoarsest], Q[kAmgCoarsest];
+    __shared__ double M[kAmgCoarsest * kAmgCoarsest];      // the matrix as it is assembled
+    __shared__ double R[kAmgCoarsest], row[2][kAmgCoarsest], col[2][kAmgCoarsest], dg[kAmgCoarsest];
     const LP<double> P = level<double>(C, C.nlev);
-    const int n = P.n;
+    const int n = P.n, tid = (int)threadIdx.x;
     if (n > kAmgCoarsest) return;   // cannot happen: the builder coarsens to <= kAmgCoarsest
+    if (tid < n) dg[tid] = P.dg[tid];
+    __syncthreads();
     double dmax = 0.0;
-    for (int i = 0; i < n; i++) dmax = fmax(dmax, fabs(P.dg[i]));
+    for (int i = 0; i < n; i++) dmax = fmax(dmax, fabs(dg[i]));
     const double cc = dmax > 0.0 ? dmax / n : 1.0;
     constexpr int kPer = kAmgCoarsest * kAmgCoarsest / kInvThreads;
-    int ei[kPer], ej[kPer];
+    for (int e = tid; e < n * n; e += kInvThreads) M[e] = cc + (e / n == e % n ? dg[e / n] : 0.0);
+    __syncthreads();
+    for (int s = tid; s < P.W * n; s += kInvThreads) {     // a row has one slot per neighbour
+        const int e = s % n, j = P.nb[s];
+        const double a = P.a[s];
+        if (j >= 0 && j < n) M[e * n + j] -= a;
+    }
+    __syncthreads();
+    double m[kPer];
+    short ei[kPer], ej[kPer];
+    const int used = (n * n + kInvThreads - 1) / kInvThreads;
 #pragma unroll
     for (int q = 0; q < kPer; q++) {
-        const int e = (int)threadIdx.x + q * kInvThreads;
-        ei[q] = e < n * n ? e / n : -1;
-        ej[q] = e < n * n ? e % n : -1;
-        if (ei[q] >= 0) M[e] = cc + (ei[q] == ej[q] ? P.dg[ei[q]] : 0.0);
+        const int e = tid + q * kInvThreads;
+        ei[q] = e < n * n ? (short)(e / n) : (short)-1;
+        ej[q] = e < n * n ? (short)(e % n) : (short)-1;
+        m[q] = e < n * n ? M[e] : 0.0;
     }
-    __syncthreads();
-    for (int e = threadIdx.x; e < n; e += blockDim.x) {
-        for (int k = 0; k < P.W; k++) {
-            const int j = P.nb[k * n + e];
-            if (j >= 0 && j < n) M[e * n + j] -= P.a[k * n + e];
-        }
-    }
-    __syncthreads();
     for (int k = 0; k < n; k++) {
-        const int t = (int)threadIdx.x;
-        if (t < n) {
-            const double p = M[k * n + k];
-            R[t] = div_rn(t == k ? 1.0 : M[k * n + t], p);   // the pivot row, scaled
-            Q[t] = M[t * n + k];                          // the pivot column, before the update
+        double *P0 = row[k & 1], *Q = col[k & 1];          // two of each: the next pivot's are written during this one's update
+#pragma unroll
+        for (int q = 0; q < kPer; q++) {
+            if (q >= used) break;
+            if (ei[q] == k) P0[ej[q]] = m[q];              // the pivot row
+            if (ej[q] == k && ei[q] >= 0) Q[ei[q]] = m[q]; // the pivot column, before the update
         }
+        __syncthreads();
+        if (tid < n) R[tid] = div_rn(tid == k ? 1.0 : P0[tid], P0[k]);
         __syncthreads();
 #pragma unroll
         for (int q = 0; q < kPer; q++) {
+            if (q >= used) break;
             const int i = ei[q], j = ej[q];
             if (i < 0) continue;
-            double &m = M[i * n + j];
-            if (i == k) m = R[j];
-            else if (j == k) m = -Q[i] * R[k];
-            else m -= Q[i] * R[j];
+            // one FP64 instruction whichever case an entry is: the pivot row,
+            // the pivot column (-Q R) or the rest (m - Q R)
+            const double rj = R[j], x = __fma_rn(-Q[i], rj, j == k ? 0.0 : m[q]);
+            m[q] = i == k ? rj : x;
         }
-        __syncthreads();
     }
 #pragma unroll
     for (int q = 0; q < kPer; q++) {
         if (ei[q] < 0) continue;
         const int e = ei[q] * n + ej[q];
-        C.cinv[e] = M[e];
-        if (C.precision >= 1) C.cinv32[e] = (float)M[e];
+        C.cinv[e] = m[q];
+        if (C.precision >= 1) C.cinv32[e] = (float)m[q];
     }
 }
 
@@ -689,6 +698,28 @@ __global__ void __launch_bounds__(kTile) k_v_restrict(const CaseDev *__restrict_
     rc[I] = restrict_row<T>(L, F.t, I);
 }
 
+// Sum of a coarse slot's fine couplings af[src[q0..q1)), in list order: kCh
+// indices and then kCh values loaded side by side (one by one, each entry was
+// two trips to L2: at 128^3 the large levels took 79 us on average and now
+// take 71 with kCh = 2, the small ones 35 and now 26 with 8; at 24^3 13.2 and
+// 9.8.  A warp per row on the small levels took 30 and 11.6).
+template <int kCh>
+__device__ __forceinline__ double gather_sum(const double *__restrict__ af, const int *__restrict__ src, int q0, int q1) {
+    double v = 0.0;
+    for (int q = q0; q < q1; q += kCh) {
+        int j[kCh];
+        double x[kCh];
+#pragma unroll
+        for (int u = 0; u < kCh; u++) j[u] = q + u < q1 ? src[q + u] : -1;
+#pragma unroll
+        for (int u = 0; u < kCh; u++) x[u] = j[u] >= 0 ? af[j[u]] : 0.0;
+#pragma unroll
+        for (int u = 0; u < kCh; u++)
+            if (j[u] >= 0) v += x[u];
+    }
+    return v;
+}
+
 // Galerkin row I, one thread per row (large levels)
 __global__ void __launch_bounds__(kTile) k_amg_gal(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles, int l) {
     CFDL_PDL_WAIT();
@@ -703,10 +734,14 @@ __global__ void __launch_bounds__(kTile) k_amg_gal(const CaseDev *__restrict__ c
     double dsum = 0.0;
     // padding slots (k >= len) keep the zeros they were created with
     const int len = L.len[I];
+    const int *__restrict__ gp = L.g_ptr, *__restrict__ gs = L.g_src;
+    int q0 = gp[I], q1 = gp[I + 1];
     for (int k = 0; k < len; k++) {
         const int s = k * n + I;
-        double v = 0.0;
-        for (int q = L.g_ptr[s]; q < L.g_ptr[s + 1]; q++) v += af[L.g_src[q]];
+        int p0 = 0, p1 = 0;                  // the next slot's list, ahead of this one's gathers
+        if (k + 1 < len) { p0 = gp[s + n]; p1 = gp[s + n + 1]; }
+        const double v = gather_sum<2>(af, gs, q0, q1);
+        q0 = p0; q1 = p1;
         L.a[s] = v;
         if (mixed) L.a32[s] = narrow_f32(v);
         dsum += v;
@@ -1034,11 +1069,11 @@ __global__ void __launch_bounds__(kTile) k_amg_galg(const CaseDev *__restrict__ 
     const bool mixed = C.precision >= 1;
     const int n = L.n;
     double dsum = 0.0;
+    const int *__restrict__ gp = L.g_ptr, *__restrict__ gs = L.g_src;
     if (ok)
         for (int k = g, len = L.len[i]; k < len; k += G) {
             const int sl = k * n + i;
-            double v = 0.0;
-            for (int q = L.g_ptr[sl]; q < L.g_ptr[sl + 1]; q++) v += af[L.g_src[q]];
+            const double v = gather_sum<8>(af, gs, gp[sl], gp[sl + 1]);
             L.a[sl] = v;
             if (mixed) L.a32[sl] = narrow_f32(v);
             dsum += v;
