@@ -632,6 +632,28 @@ __global__ void __launch_bounds__(kTile, 8) k_v_resid_mesh(const CaseDev *__rest
     const LP<double> P = level<double>(C, 0);
     P.t[i] = offsum_mesh(P, P.z, i, resid64(P.r[i], P.dg[i], P.z[i]));
 }
+// The mesh level's residual in precision 1's order of sums (flow_fp64): r - A z
+// with A z formed first, its roundings spelled out.
+template <int W, bool kGuard> __device__ __forceinline__ double amul_order(const LP<double> &P, const double *x, int i) {
+    int j[W];
+    double c[W];
+    row_slots<W, double, kGuard>(P, i, j, c);
+    double s = __fma_rn(P.dg[i], x[i], -__dmul_rn(c[0], x[j[0]]));
+#pragma unroll
+    for (int k = 1; k < W; k++) s = __fma_rn(-c[k], x[j[k]], s);
+    return s;
+}
+__global__ void __launch_bounds__(kTile) k_v_resid_order(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles) {
+    CFDL_PDL_WAIT();
+    const Tile tl = tiles[blockIdx.x];
+    const CaseDev &C = cases[tl.c];
+    if (!pactive(C)) return;
+    const int i = tl.first + (int)threadIdx.x;
+    if (i >= tl.last) return;
+    const LP<double> P = level<double>(C, 0);
+    const double y = P.W == 6 ? amul_order<6, false>(P, P.z, i) : P.W == 4 ? amul_order<4, false>(P, P.z, i) : amul_order<kMaxW, true>(P, P.z, i);
+    P.t[i] = P.r[i] - y;
+}
 __global__ void __launch_bounds__(kTile / 2, 16) k_v_resid_pair64(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles) {
     CFDL_PDL_WAIT();
     const Tile tl = tiles[blockIdx.x];
@@ -1564,9 +1586,11 @@ static void amg_setup_operators(cfdl_ctx *ctx) {
 
 // An FP64 mesh-level kernel: two rows per thread where one row per thread would
 // fill the SMs (8 CTAs of kTile threads each) more than once.  Each row's
-// arithmetic is the same either way.
-#define MESH64(NAME, K1, K2)                                                                              \
-    if (ctx->amg_smooth[0].ntiles > 8 * 152) ALAUNCH_N(NAME, K2, ctx->amg_smooth[0], kTile / 2);          \
+// arithmetic is the same either way.  KE: the coarse levels' kernel with its
+// order of sums (flow_fp64).
+#define MESH64(NAME, K1, K2, KE, ...)                                                                     \
+    if (!flow_fp64(ctx)) ALAUNCH(NAME, KE, ctx->amg_smooth[0], ##__VA_ARGS__);                            \
+    else if (ctx->amg_smooth[0].ntiles > 8 * 152) ALAUNCH_N(NAME, K2, ctx->amg_smooth[0], kTile / 2);     \
     else ALAUNCH(NAME, K1, ctx->amg_smooth[0]);
 
 template <class T> static void vcycle(cfdl_ctx *ctx) {
@@ -1594,8 +1618,8 @@ template <class T> static void vcycle(cfdl_ctx *ctx) {
         } else {
             ALAUNCH(l ? "k_v_jac0_c" : "k_v_jac0_f", k_v_jac0<T>, ctx->amg_smooth[l], l);
             if (l == 0) {
-                MESH64("k_v_jac_f", k_v_jac_mesh<false>, k_v_jac_pair64<false>)
-                MESH64("k_v_resid_f", k_v_resid_mesh, k_v_resid_pair64)
+                MESH64("k_v_jac_f", k_v_jac_mesh<false>, k_v_jac_pair64<false>, k_v_jac<double>, 0)
+                MESH64("k_v_resid_f", k_v_resid_mesh, k_v_resid_pair64, k_v_resid_order)
             } else {
                 ALAUNCH("k_v_jac_c", (k_v_jac<T>), ctx->amg_smooth[l], l);
                 ALAUNCH("k_v_resid_c", (k_v_resid<T>), ctx->amg_smooth[l], l);
@@ -1619,8 +1643,8 @@ template <class T> static void vcycle(cfdl_ctx *ctx) {
                 MESH32("k_v_jac_f", k_v_jac_pair, true, false)
                 MESH32("k_v_jac_f", k_v_jac_pair, false, false)
             } else if (l == 0) {
-                MESH64("k_v_jac_f", k_v_jac_mesh<true>, k_v_jac_pair64<true>)
-                MESH64("k_v_jac_f", k_v_jac_mesh<false>, k_v_jac_pair64<false>)
+                MESH64("k_v_jac_f", k_v_jac_mesh<true>, k_v_jac_pair64<true>, (k_v_jac<double, true>), 0)
+                MESH64("k_v_jac_f", k_v_jac_mesh<false>, k_v_jac_pair64<false>, k_v_jac<double>, 0)
             } else {
                 ALAUNCH("k_v_jac_c", (k_v_jac<T, true>), ctx->amg_smooth[l], l);
                 ALAUNCH("k_v_jac_c", (k_v_jac<T>), ctx->amg_smooth[l], l);

@@ -911,7 +911,6 @@ void ensure_face_props(cfdl_ctx *ctx) {
     CFDL_LAUNCH("k_face_props", k_face_props, faces);
     for (HostCase *hc : ctx->cases) hc->props_dirty = false;
 }
-static bool fp64_only(const cfdl_ctx *ctx) { return ctx->cases[0]->cfg.precision == 0; }
 static bool f32_assembly(const cfdl_ctx *ctx) { return ctx->cases[0]->cfg.precision == 3; }
 
 void ensure_g32(cfdl_ctx *ctx) {
@@ -927,7 +926,7 @@ static void launch_coef_uvw_faces(cfdl_ctx *ctx) {
     if (f32_assembly(ctx)) ensure_g32(ctx);
     CFDL_LAUNCH("k_coef_uvw_halo", k_coef_uvw_halo, halos);
     if (f32_assembly(ctx)) CFDL_LAUNCH("k_coef_uvw_face_f32", k_coef_uvw_face_f32, faces);
-    else if (fp64_only(ctx)) CFDL_LAUNCH("k_coef_uvw_face", k_coef_uvw_face<true>, faces);
+    else if (flow_fp64(ctx)) CFDL_LAUNCH("k_coef_uvw_face", k_coef_uvw_face<true>, faces);
     else CFDL_LAUNCH("k_coef_uvw_face", k_coef_uvw_face<false>, faces);
 }
 void launch_coef_uvw(cfdl_ctx *ctx) {
@@ -940,7 +939,7 @@ void launch_coef_uvw_init(cfdl_ctx *ctx) {
     launch_coef_uvw_faces(ctx);
     const WorkList &wl = ctx->cellsr;
     if (f32_assembly(ctx)) CFDL_LAUNCH("k_coef_uvw_init", k_coef_uvw_init<3>, cellsr, wl.d_case_first, wl.d_case_ntiles, ctx->d_partials);
-    else if (fp64_only(ctx)) CFDL_LAUNCH("k_coef_uvw_init", k_coef_uvw_init<0>, cellsr, wl.d_case_first, wl.d_case_ntiles, ctx->d_partials);
+    else if (flow_fp64(ctx)) CFDL_LAUNCH("k_coef_uvw_init", k_coef_uvw_init<0>, cellsr, wl.d_case_first, wl.d_case_ntiles, ctx->d_partials);
     else CFDL_LAUNCH("k_coef_uvw_init", k_coef_uvw_init<1>, cellsv, ctx->cellsv.d_case_first, ctx->cellsv.d_case_ntiles, ctx->d_partials);
 }
 void launch_grad(cfdl_ctx *ctx, int field) {
@@ -956,7 +955,7 @@ void launch_calc_mip(cfdl_ctx *ctx, int rc) {
         CFDL_LAUNCH("k_calc_mip", k_calc_mip_f32, faces, rc);
         return;
     }
-    if (fp64_only(ctx)) CFDL_LAUNCH("k_calc_mip", k_calc_mip<true>, faces, rc);
+    if (flow_fp64(ctx)) CFDL_LAUNCH("k_calc_mip", k_calc_mip<true>, faces, rc);
     else CFDL_LAUNCH("k_calc_mip", k_calc_mip<false>, faces, rc);
 }
 void launch_coef_p_matrix(cfdl_ctx *ctx) {
