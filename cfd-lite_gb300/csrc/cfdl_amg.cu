@@ -483,7 +483,7 @@ __global__ void __launch_bounds__(kTile) k_v_jac(const CaseDev *__restrict__ cas
     const CaseDev &C = cases[tl.c];
     if (sizeof(T) == 8 ? !pactive(C) : !mactive(C)) return;
     const int i = tl.first + (int)threadIdx.x;
-    if (i >= tl.last) return;
+    if (i >= tl.last || (sizeof(T) == 8 && l == 0 && flow_fp64(C))) return;
     const LP<T> P = level<T>(C, l);
     const T *x = kToT ? P.z : P.t;
     T *y = kToT ? P.t : P.z;
@@ -505,7 +505,7 @@ __global__ void __launch_bounds__(kTile, 8) k_v_jac_mesh(const CaseDev *__restri
     CFDL_PDL_WAIT();
     const Tile tl = tiles[blockIdx.x];
     const CaseDev &C = cases[tl.c];
-    if (!pactive(C)) return;
+    if (!pactive(C) || !flow_fp64(C)) return;
     const int i = tl.first + (int)threadIdx.x;
     if (i >= tl.last) return;
     const LP<double> P = level<double>(C, 0);
@@ -553,7 +553,7 @@ __global__ void __launch_bounds__(kTile / 2, 16) k_v_jac_pair64(const CaseDev *_
     CFDL_PDL_WAIT();
     const Tile tl = tiles[blockIdx.x];
     const CaseDev &C = cases[tl.c];
-    if (!pactive(C)) return;
+    if (!pactive(C) || !flow_fp64(C)) return;
     const int i = tl.first + 2 * (int)threadIdx.x;
     if (i >= tl.last) return;
     const LP<double> P = level<double>(C, 0);
@@ -626,7 +626,7 @@ __global__ void __launch_bounds__(kTile, 8) k_v_resid_mesh(const CaseDev *__rest
     CFDL_PDL_WAIT();
     const Tile tl = tiles[blockIdx.x];
     const CaseDev &C = cases[tl.c];
-    if (!pactive(C)) return;
+    if (!pactive(C) || !flow_fp64(C)) return;
     const int i = tl.first + (int)threadIdx.x;
     if (i >= tl.last) return;
     const LP<double> P = level<double>(C, 0);
@@ -647,7 +647,7 @@ __global__ void __launch_bounds__(kTile) k_v_resid_order(const CaseDev *__restri
     CFDL_PDL_WAIT();
     const Tile tl = tiles[blockIdx.x];
     const CaseDev &C = cases[tl.c];
-    if (!pactive(C)) return;
+    if (!pactive(C) || flow_fp64(C)) return;
     const int i = tl.first + (int)threadIdx.x;
     if (i >= tl.last) return;
     const LP<double> P = level<double>(C, 0);
@@ -658,7 +658,7 @@ __global__ void __launch_bounds__(kTile / 2, 16) k_v_resid_pair64(const CaseDev 
     CFDL_PDL_WAIT();
     const Tile tl = tiles[blockIdx.x];
     const CaseDev &C = cases[tl.c];
-    if (!pactive(C)) return;
+    if (!pactive(C) || !flow_fp64(C)) return;
     const int i = tl.first + 2 * (int)threadIdx.x;
     if (i >= tl.last) return;
     const LP<double> P = level<double>(C, 0);
@@ -1586,12 +1586,14 @@ static void amg_setup_operators(cfdl_ctx *ctx) {
 
 // An FP64 mesh-level kernel: two rows per thread where one row per thread would
 // fill the SMs (8 CTAs of kTile threads each) more than once.  Each row's
-// arithmetic is the same either way.  KE: the coarse levels' kernel with its
-// order of sums (flow_fp64).
+// arithmetic is the same either way.  KE: the form of the cases with the energy
+// equation (flow_fp64), in precision 1's order of sums.
 #define MESH64(NAME, K1, K2, KE, ...)                                                                     \
-    if (!flow_fp64(ctx)) ALAUNCH(NAME, KE, ctx->amg_smooth[0], ##__VA_ARGS__);                            \
-    else if (ctx->amg_smooth[0].ntiles > 8 * 152) ALAUNCH_N(NAME, K2, ctx->amg_smooth[0], kTile / 2);     \
-    else ALAUNCH(NAME, K1, ctx->amg_smooth[0]);
+    if (any_flow_fp64(ctx)) {                                                                             \
+        if (ctx->amg_smooth[0].ntiles > 8 * 152) ALAUNCH_N(NAME, K2, ctx->amg_smooth[0], kTile / 2);      \
+        else ALAUNCH(NAME, K1, ctx->amg_smooth[0]);                                                       \
+    }                                                                                                     \
+    if (any_ordered(ctx)) ALAUNCH(NAME, KE, ctx->amg_smooth[0], ##__VA_ARGS__);
 
 template <class T> static void vcycle(cfdl_ctx *ctx) {
     // Large levels run one thread per row (G = 1) or a few lanes per row

@@ -204,6 +204,17 @@ bool energy_on(const cfdl_ctx *ctx) {
     return false;
 }
 
+bool any_flow_fp64(const cfdl_ctx *ctx) {
+    for (const HostCase *hc : ctx->cases)
+        if (flow_fp64(hc->dev)) return true;
+    return false;
+}
+bool any_ordered(const cfdl_ctx *ctx) {
+    for (const HostCase *hc : ctx->cases)
+        if (!flow_fp64(hc->dev)) return true;
+    return false;
+}
+
 void launch_energy_bc(cfdl_ctx *ctx) {
     if (energy_on(ctx)) CFDL_LAUNCH("k_en_bc", k_en_bc, halos);
 }

@@ -333,12 +333,16 @@ void launch_set_mip0(cfdl_ctx *ctx);
 
 // energy equation (cfdl_energy.cu)
 bool energy_on(const cfdl_ctx *ctx);          // some case of the context has it
-// The flow alone in FP64: its passes order their sums as is fastest.  The energy
-// solve stops after a set number of iterations, on fine meshes far from its
-// solution, and its iterates amplify a rounding difference in the fluxes by up
-// to 1e10 (84^3 cells, Re 100: 1e-14 in u became 1e-4 in T), so with the energy
-// equation set up the passes keep the one order of precision 1.
-inline bool flow_fp64(const cfdl_ctx *ctx) { return ctx->cases[0]->cfg.precision == 0 && !energy_on(ctx); }
+// A case whose flow is solved alone in FP64: its passes order their sums as is
+// fastest.  The energy solve stops after a set number of iterations, on fine
+// meshes far from its solution, and its iterates amplify a rounding difference
+// in the fluxes by up to 1e10 (84^3 cells, Re 100: 1e-14 in u became 1e-4 in T),
+// so a case with the energy equation keeps the one order of precision 1.  A
+// context may hold cases of both kinds: each kind has its launch, which passes
+// over the other's tiles.
+__host__ __device__ inline bool flow_fp64(const CaseDev &C) { return C.precision == 0 && !C.ee; }
+bool any_flow_fp64(const cfdl_ctx *ctx);      // some case is of the first kind
+bool any_ordered(const cfdl_ctx *ctx);        // some case is not
 void launch_energy_bc(cfdl_ctx *ctx);
 void launch_energy_time(cfdl_ctx *ctx, bool run_due);   // run_due: only cases whose run cadence is due
 void launch_coef_energy(cfdl_ctx *ctx);

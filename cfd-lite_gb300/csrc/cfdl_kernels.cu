@@ -67,7 +67,7 @@ template <bool kFast>
 __global__ void __launch_bounds__(kTile) k_coef_uvw_face(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles) {
     CFDL_PDL_WAIT();
     TILE_PROLOGUE(faces)
-    if (i >= t.last) return;
+    if (i >= t.last || flow_fp64(C) != kFast) return;
     const int nf = C.nf, o = C.f_own[i], n = C.f_nb[i];
     if (n >= C.ne) return;                  // boundary faces: only their (precomputed) diffusion
     const double *g = C.fgeo, *pr = C.fprop;
@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(kTile, 4) k_coef_uvw_init(const CaseDev *__res
     CFDL_PDL_WAIT();
     const Tile t = tiles[blockIdx.x];
     const CaseDev &C = cases[t.c];
-    if (C.sc->halted) return;
+    if (C.sc->halted || flow_fp64(C) != (FORM == 0)) return;
     const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     double v[6] = {0, 0, 0, 0, 0, 0};
     if (C.W == 6) coef_init_rows<FORM, 6>(C, t, v);
@@ -641,7 +641,7 @@ template <bool kFast>
 __global__ void __launch_bounds__(kTile) k_calc_mip(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles, int rc) {
     CFDL_PDL_WAIT();
     TILE_PROLOGUE(faces)
-    if (i >= t.last) return;
+    if (i >= t.last || flow_fp64(C) != kFast) return;
     const int nf = C.nf, o = C.f_own[i], n = C.f_nb[i];
     if (n >= C.ne) return;
     const double *g = C.fgeo;
@@ -926,8 +926,10 @@ static void launch_coef_uvw_faces(cfdl_ctx *ctx) {
     if (f32_assembly(ctx)) ensure_g32(ctx);
     CFDL_LAUNCH("k_coef_uvw_halo", k_coef_uvw_halo, halos);
     if (f32_assembly(ctx)) CFDL_LAUNCH("k_coef_uvw_face_f32", k_coef_uvw_face_f32, faces);
-    else if (flow_fp64(ctx)) CFDL_LAUNCH("k_coef_uvw_face", k_coef_uvw_face<true>, faces);
-    else CFDL_LAUNCH("k_coef_uvw_face", k_coef_uvw_face<false>, faces);
+    else {
+        if (any_flow_fp64(ctx)) CFDL_LAUNCH("k_coef_uvw_face", k_coef_uvw_face<true>, faces);
+        if (any_ordered(ctx)) CFDL_LAUNCH("k_coef_uvw_face", k_coef_uvw_face<false>, faces);
+    }
 }
 void launch_coef_uvw(cfdl_ctx *ctx) {
     launch_coef_uvw_faces(ctx);
@@ -939,8 +941,10 @@ void launch_coef_uvw_init(cfdl_ctx *ctx) {
     launch_coef_uvw_faces(ctx);
     const WorkList &wl = ctx->cellsr;
     if (f32_assembly(ctx)) CFDL_LAUNCH("k_coef_uvw_init", k_coef_uvw_init<3>, cellsr, wl.d_case_first, wl.d_case_ntiles, ctx->d_partials);
-    else if (flow_fp64(ctx)) CFDL_LAUNCH("k_coef_uvw_init", k_coef_uvw_init<0>, cellsr, wl.d_case_first, wl.d_case_ntiles, ctx->d_partials);
-    else CFDL_LAUNCH("k_coef_uvw_init", k_coef_uvw_init<1>, cellsv, ctx->cellsv.d_case_first, ctx->cellsv.d_case_ntiles, ctx->d_partials);
+    else {
+        if (any_flow_fp64(ctx)) CFDL_LAUNCH("k_coef_uvw_init", k_coef_uvw_init<0>, cellsr, wl.d_case_first, wl.d_case_ntiles, ctx->d_partials);
+        if (any_ordered(ctx)) CFDL_LAUNCH("k_coef_uvw_init", k_coef_uvw_init<1>, cellsv, ctx->cellsv.d_case_first, ctx->cellsv.d_case_ntiles, ctx->d_partials);
+    }
 }
 void launch_grad(cfdl_ctx *ctx, int field) {
     if (field == 4 && f32_assembly(ctx)) CFDL_LAUNCH("k_grad3_f32", k_grad3_f32, cells);
@@ -955,8 +959,8 @@ void launch_calc_mip(cfdl_ctx *ctx, int rc) {
         CFDL_LAUNCH("k_calc_mip", k_calc_mip_f32, faces, rc);
         return;
     }
-    if (flow_fp64(ctx)) CFDL_LAUNCH("k_calc_mip", k_calc_mip<true>, faces, rc);
-    else CFDL_LAUNCH("k_calc_mip", k_calc_mip<false>, faces, rc);
+    if (any_flow_fp64(ctx)) CFDL_LAUNCH("k_calc_mip", k_calc_mip<true>, faces, rc);
+    if (any_ordered(ctx)) CFDL_LAUNCH("k_calc_mip", k_calc_mip<false>, faces, rc);
 }
 void launch_coef_p_matrix(cfdl_ctx *ctx) {
     ensure_face_props(ctx);
