@@ -227,6 +227,7 @@ int cfdl_set_config(cfdl_ctx *ctx, const cfdl_config *cfg) {
     int st = check_ctx(ctx);
     if (st) return st;
     if ((st = validate_config(cfg))) return st;
+    const bool reshape = ctx->cases[0]->cfg.precision != cfg->precision;   // the solver tiles go by the precision
     for (HostCase *hc : ctx->cases) {
         if (hc->cfg.rho != cfg->rho || hc->cfg.mu != cfg->mu) {
             hc->props_dirty = true;
@@ -238,7 +239,9 @@ int cfdl_set_config(cfdl_ctx *ctx, const cfdl_config *cfg) {
         if (cfg->precision == 3 && hc->cfg.precision != 3) hc->g32_stale = true;
         apply_config(hc, cfg);
     }
-    return upload_case_table(ctx);
+    if (!reshape) return upload_case_table(ctx);
+    if ((st = cuda_status(cudaStreamSynchronize(ctx->stream)))) return st;
+    return rebuild_worklists(ctx);
 }
 
 int cfdl_upload_fields(cfdl_ctx *ctx, const cfdl_fields *f) {
@@ -487,8 +490,10 @@ int cfdl_energy_init(cfdl_ctx *ctx, double cp, double tc, double t_init) {
     for (HostCase *hc : ctx->cases)
         if ((st = energy_init_case(ctx, hc, cp, tc, t_init))) break;
     // the device table follows the host records even after a failure part way
-    destroy_graph(ctx);   // graphs captured without (or with) the energy launches
-    const int st2 = upload_case_table(ctx);
+    // (the solver tiles go by it too; graphs captured without, or with, the
+    // energy launches are dropped with the old lists)
+    int st2 = cuda_status(cudaStreamSynchronize(ctx->stream));
+    if (!st2) st2 = rebuild_worklists(ctx);
     if (st) return st;
     if (st2) return st2;
     return cuda_status(cudaStreamSynchronize(ctx->stream));

@@ -72,6 +72,19 @@ int build_worklist(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &sizes, i
 // so a case's sums are the same alone and in a batch.
 static int rows_per_thread(int ne) { return ne <= 152 * 4 * kTile ? 1 : ne <= 2 * 152 * 4 * kTile ? 2 : 4; }
 
+// Rows per thread of the FP64 solver passes: at least `least`, and on large
+// cases as many as put the case's tiles on the chip at once (152 SMs, four
+// CTAs each).  A tile's reduction takes 17 FP64 warp adds per sum and its
+// start and end a few thousand clocks, whatever its rows: at 128^3, 14 rows per
+// thread instead of four took an outer iteration from 4585 to 4425 us, 16 (two
+// waves again) 4520; a wave of five or eight CTAs per SM gave 4530 and 4440.
+// The FP32 passes and the cases with the energy equation keep four: their sums'
+// order is part of their results (flow_fp64).
+static int rows_one_wave(int ne, int least) {
+    constexpr int wave = 152 * 4 * kTile;
+    return std::max(least, (ne + wave - 1) / wave);
+}
+
 // tiles: entities per tile of each case
 int build_worklist(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &sizes, const std::vector<int> &tiles) {
     free_worklist(wl);
@@ -459,9 +472,12 @@ int rebuild_worklists(cfdl_ctx *ctx) {
     if ((st = build_worklist(ctx, ctx->faces, nfc))) return st;
     if ((st = build_worklist(ctx, ctx->facesv, nfc, kTile * kFaceVec))) return st;
     if ((st = build_worklist(ctx, ctx->halos, nh))) return st;
-    if ((st = build_worklist(ctx, ctx->cellsv, nc, kTile * ctx->vec))) return st;
-    if ((st = build_worklist(ctx, ctx->cellse, nc, kTile * ctx->en_vec))) return st;
     std::vector<int> tiles;
+    for (const HostCase *hc : ctx->cases)
+        tiles.push_back(kTile * (ctx->vec == kVec && flow_fp64(hc->dev) ? rows_one_wave(hc->ne, kVec) : ctx->vec));
+    if ((st = build_worklist(ctx, ctx->cellsv, nc, tiles))) return st;
+    if ((st = build_worklist(ctx, ctx->cellse, nc, kTile * ctx->en_vec))) return st;
+    tiles.clear();
     for (int ne : nc) tiles.push_back(kTile * rows_per_thread(ne));
     if ((st = build_worklist(ctx, ctx->cellsr, nc, tiles))) return st;
     for (auto &wl : ctx->amg_cells) free_worklist(wl);

@@ -226,7 +226,8 @@ struct cfdl_ctx {
     cfdl::CaseDev *d_cases = nullptr;
     int d_cases_cap = 0;
     cfdl::WorkList cells, faces, halos;
-    cfdl::WorkList cellsv;               // wide tiles (kTile*vec cells) for the solver kernels
+    cfdl::WorkList cellsv;               // wide tiles (kTile*vec cells) for the solver kernels; at the default vec
+                                         // more on large FP64 flow cases (rows_one_wave)
     int vec = cfdl::kVec;                // cells per thread in those tiles (autotuned)
     cfdl::WorkList cellsr;               // tiles of the FP64 passes whose shape goes by the case's size (rows_per_thread)
     cfdl::WorkList cellse;               // tiles of the energy solve (kTile*en_vec cells)

@@ -406,7 +406,10 @@ int cfdl_run(cfdl_ctx *ctx, int max_outer, int *running);
  * snapshot of their state that it restores afterwards, keeps the fastest and
  * returns it in *best; ms[4] (optional) receives the time per outer
  * iteration of each candidate.  The shape changes the order of the partial
- * sums, so results agree across shapes to rounding, not bit for bit. */
+ * sums, so results agree across shapes to rounding, not bit for bit.  At the
+ * default, cases of precision 0 without the energy equation and with more than
+ * 622592 cells get as many cells per CTA as put the case on the chip in one
+ * wave. */
 int cfdl_set_tile(cfdl_ctx *ctx, int vec);
 int cfdl_get_tile(const cfdl_ctx *ctx);
 /* Lanes per row (1, 2 or 4; default 1) on the large coarse multigrid levels
