@@ -86,7 +86,8 @@ static int rows_one_wave(int ne, int least) {
 }
 
 // tiles: entities per tile of each case
-int build_worklist(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &sizes, const std::vector<int> &tiles) {
+// per_thread: entities per thread and sub-tile of a merged list (0: the tile's)
+int build_worklist(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &sizes, const std::vector<int> &tiles, int per_thread) {
     free_worklist(wl);
     wl.h_tiles.clear(); wl.case_first.clear(); wl.case_ntiles.clear();
     for (size_t c = 0; c < sizes.size(); c++) {
@@ -94,7 +95,7 @@ int build_worklist(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &sizes, c
         int cnt = 0;
         const int tile = tiles[c];
         for (int s = 0; s < sizes[c]; s += tile, cnt++)
-            wl.h_tiles.push_back({(int)c, s, std::min(sizes[c], s + tile), (tile + kTile - 1) / kTile});
+            wl.h_tiles.push_back({(int)c, s, std::min(sizes[c], s + tile), per_thread ? per_thread : (tile + kTile - 1) / kTile});
         wl.case_ntiles.push_back(cnt);
     }
     wl.ntiles = (int)wl.h_tiles.size();
@@ -463,6 +464,17 @@ int create_case(cfdl_ctx *ctx, const cfdl_mesh *m, const cfdl_config *cfg, HostC
     return upload_case(p, cfg, out);
 }
 
+// A list of tiles of kTile * vec entities, M to a block: as many as bring the
+// context's blocks down to one wave (152 SMs, four CTAs each), at most kMaxMerge.
+static int build_merged(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &sizes, int vec) {
+    const int rows = kTile * vec;
+    long n = 0;
+    for (int s : sizes) n += (s + rows - 1) / rows;
+    const int M = (int)std::min<long>(kMaxMerge, std::max<long>(1, (n + 152 * 4 - 1) / (152 * 4)));
+    wl.merge = {M, rows};
+    return build_worklist(ctx, wl, sizes, std::vector<int>(sizes.size(), rows * M), vec);
+}
+
 // Tile work lists over every case of the context.
 int rebuild_worklists(cfdl_ctx *ctx) {
     std::vector<int> nc, nfc, nh;
@@ -477,6 +489,7 @@ int rebuild_worklists(cfdl_ctx *ctx) {
         tiles.push_back(kTile * (ctx->vec == kVec && flow_fp64(hc->dev) ? rows_one_wave(hc->ne, kVec) : ctx->vec));
     if ((st = build_worklist(ctx, ctx->cellsv, nc, tiles))) return st;
     if ((st = build_worklist(ctx, ctx->cellse, nc, kTile * ctx->en_vec))) return st;
+    if ((st = build_merged(ctx, ctx->cellsem, nc, ctx->en_vec))) return st;
     tiles.clear();
     for (int ne : nc) tiles.push_back(kTile * rows_per_thread(ne));
     if ((st = build_worklist(ctx, ctx->cellsr, nc, tiles))) return st;
@@ -489,7 +502,8 @@ int rebuild_worklists(cfdl_ctx *ctx) {
     ctx->amg_cells.clear(); ctx->amg_smooth.clear(); ctx->amg_gcells.clear(); ctx->amg_gsmooth.clear();
     ctx->amg_restr.clear(); ctx->amg_grestr.clear(); ctx->amg_lmax = -1;
     destroy_graph(ctx);   // captured launch arguments refer to the old lists
-    int need = std::max({ctx->cells.ntiles, ctx->faces.ntiles, ctx->halos.ntiles, 1});
+    int need = std::max({ctx->cells.ntiles, ctx->faces.ntiles, ctx->halos.ntiles,
+                         ctx->cellsem.ntiles * ctx->cellsem.merge.M, 1});
     if (need > ctx->partials_cap) {
         cudaFree(ctx->d_partials);
         ctx->d_partials = nullptr;

@@ -23,61 +23,117 @@ namespace cfdl {
 // eight warps' trees of value k with every lane busy -- 4 adds for the first
 // step of all eight trees, 2, 1, 1 and 1 for the next -- and adds the eight
 // sums in order: 17 warp-adds, the same sums in the same order.
-template <int K>
-__device__ __forceinline__ void block_sums(double (&v)[K], double *out) {
+// The sum of x[0..kTile-1] (shared) by one warp: each of the kTile / 32 warps'
+// shuffle tree, then the trees' sums in warp order.
+__device__ __forceinline__ double tree_sum(const double *v) {
     constexpr int kWarps = kTile / 32;
     static_assert(kWarps == 8, "the packing below is for eight warps");
+    const int lane = threadIdx.x & 31;
+    const bool b8 = (lane & 8) != 0, b4 = (lane & 4) != 0;
+    // x[j]: lane l & 15 of tree w = 2 j + (lane >> 4) after its first step
+    double x[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const int at = (2 * j + (lane >> 4)) * 32 + (lane & 15);
+        x[j] = v[at] + v[at + 16];
+    }
+    // second step: lanes with bit 8 clear take trees j, the others j + 1
+    double y[2];
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        const double own = b8 ? x[2 * j + 1] : x[2 * j], other = b8 ? x[2 * j] : x[2 * j + 1];
+        y[j] = own + __shfl_xor_sync(0xffffffffu, other, 8);
+    }
+    double z = (b4 ? y[1] : y[0]) + __shfl_xor_sync(0xffffffffu, b4 ? y[0] : y[1], 4);
+    z += __shfl_xor_sync(0xffffffffu, z, 2);
+    z += __shfl_xor_sync(0xffffffffu, z, 1);
+    // the sum of warp w = 2 j + h, j = (bit 8) + 2 (bit 4), is in lane 16 h + 8 (j & 1) + 4 (j >> 1)
+    double s = 0.0;
+#pragma unroll
+    for (int w = 0; w < kWarps; w++)
+        s += __shfl_sync(0xffffffffu, z, 16 * (w & 1) + 8 * ((w >> 1) & 1) + 4 * (w >> 2));
+    return s;
+}
+template <int K>
+__device__ __forceinline__ void block_sums(double (&v)[K], double *out) {
     __shared__ double sm[K][kTile];
 #pragma unroll
     for (int k = 0; k < K; k++) sm[k][threadIdx.x] = v[k];
     __syncthreads();
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const bool b8 = (lane & 8) != 0, b4 = (lane & 4) != 0;
-    for (int k = wid; k < K; k += kWarps) {
-        // x[j]: lane l & 15 of tree w = 2 j + (lane >> 4) after its first step
-        double x[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int at = (2 * j + (lane >> 4)) * 32 + (lane & 15);
-            x[j] = sm[k][at] + sm[k][at + 16];
-        }
-        // second step: lanes with bit 8 clear take trees j, the others j + 1
-        double y[2];
-#pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const double own = b8 ? x[2 * j + 1] : x[2 * j], other = b8 ? x[2 * j] : x[2 * j + 1];
-            y[j] = own + __shfl_xor_sync(0xffffffffu, other, 8);
-        }
-        double z = (b4 ? y[1] : y[0]) + __shfl_xor_sync(0xffffffffu, b4 ? y[0] : y[1], 4);
-        z += __shfl_xor_sync(0xffffffffu, z, 2);
-        z += __shfl_xor_sync(0xffffffffu, z, 1);
-        // the sum of warp w = 2 j + h, j = (bit 8) + 2 (bit 4), is in lane 16 h + 8 (j & 1) + 4 (j >> 1)
-        double s = 0.0;
-#pragma unroll
-        for (int w = 0; w < kWarps; w++)
-            s += __shfl_sync(0xffffffffu, z, 16 * (w & 1) + 8 * ((w >> 1) & 1) + 4 * (w >> 2));
-        if (lane == 0) out[k] = s;
+    for (int k = threadIdx.x >> 5; k < K; k += kTile / 32) {
+        const double s = tree_sum(sm[k]);
+        if ((threadIdx.x & 31) == 0) out[k] = s;
     }
 }
-// FP32: a fixed shuffle tree per warp, then the warps' sums in warp order
-// (FP32 adds are cheap here; the order is part of the FP32 forms' results).
+// FP32: a shuffle tree per warp, then the warps' sums in warp order (the order is
+// part of the FP32 forms' results).  The trees of N values fold together: at
+// each step a lane keeps half of the values and hands the other half over, so
+// six values take 8 shuffles and adds instead of 30 (0.2% of an FP32 outer
+// iteration).  Returns the sum of value k if `mine`: one lane per value.
+template <int N, int O = 16>
+__device__ __forceinline__ float warp_sums(const float (&v)[N], int lane, int &k, bool &mine) {
+    if constexpr (N == 1) {
+        float z = v[0];
+#pragma unroll
+        for (int o = O; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+        k = 0;
+        mine = (lane & (2 * O - 1)) == 0;
+        return z;
+    } else {
+        constexpr int H = (N + 1) / 2;
+        const bool up = (lane & O) != 0;
+        float y[H];
+#pragma unroll
+        for (int j = 0; j < H; j++) {
+            const float hi = j + H < N ? v[j + H < N ? j + H : 0] : v[j];
+            y[j] = (up ? hi : v[j]) + __shfl_xor_sync(0xffffffffu, up ? v[j] : hi, O);
+        }
+        const float z = warp_sums<H, O / 2>(y, lane, k, mine);
+        if (up) k += H;
+        mine = mine && k < N;
+        return z;
+    }
+}
 template <int K>
 __device__ __forceinline__ void block_sums(float (&v)[K], float *out) {
     __shared__ float sm[K][kTile / 32];
-#pragma unroll
-    for (int k = 0; k < K; k++)
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0)
-#pragma unroll
-        for (int k = 0; k < K; k++) sm[k][wid] = v[k];
+    int k;
+    bool mine;
+    const float z = warp_sums<K>(v, threadIdx.x & 31, k, mine);
+    if (mine) sm[k][threadIdx.x >> 5] = z;
     __syncthreads();
     if (threadIdx.x < K) {
         float s = 0;
         for (int w = 0; w < kTile / 32; w++) s += sm[threadIdx.x][w];
         out[threadIdx.x] = s;
     }
+}
+
+// The second half of case_sums: the sums of a case's `ntiles` partials per value,
+// thread-strided in a fixed order with four independent accumulators (so the
+// loads overlap instead of forming one dependent chain), then the block sum.
+template <int K, class T>
+__device__ __forceinline__ void partial_sums(T (&v)[K], const T *part, int ntiles, T *s) {
+    T a1[K], a2[K], a3[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) v[k] = a1[k] = a2[k] = a3[k] = 0;
+    int i = threadIdx.x;
+    for (; i + 3 * kTile < ntiles; i += 4 * kTile)
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            const T *p = part + (size_t)k * ntiles + i;
+            v[k] += __ldcg(p);
+            a1[k] += __ldcg(p + kTile);
+            a2[k] += __ldcg(p + 2 * kTile);
+            a3[k] += __ldcg(p + 3 * kTile);
+        }
+    for (; i < ntiles; i += kTile)
+#pragma unroll
+        for (int k = 0; k < K; k++) v[k] += __ldcg(&part[(size_t)k * ntiles + i]);
+#pragma unroll
+    for (int k = 0; k < K; k++) v[k] = (v[k] + a1[k]) + (a2[k] + a3[k]);
+    block_sums<K>(v, s);
+    __syncthreads();
 }
 
 // The K sums of v over all tiles of a case, in shared s[0..K-1] of the case's
@@ -107,30 +163,85 @@ __device__ __forceinline__ bool case_sums(T (&v)[K], int *counter, T *partials, 
     }
     __syncthreads();
     if (!is_last) return false;
-    // thread-strided in a fixed order with four independent accumulators (so
-    // the loads overlap instead of forming one dependent chain), then the
-    // block sum
-    T a1[K], a2[K], a3[K];
-#pragma unroll
-    for (int k = 0; k < K; k++) v[k] = a1[k] = a2[k] = a3[k] = 0;
-    int i = threadIdx.x;
-    for (; i + 3 * kTile < ntiles; i += 4 * kTile)
-#pragma unroll
-        for (int k = 0; k < K; k++) {
-            const T *p = part + (size_t)k * ntiles + i;
-            v[k] += __ldcg(p);
-            a1[k] += __ldcg(p + kTile);
-            a2[k] += __ldcg(p + 2 * kTile);
-            a3[k] += __ldcg(p + 3 * kTile);
-        }
-    for (; i < ntiles; i += kTile)
-#pragma unroll
-        for (int k = 0; k < K; k++) v[k] += __ldcg(&part[(size_t)k * ntiles + i]);
-#pragma unroll
-    for (int k = 0; k < K; k++) v[k] = (v[k] + a1[k]) + (a2[k] + a3[k]);
-    block_sums<K>(v, s);
-    __syncthreads();
+    partial_sums<K>(v, part, ntiles, s);
     return true;
+}
+
+// Sums of a launch whose blocks each take up to M of a case's tiles in turn (a
+// merged list), tile by tile in the order of case_sums: the same bits.  A block
+// pays its start (tile, case, scalars: three dependent trips to L2), its two
+// barriers, its fence and its count once for M tiles: an outer iteration with
+// the energy solve (256 cells a tile) at 77^3 took 3530 us and takes 3200.  The
+// FP32 flow solves (1024 cells a tile) did not gain by it.  After each tile
+// put_sums files its values; merged_sums ends the block as case_sums does, over
+// the partials of all `nsub` tiles of the case.  kSub: the most tiles a block
+// may take.
+template <class T> constexpr int kSumWidth = sizeof(T) == 4 ? kTile / 32 : kTile;
+template <int K, class T, int kSub> __device__ __forceinline__ T *sum_buf() {
+    __shared__ T buf[kSub * K * kSumWidth<T>];
+    return buf;
+}
+template <int K, int kSub> __device__ __forceinline__ void put_sums(float (&v)[K], int m) {
+    int k;
+    bool mine;
+    const float z = warp_sums<K>(v, threadIdx.x & 31, k, mine);
+    if (mine) sum_buf<K, float, kSub>()[(m * K + k) * kSumWidth<float> + (threadIdx.x >> 5)] = z;
+}
+template <int K, int kSub> __device__ __forceinline__ void put_sums(double (&v)[K], int m) {
+    double *buf = sum_buf<K, double, kSub>() + m * K * kSumWidth<double>;
+#pragma unroll
+    for (int k = 0; k < K; k++) buf[k * kSumWidth<double> + threadIdx.x] = v[k];
+}
+template <int K, class T, int kSub>
+__device__ __forceinline__ bool merged_sums(int nm, int *counter, T *partials, int tile0, int ntiles, int M, int nsub, T *s) {
+    __shared__ int is_last;
+    T *part = partials + (size_t)tile0 * M * kNPart;
+    const int at = ((int)blockIdx.x - tile0) * M, lane = threadIdx.x & 31;
+    T *buf = sum_buf<K, T, kSub>();
+    __syncthreads();
+    if (sizeof(T) == 8) {
+        // each value's tree by one warp, its sum left in the buffer's first entry
+        for (int q = threadIdx.x >> 5; q < nm * K; q += kTile / 32) {
+            const double x = tree_sum((const double *)buf + q * kSumWidth<T>);
+            if (lane == 0) buf[q * kSumWidth<T>] = (T)x;
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x < 32) {
+        for (int q = lane; q < nm * K; q += 32) {
+            T x = buf[q * kSumWidth<T>];
+            if (sizeof(T) == 4) {
+                x = (T)0 + x;
+#pragma unroll
+                for (int w = 1; w < kTile / 32; w++) x += buf[q * kSumWidth<T> + w];
+            }
+            __stcg(&part[(size_t)(q % K) * nsub + at + q / K], x);
+        }
+        __syncwarp();
+        if (lane == 0) {
+            __threadfence();
+            const bool last = atomicAdd(counter, 1) == ntiles - 1;
+            if (last) { *counter = 0; __threadfence(); }
+            is_last = last;
+        }
+    }
+    __syncthreads();
+    if (!is_last) return false;
+    T v[K];
+    partial_sums<K>(v, part, nsub, s);
+    return true;
+}
+
+// the tiles u of a block's tile t in a merged list, counted in nm, at most kSub
+#define FOR_SUBTILES(u, t, mg, nm, kSub)                                                               \
+    int nm = 0;                                                                                        \
+    for (Tile u{(t).c, (t).first, (kSub) == 1 ? (t).last : min((t).last, (t).first + (mg).rows), (t).pad}; nm < (kSub) && u.first < (t).last; \
+         u.first += (mg).rows, u.last = min((t).last, u.last + (mg).rows), nm++)
+// case_sums of a plain list (kSub 1) or merged_sums of a merged one
+template <int K, int kSub, class T>
+__device__ __forceinline__ bool tile_sums(T (&v)[K], int nm, int *counter, T *partials, int tile0, int ntiles, const Merge &mg, int ne, T *s) {
+    if constexpr (kSub == 1) return case_sums<K>(v, counter, partials, tile0, ntiles, s);
+    else return merged_sums<K, T, kSub>(nm, counter, partials, tile0, ntiles, mg.M, (ne + mg.rows - 1) / mg.rows, s);
 }
 
 // Start of a case's momentum solve from s[0..2] = sum b'^2 and s[3..5] =

@@ -182,9 +182,14 @@ struct CaseDev {
 // thread (1 for the kTile-entity lists, the solver tile shape for cellsv).
 struct Tile { int c, first, last, pad; };
 
+// A merged list's blocks: up to M tiles of `rows` entities, taken in turn.
+struct Merge { int M, rows; };
+constexpr int kMaxMerge = 4;            // most tiles a block takes (a shared buffer holds their values)
+
 // One work list per entity type, with each case's tile range for reductions.
 struct WorkList {
     int ntiles = 0;
+    Merge merge{1, 1 << 30};            // merged lists: see merged_sums (cfdl_device.cuh)
     Tile *d_tiles = nullptr;
     int *d_case_first = nullptr, *d_case_ntiles = nullptr;
     std::vector<Tile> h_tiles;
@@ -231,6 +236,7 @@ struct cfdl_ctx {
     int vec = cfdl::kVec;                // cells per thread in those tiles (autotuned)
     cfdl::WorkList cellsr;               // tiles of the FP64 passes whose shape goes by the case's size (rows_per_thread)
     cfdl::WorkList cellse;               // tiles of the energy solve (kTile*en_vec cells)
+    cfdl::WorkList cellsem;              // the same tiles, merged
     cfdl::WorkList facesv;               // wide face tiles (kTile*kFaceVec faces) for face reductions
     int en_vec = 1;                      // cells per thread in those tiles (autotuned with the energy equation)
     int last_iters_m = 0, last_iters_p = 0, last_iters_e = 0;   // previous inner iteration counts (poll scheduling)
@@ -414,7 +420,7 @@ int solve_pressure_amg(cfdl_ctx *ctx);
 int solve_pressure_mixed(cfdl_ctx *ctx);
 void free_worklist(WorkList &wl);
 int build_worklist(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &sizes, int tile = kTile);
-int build_worklist(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &sizes, const std::vector<int> &tiles);
+int build_worklist(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &sizes, const std::vector<int> &tiles, int per_thread = 0);
 int read_stats(cfdl_ctx *ctx, int c, cfdl_stats *st);
 int poll_kind(cfdl_ctx *ctx, int kind, int *maxit);
 int poll_chunk(int done, int expected);

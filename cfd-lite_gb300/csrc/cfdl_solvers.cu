@@ -165,6 +165,8 @@ template <int NC> __device__ __forceinline__ bool lanes_active(const KLanes *L) 
 // one 16-byte load instead of three: its SpMV was bound by the latency and the
 // number of its loads (A ph 67.7 -> 53 us at 128^3, A sh 63.2 -> 49).
 template <class T, int NC> constexpr bool kInter = sizeof(T) == 4 && NC == 3;
+// most tiles a block takes in turn: the energy solve's small tiles are merged
+template <class T, int NC> constexpr int kMaxSub = NC == 1 ? kMaxMerge : 1;
 
 // (A x)_i of the three components in FP32, x interleaved: d x_i - sum_k c_k x_k
 // in slot order.  Index and coefficient loads do not wait for one another.
@@ -260,33 +262,38 @@ __global__ void __launch_bounds__(kTile) k_mom_p(const CaseDev *__restrict__ cas
 
 // v = A ph; alpha = rho / (rh, v)
 template <class T, int NC, bool k16 = false>
-__global__ void __launch_bounds__(kTile, 5) k_mom_v(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles,
-                                                 const int *__restrict__ cfirst, const int *__restrict__ cnt, T *partials) {
+__global__ void __launch_bounds__(kTile, sizeof(T) == 8 && NC == 1 ? 4 : 5) k_mom_v(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles,
+                                                 const int *__restrict__ cfirst, const int *__restrict__ cnt, T *partials, Merge mg) {
     CFDL_PDL_WAIT();
     TILE_HEAD
     const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     KLanes *L = lanes<NC>(S);
     if (!lanes_active<NC>(L)) return;
     const MomVec<T> M = mom_vec<T, NC>(C);
-    T v[NC];
     int act[NC];
 #pragma unroll
-    for (int q = 0; q < NC; q++) { v[q] = 0; act[q] = L->active[q]; }
-    FOR_CELLS(t) {
-        T y[NC], rh[NC];   // one pass over the row for the components
-        if constexpr (kInter<T, NC>) row3<k16>(C, (const float4 *)M.ph, i, y);
-        else ell_row<NC, T>(C.hf_nb, M.a, M.ap[i], M.ph, ne, ne, C.W, i, y);
+    for (int q = 0; q < NC; q++) act[q] = L->active[q];
+    T v[NC];
+    FOR_SUBTILES(u, t, mg, nm, (kMaxSub<T, NC>)) {
 #pragma unroll
-        for (int q = 0; q < NC; q++) rh[q] = act[q] ? M.rh[q * ne + i] : (T)0;   // loads before the stores
+        for (int q = 0; q < NC; q++) v[q] = 0;
+        FOR_CELLS(u) {
+            T y[NC], rh[NC];   // one pass over the row for the components
+            if constexpr (kInter<T, NC>) row3<k16>(C, (const float4 *)M.ph, i, y);
+            else ell_row<NC, T>(C.hf_nb, M.a, M.ap[i], M.ph, ne, ne, C.W, i, y);
 #pragma unroll
-        for (int q = 0; q < NC; q++) {
-            if (!act[q]) continue;
-            M.v[q * ne + i] = y[q];
-            v[q] += rh[q] * y[q];
+            for (int q = 0; q < NC; q++) rh[q] = act[q] ? M.rh[q * ne + i] : (T)0;   // loads before the stores
+#pragma unroll
+            for (int q = 0; q < NC; q++) {
+                if (!act[q]) continue;
+                M.v[q * ne + i] = y[q];
+                v[q] += rh[q] * y[q];
+            }
         }
+        if (kMaxSub<T, NC> > 1) put_sums<NC, kMaxSub<T, NC>>(v, nm);
     }
     __shared__ T s[NC];
-    if (case_sums<NC>(v, &C.counters[CNT_M2], partials, tile0, ntiles, s)) {
+    if (tile_sums<NC, kMaxSub<T, NC>>(v, nm, &C.counters[CNT_M2], partials, tile0, ntiles, mg, ne, s)) {
         if (threadIdx.x < NC && L->active[threadIdx.x]) {   // one thread per component
             const int q = threadIdx.x;
             const double sq = (double)s[q];
@@ -300,56 +307,62 @@ __global__ void __launch_bounds__(kTile, 5) k_mom_v(const CaseDev *__restrict__ 
 // s = r - alpha v; sh = s / ap; early exit when ||s|| <= tol
 template <class T, int NC>
 __global__ void __launch_bounds__(kTile) k_mom_s(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles,
-                                                 const int *__restrict__ cfirst, const int *__restrict__ cnt, T *partials) {
+                                                 const int *__restrict__ cfirst, const int *__restrict__ cnt, T *partials, Merge mg) {
     CFDL_PDL_WAIT();
     TILE_HEAD
     const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     KLanes *L = lanes<NC>(S);
     if (!lanes_active<NC>(L)) return;
     const MomVec<T> M = mom_vec<T, NC>(C);
-    T v[NC], al[NC];
+    T al[NC];
     int act[NC];
 #pragma unroll
-    for (int q = 0; q < NC; q++) { v[q] = 0; act[q] = L->active[q]; al[q] = (T)L->alpha[q]; }
-    FOR_CELLS(t) {
-        const T rap = M.rap[i];
-        if (sizeof(T) == 4) {
-            // FP32: the row's loads, every component's, before its stores
-            // (36 -> 27 us a launch at 128^3; the FP64 form measured slower
-            // this way, 63 -> 68 us, and keeps one component at a time)
-            T rr[NC], vv[NC];
+    for (int q = 0; q < NC; q++) { act[q] = L->active[q]; al[q] = (T)L->alpha[q]; }
+    T v[NC];
+    FOR_SUBTILES(u, t, mg, nm, (kMaxSub<T, NC>)) {
 #pragma unroll
-            for (int q = 0; q < NC; q++) {
-                rr[q] = act[q] ? M.r[q * ne + i] : (T)0;
-                vv[q] = act[q] ? M.v[q * ne + i] : (T)0;
-            }
-            T sh[NC];
+        for (int q = 0; q < NC; q++) v[q] = 0;
+        FOR_CELLS(u) {
+            const T rap = M.rap[i];
+            if (sizeof(T) == 4) {
+                // FP32: the row's loads, every component's, before its stores
+                // (36 -> 27 us a launch at 128^3; the FP64 form measured slower
+                // this way, 63 -> 68 us, and keeps one component at a time)
+                T rr[NC], vv[NC];
 #pragma unroll
-            for (int q = 0; q < NC; q++) {
-                sh[q] = 0;
-                if (!act[q]) continue;
-                const int j = q * ne + i;
-                const T sv = rr[q] - al[q] * vv[q];
-                M.s[j] = sv;
-                sh[q] = sv * rap;
-                if (!kInter<T, NC>) M.sh[j] = sh[q];
-                v[q] += sv * sv;
-            }
-            if (kInter<T, NC>) ((float4 *)M.sh)[i] = make_float4(sh[0], sh[1 % NC], sh[2 % NC], 0.f);
-        } else {
+                for (int q = 0; q < NC; q++) {
+                    rr[q] = act[q] ? M.r[q * ne + i] : (T)0;
+                    vv[q] = act[q] ? M.v[q * ne + i] : (T)0;
+                }
+                T sh[NC];
 #pragma unroll
-            for (int q = 0; q < NC; q++) {
-                if (!act[q]) continue;
-                const int j = q * ne + i;
-                const T sv = M.r[j] - al[q] * M.v[j];
-                M.s[j] = sv;
-                M.sh[j] = sv * rap;
-                v[q] += sv * sv;
+                for (int q = 0; q < NC; q++) {
+                    sh[q] = 0;
+                    if (!act[q]) continue;
+                    const int j = q * ne + i;
+                    const T sv = rr[q] - al[q] * vv[q];
+                    M.s[j] = sv;
+                    sh[q] = sv * rap;
+                    if (!kInter<T, NC>) M.sh[j] = sh[q];
+                    v[q] += sv * sv;
+                }
+                if (kInter<T, NC>) ((float4 *)M.sh)[i] = make_float4(sh[0], sh[1 % NC], sh[2 % NC], 0.f);
+            } else {
+#pragma unroll
+                for (int q = 0; q < NC; q++) {
+                    if (!act[q]) continue;
+                    const int j = q * ne + i;
+                    const T sv = M.r[j] - al[q] * M.v[j];
+                    M.s[j] = sv;
+                    M.sh[j] = sv * rap;
+                    v[q] += sv * sv;
+                }
             }
         }
+        if (kMaxSub<T, NC> > 1) put_sums<NC, kMaxSub<T, NC>>(v, nm);
     }
     __shared__ T s[NC];
-    if (case_sums<NC>(v, &C.counters[CNT_M3], partials, tile0, ntiles, s)) {
+    if (tile_sums<NC, kMaxSub<T, NC>>(v, nm, &C.counters[CNT_M3], partials, tile0, ntiles, mg, ne, s)) {
         const int q = threadIdx.x;
         if (q < NC && L->active[q]) L->half[q] = sqrt((double)s[q]) <= L->tol[q];
     }
@@ -357,35 +370,40 @@ __global__ void __launch_bounds__(kTile) k_mom_s(const CaseDev *__restrict__ cas
 
 // t = A sh; omega = (t,s)/(t,t)
 template <class T, int NC, bool k16 = false>
-__global__ void __launch_bounds__(kTile, 5) k_mom_t(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles,
-                                                 const int *__restrict__ cfirst, const int *__restrict__ cnt, T *partials) {
+__global__ void __launch_bounds__(kTile, sizeof(T) == 8 && NC == 1 ? 4 : 5) k_mom_t(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles,
+                                                 const int *__restrict__ cfirst, const int *__restrict__ cnt, T *partials, Merge mg) {
     CFDL_PDL_WAIT();
     TILE_HEAD
     const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     KLanes *L = lanes<NC>(S);
     if (!lanes_active<NC>(L)) return;
     const MomVec<T> M = mom_vec<T, NC>(C);
-    T v[2 * NC];
     int act[NC];
 #pragma unroll
-    for (int q = 0; q < NC; q++) { v[q] = v[NC + q] = 0; act[q] = L->active[q] && !L->half[q]; }
-    FOR_CELLS(t) {
-        T y[NC], sv[NC];
-        if constexpr (kInter<T, NC>) row3<k16>(C, (const float4 *)M.sh, i, y);
-        else ell_row<NC, T>(C.hf_nb, M.a, M.ap[i], M.sh, ne, ne, C.W, i, y);
+    for (int q = 0; q < NC; q++) act[q] = L->active[q] && !L->half[q];
+    T v[2 * NC];
+    FOR_SUBTILES(u, t, mg, nm, (kMaxSub<T, NC>)) {
 #pragma unroll
-        for (int q = 0; q < NC; q++) sv[q] = act[q] ? M.s[q * ne + i] : (T)0;   // loads before the stores
+        for (int q = 0; q < 2 * NC; q++) v[q] = 0;
+        FOR_CELLS(u) {
+            T y[NC], sv[NC];
+            if constexpr (kInter<T, NC>) row3<k16>(C, (const float4 *)M.sh, i, y);
+            else ell_row<NC, T>(C.hf_nb, M.a, M.ap[i], M.sh, ne, ne, C.W, i, y);
 #pragma unroll
-        for (int q = 0; q < NC; q++) {
-            if (!act[q]) continue;
-            const int j = q * ne + i;
-            M.t[j] = y[q];
-            v[q] += y[q] * sv[q];
-            v[NC + q] += y[q] * y[q];
+            for (int q = 0; q < NC; q++) sv[q] = act[q] ? M.s[q * ne + i] : (T)0;   // loads before the stores
+#pragma unroll
+            for (int q = 0; q < NC; q++) {
+                if (!act[q]) continue;
+                const int j = q * ne + i;
+                M.t[j] = y[q];
+                v[q] += y[q] * sv[q];
+                v[NC + q] += y[q] * y[q];
+            }
         }
+        if (kMaxSub<T, NC> > 1) put_sums<2 * NC, kMaxSub<T, NC>>(v, nm);
     }
     __shared__ T s[2 * NC];
-    if (case_sums<2 * NC>(v, &C.counters[CNT_M4], partials, tile0, ntiles, s)) {
+    if (tile_sums<2 * NC, kMaxSub<T, NC>>(v, nm, &C.counters[CNT_M4], partials, tile0, ntiles, mg, ne, s)) {
         const int q = threadIdx.x;
         if (q < NC && L->active[q]) {
             const double ts = (double)s[q], tt = (double)s[NC + q];
@@ -397,67 +415,73 @@ __global__ void __launch_bounds__(kTile, 5) k_mom_t(const CaseDev *__restrict__ 
 // x += alpha ph + omega sh; r = s - omega t; rho' = (rh, r); beta
 template <class T, int NC>
 __global__ void __launch_bounds__(kTile, 4) k_mom_x(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles,
-                                                 const int *__restrict__ cfirst, const int *__restrict__ cnt, T *partials) {
+                                                 const int *__restrict__ cfirst, const int *__restrict__ cnt, T *partials, Merge mg) {
     CFDL_PDL_WAIT();
     TILE_HEAD
     const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     KLanes *L = lanes<NC>(S);
     if (!lanes_active<NC>(L)) return;
     const MomVec<T> M = mom_vec<T, NC>(C);
-    T v[2 * NC], al[NC], om[NC];
+    T al[NC], om[NC];
     int act[NC];
 #pragma unroll
     for (int q = 0; q < NC; q++) {
-        v[q] = v[NC + q] = 0; act[q] = L->active[q]; al[q] = (T)L->alpha[q]; om[q] = (T)L->omega[q];
+        act[q] = L->active[q]; al[q] = (T)L->alpha[q]; om[q] = (T)L->omega[q];
     }
-    if (sizeof(T) == 8 && NC == 3) {
-        // FP64: one component's loads at a time; all eighteen together spilled
-        // 200 bytes under four CTAs per SM (128^3: an outer iteration 0.4%)
-        FOR_CELLS(t) {
+    T v[2 * NC];
+    FOR_SUBTILES(u, t, mg, nm, (kMaxSub<T, NC>)) {
+#pragma unroll
+        for (int q = 0; q < 2 * NC; q++) v[q] = 0;
+        if (sizeof(T) == 8 && NC == 3) {
+            // FP64: one component's loads at a time; all eighteen together spilled
+            // 200 bytes under four CTAs per SM (128^3: an outer iteration 0.4%)
+            FOR_CELLS(u) {
+#pragma unroll
+                for (int q = 0; q < NC; q++) {
+                    if (!act[q]) continue;
+                    const int j = q * ne + i;
+                    const T xv = M.x[q][i], ph = M.ph[j], sh = M.sh[j], sv = M.s[j], rh = M.rh[j];
+                    const T tv = om[q] != (T)0 ? M.t[j] : (T)0;
+                    M.x[q][i] = xv + al[q] * ph + om[q] * sh;
+                    const T r = om[q] == (T)0 ? sv : sv - om[q] * tv;
+                    M.r[j] = r;
+                    v[q] += r * r;
+                    v[NC + q] += rh * r;
+                }
+            }
+        } else
+        FOR_CELLS(u) {
+            // the row's loads, every component's, before its stores
+            T xv[NC], ph[NC], sh[NC], sv[NC], tv[NC], rh[NC];
+#pragma unroll
+            for (int q = 0; q < NC; q++) {
+                const int j = q * ne + i;
+                xv[q] = ph[q] = sh[q] = sv[q] = tv[q] = rh[q] = 0;
+                if (!act[q]) continue;
+                xv[q] = M.x[q][i]; sv[q] = M.s[j]; rh[q] = M.rh[j];
+                if (!kInter<T, NC>) { ph[q] = M.ph[j]; sh[q] = M.sh[j]; }
+                if (om[q] != (T)0) tv[q] = M.t[j];
+            }
+            if constexpr (kInter<T, NC>) {
+                const float4 a = ((const float4 *)M.ph)[i], b = ((const float4 *)M.sh)[i];
+                ph[0] = a.x; ph[1] = a.y; ph[2] = a.z;
+                sh[0] = b.x; sh[1] = b.y; sh[2] = b.z;
+            }
 #pragma unroll
             for (int q = 0; q < NC; q++) {
                 if (!act[q]) continue;
                 const int j = q * ne + i;
-                const T xv = M.x[q][i], ph = M.ph[j], sh = M.sh[j], sv = M.s[j], rh = M.rh[j];
-                const T tv = om[q] != (T)0 ? M.t[j] : (T)0;
-                M.x[q][i] = xv + al[q] * ph + om[q] * sh;
-                const T r = om[q] == (T)0 ? sv : sv - om[q] * tv;
+                M.x[q][i] = xv[q] + al[q] * ph[q] + om[q] * sh[q];
+                const T r = om[q] == (T)0 ? sv[q] : sv[q] - om[q] * tv[q];
                 M.r[j] = r;
                 v[q] += r * r;
-                v[NC + q] += rh * r;
+                v[NC + q] += rh[q] * r;
             }
         }
-    } else
-    FOR_CELLS(t) {
-        // the row's loads, every component's, before its stores
-        T xv[NC], ph[NC], sh[NC], sv[NC], tv[NC], rh[NC];
-#pragma unroll
-        for (int q = 0; q < NC; q++) {
-            const int j = q * ne + i;
-            xv[q] = ph[q] = sh[q] = sv[q] = tv[q] = rh[q] = 0;
-            if (!act[q]) continue;
-            xv[q] = M.x[q][i]; sv[q] = M.s[j]; rh[q] = M.rh[j];
-            if (!kInter<T, NC>) { ph[q] = M.ph[j]; sh[q] = M.sh[j]; }
-            if (om[q] != (T)0) tv[q] = M.t[j];
-        }
-        if constexpr (kInter<T, NC>) {
-            const float4 a = ((const float4 *)M.ph)[i], b = ((const float4 *)M.sh)[i];
-            ph[0] = a.x; ph[1] = a.y; ph[2] = a.z;
-            sh[0] = b.x; sh[1] = b.y; sh[2] = b.z;
-        }
-#pragma unroll
-        for (int q = 0; q < NC; q++) {
-            if (!act[q]) continue;
-            const int j = q * ne + i;
-            M.x[q][i] = xv[q] + al[q] * ph[q] + om[q] * sh[q];
-            const T r = om[q] == (T)0 ? sv[q] : sv[q] - om[q] * tv[q];
-            M.r[j] = r;
-            v[q] += r * r;
-            v[NC + q] += rh[q] * r;
-        }
+        if (kMaxSub<T, NC> > 1) put_sums<2 * NC, kMaxSub<T, NC>>(v, nm);
     }
     __shared__ T s[2 * NC];
-    if (case_sums<2 * NC>(v, &C.counters[CNT_M5], partials, tile0, ntiles, s)) {
+    if (tile_sums<2 * NC, kMaxSub<T, NC>>(v, nm, &C.counters[CNT_M5], partials, tile0, ntiles, mg, ne, s)) {
         const int q = threadIdx.x;
         if (q < NC && L->active[q]) {
             const int cap = C.solve_mode == 0 ? C.nit : C.tight_maxit;
@@ -725,7 +749,7 @@ static int max_cap(cfdl_ctx *ctx) {
 
 static void mom_init(cfdl_ctx *ctx) { CFDL_LAUNCH("k_mom_init", k_mom_init, cellsv, RED); }
 
-#define RED32 ctx->cellsv.d_case_first, ctx->cellsv.d_case_ntiles, (float *)ctx->d_partials
+#define RED32 ctx->cellsv.d_case_first, ctx->cellsv.d_case_ntiles, (float *)ctx->d_partials, ctx->cellsv.merge
 
 void mom_iter(cfdl_ctx *ctx) {
     if (ctx->cases[0]->cfg.precision >= 2) {
@@ -741,10 +765,10 @@ void mom_iter(cfdl_ctx *ctx) {
         return;
     }
     CFDL_LAUNCH("k_mom_p", (k_mom_p<double, 3>), cellsv);
-    CFDL_LAUNCH("k_mom_v", (k_mom_v<double, 3>), cellsv, RED);
-    CFDL_LAUNCH("k_mom_s", (k_mom_s<double, 3>), cellsv, RED);
-    CFDL_LAUNCH("k_mom_t", (k_mom_t<double, 3>), cellsv, RED);
-    CFDL_LAUNCH("k_mom_x", (k_mom_x<double, 3>), cellsv, RED);
+    CFDL_LAUNCH("k_mom_v", (k_mom_v<double, 3>), cellsv, RED, ctx->cellsv.merge);
+    CFDL_LAUNCH("k_mom_s", (k_mom_s<double, 3>), cellsv, RED, ctx->cellsv.merge);
+    CFDL_LAUNCH("k_mom_t", (k_mom_t<double, 3>), cellsv, RED, ctx->cellsv.merge);
+    CFDL_LAUNCH("k_mom_x", (k_mom_x<double, 3>), cellsv, RED, ctx->cellsv.merge);
 }
 
 // Jacobi-preconditioned BiCGStab on the energy system, with the momentum
@@ -777,21 +801,22 @@ void energy_finish(cfdl_ctx *ctx) {
 
 // one BiCGStab iteration of the energy solve (one right-hand side; FP64, or
 // FP32 on the correction for precision >= 2)
-#define REDE32 ctx->cellse.d_case_first, ctx->cellse.d_case_ntiles, (float *)ctx->d_partials
+#define REDEM ctx->cellsem.d_case_first, ctx->cellsem.d_case_ntiles, ctx->d_partials, ctx->cellsem.merge
+#define REDEM32 ctx->cellsem.d_case_first, ctx->cellsem.d_case_ntiles, (float *)ctx->d_partials, ctx->cellsem.merge
 void energy_iter(cfdl_ctx *ctx) {
     if (ctx->cases[0]->cfg.precision >= 2) {
         CFDL_LAUNCH("k_en_p", (k_mom_p<float, 1>), cellse);
-        CFDL_LAUNCH("k_en_v", (k_mom_v<float, 1>), cellse, REDE32);
-        CFDL_LAUNCH("k_en_s", (k_mom_s<float, 1>), cellse, REDE32);
-        CFDL_LAUNCH("k_en_t", (k_mom_t<float, 1>), cellse, REDE32);
-        CFDL_LAUNCH("k_en_x", (k_mom_x<float, 1>), cellse, REDE32);
+        CFDL_LAUNCH("k_en_v", (k_mom_v<float, 1>), cellsem, REDEM32);
+        CFDL_LAUNCH("k_en_s", (k_mom_s<float, 1>), cellsem, REDEM32);
+        CFDL_LAUNCH("k_en_t", (k_mom_t<float, 1>), cellsem, REDEM32);
+        CFDL_LAUNCH("k_en_x", (k_mom_x<float, 1>), cellsem, REDEM32);
         return;
     }
     CFDL_LAUNCH("k_en_p", (k_mom_p<double, 1>), cellse);
-    CFDL_LAUNCH("k_en_v", (k_mom_v<double, 1>), cellse, REDE);
-    CFDL_LAUNCH("k_en_s", (k_mom_s<double, 1>), cellse, REDE);
-    CFDL_LAUNCH("k_en_t", (k_mom_t<double, 1>), cellse, REDE);
-    CFDL_LAUNCH("k_en_x", (k_mom_x<double, 1>), cellse, REDE);
+    CFDL_LAUNCH("k_en_v", (k_mom_v<double, 1>), cellsem, REDEM);
+    CFDL_LAUNCH("k_en_s", (k_mom_s<double, 1>), cellsem, REDEM);
+    CFDL_LAUNCH("k_en_t", (k_mom_t<double, 1>), cellsem, REDEM);
+    CFDL_LAUNCH("k_en_x", (k_mom_x<double, 1>), cellsem, REDEM);
 }
 
 // the end of the momentum solve: precision 2 applies its FP32 correction
