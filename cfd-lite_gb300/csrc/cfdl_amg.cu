@@ -103,16 +103,16 @@ __device__ __forceinline__ double cg_aq_rows(const LP<double> &P, const double *
     }
     return v;
 }
-// CG's (r, z), two rows per step
-template <class T>
-__device__ __forceinline__ T cg_rz_rows(const T *r, const T *z, const Tile &t) {
-    T v = 0;
+// CG's (r, z), two rows per step; its roundings spelled out (the split form
+// has to have them)
+__device__ __forceinline__ float cg_rz_rows(const float *r, const float *z, const Tile &t) {
+    float v = 0;
     FOR_ROW_PAIRS(t) {
-        T r0 = 0, z0 = 0, r1 = 0, z1 = 0;
+        float r0 = 0, z0 = 0, r1 = 0, z1 = 0;
         if (ok0) { r0 = r[i0]; z0 = z[i0]; }
         if (ok1) { r1 = r[i1]; z1 = z[i1]; }
-        if (ok0) v += r0 * z0;
-        if (ok1) v += r1 * z1;
+        if (ok0) v = __fmaf_rn(r0, z0, v);
+        if (ok1) v = __fadd_rn(v, __fmul_rn(r1, z1));
     }
     return v;
 }
@@ -136,8 +136,8 @@ __device__ __forceinline__ T cg_x_rows(T *x, const T *p, T *r, const T *q, T a, 
         T x0 = 0, p0 = 0, r0 = 0, q0 = 0, x1 = 0, p1 = 0, r1 = 0, q1 = 0;
         if (ok0) { x0 = x[i0]; p0 = p[i0]; r0 = r[i0]; q0 = q[i0]; }
         if (ok1) { x1 = x[i1]; p1 = p[i1]; r1 = r[i1]; q1 = q[i1]; }
-        if (ok0) { x[i0] = x0 + a * p0; const T rr = r0 - a * q0; r[i0] = rr; v += rr * rr; }
-        if (ok1) { x[i1] = x1 + a * p1; const T rr = r1 - a * q1; r[i1] = rr; v += rr * rr; }
+        if (ok0) { x[i0] = x0 + a * p0; const T rr = r0 - a * q0; r[i0] = rr; v = fma_rn(rr, rr, v); }
+        if (ok1) { x[i1] = x1 + a * p1; const T rr = r1 - a * q1; r[i1] = rr; v = fma_rn(rr, rr, v); }
     }
     return v;
 }
@@ -289,6 +289,36 @@ __device__ __forceinline__ float2 pair_amul(const LP<float> &P, const float *x, 
 #pragma unroll
     for (int k = 1; k < W; k++) { s.x = __fmaf_rn(-c[0][k], v[0][k], s.x); s.y = __fmaf_rn(-c[1][k], v[1][k], s.y); }
     return s;
+}
+// one row of A x, with pair_amul's roundings
+template <int W, bool k16, bool kGuard>
+__device__ __forceinline__ float row_amul(const LP<float> &P, const float *x, int i) {
+    int j[W];
+    float c[W], v[W];
+#pragma unroll
+    for (int k = 0; k < W; k++) {
+        int jj = -1;
+        float a = 0.f;
+        if (!kGuard || k < P.W) {
+            if (k16) { const int d = P.nb16[k * P.ld + i]; jj = d == (int)kNb16None ? -1 : i + d; }
+            else jj = P.nb[k * P.n + i];
+            a = P.a[k * P.ld + i];
+        }
+        const bool ok = (unsigned)jj < (unsigned)P.n;
+        j[k] = ok ? jj : i;
+        c[k] = ok ? a : 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k < W; k++) v[k] = x[j[k]];
+    float s = __fmaf_rn(P.dg[i], x[i], -__fmul_rn(c[0], v[0]));
+#pragma unroll
+    for (int k = 1; k < W; k++) s = __fmaf_rn(-c[k], v[k], s);
+    return s;
+}
+template <bool k16> __device__ __forceinline__ float row_amul_mesh(const LP<float> &P, const float *x, int i) {
+    if (P.W == 6) return row_amul<6, k16, false>(P, x, i);
+    if (P.W == 4) return row_amul<4, k16, false>(P, x, i);
+    return row_amul<kMaxW, k16, true>(P, x, i);
 }
 template <bool k16, bool kRd = false> __device__ __forceinline__ float2 pair_offsum_mesh(const LP<float> &P, const float *x, int i) {
     if (P.W == 6) return pair_offsum<6, k16, false, kRd>(P, x, i);
@@ -1140,6 +1170,7 @@ __global__ void __launch_bounds__(kTile) k_apc_init(const CaseDev *__restrict__ 
 }
 
 // beta = (r,z)/(r,z)_old (0 on the first iteration)
+template <bool kSpl>
 __global__ void __launch_bounds__(kTile) k_apc_rz(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles,
                                                   const int *__restrict__ cfirst, const int *__restrict__ cnt, double *partials) {
     CFDL_PDL_WAIT();
@@ -1148,12 +1179,24 @@ __global__ void __launch_bounds__(kTile) k_apc_rz(const CaseDev *__restrict__ ca
     SolveScalars *S = C.sc;
     const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     if (!S->active_p) return;
-    // one row per step in FP64: the paired form (cg_rz_rows) measured slower
-    // here (21.4 against 18.8 us a launch at 128^3)
-    double v[1] = {0.0};
-    FOR_CELLS(t) v[0] += C.kr[i] * C.ks[i];
     __shared__ double s[1];
-    if (case_sums<1>(v, &C.counters[CNT_A1], partials, tile0, ntiles, s)) {
+    bool last;
+    if constexpr (kSpl) {
+        double a[1] = {0}, b[1] = {0};
+        const int i = split_row(t);
+        if (i < t.last) {
+            a[0] = C.kr[i];
+            b[0] = C.ks[i];
+        }
+        last = split_sums<1>(a, b, &C.counters[CNT_A1], partials, tile0, ntiles, s);
+    } else {
+        // one row per step in FP64: the paired form (cg_rz_rows) measured slower
+        // here (21.4 against 18.8 us a launch at 128^3)
+        double v[1] = {0.0};
+        FOR_CELLS(t) v[0] += C.kr[i] * C.ks[i];
+        last = case_sums<1>(v, &C.counters[CNT_A1], partials, tile0, ntiles, s);
+    }
+    if (last) {
         if (threadIdx.x == 0) {
             S->beta_p = S->iters_p == 0 || S->rz == 0.0 ? 0.0 : s[0] / S->rz;
             S->rz = s[0];
@@ -1173,6 +1216,7 @@ __global__ void __launch_bounds__(kTile) k_apc_p(const CaseDev *__restrict__ cas
 }
 
 // q = A p; alpha = rz / (p, q)
+template <bool kSpl>
 __global__ void __launch_bounds__(kTile) k_apc_q(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles,
                                                  const int *__restrict__ cfirst, const int *__restrict__ cnt, double *partials) {
     CFDL_PDL_WAIT();
@@ -1181,9 +1225,22 @@ __global__ void __launch_bounds__(kTile) k_apc_q(const CaseDev *__restrict__ cas
     SolveScalars *S = C.sc;
     const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     if (!S->active_p) return;
-    double v[1] = {cg_aq_rows(level<double>(C, 0), C.kp, C.kv, t)};
     __shared__ double s[1];
-    if (case_sums<1>(v, &C.counters[CNT_A2], partials, tile0, ntiles, s)) {
+    bool last;
+    if constexpr (kSpl) {
+        double a[1] = {0}, b[1] = {0};
+        const int i = split_row(t);
+        if (i < t.last) {
+            b[0] = amul<double>(level<double>(C, 0), C.kp, i);
+            a[0] = C.kp[i];
+            C.kv[i] = b[0];
+        }
+        last = split_sums<1>(a, b, &C.counters[CNT_A2], partials, tile0, ntiles, s);
+    } else {
+        double v[1] = {cg_aq_rows(level<double>(C, 0), C.kp, C.kv, t)};
+        last = case_sums<1>(v, &C.counters[CNT_A2], partials, tile0, ntiles, s);
+    }
+    if (last) {
         if (threadIdx.x == 0) {
             if (!(s[0] > 0.0) || !isfinite(s[0])) {
                 // runs only while ||r|| is above the tolerance, where p.Ap > 0 for the SPD system
@@ -1196,6 +1253,7 @@ __global__ void __launch_bounds__(kTile) k_apc_q(const CaseDev *__restrict__ cas
 }
 
 // x += alpha p; r -= alpha q; ||r||
+template <bool kSpl>
 __global__ void __launch_bounds__(kTile) k_apc_x(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles,
                                                  const int *__restrict__ cfirst, const int *__restrict__ cnt, double *partials) {
     CFDL_PDL_WAIT();
@@ -1204,18 +1262,31 @@ __global__ void __launch_bounds__(kTile) k_apc_x(const CaseDev *__restrict__ cas
     SolveScalars *S = C.sc;
     const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     if (!S->active_p) return;
-    // one row per step in FP64: the paired form (cg_x_rows, 48 registers
-    // against 32) measured slower here (31.9 against 28.5 us a launch)
-    double v[1] = {0};
-    FOR_CELLS(t) {
-        const double a = S->alpha_p;
-        C.phic[i] = C.phic[i] + a * C.kp[i];
-        const double r = C.kr[i] - a * C.kv[i];
-        C.kr[i] = r;
-        v[0] += r * r;
-    }
     __shared__ double s[1];
-    if (case_sums<1>(v, &C.counters[CNT_A3], partials, tile0, ntiles, s)) {
+    bool last;
+    if constexpr (kSpl) {
+        double a[1] = {0}, b[1] = {0};
+        const int i = split_row(t);
+        if (i < t.last) {
+            const double al = S->alpha_p, x = C.phic[i], p = C.kp[i], r = C.kr[i] - al * C.kv[i];
+            C.phic[i] = x + al * p;
+            C.kr[i] = a[0] = b[0] = r;
+        }
+        last = split_sums<1>(a, b, &C.counters[CNT_A3], partials, tile0, ntiles, s);
+    } else {
+        // one row per step in FP64: the paired form (cg_x_rows, 48 registers
+        // against 32) measured slower here (31.9 against 28.5 us a launch)
+        double v[1] = {0};
+        FOR_CELLS(t) {
+            const double a = S->alpha_p;
+            C.phic[i] = C.phic[i] + a * C.kp[i];
+            const double r = C.kr[i] - a * C.kv[i];
+            C.kr[i] = r;
+            v[0] += r * r;
+        }
+        last = case_sums<1>(v, &C.counters[CNT_A3], partials, tile0, ntiles, s);
+    }
+    if (last) {
         if (threadIdx.x == 0) {
             const int cap = C.solve_mode == 0 ? C.nit : C.tight_maxit;
             const double rn = sqrt(s[0]);
@@ -1658,6 +1729,8 @@ template <class T> static void vcycle(cfdl_ctx *ctx) {
 void launch_pc_mean(cfdl_ctx *ctx);
 
 #define RED ctx->cellsv.d_case_first, ctx->cellsv.d_case_ntiles, ctx->d_partials
+#define REDS ctx->cellss.d_case_first, ctx->cellss.d_case_ntiles, ctx->d_partials
+#define REDS32 ctx->cellss.d_case_first, ctx->cellss.d_case_ntiles, (float *)ctx->d_partials
 #define RED32 ctx->cellsv.d_case_first, ctx->cellsv.d_case_ntiles, (float *)ctx->d_partials
 
 // What the pressure solve needs of its matrix, once the matrix exists: the
@@ -1679,10 +1752,17 @@ void apc_init(cfdl_ctx *ctx) {
 // one preconditioned CG iteration
 void apc_iter(cfdl_ctx *ctx) {
     vcycle<double>(ctx);
-    ALAUNCH("k_apc_rz", k_apc_rz, ctx->cellsv, RED);
+    if (ctx->cellss.ntiles) {
+        ALAUNCH("k_apc_rz", k_apc_rz<true>, ctx->cellss, REDS);
+        ALAUNCH("k_apc_p", k_apc_p, ctx->cells);
+        ALAUNCH("k_apc_q", k_apc_q<true>, ctx->cellss, REDS);
+        ALAUNCH("k_apc_x", k_apc_x<true>, ctx->cellss, REDS);
+        return;
+    }
+    ALAUNCH("k_apc_rz", k_apc_rz<false>, ctx->cellsv, RED);
     ALAUNCH("k_apc_p", k_apc_p, ctx->cellsv);
-    ALAUNCH("k_apc_q", k_apc_q, ctx->cellsv, RED);
-    ALAUNCH("k_apc_x", k_apc_x, ctx->cellsv, RED);
+    ALAUNCH("k_apc_q", k_apc_q<false>, ctx->cellsv, RED);
+    ALAUNCH("k_apc_x", k_apc_x<false>, ctx->cellsv, RED);
 }
 
 int solve_pressure_amg(cfdl_ctx *ctx) {
@@ -1782,6 +1862,7 @@ __global__ void __launch_bounds__(kTile) k_mx_jacobi(const CaseDev *__restrict__
     FOR_CELLS(t) C.fz[i] = C.fr[i] * C.frap_p[i];
 }
 
+template <bool kSpl>
 __global__ void __launch_bounds__(kTile) k_mx_rz(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles,
                                                  const int *__restrict__ cfirst, const int *__restrict__ cnt, float *partials) {
     CFDL_PDL_WAIT();
@@ -1790,9 +1871,24 @@ __global__ void __launch_bounds__(kTile) k_mx_rz(const CaseDev *__restrict__ cas
     SolveScalars *S = C.sc;
     const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     if (!S->active32) return;
-    float v[1] = {cg_rz_rows<float>(C.fr, C.fz, t)};
     __shared__ float s[1];
-    if (case_sums<1>(v, &C.counters[CNT_A2], partials, tile0, ntiles, s)) {
+    bool last;
+    if constexpr (kSpl) {
+        float a[1] = {0}, b[1] = {0};
+        const int i = split_row(t);
+        if (i < t.last) {
+            // cg_rz_rows' roundings: a pair's second product is rounded by itself
+            const float r = C.fr[i], z = C.fz[i];
+            const bool second = threadIdx.x / (kTile / kSplit) % 2;
+            a[0] = second ? __fmul_rn(r, z) : r;
+            b[0] = second ? 1.f : z;
+        }
+        last = split_sums<1>(a, b, &C.counters[CNT_A2], partials, tile0, ntiles, s);
+    } else {
+        float v[1] = {cg_rz_rows(C.fr, C.fz, t)};
+        last = case_sums<1>(v, &C.counters[CNT_A2], partials, tile0, ntiles, s);
+    }
+    if (last) {
         if (threadIdx.x == 0) {
             S->beta32 = S->iters32 == 0 || S->rz32 == 0.f ? 0.f : s[0] / S->rz32;
             S->rz32 = s[0];
@@ -1810,7 +1906,7 @@ __global__ void __launch_bounds__(kTile) k_mx_p(const CaseDev *__restrict__ case
     cg_p_rows<float>(C.fz, C.fp, S->iters32 == 0, S->beta32, t);
 }
 
-template <bool k16>
+template <bool k16, bool kSpl>
 __global__ void __launch_bounds__(kTile) k_mx_q(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles,
                                                 const int *__restrict__ cfirst, const int *__restrict__ cnt, float *partials) {
     CFDL_PDL_WAIT();
@@ -1819,28 +1915,41 @@ __global__ void __launch_bounds__(kTile) k_mx_q(const CaseDev *__restrict__ case
     SolveScalars *S = C.sc;
     const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     if (!S->active32) return;
-    // rows in pairs (pair_slots); then (p, q), each thread its rows 256 apart in
-    // row order, which is the order of the FP32 sums
-    __shared__ __align__(8) float qs[2 * kTile];
     const LP<float> P = level<float>(C, 0);
     const float *p = C.fp;
-    const int tid = (int)threadIdx.x;
-    float v[1] = {0.f};
-    for (int c0 = t.first; c0 < t.last; c0 += 2 * kTile) {
-        const int i = c0 + 2 * tid, i0 = c0 + tid, i1 = i0 + kTile;
-        if (i < t.last) {
-            const float2 y = pair_amul_mesh<k16>(P, p, i);
-            *(float2 *)&C.fq[i] = y;
-            *(float2 *)&qs[2 * tid] = y;
-        }
-        const float p0 = i0 < t.last ? p[i0] : 0.f, p1 = i1 < t.last ? p[i1] : 0.f;
-        __syncthreads();
-        if (i0 < t.last) v[0] += p0 * qs[tid];
-        if (i1 < t.last) v[0] += p1 * qs[tid + kTile];
-        __syncthreads();
-    }
     __shared__ float s[1];
-    if (case_sums<1>(v, &C.counters[CNT_A3], partials, tile0, ntiles, s)) {
+    bool last;
+    if constexpr (kSpl) {
+        float a[1] = {0.f}, b[1] = {0.f};
+        const int i = split_row(t);
+        if (i < t.last) {
+            b[0] = row_amul_mesh<k16>(P, p, i);
+            a[0] = p[i];
+            C.fq[i] = b[0];
+        }
+        last = split_sums<1>(a, b, &C.counters[CNT_A3], partials, tile0, ntiles, s);
+    } else {
+        // rows in pairs (pair_slots); then (p, q), each thread its rows 256 apart in
+        // row order, which is the order of the FP32 sums
+        __shared__ __align__(8) float qs[2 * kTile];
+        const int tid = (int)threadIdx.x;
+        float v[1] = {0.f};
+        for (int c0 = t.first; c0 < t.last; c0 += 2 * kTile) {
+            const int i = c0 + 2 * tid, i0 = c0 + tid, i1 = i0 + kTile;
+            if (i < t.last) {
+                const float2 y = pair_amul_mesh<k16>(P, p, i);
+                *(float2 *)&C.fq[i] = y;
+                *(float2 *)&qs[2 * tid] = y;
+            }
+            const float p0 = i0 < t.last ? p[i0] : 0.f, p1 = i1 < t.last ? p[i1] : 0.f;
+            __syncthreads();
+            if (i0 < t.last) v[0] += p0 * qs[tid];
+            if (i1 < t.last) v[0] += p1 * qs[tid + kTile];
+            __syncthreads();
+        }
+        last = case_sums<1>(v, &C.counters[CNT_A3], partials, tile0, ntiles, s);
+    }
+    if (last) {
         if (threadIdx.x == 0) {
             if (!(s[0] > 0.f) || !isfinite(s[0])) S->active32 = 0;
             else S->alpha32 = S->rz32 / s[0];
@@ -1848,6 +1957,7 @@ __global__ void __launch_bounds__(kTile) k_mx_q(const CaseDev *__restrict__ case
     }
 }
 
+template <bool kSpl>
 __global__ void __launch_bounds__(kTile) k_mx_x(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles,
                                                 const int *__restrict__ cfirst, const int *__restrict__ cnt, float *partials) {
     CFDL_PDL_WAIT();
@@ -1856,9 +1966,22 @@ __global__ void __launch_bounds__(kTile) k_mx_x(const CaseDev *__restrict__ case
     SolveScalars *S = C.sc;
     const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     if (!S->active32) return;
-    float v[1] = {cg_x_rows<float>(C.fx, C.fp, C.fr, C.fq, S->alpha32, t)};
     __shared__ float s[1];
-    if (case_sums<1>(v, &C.counters[CNT_A4], partials, tile0, ntiles, s)) {
+    bool last;
+    if constexpr (kSpl) {
+        float a[1] = {0}, b[1] = {0};
+        const int i = split_row(t);
+        if (i < t.last) {
+            const float al = S->alpha32, x = C.fx[i], p = C.fp[i], r = C.fr[i] - al * C.fq[i];
+            C.fx[i] = x + al * p;
+            C.fr[i] = a[0] = b[0] = r;
+        }
+        last = split_sums<1>(a, b, &C.counters[CNT_A4], partials, tile0, ntiles, s);
+    } else {
+        float v[1] = {cg_x_rows<float>(C.fx, C.fp, C.fr, C.fq, S->alpha32, t)};
+        last = case_sums<1>(v, &C.counters[CNT_A4], partials, tile0, ntiles, s);
+    }
+    if (last) {
         if (threadIdx.x == 0) {
             const float rn = sqrtf(s[0]);
             S->rnorm32 = rn;
@@ -1879,6 +2002,7 @@ __global__ void __launch_bounds__(kTile) k_mx_apply(const CaseDev *__restrict__ 
 }
 
 // FP64 true residual r = (b - mean) - A x and the outer stopping test
+template <bool kSpl>
 __global__ void __launch_bounds__(kTile) k_mx_res(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles,
                                                   const int *__restrict__ cfirst, const int *__restrict__ cnt, double *partials) {
     CFDL_PDL_WAIT();
@@ -1887,19 +2011,33 @@ __global__ void __launch_bounds__(kTile) k_mx_res(const CaseDev *__restrict__ ca
     SolveScalars *S = C.sc;
     const int tile0 = cfirst[t.c], ntiles = cnt[t.c];
     if (!S->active_p) return;
-    // two rows per step, both rows' loads before either store
-    double v[1] = {0};
-    const LP<double> P = level<double>(C, 0);
-    const double mb = S->mean_b;
-    FOR_ROW_PAIRS(t) {
-        double r0 = 0.0, r1 = 0.0;
-        if (ok0) r0 = (C.b[i0] - mb) - amul<double>(P, C.phic, i0);
-        if (ok1) r1 = (C.b[i1] - mb) - amul<double>(P, C.phic, i1);
-        if (ok0) { C.kr[i0] = r0; v[0] += r0 * r0; }
-        if (ok1) { C.kr[i1] = r1; v[0] += r1 * r1; }
-    }
     __shared__ double s[1];
-    if (case_sums<1>(v, &C.counters[CNT_M0], partials, tile0, ntiles, s)) {
+    bool last;
+    if constexpr (kSpl) {
+        double a[1] = {0}, b[1] = {0};
+        const int i = split_row(t);
+        if (i < t.last) {
+            const LP<double> P = level<double>(C, 0);
+            const double y = P.W == 6 ? amul_order<6, false>(P, C.phic, i) : P.W == 4 ? amul_order<4, false>(P, C.phic, i) : amul<double>(P, C.phic, i);
+            a[0] = b[0] = (C.b[i] - S->mean_b) - y;
+            C.kr[i] = a[0];
+        }
+        last = split_sums<1>(a, b, &C.counters[CNT_M0], partials, tile0, ntiles, s);
+    } else {
+        // two rows per step, both rows' loads before either store
+        double v[1] = {0};
+        const LP<double> P = level<double>(C, 0);
+        const double mb = S->mean_b;
+        FOR_ROW_PAIRS(t) {
+            double r0 = 0.0, r1 = 0.0;
+            if (ok0) r0 = (C.b[i0] - mb) - amul<double>(P, C.phic, i0);
+            if (ok1) r1 = (C.b[i1] - mb) - amul<double>(P, C.phic, i1);
+            if (ok0) { C.kr[i0] = r0; v[0] += r0 * r0; }
+            if (ok1) { C.kr[i1] = r1; v[0] += r1 * r1; }
+        }
+        last = case_sums<1>(v, &C.counters[CNT_M0], partials, tile0, ntiles, s);
+    }
+    if (last) {
         if (threadIdx.x == 0) {
             const double rn = sqrt(s[0]);
             S->rnorm_p = rn;
@@ -1924,15 +2062,25 @@ void mx_start(cfdl_ctx *ctx) { ALAUNCH("k_mx_start", k_mx_start, ctx->cellsv, RE
 void mx_inner_iter(cfdl_ctx *ctx) {
     if (ctx->cases[0]->cfg.precond == 1) vcycle<float>(ctx);
     else ALAUNCH("k_mx_jacobi", k_mx_jacobi, ctx->cellsv);
-    ALAUNCH("k_mx_rz", k_mx_rz, ctx->cellsv, RED32);
+    const bool n16 = ctx->amg_nb16;
+    if (ctx->cellss.ntiles) {
+        ALAUNCH("k_mx_rz", k_mx_rz<true>, ctx->cellss, REDS32);
+        ALAUNCH("k_mx_p", k_mx_p, ctx->cells);
+        if (n16) ALAUNCH("k_mx_q", (k_mx_q<true, true>), ctx->cellss, REDS32);
+        else ALAUNCH("k_mx_q", (k_mx_q<false, true>), ctx->cellss, REDS32);
+        ALAUNCH("k_mx_x", k_mx_x<true>, ctx->cellss, REDS32);
+        return;
+    }
+    ALAUNCH("k_mx_rz", k_mx_rz<false>, ctx->cellsv, RED32);
     ALAUNCH("k_mx_p", k_mx_p, ctx->cellsv);
-    if (ctx->amg_nb16) ALAUNCH("k_mx_q", k_mx_q<true>, ctx->cellsv, RED32);
-    else ALAUNCH("k_mx_q", k_mx_q<false>, ctx->cellsv, RED32);
-    ALAUNCH("k_mx_x", k_mx_x, ctx->cellsv, RED32);
+    if (n16) ALAUNCH("k_mx_q", (k_mx_q<true, false>), ctx->cellsv, RED32);
+    else ALAUNCH("k_mx_q", (k_mx_q<false, false>), ctx->cellsv, RED32);
+    ALAUNCH("k_mx_x", k_mx_x<false>, ctx->cellsv, RED32);
 }
 void mx_finish(cfdl_ctx *ctx) {
     ALAUNCH("k_mx_apply", k_mx_apply, ctx->cellsv);
-    ALAUNCH("k_mx_res", k_mx_res, ctx->cellsv, RED);
+    if (ctx->cellss.ntiles) ALAUNCH("k_mx_res", k_mx_res<true>, ctx->cellss, REDS);
+    else ALAUNCH("k_mx_res", k_mx_res<false>, ctx->cellsv, RED);
 }
 
 int solve_pressure_mixed(cfdl_ctx *ctx) {

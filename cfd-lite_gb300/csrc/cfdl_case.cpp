@@ -87,15 +87,17 @@ static int rows_one_wave(int ne, int least) {
 
 // tiles: entities per tile of each case
 // per_thread: entities per thread and sub-tile of a merged list (0: the tile's)
-int build_worklist(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &sizes, const std::vector<int> &tiles, int per_thread) {
+// split: blocks to a tile of a split list
+int build_worklist(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &sizes, const std::vector<int> &tiles, int per_thread, int split) {
     free_worklist(wl);
     wl.h_tiles.clear(); wl.case_first.clear(); wl.case_ntiles.clear();
     for (size_t c = 0; c < sizes.size(); c++) {
         wl.case_first.push_back((int)wl.h_tiles.size());
         int cnt = 0;
         const int tile = tiles[c];
-        for (int s = 0; s < sizes[c]; s += tile, cnt++)
-            wl.h_tiles.push_back({(int)c, s, std::min(sizes[c], s + tile), per_thread ? per_thread : (tile + kTile - 1) / kTile});
+        for (int s = 0; s < sizes[c]; s += tile)
+            for (int j = 0; j < split; j++, cnt++)
+                wl.h_tiles.push_back({(int)c, s, std::min(sizes[c], s + tile), split > 1 ? j : per_thread ? per_thread : (tile + kTile - 1) / kTile});
         wl.case_ntiles.push_back(cnt);
     }
     wl.ntiles = (int)wl.h_tiles.size();
@@ -475,6 +477,20 @@ static int build_merged(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &siz
     return build_worklist(ctx, wl, sizes, std::vector<int>(sizes.size(), rows * M), vec);
 }
 
+// The solver tiles of a small context, kSplit blocks to a tile (Tile::pad: the
+// block's place among them); empty for a larger one.  The line lies where the
+// split blocks are four to an SM in FP64 and three in the mixed forms, in outer
+// iterations, split against whole tiles: FP64 at 32^3 cells 452 against 517 us,
+// 45^3 640 / 717, 53^3 (584 blocks) 759 / 766; FP32 assembly and solves at 24^3
+// 334 / 368, 45^3 (356 blocks) 526 / 529, 53^3 645 / 638.
+static int build_split(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &sizes) {
+    long n = 0;
+    for (int s : sizes) n += (s + kTile * kVec - 1) / (kTile * kVec);
+    const bool fp64 = !ctx->cases.empty() && ctx->cases[0]->cfg.precision == 0;
+    const bool on = ctx->vec == kVec && n * kSplit <= 152 * (fp64 ? 4 : 3);
+    return build_worklist(ctx, wl, on ? sizes : std::vector<int>(sizes.size(), 0), std::vector<int>(sizes.size(), kTile * kVec), 0, kSplit);
+}
+
 // Tile work lists over every case of the context.
 int rebuild_worklists(cfdl_ctx *ctx) {
     std::vector<int> nc, nfc, nh;
@@ -490,6 +506,7 @@ int rebuild_worklists(cfdl_ctx *ctx) {
     if ((st = build_worklist(ctx, ctx->cellsv, nc, tiles))) return st;
     if ((st = build_worklist(ctx, ctx->cellse, nc, kTile * ctx->en_vec))) return st;
     if ((st = build_merged(ctx, ctx->cellsem, nc, ctx->en_vec))) return st;
+    if ((st = build_split(ctx, ctx->cellss, nc))) return st;
     tiles.clear();
     for (int ne : nc) tiles.push_back(kTile * rows_per_thread(ne));
     if ((st = build_worklist(ctx, ctx->cellsr, nc, tiles))) return st;
@@ -502,7 +519,7 @@ int rebuild_worklists(cfdl_ctx *ctx) {
     ctx->amg_cells.clear(); ctx->amg_smooth.clear(); ctx->amg_gcells.clear(); ctx->amg_gsmooth.clear();
     ctx->amg_restr.clear(); ctx->amg_grestr.clear(); ctx->amg_lmax = -1;
     destroy_graph(ctx);   // captured launch arguments refer to the old lists
-    int need = std::max({ctx->cells.ntiles, ctx->faces.ntiles, ctx->halos.ntiles,
+    int need = std::max({ctx->cells.ntiles, ctx->faces.ntiles, ctx->halos.ntiles, ctx->cellss.ntiles,
                          ctx->cellsem.ntiles * ctx->cellsem.merge.M, 1});
     if (need > ctx->partials_cap) {
         cudaFree(ctx->d_partials);

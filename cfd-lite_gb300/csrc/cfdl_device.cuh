@@ -70,10 +70,10 @@ __device__ __forceinline__ void block_sums(double (&v)[K], double *out) {
 // each step a lane keeps half of the values and hands the other half over, so
 // six values take 8 shuffles and adds instead of 30 (0.2% of an FP32 outer
 // iteration).  Returns the sum of value k if `mine`: one lane per value.
-template <int N, int O = 16>
-__device__ __forceinline__ float warp_sums(const float (&v)[N], int lane, int &k, bool &mine) {
+template <int N, int O = 16, class T>
+__device__ __forceinline__ T warp_sums(const T (&v)[N], int lane, int &k, bool &mine) {
     if constexpr (N == 1) {
-        float z = v[0];
+        T z = v[0];
 #pragma unroll
         for (int o = O; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
         k = 0;
@@ -82,13 +82,13 @@ __device__ __forceinline__ float warp_sums(const float (&v)[N], int lane, int &k
     } else {
         constexpr int H = (N + 1) / 2;
         const bool up = (lane & O) != 0;
-        float y[H];
+        T y[H];
 #pragma unroll
         for (int j = 0; j < H; j++) {
-            const float hi = j + H < N ? v[j + H < N ? j + H : 0] : v[j];
+            const T hi = j + H < N ? v[j + H < N ? j + H : 0] : v[j];
             y[j] = (up ? hi : v[j]) + __shfl_xor_sync(0xffffffffu, up ? v[j] : hi, O);
         }
-        const float z = warp_sums<H, O / 2>(y, lane, k, mine);
+        const T z = warp_sums<H, O / 2>(y, lane, k, mine);
         if (up) k += H;
         mine = mine && k < N;
         return z;
@@ -242,6 +242,73 @@ template <int K, int kSub, class T>
 __device__ __forceinline__ bool tile_sums(T (&v)[K], int nm, int *counter, T *partials, int tile0, int ntiles, const Merge &mg, int ne, T *s) {
     if constexpr (kSub == 1) return case_sums<K>(v, counter, partials, tile0, ntiles, s);
     else return merged_sums<K, T, kSub>(nm, counter, partials, tile0, ntiles, mg.M, (ne + mg.rows - 1) / mg.rows, s);
+}
+
+// A small context leaves most SMs idle with 1024 cells to a block, and each
+// thread there goes through its four rows one after the other.  In a split list
+// kSplit blocks share a tile: block j takes the columns of threads 64 j to
+// 64 j + 63, one row per thread (split_row), and split_sums chains each column's
+// products in row order, forms the two warps' trees and files them, so the sums
+// have the bits of case_sums.  a, b: the factors of the row's share of each sum.
+// At 32^3 cells a launch of the FP64 A ph went from 17 to 10 us, at 24^3 the
+// FP32 one from 10 to 6.6.
+__device__ __forceinline__ int split_row(const Tile &t) {
+    constexpr int cols = kTile / kSplit;
+    return t.first + (int)threadIdx.x / cols * kTile + t.pad * cols + (int)threadIdx.x % cols;
+}
+template <class T> __device__ __forceinline__ T fma_rn(T a, T b, T c) {
+    if constexpr (sizeof(T) == 4) return __fmaf_rn(a, b, c);
+    else return __fma_rn(a, b, c);
+}
+template <int K, class T>
+__device__ __forceinline__ bool split_sums(const T (&a)[K], const T (&b)[K], int *counter, T *partials, int tile0, int nblocks, T *s) {
+    constexpr int cols = kTile / kSplit, kWarps = kTile / 32;
+    __shared__ T sa[K][kTile], sb[K][kTile];
+    __shared__ int is_last;
+    const int tid = (int)threadIdx.x, ntiles = nblocks / kSplit, at = (int)blockIdx.x - tile0;
+#pragma unroll
+    for (int k = 0; k < K; k++) { sa[k][tid] = a[k]; sb[k][tid] = b[k]; }
+    __syncthreads();
+    T *part = partials + (size_t)tile0 * kNPart;           // [K][ntiles][kWarps]
+    if (tid < cols) {
+        T v[K];
+#pragma unroll
+        for (int k = 0; k < K; k++) v[k] = 0;
+#pragma unroll
+        for (int g = 0; g < kSplit; g++)
+#pragma unroll
+            for (int k = 0; k < K; k++) v[k] = fma_rn(sa[k][g * cols + tid], sb[k][g * cols + tid], v[k]);
+        int k;
+        bool mine;
+        const T z = warp_sums<K>(v, tid & 31, k, mine);
+        if (mine) __stcg(&part[((size_t)k * ntiles + at / kSplit) * kWarps + at % kSplit * (cols / 32) + (tid >> 5)], z);
+    }
+    __syncthreads();
+    if (tid == 0) {
+        __threadfence();
+        const bool last = atomicAdd(counter, 1) == nblocks - 1;
+        if (last) { *counter = 0; __threadfence(); }
+        is_last = last;
+    }
+    __syncthreads();
+    if (!is_last) return false;
+    T v[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) v[k] = 0;
+    for (int i = tid; i < ntiles; i += kTile)
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            const T *q = part + ((size_t)k * ntiles + i) * kWarps;
+            T w[kWarps], x = 0;
+#pragma unroll
+            for (int u = 0; u < kWarps; u++) w[u] = __ldcg(q + u);
+#pragma unroll
+            for (int u = 0; u < kWarps; u++) x += w[u];
+            v[k] += x;
+        }
+    block_sums<K>(v, s);
+    __syncthreads();
+    return true;
 }
 
 // Start of a case's momentum solve from s[0..2] = sum b'^2 and s[3..5] =

@@ -184,6 +184,8 @@ struct Tile { int c, first, last, pad; };
 
 // A merged list's blocks: up to M tiles of `rows` entities, taken in turn.
 struct Merge { int M, rows; };
+constexpr int kSplit = 4;               // blocks that share a tile of a split list, one row per thread
+static_assert(kSplit == kVec && kTile / kSplit % 32 == 0, "split_sums");
 constexpr int kMaxMerge = 4;            // most tiles a block takes (a shared buffer holds their values)
 
 // One work list per entity type, with each case's tile range for reductions.
@@ -237,6 +239,7 @@ struct cfdl_ctx {
     cfdl::WorkList cellsr;               // tiles of the FP64 passes whose shape goes by the case's size (rows_per_thread)
     cfdl::WorkList cellse;               // tiles of the energy solve (kTile*en_vec cells)
     cfdl::WorkList cellsem;              // the same tiles, merged
+    cfdl::WorkList cellss;               // cellsv's tiles, split (empty where they are not: see split_sums)
     cfdl::WorkList facesv;               // wide face tiles (kTile*kFaceVec faces) for face reductions
     int en_vec = 1;                      // cells per thread in those tiles (autotuned with the energy equation)
     int last_iters_m = 0, last_iters_p = 0, last_iters_e = 0;   // previous inner iteration counts (poll scheduling)
@@ -420,7 +423,7 @@ int solve_pressure_amg(cfdl_ctx *ctx);
 int solve_pressure_mixed(cfdl_ctx *ctx);
 void free_worklist(WorkList &wl);
 int build_worklist(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &sizes, int tile = kTile);
-int build_worklist(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &sizes, const std::vector<int> &tiles, int per_thread = 0);
+int build_worklist(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &sizes, const std::vector<int> &tiles, int per_thread = 0, int split = 1);
 int read_stats(cfdl_ctx *ctx, int c, cfdl_stats *st);
 int poll_kind(cfdl_ctx *ctx, int kind, int *maxit);
 int poll_chunk(int done, int expected);

@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(kTile) k_mom_p(const CaseDev *__restrict__ cas
 }
 
 // v = A ph; alpha = rho / (rh, v)
-template <class T, int NC, bool k16 = false>
+template <class T, int NC, bool k16 = false, bool kSpl = false>
 __global__ void __launch_bounds__(kTile, sizeof(T) == 8 && NC == 1 ? 4 : 5) k_mom_v(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles,
                                                  const int *__restrict__ cfirst, const int *__restrict__ cnt, T *partials, Merge mg) {
     CFDL_PDL_WAIT();
@@ -273,27 +273,40 @@ __global__ void __launch_bounds__(kTile, sizeof(T) == 8 && NC == 1 ? 4 : 5) k_mo
     int act[NC];
 #pragma unroll
     for (int q = 0; q < NC; q++) act[q] = L->active[q];
-    T v[NC];
-    FOR_SUBTILES(u, t, mg, nm, (kMaxSub<T, NC>)) {
+    // row i; add(k, a, b): its share a b of sum k
+    auto row = [&](int i, auto &&add) {
+        T y[NC], rh[NC];   // one pass over the row for the components
+        if constexpr (kInter<T, NC>) row3<k16>(C, (const float4 *)M.ph, i, y);
+        else ell_row<NC, T>(C.hf_nb, M.a, M.ap[i], M.ph, ne, ne, C.W, i, y);
 #pragma unroll
-        for (int q = 0; q < NC; q++) v[q] = 0;
-        FOR_CELLS(u) {
-            T y[NC], rh[NC];   // one pass over the row for the components
-            if constexpr (kInter<T, NC>) row3<k16>(C, (const float4 *)M.ph, i, y);
-            else ell_row<NC, T>(C.hf_nb, M.a, M.ap[i], M.ph, ne, ne, C.W, i, y);
+        for (int q = 0; q < NC; q++) rh[q] = act[q] ? M.rh[q * ne + i] : (T)0;   // loads before the stores
 #pragma unroll
-            for (int q = 0; q < NC; q++) rh[q] = act[q] ? M.rh[q * ne + i] : (T)0;   // loads before the stores
-#pragma unroll
-            for (int q = 0; q < NC; q++) {
-                if (!act[q]) continue;
-                M.v[q * ne + i] = y[q];
-                v[q] += rh[q] * y[q];
-            }
+        for (int q = 0; q < NC; q++) {
+            if (!act[q]) continue;
+            M.v[q * ne + i] = y[q];
+            add(q, rh[q], y[q]);
         }
-        if (kMaxSub<T, NC> > 1) put_sums<NC, kMaxSub<T, NC>>(v, nm);
-    }
+    };
     __shared__ T s[NC];
-    if (tile_sums<NC, kMaxSub<T, NC>>(v, nm, &C.counters[CNT_M2], partials, tile0, ntiles, mg, ne, s)) {
+    bool last;
+    if constexpr (kSpl) {
+        T a[NC], b[NC];
+#pragma unroll
+        for (int q = 0; q < NC; q++) a[q] = b[q] = 0;
+        const int i = split_row(t);
+        if (i < t.last) row(i, [&](int q, T x, T y) { a[q] = x; b[q] = y; });
+        last = split_sums<NC>(a, b, &C.counters[CNT_M2], partials, tile0, ntiles, s);
+    } else {
+        T v[NC];
+        FOR_SUBTILES(u, t, mg, nm, (kMaxSub<T, NC>)) {
+#pragma unroll
+            for (int q = 0; q < NC; q++) v[q] = 0;
+            FOR_CELLS(u) row(i, [&](int q, T x, T y) { v[q] += x * y; });
+            if (kMaxSub<T, NC> > 1) put_sums<NC, kMaxSub<T, NC>>(v, nm);
+        }
+        last = tile_sums<NC, kMaxSub<T, NC>>(v, nm, &C.counters[CNT_M2], partials, tile0, ntiles, mg, ne, s);
+    }
+    if (last) {
         if (threadIdx.x < NC && L->active[threadIdx.x]) {   // one thread per component
             const int q = threadIdx.x;
             const double sq = (double)s[q];
@@ -305,7 +318,7 @@ __global__ void __launch_bounds__(kTile, sizeof(T) == 8 && NC == 1 ? 4 : 5) k_mo
 }
 
 // s = r - alpha v; sh = s / ap; early exit when ||s|| <= tol
-template <class T, int NC>
+template <class T, int NC, bool kSpl = false>
 __global__ void __launch_bounds__(kTile) k_mom_s(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles,
                                                  const int *__restrict__ cfirst, const int *__restrict__ cnt, T *partials, Merge mg) {
     CFDL_PDL_WAIT();
@@ -318,58 +331,71 @@ __global__ void __launch_bounds__(kTile) k_mom_s(const CaseDev *__restrict__ cas
     int act[NC];
 #pragma unroll
     for (int q = 0; q < NC; q++) { act[q] = L->active[q]; al[q] = (T)L->alpha[q]; }
-    T v[NC];
-    FOR_SUBTILES(u, t, mg, nm, (kMaxSub<T, NC>)) {
+    // row i; add(k, a, b): its share a b of sum k
+    auto row = [&](int i, auto &&add) {
+        const T rap = M.rap[i];
+        if (sizeof(T) == 4) {
+            // FP32: the row's loads, every component's, before its stores
+            // (36 -> 27 us a launch at 128^3; the FP64 form measured slower
+            // this way, 63 -> 68 us, and keeps one component at a time)
+            T rr[NC], vv[NC];
 #pragma unroll
-        for (int q = 0; q < NC; q++) v[q] = 0;
-        FOR_CELLS(u) {
-            const T rap = M.rap[i];
-            if (sizeof(T) == 4) {
-                // FP32: the row's loads, every component's, before its stores
-                // (36 -> 27 us a launch at 128^3; the FP64 form measured slower
-                // this way, 63 -> 68 us, and keeps one component at a time)
-                T rr[NC], vv[NC];
+            for (int q = 0; q < NC; q++) {
+                rr[q] = act[q] ? M.r[q * ne + i] : (T)0;
+                vv[q] = act[q] ? M.v[q * ne + i] : (T)0;
+            }
+            T sh[NC];
 #pragma unroll
-                for (int q = 0; q < NC; q++) {
-                    rr[q] = act[q] ? M.r[q * ne + i] : (T)0;
-                    vv[q] = act[q] ? M.v[q * ne + i] : (T)0;
-                }
-                T sh[NC];
+            for (int q = 0; q < NC; q++) {
+                sh[q] = 0;
+                if (!act[q]) continue;
+                const int j = q * ne + i;
+                const T sv = rr[q] - al[q] * vv[q];
+                M.s[j] = sv;
+                sh[q] = sv * rap;
+                if (!kInter<T, NC>) M.sh[j] = sh[q];
+                add(q, sv, sv);
+            }
+            if (kInter<T, NC>) ((float4 *)M.sh)[i] = make_float4(sh[0], sh[1 % NC], sh[2 % NC], 0.f);
+        } else {
 #pragma unroll
-                for (int q = 0; q < NC; q++) {
-                    sh[q] = 0;
-                    if (!act[q]) continue;
-                    const int j = q * ne + i;
-                    const T sv = rr[q] - al[q] * vv[q];
-                    M.s[j] = sv;
-                    sh[q] = sv * rap;
-                    if (!kInter<T, NC>) M.sh[j] = sh[q];
-                    v[q] += sv * sv;
-                }
-                if (kInter<T, NC>) ((float4 *)M.sh)[i] = make_float4(sh[0], sh[1 % NC], sh[2 % NC], 0.f);
-            } else {
-#pragma unroll
-                for (int q = 0; q < NC; q++) {
-                    if (!act[q]) continue;
-                    const int j = q * ne + i;
-                    const T sv = M.r[j] - al[q] * M.v[j];
-                    M.s[j] = sv;
-                    M.sh[j] = sv * rap;
-                    v[q] += sv * sv;
-                }
+            for (int q = 0; q < NC; q++) {
+                if (!act[q]) continue;
+                const int j = q * ne + i;
+                const T sv = M.r[j] - al[q] * M.v[j];
+                M.s[j] = sv;
+                M.sh[j] = sv * rap;
+                add(q, sv, sv);
             }
         }
-        if (kMaxSub<T, NC> > 1) put_sums<NC, kMaxSub<T, NC>>(v, nm);
-    }
+    };
     __shared__ T s[NC];
-    if (tile_sums<NC, kMaxSub<T, NC>>(v, nm, &C.counters[CNT_M3], partials, tile0, ntiles, mg, ne, s)) {
+    bool last;
+    if constexpr (kSpl) {
+        T a[NC], b[NC];
+#pragma unroll
+        for (int q = 0; q < NC; q++) a[q] = b[q] = 0;
+        const int i = split_row(t);
+        if (i < t.last) row(i, [&](int q, T x, T y) { a[q] = x; b[q] = y; });
+        last = split_sums<NC>(a, b, &C.counters[CNT_M3], partials, tile0, ntiles, s);
+    } else {
+        T v[NC];
+        FOR_SUBTILES(u, t, mg, nm, (kMaxSub<T, NC>)) {
+#pragma unroll
+            for (int q = 0; q < NC; q++) v[q] = 0;
+            FOR_CELLS(u) row(i, [&](int q, T x, T y) { v[q] += x * y; });
+            if (kMaxSub<T, NC> > 1) put_sums<NC, kMaxSub<T, NC>>(v, nm);
+        }
+        last = tile_sums<NC, kMaxSub<T, NC>>(v, nm, &C.counters[CNT_M3], partials, tile0, ntiles, mg, ne, s);
+    }
+    if (last) {
         const int q = threadIdx.x;
         if (q < NC && L->active[q]) L->half[q] = sqrt((double)s[q]) <= L->tol[q];
     }
 }
 
 // t = A sh; omega = (t,s)/(t,t)
-template <class T, int NC, bool k16 = false>
+template <class T, int NC, bool k16 = false, bool kSpl = false>
 __global__ void __launch_bounds__(kTile, sizeof(T) == 8 && NC == 1 ? 4 : 5) k_mom_t(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles,
                                                  const int *__restrict__ cfirst, const int *__restrict__ cnt, T *partials, Merge mg) {
     CFDL_PDL_WAIT();
@@ -381,29 +407,42 @@ __global__ void __launch_bounds__(kTile, sizeof(T) == 8 && NC == 1 ? 4 : 5) k_mo
     int act[NC];
 #pragma unroll
     for (int q = 0; q < NC; q++) act[q] = L->active[q] && !L->half[q];
-    T v[2 * NC];
-    FOR_SUBTILES(u, t, mg, nm, (kMaxSub<T, NC>)) {
+    // row i; add(k, a, b): its share a b of sum k
+    auto row = [&](int i, auto &&add) {
+        T y[NC], sv[NC];
+        if constexpr (kInter<T, NC>) row3<k16>(C, (const float4 *)M.sh, i, y);
+        else ell_row<NC, T>(C.hf_nb, M.a, M.ap[i], M.sh, ne, ne, C.W, i, y);
 #pragma unroll
-        for (int q = 0; q < 2 * NC; q++) v[q] = 0;
-        FOR_CELLS(u) {
-            T y[NC], sv[NC];
-            if constexpr (kInter<T, NC>) row3<k16>(C, (const float4 *)M.sh, i, y);
-            else ell_row<NC, T>(C.hf_nb, M.a, M.ap[i], M.sh, ne, ne, C.W, i, y);
+        for (int q = 0; q < NC; q++) sv[q] = act[q] ? M.s[q * ne + i] : (T)0;   // loads before the stores
 #pragma unroll
-            for (int q = 0; q < NC; q++) sv[q] = act[q] ? M.s[q * ne + i] : (T)0;   // loads before the stores
-#pragma unroll
-            for (int q = 0; q < NC; q++) {
-                if (!act[q]) continue;
-                const int j = q * ne + i;
-                M.t[j] = y[q];
-                v[q] += y[q] * sv[q];
-                v[NC + q] += y[q] * y[q];
-            }
+        for (int q = 0; q < NC; q++) {
+            if (!act[q]) continue;
+            const int j = q * ne + i;
+            M.t[j] = y[q];
+            add(q, y[q], sv[q]);
+            add(NC + q, y[q], y[q]);
         }
-        if (kMaxSub<T, NC> > 1) put_sums<2 * NC, kMaxSub<T, NC>>(v, nm);
-    }
+    };
     __shared__ T s[2 * NC];
-    if (tile_sums<2 * NC, kMaxSub<T, NC>>(v, nm, &C.counters[CNT_M4], partials, tile0, ntiles, mg, ne, s)) {
+    bool last;
+    if constexpr (kSpl) {
+        T a[2 * NC], b[2 * NC];
+#pragma unroll
+        for (int q = 0; q < 2 * NC; q++) a[q] = b[q] = 0;
+        const int i = split_row(t);
+        if (i < t.last) row(i, [&](int q, T x, T y) { a[q] = x; b[q] = y; });
+        last = split_sums<2 * NC>(a, b, &C.counters[CNT_M4], partials, tile0, ntiles, s);
+    } else {
+        T v[2 * NC];
+        FOR_SUBTILES(u, t, mg, nm, (kMaxSub<T, NC>)) {
+#pragma unroll
+            for (int q = 0; q < 2 * NC; q++) v[q] = 0;
+            FOR_CELLS(u) row(i, [&](int q, T x, T y) { v[q] += x * y; });
+            if (kMaxSub<T, NC> > 1) put_sums<2 * NC, kMaxSub<T, NC>>(v, nm);
+        }
+        last = tile_sums<2 * NC, kMaxSub<T, NC>>(v, nm, &C.counters[CNT_M4], partials, tile0, ntiles, mg, ne, s);
+    }
+    if (last) {
         const int q = threadIdx.x;
         if (q < NC && L->active[q]) {
             const double ts = (double)s[q], tt = (double)s[NC + q];
@@ -413,7 +452,7 @@ __global__ void __launch_bounds__(kTile, sizeof(T) == 8 && NC == 1 ? 4 : 5) k_mo
 }
 
 // x += alpha ph + omega sh; r = s - omega t; rho' = (rh, r); beta
-template <class T, int NC>
+template <class T, int NC, bool kSpl = false>
 __global__ void __launch_bounds__(kTile, 4) k_mom_x(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles,
                                                  const int *__restrict__ cfirst, const int *__restrict__ cnt, T *partials, Merge mg) {
     CFDL_PDL_WAIT();
@@ -428,29 +467,24 @@ __global__ void __launch_bounds__(kTile, 4) k_mom_x(const CaseDev *__restrict__ 
     for (int q = 0; q < NC; q++) {
         act[q] = L->active[q]; al[q] = (T)L->alpha[q]; om[q] = (T)L->omega[q];
     }
-    T v[2 * NC];
-    FOR_SUBTILES(u, t, mg, nm, (kMaxSub<T, NC>)) {
-#pragma unroll
-        for (int q = 0; q < 2 * NC; q++) v[q] = 0;
+    // row i; add(k, a, b): its share a b of sum k
+    auto row = [&](int i, auto &&add) {
         if (sizeof(T) == 8 && NC == 3) {
             // FP64: one component's loads at a time; all eighteen together spilled
             // 200 bytes under four CTAs per SM (128^3: an outer iteration 0.4%)
-            FOR_CELLS(u) {
 #pragma unroll
-                for (int q = 0; q < NC; q++) {
-                    if (!act[q]) continue;
-                    const int j = q * ne + i;
-                    const T xv = M.x[q][i], ph = M.ph[j], sh = M.sh[j], sv = M.s[j], rh = M.rh[j];
-                    const T tv = om[q] != (T)0 ? M.t[j] : (T)0;
-                    M.x[q][i] = xv + al[q] * ph + om[q] * sh;
-                    const T r = om[q] == (T)0 ? sv : sv - om[q] * tv;
-                    M.r[j] = r;
-                    v[q] += r * r;
-                    v[NC + q] += rh * r;
-                }
+            for (int q = 0; q < NC; q++) {
+                if (!act[q]) continue;
+                const int j = q * ne + i;
+                const T xv = M.x[q][i], ph = M.ph[j], sh = M.sh[j], sv = M.s[j], rh = M.rh[j];
+                const T tv = om[q] != (T)0 ? M.t[j] : (T)0;
+                M.x[q][i] = xv + al[q] * ph + om[q] * sh;
+                const T r = om[q] == (T)0 ? sv : sv - om[q] * tv;
+                M.r[j] = r;
+                add(q, r, r);
+                add(NC + q, rh, r);
             }
-        } else
-        FOR_CELLS(u) {
+        } else {
             // the row's loads, every component's, before its stores
             T xv[NC], ph[NC], sh[NC], sv[NC], tv[NC], rh[NC];
 #pragma unroll
@@ -474,14 +508,31 @@ __global__ void __launch_bounds__(kTile, 4) k_mom_x(const CaseDev *__restrict__ 
                 M.x[q][i] = xv[q] + al[q] * ph[q] + om[q] * sh[q];
                 const T r = om[q] == (T)0 ? sv[q] : sv[q] - om[q] * tv[q];
                 M.r[j] = r;
-                v[q] += r * r;
-                v[NC + q] += rh[q] * r;
+                add(q, r, r);
+                add(NC + q, rh[q], r);
             }
         }
-        if (kMaxSub<T, NC> > 1) put_sums<2 * NC, kMaxSub<T, NC>>(v, nm);
-    }
+    };
     __shared__ T s[2 * NC];
-    if (tile_sums<2 * NC, kMaxSub<T, NC>>(v, nm, &C.counters[CNT_M5], partials, tile0, ntiles, mg, ne, s)) {
+    bool last;
+    if constexpr (kSpl) {
+        T a[2 * NC], b[2 * NC];
+#pragma unroll
+        for (int q = 0; q < 2 * NC; q++) a[q] = b[q] = 0;
+        const int i = split_row(t);
+        if (i < t.last) row(i, [&](int q, T x, T y) { a[q] = x; b[q] = y; });
+        last = split_sums<2 * NC>(a, b, &C.counters[CNT_M5], partials, tile0, ntiles, s);
+    } else {
+        T v[2 * NC];
+        FOR_SUBTILES(u, t, mg, nm, (kMaxSub<T, NC>)) {
+#pragma unroll
+            for (int q = 0; q < 2 * NC; q++) v[q] = 0;
+            FOR_CELLS(u) row(i, [&](int q, T x, T y) { v[q] += x * y; });
+            if (kMaxSub<T, NC> > 1) put_sums<2 * NC, kMaxSub<T, NC>>(v, nm);
+        }
+        last = tile_sums<2 * NC, kMaxSub<T, NC>>(v, nm, &C.counters[CNT_M5], partials, tile0, ntiles, mg, ne, s);
+    }
+    if (last) {
         const int q = threadIdx.x;
         if (q < NC && L->active[q]) {
             const int cap = C.solve_mode == 0 ? C.nit : C.tight_maxit;
@@ -749,12 +800,24 @@ static int max_cap(cfdl_ctx *ctx) {
 
 static void mom_init(cfdl_ctx *ctx) { CFDL_LAUNCH("k_mom_init", k_mom_init, cellsv, RED); }
 
+#define REDS ctx->cellss.d_case_first, ctx->cellss.d_case_ntiles, ctx->d_partials, ctx->cellss.merge
+#define REDS32 ctx->cellss.d_case_first, ctx->cellss.d_case_ntiles, (float *)ctx->d_partials, ctx->cellss.merge
 #define RED32 ctx->cellsv.d_case_first, ctx->cellsv.d_case_ntiles, (float *)ctx->d_partials, ctx->cellsv.merge
 
 void mom_iter(cfdl_ctx *ctx) {
     if (ctx->cases[0]->cfg.precision >= 2) {
         bool n16 = ctx->amg_nb16;           // the 16-bit neighbour offsets, where every case has them
         for (const HostCase *hc : ctx->cases) n16 = n16 && hc->dev.nb16;   // (one added since may not)
+        if (ctx->cellss.ntiles) {
+            CFDL_LAUNCH("k_mom_p", (k_mom_p<float, 3>), cells);
+            if (n16) CFDL_LAUNCH("k_mom_v", (k_mom_v<float, 3, true, true>), cellss, REDS32);
+            else CFDL_LAUNCH("k_mom_v", (k_mom_v<float, 3, false, true>), cellss, REDS32);
+            CFDL_LAUNCH("k_mom_s", (k_mom_s<float, 3, true>), cellss, REDS32);
+            if (n16) CFDL_LAUNCH("k_mom_t", (k_mom_t<float, 3, true, true>), cellss, REDS32);
+            else CFDL_LAUNCH("k_mom_t", (k_mom_t<float, 3, false, true>), cellss, REDS32);
+            CFDL_LAUNCH("k_mom_x", (k_mom_x<float, 3, true>), cellss, REDS32);
+            return;
+        }
         CFDL_LAUNCH("k_mom_p", (k_mom_p<float, 3>), cellsv);
         if (n16) CFDL_LAUNCH("k_mom_v", (k_mom_v<float, 3, true>), cellsv, RED32);
         else CFDL_LAUNCH("k_mom_v", (k_mom_v<float, 3, false>), cellsv, RED32);
@@ -762,6 +825,14 @@ void mom_iter(cfdl_ctx *ctx) {
         if (n16) CFDL_LAUNCH("k_mom_t", (k_mom_t<float, 3, true>), cellsv, RED32);
         else CFDL_LAUNCH("k_mom_t", (k_mom_t<float, 3, false>), cellsv, RED32);
         CFDL_LAUNCH("k_mom_x", (k_mom_x<float, 3>), cellsv, RED32);
+        return;
+    }
+    if (ctx->cellss.ntiles) {
+        CFDL_LAUNCH("k_mom_p", (k_mom_p<double, 3>), cells);
+        CFDL_LAUNCH("k_mom_v", (k_mom_v<double, 3, false, true>), cellss, REDS);
+        CFDL_LAUNCH("k_mom_s", (k_mom_s<double, 3, true>), cellss, REDS);
+        CFDL_LAUNCH("k_mom_t", (k_mom_t<double, 3, false, true>), cellss, REDS);
+        CFDL_LAUNCH("k_mom_x", (k_mom_x<double, 3, true>), cellss, REDS);
         return;
     }
     CFDL_LAUNCH("k_mom_p", (k_mom_p<double, 3>), cellsv);
