@@ -213,8 +213,8 @@ int upload_all(HostCase *hc, const cfdl_config *cfg, const FillVec<int> &hf_nb, 
     if ((st = zeros(hc, &d.fdiag_p, ld))) return st;
     if ((st = zeros(hc, &d.frap_p, ld))) return st;
     if ((st = zeros(hc, &d.fdiff, (size_t)nf))) return st;
-    if ((st = zeros(hc, &d.fmip, (size_t)nf))) return st;
     if ((st = zeros(hc, &d.fS, 3 * (size_t)nf))) return st;
+    d.fmip = d.fS + 2 * (size_t)nf;      // fS's readers are done when dc is there (its FP32 form ends before this plane)
     if ((st = zeros(hc, &d.hbc, 4 * (size_t)nbf))) return st;
     if ((st = zeros(hc, &d.fprop, (size_t)PR_N * nf))) return st;
     double **kv[] = {&d.kr, &d.krh, &d.kp, &d.kph, &d.kv, &d.ks, &d.ksh, &d.kt};

@@ -135,7 +135,7 @@ struct CaseDev {
     float *fdiag_p, *fanb_p, *frap_p;     // fanb_p [W][ld32]; the FP32 vectors have ld32 elements
     // face intermediates of the assemblies
     double *fdiff, *fS;                   // [nf] pressure face coefficient, [3][nf] explicit momentum face terms
-    double *fmip;                         // [nf] rho_face area/(dr.n) dc_ip: update_uvwp's flux factor, left by k_coef_p_face
+    double *fmip;                         // [nf] rho_face area/(dr.n) dc_ip: update_uvwp's flux factor, left by k_coef_p_face in fS's third plane
     double *hbc;                          // [4][nbf] per halo: the wall diffusion added to ap and anb, and the
                                           // three momentum sources of the BC loop (k_coef_uvw_halo)
     double *fprop;                        // [PR_N][nf] property planes
