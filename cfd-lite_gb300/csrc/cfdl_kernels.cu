@@ -521,52 +521,65 @@ __global__ void __launch_bounds__(kTile) k_grad(const CaseDev *__restrict__ case
 __global__ void __launch_bounds__(kTile, 3) k_grad3_f32(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles) {
     CFDL_PDL_WAIT();
     TILE_PROLOGUE(cells)
-    if (i >= t.last) return;
-    const int ne = C.ne, W = C.W;
-    const double *phi[3] = {C.u, C.v, C.w};
-    double *grad[3] = {C.gu, C.gv, C.gw};
-    double pe[3];
-    float g[3][3];
+    __shared__ float sg[3][3 * kTile];
+    if (i < t.last) {
+        const int ne = C.ne, W = C.W;
+        const double *phi[3] = {C.u, C.v, C.w};
+        double pe[3];
+        float g[3][3];
 #pragma unroll
-    for (int q = 0; q < 3; q++) { pe[q] = phi[q][i]; g[q][0] = g[q][1] = g[q][2] = 0.f; }
-    // Every slot's loads are issued before the first is used: a loop that
-    // stopped at the first padding slot had to wait for each slot's index
-    // before it could load the next slot, six dependent trips to memory.  A
-    // row's slots end at its first padding slot (live), as that loop did.
-    // With 3 CTAs per SM (80 registers) this measured 203 -> 151 us at 128^3.
-    int nb[kMaxW];
-    bool live[kMaxW];
-    float G[3][kMaxW];
-    bool on = true;
+        for (int q = 0; q < 3; q++) { pe[q] = phi[q][i]; g[q][0] = g[q][1] = g[q][2] = 0.f; }
+        // Every slot's loads are issued before the first is used: a loop that
+        // stopped at the first padding slot had to wait for each slot's index
+        // before it could load the next slot, six dependent trips to memory.  A
+        // row's slots end at its first padding slot (live), as that loop did.
+        // With 3 CTAs per SM (80 registers) this measured 203 -> 151 us at 128^3.
+        int nb[kMaxW];
+        bool live[kMaxW];
+        float G[3][kMaxW];
+        bool on = true;
 #pragma unroll
-    for (int k = 0; k < kMaxW; k++) {
-        const int j = k < W ? C.hf_nb[k * ne + i] : -1;
+        for (int k = 0; k < kMaxW; k++) {
+            const int j = k < W ? C.hf_nb[k * ne + i] : -1;
 #pragma unroll
-        for (int m = 0; m < 3; m++) G[m][k] = k < W ? C.G32[(m * W + k) * ne + i] : 0.f;
-        on = on && j >= 0;
-        live[k] = on;
-        nb[k] = on ? j : i;
+            for (int m = 0; m < 3; m++) G[m][k] = k < W ? C.G32[(m * W + k) * ne + i] : 0.f;
+            on = on && j >= 0;
+            live[k] = on;
+            nb[k] = on ? j : i;
+        }
+        double pn[3][kMaxW];
+#pragma unroll
+        for (int k = 0; k < kMaxW; k++)
+#pragma unroll
+            for (int q = 0; q < 3; q++) pn[q][k] = phi[q][nb[k]];
+#pragma unroll
+        for (int k = 0; k < kMaxW; k++) {
+            if (!live[k]) continue;
+#pragma unroll
+            for (int q = 0; q < 3; q++) {
+                const float d = narrow_f32(pn[q][k] - pe[q]);
+                g[q][0] += G[0][k] * d; g[q][1] += G[1][k] * d; g[q][2] += G[2][k] * d;
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 3; q++)
+#pragma unroll
+            for (int m = 0; m < 3; m++) sg[q][3 * threadIdx.x + m] = g[q][m];
     }
-    double pn[3][kMaxW];
-#pragma unroll
-    for (int k = 0; k < kMaxW; k++)
-#pragma unroll
-        for (int q = 0; q < 3; q++) pn[q][k] = phi[q][nb[k]];
-#pragma unroll
-    for (int k = 0; k < kMaxW; k++) {
-        if (!live[k]) continue;
+    // the tile's gradients, three to a cell, are one range of each plane: written
+    // in its order (a cell's three by its own thread touched each sector of the
+    // planes several times: an outer iteration at 128^3 2922 us, 2900 so; the
+    // FP64 gradients, bound by their FP64 instructions, lose by it)
+    __syncthreads();
+    double *grad[3] = {C.gu, C.gv, C.gw};
+    const size_t at = 3 * (size_t)t.first;
+    for (int e = threadIdx.x; e < 3 * (t.last - t.first); e += kTile)
 #pragma unroll
         for (int q = 0; q < 3; q++) {
-            const float d = narrow_f32(pn[q][k] - pe[q]);
-            g[q][0] += G[0][k] * d; g[q][1] += G[1][k] * d; g[q][2] += G[2][k] * d;
+            const float g = sg[q][e];
+            C.g32[(size_t)q * 3 * C.ne + at + e] = g;
+            grad[q][at + e] = widen_f64(g);
         }
-    }
-#pragma unroll
-    for (int q = 0; q < 3; q++) {
-        float *g32 = C.g32 + (size_t)q * 3 * ne + 3 * i;
-#pragma unroll
-        for (int m = 0; m < 3; m++) { g32[m] = g[q][m]; grad[q][3 * i + m] = widen_f64(g[q][m]); }
-    }
 }
 
 // precision 3: g32 from gu, gv, gw after they were written from outside
