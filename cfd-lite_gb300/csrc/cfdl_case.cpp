@@ -65,12 +65,14 @@ int build_worklist(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &sizes, i
     return build_worklist(ctx, wl, sizes, std::vector<int>(sizes.size(), tile));
 }
 
-// Rows per thread of an FP64 pass with a reduction: one while the case's tiles
-// then fit the chip at once (152 SMs, four CTAs each), as a small case is bound
-// by its chain of latencies and by the SMs it leaves idle; four on large ones,
-// where the block's reduction is paid once for them.  It goes by the case alone,
-// so a case's sums are the same alone and in a batch.
-static int rows_per_thread(int ne) { return ne <= 152 * 4 * kTile ? 1 : ne <= 2 * 152 * 4 * kTile ? 2 : 4; }
+// Rows per thread of the fused momentum assembly, which has a reduction at its
+// end: one while the case's tiles then fit the chip at once (152 SMs, four CTAs
+// each), as a small case is bound by its chain of latencies and by the SMs it
+// leaves idle; else two: the block's reduction against the last wave (128^3, an
+// outer iteration of precision 3: 2926 us with one, 2915 with two, 2924 with
+// four or seven; tets of 45^3, 1367, 1365, 1371).  It goes by the case alone, so
+// a case's sums are the same alone and in a batch.
+static int rows_per_thread(int ne) { return ne <= 152 * 4 * kTile ? 1 : 2; }
 
 // Rows per thread of the FP64 solver passes: at least `least`, and on large
 // cases as many as put the case's tiles on the chip at once (152 SMs, four
@@ -507,6 +509,9 @@ int rebuild_worklists(cfdl_ctx *ctx) {
     if ((st = build_worklist(ctx, ctx->cellse, nc, kTile * ctx->en_vec))) return st;
     if ((st = build_merged(ctx, ctx->cellsem, nc, ctx->en_vec))) return st;
     if ((st = build_split(ctx, ctx->cellss, nc))) return st;
+    tiles.clear();
+    for (int ne : nc) tiles.push_back(kTile * (ctx->vec == kVec ? rows_one_wave(ne, kVec) : ctx->vec));
+    if ((st = build_worklist(ctx, ctx->cellsw, nc, tiles))) return st;
     tiles.clear();
     for (int ne : nc) tiles.push_back(kTile * rows_per_thread(ne));
     if ((st = build_worklist(ctx, ctx->cellsr, nc, tiles))) return st;

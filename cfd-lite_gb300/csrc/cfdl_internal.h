@@ -236,7 +236,8 @@ struct cfdl_ctx {
     cfdl::WorkList cellsv;               // wide tiles (kTile*vec cells) for the solver kernels; at the default vec
                                          // more on large FP64 flow cases (rows_one_wave)
     int vec = cfdl::kVec;                // cells per thread in those tiles (autotuned)
-    cfdl::WorkList cellsr;               // tiles of the FP64 passes whose shape goes by the case's size (rows_per_thread)
+    cfdl::WorkList cellsw;               // as cellsv for flow cases in FP64, in every form: for FP64 sums that are only compared
+    cfdl::WorkList cellsr;               // tiles of the fused momentum assembly (rows_per_thread)
     cfdl::WorkList cellse;               // tiles of the energy solve (kTile*en_vec cells)
     cfdl::WorkList cellsem;              // the same tiles, merged
     cfdl::WorkList cellss;               // cellsv's tiles, split (empty where they are not: see split_sums)
