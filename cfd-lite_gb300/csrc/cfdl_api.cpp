@@ -267,7 +267,7 @@ int cfdl_ctx_destroy(cfdl_ctx *ctx) {
     free_worklist(ctx->cellsv);
     free_worklist(ctx->cellse);
     free_worklist(ctx->cellsr);
-    free_worklist(ctx->cellsem); free_worklist(ctx->cellss); free_worklist(ctx->cellsw);
+    free_worklist(ctx->cellsem); free_worklist(ctx->cellss); free_worklist(ctx->cellsw); free_worklist(ctx->facesw);
     free_worklist(ctx->facesv);
     for (auto &wl : ctx->amg_cells) free_worklist(wl);
     for (auto &wl : ctx->amg_smooth) free_worklist(wl);

@@ -500,6 +500,12 @@ int rebuild_worklists(cfdl_ctx *ctx) {
     int st;
     if ((st = build_worklist(ctx, ctx->cells, nc))) return st;
     if ((st = build_worklist(ctx, ctx->faces, nfc))) return st;
+    // four faces per thread where that still fills the chip (8 CTAs per SM): a
+    // face pass of one face per thread spends a fifth of its time starting CTAs
+    // (128^3: 24 000 of them; an outer iteration of precision 3 2888 us, with two
+    // or four faces per thread 2867, with eight 2879; FP64 4424 and 4412).  A face
+    // is computed by itself, so the bits do not depend on it.
+    if ((st = build_worklist(ctx, ctx->facesw, nfc, kTile * (ctx->faces.ntiles >= 4 * 8 * 152 ? 4 : 1)))) return st;
     if ((st = build_worklist(ctx, ctx->facesv, nfc, kTile * kFaceVec))) return st;
     if ((st = build_worklist(ctx, ctx->halos, nh))) return st;
     std::vector<int> tiles;

@@ -241,6 +241,7 @@ struct cfdl_ctx {
     cfdl::WorkList cellse;               // tiles of the energy solve (kTile*en_vec cells)
     cfdl::WorkList cellsem;              // the same tiles, merged
     cfdl::WorkList cellss;               // cellsv's tiles, split (empty where they are not: see split_sums)
+    cfdl::WorkList facesw;               // face tiles of the passes bound by their CTAs' start: wider on large contexts
     cfdl::WorkList facesv;               // wide face tiles (kTile*kFaceVec faces) for face reductions
     int en_vec = 1;                      // cells per thread in those tiles (autotuned with the energy equation)
     int last_iters_m = 0, last_iters_p = 0, last_iters_e = 0;   // previous inner iteration counts (poll scheduling)

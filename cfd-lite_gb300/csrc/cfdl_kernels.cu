@@ -14,10 +14,12 @@
 namespace cfdl {
 namespace {
 
-#define TILE_PROLOGUE(WL)                         \
+#define TILE_HEAD_ENTITIES                        \
     const Tile t = tiles[blockIdx.x];             \
     const CaseDev &C = cases[t.c];                \
-    if (C.sc->halted) return;                     \
+    if (C.sc->halted) return;
+#define TILE_PROLOGUE(WL)                         \
+    TILE_HEAD_ENTITIES                            \
     const int i = t.first + (int)threadIdx.x;
 
 // ---------------------------------------------------------------------------
@@ -141,25 +143,26 @@ __global__ void __launch_bounds__(kTile) k_face_props(const CaseDev *__restrict_
 // gradients and planes, with no FP64 instruction; fS holds them as FP32.
 __global__ void __launch_bounds__(kTile) k_coef_uvw_face_f32(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles) {
     CFDL_PDL_WAIT();
-    TILE_PROLOGUE(faces)
-    if (i >= t.last) return;
-    const int nf = C.nf, ne = C.ne, o = C.f_own[i], n = C.f_nb[i];
-    if (n >= ne) return;
-    const float *pf = C.fprop32;
-    const float wt = pf[i], omw = 1.0f - wt;
-    const float A0 = pf[nf + i], A1 = pf[2 * nf + i], A2 = pf[3 * nf + i];
-    const float E0 = pf[4 * nf + i], E1 = pf[5 * nf + i], E2 = pf[6 * nf + i];
-    float gi[3][3];
+    TILE_HEAD_ENTITIES
+    FOR_CELLS(t) {
+        const int nf = C.nf, ne = C.ne, o = C.f_own[i], n = C.f_nb[i];
+        if (n >= ne) continue;
+        const float *pf = C.fprop32;
+        const float wt = pf[i], omw = 1.0f - wt;
+        const float A0 = pf[nf + i], A1 = pf[2 * nf + i], A2 = pf[3 * nf + i];
+        const float E0 = pf[4 * nf + i], E1 = pf[5 * nf + i], E2 = pf[6 * nf + i];
+        float gi[3][3];
 #pragma unroll
-    for (int q = 0; q < 3; q++) {
-        const float *g = C.g32 + (size_t)q * 3 * ne;
+        for (int q = 0; q < 3; q++) {
+            const float *g = C.g32 + (size_t)q * 3 * ne;
 #pragma unroll
-        for (int m = 0; m < 3; m++) gi[q][m] = omw * g[3 * o + m] + wt * g[3 * n + m];
+            for (int m = 0; m < 3; m++) gi[q][m] = omw * g[3 * o + m] + wt * g[3 * n + m];
+        }
+        float *fS = (float *)C.fS;
+#pragma unroll
+        for (int m = 0; m < 3; m++)
+            fS[m * nf + i] = (gi[0][m] * A0 + gi[1][m] * A1 + gi[2][m] * A2) + (gi[m][0] * E0 + gi[m][1] * E1 + gi[m][2] * E2);
     }
-    float *fS = (float *)C.fS;
-#pragma unroll
-    for (int m = 0; m < 3; m++)
-        fS[m * nf + i] = (gi[0][m] * A0 + gi[1][m] * A1 + gi[2][m] * A2) + (gi[m][0] * E0 + gi[m][1] * E1 + gi[m][2] * E2);
 }
 
 // calc_coef_uvw, boundary-condition loop (mod_uvwp.f90:242-273), one thread
@@ -703,35 +706,36 @@ __global__ void __launch_bounds__(kTile) k_calc_mip(const CaseDev *__restrict__ 
 // of an unsteady case stays FP64.
 __global__ void __launch_bounds__(kTile) k_calc_mip_f32(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles, int rc) {
     CFDL_PDL_WAIT();
-    TILE_PROLOGUE(faces)
-    if (i >= t.last) return;
-    const int nf = C.nf, o = C.f_own[i], n = C.f_nb[i];
-    if (n >= C.ne) return;
-    const double *g = C.fgeo;
-    const double wt = g[FG_WT * nf + i], omw = 1.0 - wt;
-    const double A0 = g[FG_AX * nf + i], A1 = g[FG_AY * nf + i], A2 = g[FG_AZ * nf + i];
-    const double vx = omw * C.u[o] + wt * C.u[n], vy = omw * C.v[o] + wt * C.v[n], vz = omw * C.w[o] + wt * C.w[n];
-    const double rhoip = C.fprop[PR_RHO * nf + i];
-    double mip = (vx * A0 + vy * A1 + vz * A2) * rhoip;
-    if (rc) {
-        const float *pf = C.fprop32;
-        const float wf = pf[i], omf = 1.0f - wf;
-        const float D0 = pf[7 * nf + i], D1 = pf[8 * nf + i], D2 = pf[9 * nf + i];
-        const float *gp = C.gp32;
-        const float gx = omf * gp[3 * o] + wf * gp[3 * n];
-        const float gy = omf * gp[3 * o + 1] + wf * gp[3 * n + 1];
-        const float gz = omf * gp[3 * o + 2] + wf * gp[3 * n + 2];
-        const float dip = omf * C.d32[o] + wf * C.d32[n];
-        const float dp = narrow_f32(C.p[n] - C.p[o]);
-        const float corr = dip * pf[10 * nf + i] * (dp - (gx * D0 + gy * D1 + gz * D2));
-        mip = mip - widen_f64(corr);
-        if (!C.steady) {
-            const double dip64 = omw * C.d[o] + wt * C.d[n];
-            const double ux = omw * C.u0[o] + wt * C.u0[n], uy = omw * C.v0[o] + wt * C.v0[n], uz = omw * C.w0[o] + wt * C.w0[n];
-            mip = mip - rhoip * dip64 * C.rdt * (C.mip0[i] - (ux * A0 + uy * A1 + uz * A2) * rhoip);
+    TILE_HEAD_ENTITIES
+    FOR_CELLS(t) {
+        const int nf = C.nf, o = C.f_own[i], n = C.f_nb[i];
+        if (n >= C.ne) continue;
+        const double *g = C.fgeo;
+        const double wt = g[FG_WT * nf + i], omw = 1.0 - wt;
+        const double A0 = g[FG_AX * nf + i], A1 = g[FG_AY * nf + i], A2 = g[FG_AZ * nf + i];
+        const double vx = omw * C.u[o] + wt * C.u[n], vy = omw * C.v[o] + wt * C.v[n], vz = omw * C.w[o] + wt * C.w[n];
+        const double rhoip = C.fprop[PR_RHO * nf + i];
+        double mip = (vx * A0 + vy * A1 + vz * A2) * rhoip;
+        if (rc) {
+            const float *pf = C.fprop32;
+            const float wf = pf[i], omf = 1.0f - wf;
+            const float D0 = pf[7 * nf + i], D1 = pf[8 * nf + i], D2 = pf[9 * nf + i];
+            const float *gp = C.gp32;
+            const float gx = omf * gp[3 * o] + wf * gp[3 * n];
+            const float gy = omf * gp[3 * o + 1] + wf * gp[3 * n + 1];
+            const float gz = omf * gp[3 * o + 2] + wf * gp[3 * n + 2];
+            const float dip = omf * C.d32[o] + wf * C.d32[n];
+            const float dp = narrow_f32(C.p[n] - C.p[o]);
+            const float corr = dip * pf[10 * nf + i] * (dp - (gx * D0 + gy * D1 + gz * D2));
+            mip = mip - widen_f64(corr);
+            if (!C.steady) {
+                const double dip64 = omw * C.d[o] + wt * C.d[n];
+                const double ux = omw * C.u0[o] + wt * C.u0[n], uy = omw * C.v0[o] + wt * C.v0[n], uz = omw * C.w0[o] + wt * C.w0[n];
+                mip = mip - rhoip * dip64 * C.rdt * (C.mip0[i] - (ux * A0 + uy * A1 + uz * A2) * rhoip);
+            }
         }
+        C.mip[i] = mip;
     }
-    C.mip[i] = mip;
 }
 
 // ---------------------------------------------------------------------------
@@ -741,14 +745,15 @@ __global__ void __launch_bounds__(kTile) k_calc_mip_f32(const CaseDev *__restric
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kTile) k_coef_p_face(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles) {
     CFDL_PDL_WAIT();
-    TILE_PROLOGUE(faces)
-    if (i >= t.last) return;
-    const int nf = C.nf, o = C.f_own[i], n = C.f_nb[i];
-    if (n >= C.ne) { C.fdiff[i] = 0.0; return; }
-    const double wt = C.fgeo[FG_WT * nf + i], omw = 1.0 - wt;
-    const double dip = omw * C.dc[o] + wt * C.dc[n];
-    C.fdiff[i] = dip * C.fprop[PR_RHOADN * nf + i];
-    C.fmip[i] = C.fprop[PR_RHOMADN * nf + i] * dip;
+    TILE_HEAD_ENTITIES
+    FOR_CELLS(t) {
+        const int nf = C.nf, o = C.f_own[i], n = C.f_nb[i];
+        if (n >= C.ne) { C.fdiff[i] = 0.0; continue; }
+        const double wt = C.fgeo[FG_WT * nf + i], omw = 1.0 - wt;
+        const double dip = omw * C.dc[o] + wt * C.dc[n];
+        C.fdiff[i] = dip * C.fprop[PR_RHOADN * nf + i];
+        C.fmip[i] = C.fprop[PR_RHOMADN * nf + i] * dip;
+    }
 }
 
 // the matrix: anb = the face coefficient on interior slots (0 on walls,
@@ -887,11 +892,12 @@ __global__ void __launch_bounds__(kTile) k_update_faces(const CaseDev *__restric
 // product and store take k_coef_p_face from 66 to 81 beside the momentum solve)
 __global__ void __launch_bounds__(kTile) k_update_faces_fresh(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles) {
     CFDL_PDL_WAIT();
-    TILE_PROLOGUE(faces)
-    if (i >= t.last) return;
-    const int o = C.f_own[i], n = C.f_nb[i];
-    if (n >= C.ne) return;
-    C.mip[i] = C.mip[i] - C.fmip[i] * (C.phic[n] - C.phic[o]);
+    TILE_HEAD_ENTITIES
+    FOR_CELLS(t) {
+        const int o = C.f_own[i], n = C.f_nb[i];
+        if (n >= C.ne) continue;
+        C.mip[i] = C.mip[i] - C.fmip[i] * (C.phic[n] - C.phic[o]);
+    }
 }
 
 // update_time, mod_physics.f90:101-112
@@ -938,7 +944,7 @@ static void launch_coef_uvw_faces(cfdl_ctx *ctx) {
     for (HostCase *hc : ctx->cases) hc->coef_is_pressure = false;
     if (f32_assembly(ctx)) ensure_g32(ctx);
     CFDL_LAUNCH("k_coef_uvw_halo", k_coef_uvw_halo, halos);
-    if (f32_assembly(ctx)) CFDL_LAUNCH("k_coef_uvw_face_f32", k_coef_uvw_face_f32, faces);
+    if (f32_assembly(ctx)) CFDL_LAUNCH("k_coef_uvw_face_f32", k_coef_uvw_face_f32, facesw);
     else {
         if (any_flow_fp64(ctx)) CFDL_LAUNCH("k_coef_uvw_face", k_coef_uvw_face<true>, faces);
         if (any_ordered(ctx)) CFDL_LAUNCH("k_coef_uvw_face", k_coef_uvw_face<false>, faces);
@@ -969,7 +975,7 @@ void launch_calc_mip(cfdl_ctx *ctx, int rc) {
     ensure_face_props(ctx);
     if (rc && f32_assembly(ctx)) {
         ensure_g32(ctx);
-        CFDL_LAUNCH("k_calc_mip", k_calc_mip_f32, faces, rc);
+        CFDL_LAUNCH("k_calc_mip", k_calc_mip_f32, facesw, rc);
         return;
     }
     if (any_flow_fp64(ctx)) CFDL_LAUNCH("k_calc_mip", k_calc_mip<true>, faces, rc);
@@ -977,7 +983,7 @@ void launch_calc_mip(cfdl_ctx *ctx, int rc) {
 }
 void launch_coef_p_matrix(cfdl_ctx *ctx) {
     ensure_face_props(ctx);
-    CFDL_LAUNCH("k_coef_p_face", k_coef_p_face, faces);
+    CFDL_LAUNCH("k_coef_p_face", k_coef_p_face, facesw);
     CFDL_LAUNCH("k_coef_p_mat", k_coef_p_mat, cells);
 }
 void launch_coef_p_rhs(cfdl_ctx *ctx) {
@@ -1002,7 +1008,7 @@ void launch_adjust_pc(cfdl_ctx *ctx) {
 void launch_update_uvwp(cfdl_ctx *ctx, bool fresh) {
     ensure_face_props(ctx);
     CFDL_LAUNCH("k_update_cells", k_update_cells, cells);
-    if (fresh) CFDL_LAUNCH("k_update_faces", k_update_faces_fresh, faces);
+    if (fresh) CFDL_LAUNCH("k_update_faces", k_update_faces_fresh, facesw);
     else CFDL_LAUNCH("k_update_faces", k_update_faces, faces);
 }
 void launch_update_time(cfdl_ctx *ctx) {
