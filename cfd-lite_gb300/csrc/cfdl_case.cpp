@@ -76,7 +76,7 @@ static int rows_per_thread(int ne) { return ne <= 152 * 4 * kTile ? 1 : 2; }
 
 // Rows per thread of the FP64 solver passes: at least `least`, and on large
 // cases as many as put the case's tiles on the chip at once (152 SMs, four
-// CTAs each).  A tile's reduction takes 17 FP64 warp adds per sum and its
+// CTAs each).  A tile's reduction takes 9 FP64 warp adds per sum and its
 // start and end a few thousand clocks, whatever its rows: at 128^3, 14 rows per
 // thread instead of four took an outer iteration from 4585 to 4425 us, 16 (two
 // waves again) 4520; a wave of five or eight CTAs per SM gave 4530 and 4440.

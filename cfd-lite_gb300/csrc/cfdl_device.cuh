@@ -11,7 +11,7 @@ namespace cfdl {
 #define CFDL_PDL_WAIT() asm volatile("griddepcontrol.wait;" ::: "memory")
 
 // Deterministic sums over the kTile threads of a block: K sums of v land in
-// shared out[0..K-1] (valid after the caller's next barrier).  The order is a
+// shared out[0..K-1] (written by the first warp; the others read it after a barrier).  The order is a
 // fixed tree over each warp's 32 values (lane l with l+16, then l+8, ...),
 // then the warps' sums in warp order.
 //
@@ -21,13 +21,16 @@ namespace cfdl {
 // steps, then the warps), more than the rows' own arithmetic when a thread has
 // few rows.  Here each thread stores its K values and warp k alone forms the
 // eight warps' trees of value k with every lane busy -- 4 adds for the first
-// step of all eight trees, 2, 1, 1 and 1 for the next -- and adds the eight
-// sums in order: 17 warp-adds, the same sums in the same order.
-// The sum of x[0..kTile-1] (shared) by one warp: each of the kTile / 32 warps'
-// shuffle tree, then the trees' sums in warp order.
-__device__ __forceinline__ double tree_sum(const double *v) {
-    constexpr int kWarps = kTile / 32;
-    static_assert(kWarps == 8, "the packing below is for eight warps");
+// step of all eight trees, 2, 1, 1 and 1 for the next -- and the eight sums of
+// all K values are added in order by one warp, a lane to a value: 9 K + 8
+// warp-adds, the same sums in the same order.  (With each warp adding its own
+// value's eight, 17 K, an FP64 outer iteration took 0.5% longer at 128^3, 0.8%
+// in a batch, 2.7% with the energy solve on 77^3 cells.)
+// One warp's part of the sum of v[0..kTile-1] (shared): the shuffle trees of the
+// block's kTile / 32 warps, packed so that they take 9 warp adds; the sum of
+// warp w's tree is left in dst[w].
+__device__ __forceinline__ void warp_trees(const double *v, double *dst) {
+    static_assert(kTile / 32 == 8, "the packing below is for eight warps");
     const int lane = threadIdx.x & 31;
     const bool b8 = (lane & 8) != 0, b4 = (lane & 4) != 0;
     // x[j]: lane l & 15 of tree w = 2 j + (lane >> 4) after its first step
@@ -48,21 +51,25 @@ __device__ __forceinline__ double tree_sum(const double *v) {
     z += __shfl_xor_sync(0xffffffffu, z, 2);
     z += __shfl_xor_sync(0xffffffffu, z, 1);
     // the sum of warp w = 2 j + h, j = (bit 8) + 2 (bit 4), is in lane 16 h + 8 (j & 1) + 4 (j >> 1)
-    double s = 0.0;
-#pragma unroll
-    for (int w = 0; w < kWarps; w++)
-        s += __shfl_sync(0xffffffffu, z, 16 * (w & 1) + 8 * ((w >> 1) & 1) + 4 * (w >> 2));
-    return s;
+    if ((lane & 3) == 0) dst[2 * ((lane >> 3 & 1) + 2 * (lane >> 2 & 1)) + (lane >> 4)] = z;
 }
+// out[k] is written by thread k of the first warp
 template <int K>
 __device__ __forceinline__ void block_sums(double (&v)[K], double *out) {
-    __shared__ double sm[K][kTile];
+    constexpr int kWarps = kTile / 32;
+    __shared__ double sm[K][kTile], ws[K][kWarps];
 #pragma unroll
     for (int k = 0; k < K; k++) sm[k][threadIdx.x] = v[k];
     __syncthreads();
-    for (int k = threadIdx.x >> 5; k < K; k += kTile / 32) {
-        const double s = tree_sum(sm[k]);
-        if ((threadIdx.x & 31) == 0) out[k] = s;
+    for (int k = threadIdx.x >> 5; k < K; k += kWarps) warp_trees(sm[k], ws[k]);
+    __syncthreads();
+    // the trees' sums in warp order, all values in one warp's lanes: 8 adds for
+    // the K of them, not 8 for each
+    if (threadIdx.x < K) {
+        double s = 0.0;
+#pragma unroll
+        for (int w = 0; w < kWarps; w++) s += ws[threadIdx.x][w];
+        out[threadIdx.x] = s;
     }
 }
 // FP32: a shuffle tree per warp, then the warps' sums in warp order (the order is
@@ -152,7 +159,7 @@ __device__ __forceinline__ bool case_sums(T (&v)[K], int *counter, T *partials, 
     T *part = partials + (size_t)tile0 * kNPart;
     const int tile = (int)blockIdx.x - tile0;
     block_sums<K>(v, s);
-    __syncthreads();
+    if (threadIdx.x < 32) __syncwarp();      // s is the first warp's
     if (threadIdx.x == 0) {
 #pragma unroll
         for (int k = 0; k < K; k++) __stcg(&part[(size_t)k * ntiles + tile], s[k]);
@@ -199,22 +206,16 @@ __device__ __forceinline__ bool merged_sums(int nm, int *counter, T *partials, i
     const int at = ((int)blockIdx.x - tile0) * M, lane = threadIdx.x & 31;
     T *buf = sum_buf<K, T, kSub>();
     __syncthreads();
-    if (sizeof(T) == 8) {
-        // each value's tree by one warp, its sum left in the buffer's first entry
-        for (int q = threadIdx.x >> 5; q < nm * K; q += kTile / 32) {
-            const double x = tree_sum((const double *)buf + q * kSumWidth<T>);
-            if (lane == 0) buf[q * kSumWidth<T>] = (T)x;
-        }
+    if constexpr (sizeof(T) == 8) {
+        for (int q = threadIdx.x >> 5; q < nm * K; q += kTile / 32)
+            warp_trees(buf + q * kSumWidth<T>, buf + q * kSumWidth<T>);   // read before it is written
         __syncthreads();
     }
     if (threadIdx.x < 32) {
         for (int q = lane; q < nm * K; q += 32) {
-            T x = buf[q * kSumWidth<T>];
-            if (sizeof(T) == 4) {
-                x = (T)0 + x;
+            T x = 0;
 #pragma unroll
-                for (int w = 1; w < kTile / 32; w++) x += buf[q * kSumWidth<T> + w];
-            }
+            for (int w = 0; w < kTile / 32; w++) x += buf[q * kSumWidth<T> + w];
             __stcg(&part[(size_t)(q % K) * nsub + at + q / K], x);
         }
         __syncwarp();
