@@ -1910,8 +1910,12 @@ __global__ void __launch_bounds__(kTile) k_mx_p(const CaseDev *__restrict__ case
     cg_p_rows<float>(C.fz, C.fp, S->iters32 == 0, S->beta32, t);
 }
 
+// q = A p; alpha = rz / (p, q).  Bound by the latency of its gathers: six CTAs
+// per SM (40 registers) instead of the four of the compiler's 62 took a mixed
+// pressure solve on 176^3 cells from 12560 to 12285 us; seven and eight
+// 12390.  With int32 indices 40 registers would spill.
 template <bool k16, bool kSpl>
-__global__ void __launch_bounds__(kTile) k_mx_q(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles,
+__global__ void __launch_bounds__(kTile, k16 ? 6 : 4) k_mx_q(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles,
                                                 const int *__restrict__ cfirst, const int *__restrict__ cnt, float *partials) {
     CFDL_PDL_WAIT();
     const Tile t = tiles[blockIdx.x];
@@ -1935,22 +1939,16 @@ __global__ void __launch_bounds__(kTile) k_mx_q(const CaseDev *__restrict__ case
     } else {
         // rows in pairs (pair_slots); then (p, q), each thread its rows 256 apart in
         // row order, which is the order of the FP32 sums
-        __shared__ __align__(8) float qs[2 * kTile];
+        __shared__ __align__(8) float qs[8 * kTile];     // a tile has at most 8 rows per thread
         const int tid = (int)threadIdx.x;
-        float v[1] = {0.f};
-        for (int c0 = t.first; c0 < t.last; c0 += 2 * kTile) {
-            const int i = c0 + 2 * tid, i0 = c0 + tid, i1 = i0 + kTile;
-            if (i < t.last) {
-                const float2 y = pair_amul_mesh<k16>(P, p, i);
-                *(float2 *)&C.fq[i] = y;
-                *(float2 *)&qs[2 * tid] = y;
-            }
-            const float p0 = i0 < t.last ? p[i0] : 0.f, p1 = i1 < t.last ? p[i1] : 0.f;
-            __syncthreads();
-            if (i0 < t.last) v[0] += p0 * qs[tid];
-            if (i1 < t.last) v[0] += p1 * qs[tid + kTile];
-            __syncthreads();
+        for (int i = t.first + 2 * tid; i < t.last; i += 2 * kTile) {
+            const float2 y = pair_amul_mesh<k16>(P, p, i);
+            *(float2 *)&C.fq[i] = y;
+            *(float2 *)&qs[i - t.first] = y;
         }
+        __syncthreads();
+        float v[1] = {0.f};
+        FOR_CELLS(t) v[0] += p[i] * qs[i - t.first];
         last = case_sums<1>(v, &C.counters[CNT_A3], partials, tile0, ntiles, s);
     }
     if (last) {
