@@ -61,10 +61,10 @@ __global__ void __launch_bounds__(kTile) k_bc(const CaseDev *__restrict__ cases,
 // diffusion mu*area/ds of the BC loop (mod_uvwp.f90:257).
 // ---------------------------------------------------------------------------
 // Bound by the FP64 pipe (4.5 us per instruction and 2.1M faces).  kFast
-// (precision 0): interpolation as go + wt (gn - go) and each component's six
+// (flow_fp64): interpolation as go + wt (gn - go) and each component's six
 // products as one chain, 36 FP64 instructions a face instead of 40
-// (445 -> 392 us at 128^3); the mixed forms keep the other order, on
-// which their FP32 roundings depend.
+// (445 -> 392 us at 128^3); the others keep the one order on which the mixed
+// forms' FP32 roundings and the energy solve depend.
 template <bool kFast>
 __global__ void __launch_bounds__(kTile) k_coef_uvw_face(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles) {
     CFDL_PDL_WAIT();
@@ -288,8 +288,8 @@ __global__ void __launch_bounds__(kTile) k_coef_uvw_cell(const CaseDev *__restri
 // instructions: rows without a boundary slot (the whole warp's) start their
 // sums from the first slot and skip the boundary terms, and sum b'^2 is formed
 // in tight mode only (otherwise it is only asked whether it is finite, see
-// kBigExp).  FORM 0 (precision 0) also takes its quotients by reciprocals
-// (rcp_near) and chains its sums.  FORM 1 (precision 1 and 2) and 3 (FP32
+// kBigExp).  FORM 0 (flow_fp64) also takes its quotients by reciprocals
+// (rcp_near) and chains its sums.  FORM 1 (precision 1 and 2, and FP64 with the energy equation) and 3 (FP32
 // explicit face terms) keep every rounding of the two kernels, spelled out
 // where the compiler could contract either of two products (div_rn rounds as
 // the division does).  At four CTAs per SM it
@@ -646,11 +646,11 @@ __global__ void k_check_conversions(int n, unsigned *bad) {
 
 // ---------------------------------------------------------------------------
 // calc_mip, mod_uvwp.f90:438-490.  One thread per face; boundary faces keep
-// the value their BC set.  Bound by the FP64 pipe.  kFast (precision 0): each
+// the value their BC set.  Bound by the FP64 pipe.  kFast (flow_fp64): each
 // side's dot products first, then one interpolation, so a vector's three
 // components cost 8 FP64 instructions instead of 9 and 1 - wt is not formed:
-// 23 a face instead of 26 (262 -> 228 us at 128^3); the mixed forms
-// keep the order their FP32 roundings depend on.
+// 23 a face instead of 26 (262 -> 228 us at 128^3); the others keep the one
+// order (see k_coef_uvw_face).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ double lerp64(double a, double b, double wt) { return a + wt * (b - a); }
 template <bool kFast>

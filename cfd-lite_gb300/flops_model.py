@@ -24,6 +24,11 @@ for them:
   k_mom_*          BiCGStab with three active right-hand sides
   k_v_* , k_apc_q  the pressure solve's mesh-level rows
 
+The counts are those of the forms that keep one order of sums (precision 1,
+and FP64 cases with the energy equation).  The FP64 flow alone executes fewer:
+36 per face in k_coef_uvw_face, three fewer in k_calc_mip, 8 and 7 per row in the
+mesh-level sweep and residual; its fractions of the pipe are high by as much.
+
 W = faces per cell; per-cell figures of the W-slot rows are scaled from the
 hex counts by W / 6.
 """
