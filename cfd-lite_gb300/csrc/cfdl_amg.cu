@@ -42,8 +42,6 @@ namespace {
 // cavity against 0.8 / 0.8: 2% less time per outer iteration, FP64 and
 // mixed alike (Chebyshev on [0.5, 2] 1%, [0.4, 2] 1% more; a coarse
 // over-correction of 2 instead of 3: 22% more).
-constexpr double kOmega = 0.557;   // first sweep
-constexpr double kOmega2 = 1.242;  // second sweep
 constexpr double kOverCorrect = 3.0;   // scaling of the prolongated coarse correction
 constexpr int kG = 8;                  // lanes per row on the small coarse levels
 constexpr int kGroupedRows = 65536;    // levels below this many rows (per case) run grouped
@@ -385,31 +383,20 @@ __device__ __forceinline__ bool mactive(const CaseDev &C) { return C.sc->active3
 // diagonal is therefore the sum of its row's off-diagonal couplings -- no
 // pass over the aggregate's members or its internal couplings.
 
-// level-0 diagonal inverse and the FP32 copies the mixed form needs
+// prep_row of every row of a matrix that came from elsewhere (k_coef_p_mat does
+// it for its own)
 __global__ void __launch_bounds__(kTile) k_amg_prep0(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles) {
     CFDL_PDL_WAIT();
     const Tile t = tiles[blockIdx.x];
     const CaseDev &C = cases[t.c];
     const int i = t.first + (int)threadIdx.x;
     if (i >= t.last || C.sc->halted) return;
-    const double ap = C.ap_p[i];
-    const bool mixed = C.precision >= 1;
     // the row's loads before its stores (a store holds back the loads after it)
+    const double ap = C.ap_p[i];
     double a[kMaxW];
 #pragma unroll
-    for (int k = 0; k < kMaxW; k++) a[k] = mixed && k < C.W ? C.anb_p[k * C.ne + i] : 0.0;
-    const double rd = div_rn(kOmega, ap);
-    C.rap_p[i] = rd;
-    if (!mixed) C.rap2_p[i] = rd * (kOmega2 / kOmega);
-    if (mixed) {
-        // the FP32 copies converted in the integer pipe (GB300 runs the hardware
-        // conversions at its FP64 rate)
-        C.fdiag_p[i] = narrow_f32(ap);
-        C.frap_p[i] = narrow_f32(rd);
-#pragma unroll
-        for (int k = 0; k < kMaxW; k++)
-            if (k < C.W) C.fanb_p[k * C.ld32 + i] = narrow_f32(a[k]);
-    }
+    for (int k = 0; k < kMaxW; k++) a[k] = C.precision >= 1 && k < C.W ? C.anb_p[k * C.ne + i] : 0.0;
+    prep_row(C, i, ap, a);
 }
 
 // Dense inverse of A_L + c 11^T at each case's coarsest level (one CTA per
@@ -1626,8 +1613,8 @@ template <class T> static void launch_tail(cfdl_ctx *ctx) {
 }
 
 // Coarse operators of every level and the coarsest inverse.
-static void amg_setup_operators(cfdl_ctx *ctx) {
-    ALAUNCH("k_amg_prep0", k_amg_prep0, ctx->cells);
+static void amg_setup_operators(cfdl_ctx *ctx, bool prepped) {
+    if (!prepped) ALAUNCH("k_amg_prep0", k_amg_prep0, ctx->cells);
     for (int l = 1; l <= ctx->amg_lmax; l++) {
         switch (ctx->amg_grouped[l]) {
         case 8: ALAUNCH("k_amg_gal", k_amg_galg<8>, ctx->amg_gcells[l], l); break;
@@ -1741,10 +1728,11 @@ void launch_pc_mean(cfdl_ctx *ctx);
 // multigrid operators (AMG), or the level-0 FP32 copies and 1/ap (mixed
 // Jacobi); the FP64 Jacobi form needs nothing.  In solve_uvwp this runs
 // beside the momentum solve (cfdl_graph.cu): it depends on dc only.
-void pressure_operators(cfdl_ctx *ctx) {
+void pressure_operators(cfdl_ctx *ctx, bool prepped) {
     const cfdl_config &c = ctx->cases[0]->cfg;
-    if (c.precond == 1) amg_setup_operators(ctx);
-    else if (c.precision >= 1) ALAUNCH("k_amg_prep0", k_amg_prep0, ctx->cells);
+    prepped = prepped && c.precision >= 1;       // as launch_coef_p_matrix
+    if (c.precond == 1) amg_setup_operators(ctx, prepped);
+    else if (c.precision >= 1 && !prepped) ALAUNCH("k_amg_prep0", k_amg_prep0, ctx->cells);
 }
 
 // FP64 AMG-PCG: zero-mean right-hand side, x = 0 (operators already built)

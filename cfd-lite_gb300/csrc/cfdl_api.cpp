@@ -148,8 +148,8 @@ int solve_uvwp_all(cfdl_ctx *ctx) {
     int st;
     if (ctx->cases[0]->cfg.precond == 1 && (st = ensure_amg(ctx))) return st;
     launch_coef_uvw_init(ctx);
-    launch_coef_p_matrix(ctx);
-    pressure_operators(ctx);
+    launch_coef_p_matrix(ctx, true);
+    pressure_operators(ctx, true);
     if ((st = solve_momentum_started(ctx))) return st;
     launch_grad(ctx, 4);
     if (ctx->ev_mom) cudaEventRecord(ctx->ev_mom, ctx->stream);

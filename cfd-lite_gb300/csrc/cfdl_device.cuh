@@ -460,4 +460,26 @@ __device__ __forceinline__ double div_rn(double b, double a) {
     return __fma_rn(__fma_rn(-a, q, b), y, q);
 }
 
+// the mesh level of the pressure multigrid: weights of the two sweeps
+constexpr double kOmega = 0.557;   // first sweep
+constexpr double kOmega2 = 1.242;  // second sweep
+
+// What the pressure solve needs of row i of its matrix (diagonal ap, couplings
+// a): the diagonal's inverse under the sweep weights and, in the mixed forms,
+// the FP32 copies, converted in the integer pipe (GB300 runs the hardware
+// conversions at its FP64 rate).
+__device__ __forceinline__ void prep_row(const CaseDev &C, int i, double ap, const double (&a)[kMaxW]) {
+    const bool mixed = C.precision >= 1;
+    const double rd = div_rn(kOmega, ap);
+    C.rap_p[i] = rd;
+    if (!mixed) C.rap2_p[i] = rd * (kOmega2 / kOmega);
+    if (mixed) {
+        C.fdiag_p[i] = narrow_f32(ap);
+        C.frap_p[i] = narrow_f32(rd);
+#pragma unroll
+        for (int k = 0; k < kMaxW; k++)
+            if (k < C.W) C.fanb_p[k * C.ld32 + i] = narrow_f32(a[k]);
+    }
+}
+
 }  // namespace cfdl

@@ -204,8 +204,8 @@ static int append_uvwp(Builder &b, cudaGraph_t G, cudaGraphNode_t *prev, Pre pre
     {
         const cudaGraphNode_t dep[1] = {*prev};
         if ((st = b.segment_after(G, dep, 1, [&] {
-                 launch_coef_p_matrix(ctx);
-                 pressure_operators(ctx);
+                 launch_coef_p_matrix(ctx, true);
+                 pressure_operators(ctx, true);
              }, &k, &branch)))
             return st;
         *static_k += k;

@@ -336,7 +336,7 @@ void launch_coef_uvw_init(cfdl_ctx *ctx);      // with the start of the momentum
 void launch_grad(cfdl_ctx *ctx, int field);     // 0 u, 1 v, 2 w, 3 phic, 4 = u,v,w fused, 5 = energy t, phi
 void launch_calc_mip(cfdl_ctx *ctx, int rhie_chow);
 void launch_coef_p(cfdl_ctx *ctx);             // matrix and right-hand side
-void launch_coef_p_matrix(cfdl_ctx *ctx);      // face coefficients, ap_p/anb_p (needs dc only)
+void launch_coef_p_matrix(cfdl_ctx *ctx, bool prep);   // face coefficients, ap_p/anb_p (needs dc only); prep: in the mixed forms also prep_row
 void launch_coef_p_rhs(cfdl_ctx *ctx);         // b (needs the fluxes of calc_mip)
 void launch_adjust_pc(cfdl_ctx *ctx);
 void launch_update_uvwp(cfdl_ctx *ctx, bool fresh);
@@ -418,7 +418,7 @@ int solve_momentum(cfdl_ctx *ctx);
 int solve_momentum_started(cfdl_ctx *ctx);      // after launch_coef_uvw_init
 int solve_pressure(cfdl_ctx *ctx);              // operators (multigrid / FP32 copies) + solve
 int solve_pressure_prepared(cfdl_ctx *ctx);     // the solve, operators already built
-void pressure_operators(cfdl_ctx *ctx);         // what the pressure solve needs of its matrix
+void pressure_operators(cfdl_ctx *ctx, bool prepped);   // what the pressure solve needs of its matrix (prepped: the rows are there)
 // AMG-preconditioned pressure solve (cfdl_amg.cu)
 int ensure_amg(cfdl_ctx *ctx);
 int solve_pressure_amg(cfdl_ctx *ctx);

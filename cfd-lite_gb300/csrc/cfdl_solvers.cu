@@ -935,7 +935,7 @@ int solve_pressure(cfdl_ctx *ctx) {
     if (ctx->cells.ntiles == 0) return CFDL_OK;
     int st;
     if (ctx->cases[0]->cfg.precond == 1 && (st = ensure_amg(ctx))) return st;
-    pressure_operators(ctx);
+    pressure_operators(ctx, false);
     return solve_pressure_prepared(ctx);
 }
 
