@@ -1927,7 +1927,7 @@ __global__ void __launch_bounds__(kTile, k16 ? 6 : 4) k_mx_q(const CaseDev *__re
     } else {
         // rows in pairs (pair_slots); then (p, q), each thread its rows 256 apart in
         // row order, which is the order of the FP32 sums
-        __shared__ __align__(8) float qs[8 * kTile];     // a tile has at most 8 rows per thread
+        __shared__ __align__(8) float qs[kMixedRows * kTile];   // solve_pressure_prepared and append_uvwp refuse wider tiles
         const int tid = (int)threadIdx.x;
         for (int i = t.first + 2 * tid; i < t.last; i += 2 * kTile) {
             const float2 y = pair_amul_mesh<k16>(P, p, i);

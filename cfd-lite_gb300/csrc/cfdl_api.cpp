@@ -16,8 +16,6 @@ using namespace cfdl;
 
 namespace {
 
-int check_ctx(const cfdl_ctx *ctx) { return ctx && !ctx->cases.empty() ? CFDL_OK : CFDL_ERR_INVALID; }
-
 int validate_config(const cfdl_config *c) {
     if (!c) return CFDL_ERR_INVALID;
     if (!(c->rho > 0) || !(c->mu >= 0) || !(c->dt > 0) || !(c->alpha_u > 0 && c->alpha_u <= 1) ||
@@ -227,21 +225,44 @@ int cfdl_set_config(cfdl_ctx *ctx, const cfdl_config *cfg) {
     int st = check_ctx(ctx);
     if (st) return st;
     if ((st = validate_config(cfg))) return st;
-    const bool reshape = ctx->cases[0]->cfg.precision != cfg->precision;   // the solver tiles go by the precision
-    for (HostCase *hc : ctx->cases) {
-        if (hc->cfg.rho != cfg->rho || hc->cfg.mu != cfg->mu) {
-            hc->props_dirty = true;
-            std::vector<double> rho(hc->ne, cfg->rho), mu(hc->ne, cfg->mu);
-            if ((st = cuda_status(cudaMemcpy(hc->dev.rho, rho.data(), hc->ne * sizeof(double), cudaMemcpyHostToDevice)))) return st;
-            if ((st = cuda_status(cudaMemcpy(hc->dev.mu, mu.data(), hc->ne * sizeof(double), cudaMemcpyHostToDevice)))) return st;
-        }
-        if (cfg->precision == 3 && (st = ensure_f32_assembly(hc, ctx->stream))) return st;
-        if (cfg->precision == 3 && hc->cfg.precision != 3) hc->g32_stale = true;
-        apply_config(hc, cfg);
-    }
-    if (!reshape) return upload_case_table(ctx);
     if ((st = cuda_status(cudaStreamSynchronize(ctx->stream)))) return st;
-    return rebuild_worklists(ctx);
+    // what can run out of memory first, for every case, and then every case's
+    // parameters: the lists and the kernels' forms go by them together
+    if (cfg->precision == 3)
+        for (HostCase *hc : ctx->cases)
+            if ((st = ensure_f32_assembly(hc, ctx->stream))) return st;
+    std::vector<cfdl_config> old;
+    std::vector<double> rho, mu;
+    bool reshape = false;                   // the solver tiles go by the precision
+    try {
+        size_t most = 0;
+        for (const HostCase *hc : ctx->cases) {
+            old.push_back(hc->cfg);
+            reshape |= hc->cfg.precision != cfg->precision;
+            if (hc->cfg.rho != cfg->rho || hc->cfg.mu != cfg->mu) most = std::max(most, (size_t)hc->ne);
+        }
+        rho.assign(most, cfg->rho);
+        mu.assign(most, cfg->mu);
+    } catch (const std::bad_alloc &) {
+        return CFDL_ERR_OOM;
+    }
+    for (HostCase *hc : ctx->cases) apply_config(hc, cfg);
+    st = reshape ? rebuild_worklists(ctx) : upload_case_table(ctx);
+    if (st) {                               // the old parameters stand; the next call restores their lists
+        for (size_t c = 0; c < old.size(); c++) apply_config(ctx->cases[c], &old[c]);
+        ctx->lists_stale = true;
+        return st;
+    }
+    for (size_t c = 0; c < old.size(); c++) {
+        HostCase *hc = ctx->cases[c];
+        // the FP32 planes and gradients are filled by what fills the FP64 ones
+        if (cfg->precision == 3 && old[c].precision != 3) hc->g32_stale = hc->props_dirty = true;
+        if (old[c].rho == cfg->rho && old[c].mu == cfg->mu) continue;
+        hc->props_dirty = true;
+        if ((st = cuda_status(cudaMemcpy(hc->dev.rho, rho.data(), hc->ne * sizeof(double), cudaMemcpyHostToDevice)))) return st;
+        if ((st = cuda_status(cudaMemcpy(hc->dev.mu, mu.data(), hc->ne * sizeof(double), cudaMemcpyHostToDevice)))) return st;
+    }
+    return CFDL_OK;
 }
 
 int cfdl_upload_fields(cfdl_ctx *ctx, const cfdl_fields *f) {
@@ -594,7 +615,11 @@ int cfdl_case_add(cfdl_ctx *ctx, const cfdl_mesh *mesh, const cfdl_config *cfg, 
     hc->id = ctx->next_id++;
     ctx->cases.push_back(hc);
     // construct_uvwp on zero fields leaves mip = mip0 = 0, as allocated
-    if ((st = rebuild_worklists(ctx))) return st;
+    if ((st = rebuild_worklists(ctx))) {    // the context goes on without the case
+        ctx->cases.pop_back();
+        destroy_case(hc);
+        return st;
+    }
     if (id) *id = hc->id;
     return CFDL_OK;
 }

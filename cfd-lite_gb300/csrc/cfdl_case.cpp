@@ -36,11 +36,20 @@ int cuda_status(cudaError_t e) {
     return CFDL_ERR_CUDA;
 }
 
-int case_alloc(HostCase *hc, void **p, size_t bytes) {
+// cfdl_fail_alloc: allocations of this thread until the one that fails (negative: none does)
+static thread_local int fail_alloc_in = -1;
+
+int dev_alloc(void **p, size_t bytes) {
     *p = nullptr;
-    if (bytes == 0) bytes = 16;
+    if (fail_alloc_in >= 0 && fail_alloc_in-- == 0) return CFDL_ERR_OOM;
     cudaError_t e = cudaMalloc(p, bytes);
     if (e != cudaSuccess) { *p = nullptr; cudaGetLastError(); return cuda_status(e); }
+    return CFDL_OK;
+}
+
+int case_alloc(HostCase *hc, void **p, size_t bytes) {
+    if (bytes == 0) bytes = 16;
+    if (int st = dev_alloc(p, bytes)) return st;
     hc->allocs.push_back(*p);
     hc->bytes += bytes;
     return CFDL_OK;
@@ -58,6 +67,7 @@ void free_worklist(WorkList &wl) {
     cudaFree(wl.d_tiles); cudaFree(wl.d_case_first); cudaFree(wl.d_case_ntiles);
     wl.d_tiles = nullptr; wl.d_case_first = nullptr; wl.d_case_ntiles = nullptr;
     wl.ntiles = 0;
+    wl.rows = 0;
 }
 
 // Tile list over per-case entity counts (sizes[c] = 0 leaves case c out).
@@ -97,6 +107,7 @@ int build_worklist(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &sizes, c
         wl.case_first.push_back((int)wl.h_tiles.size());
         int cnt = 0;
         const int tile = tiles[c];
+        if (sizes[c] > 0) wl.rows = std::max(wl.rows, split > 1 ? 1 : per_thread ? per_thread : (tile + kTile - 1) / kTile);
         for (int s = 0; s < sizes[c]; s += tile)
             for (int j = 0; j < split; j++, cnt++)
                 wl.h_tiles.push_back({(int)c, s, std::min(sizes[c], s + tile), split > 1 ? j : per_thread ? per_thread : (tile + kTile - 1) / kTile});
@@ -105,9 +116,9 @@ int build_worklist(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &sizes, c
     wl.ntiles = (int)wl.h_tiles.size();
     size_t nt = std::max<size_t>(1, wl.h_tiles.size()), ncs = std::max<size_t>(1, sizes.size());
     int st;
-    if ((st = cuda_status(cudaMalloc(&wl.d_tiles, nt * sizeof(Tile))))) return st;
-    if ((st = cuda_status(cudaMalloc(&wl.d_case_first, ncs * sizeof(int))))) return st;
-    if ((st = cuda_status(cudaMalloc(&wl.d_case_ntiles, ncs * sizeof(int))))) return st;
+    if ((st = dev_alloc((void **)&wl.d_tiles, nt * sizeof(Tile)))) return st;
+    if ((st = dev_alloc((void **)&wl.d_case_first, ncs * sizeof(int)))) return st;
+    if ((st = dev_alloc((void **)&wl.d_case_ntiles, ncs * sizeof(int)))) return st;
     if (!wl.h_tiles.empty()) {
         if ((st = cuda_status(cudaMemcpy(wl.d_tiles, wl.h_tiles.data(), wl.h_tiles.size() * sizeof(Tile), cudaMemcpyHostToDevice)))) return st;
         if ((st = cuda_status(cudaMemcpy(wl.d_case_first, wl.case_first.data(), wl.case_first.size() * sizeof(int), cudaMemcpyHostToDevice)))) return st;
@@ -494,7 +505,8 @@ static int build_split(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &size
 }
 
 // Tile work lists over every case of the context.
-int rebuild_worklists(cfdl_ctx *ctx) {
+static int rebuild_lists(cfdl_ctx *ctx) {
+    destroy_graph(ctx);   // captured launch arguments refer to the old lists
     std::vector<int> nc, nfc, nh;
     for (const HostCase *hc : ctx->cases) { nc.push_back(hc->ne); nfc.push_back(hc->nf); nh.push_back(hc->nbf); }
     int st;
@@ -529,13 +541,12 @@ int rebuild_worklists(cfdl_ctx *ctx) {
     for (auto &wl : ctx->amg_grestr) free_worklist(wl);
     ctx->amg_cells.clear(); ctx->amg_smooth.clear(); ctx->amg_gcells.clear(); ctx->amg_gsmooth.clear();
     ctx->amg_restr.clear(); ctx->amg_grestr.clear(); ctx->amg_lmax = -1;
-    destroy_graph(ctx);   // captured launch arguments refer to the old lists
     int need = std::max({ctx->cells.ntiles, ctx->faces.ntiles, ctx->halos.ntiles, ctx->cellss.ntiles,
                          ctx->cellsem.ntiles * ctx->cellsem.merge.M, 1});
     if (need > ctx->partials_cap) {
         cudaFree(ctx->d_partials);
         ctx->d_partials = nullptr;
-        int st = cuda_status(cudaMalloc(&ctx->d_partials, (size_t)need * kNPart * sizeof(double)));
+        int st = dev_alloc((void **)&ctx->d_partials, (size_t)need * kNPart * sizeof(double));
         if (st) { ctx->partials_cap = 0; return st; }
         ctx->partials_cap = need;
     }
@@ -545,11 +556,34 @@ int rebuild_worklists(cfdl_ctx *ctx) {
         ctx->h_flags = nullptr; ctx->d_flags = nullptr;
         int cap = std::max(ncases, 8);
         int st = cuda_status(cudaMallocHost(&ctx->h_flags, (size_t)cap * 4 * sizeof(int)));
-        if (!st) st = cuda_status(cudaMalloc(&ctx->d_flags, (size_t)cap * 4 * sizeof(int)));
+        if (!st) st = dev_alloc((void **)&ctx->d_flags, (size_t)cap * 4 * sizeof(int));
         if (st) { ctx->h_flags_cap = 0; return st; }
         ctx->h_flags_cap = cap;
     }
     return upload_case_table(ctx);
+}
+
+// The lists and the case table from the cases as they are.  Until all of it is
+// done the context is stale: nothing is launched over lists that belong to
+// other cases or another precision.
+int rebuild_worklists(cfdl_ctx *ctx) {
+    ctx->lists_stale = true;
+    int st;
+    try {
+        st = rebuild_lists(ctx);
+    } catch (const std::bad_alloc &) {
+        st = CFDL_ERR_OOM;
+    }
+    if (st) return st;
+    ctx->lists_stale = false;
+    return CFDL_OK;
+}
+
+int check_ctx(cfdl_ctx *ctx) {
+    if (!ctx || ctx->cases.empty()) return CFDL_ERR_INVALID;
+    if (!ctx->lists_stale) return CFDL_OK;
+    if (int st = cuda_status(cudaStreamSynchronize(ctx->stream))) return st;
+    return rebuild_worklists(ctx);
 }
 
 int upload_case_table(cfdl_ctx *ctx) {
@@ -558,7 +592,7 @@ int upload_case_table(cfdl_ctx *ctx) {
         cudaFree(ctx->d_cases);
         ctx->d_cases = nullptr;
         int cap = std::max(n, 8);
-        int st = cuda_status(cudaMalloc(&ctx->d_cases, (size_t)cap * sizeof(CaseDev)));
+        int st = dev_alloc((void **)&ctx->d_cases, (size_t)cap * sizeof(CaseDev));
         if (st) { ctx->d_cases_cap = 0; return st; }
         ctx->d_cases_cap = cap;
     }
@@ -571,3 +605,8 @@ int upload_case_table(cfdl_ctx *ctx) {
 }
 
 }  // namespace cfdl
+
+extern "C" int cfdl_fail_alloc(int n) {
+    cfdl::fail_alloc_in = n;
+    return CFDL_OK;
+}

@@ -187,6 +187,7 @@ static int append_uvwp(Builder &b, cudaGraph_t G, cudaGraphNode_t *prev, Pre pre
     const cfdl_config &cfg = ctx->cases[0]->cfg;
     int st;
     int64_t k = 0;
+    if (cfg.precision >= 1 && ctx->cellsv.rows > kMixedRows) return CFDL_ERR_INVALID;
     cudaGraphConditionalHandle hm, hp;
     if ((st = cuda_status(cudaGraphConditionalHandleCreate(&hm, G, 0, 0)))) return st;
     if ((st = cuda_status(cudaGraphConditionalHandleCreate(&hp, G, 0, 0)))) return st;

@@ -186,6 +186,7 @@ struct Tile { int c, first, last, pad; };
 struct Merge { int M, rows; };
 constexpr int kSplit = 4;               // blocks that share a tile of a split list, one row per thread
 static_assert(kSplit == kVec && kTile / kSplit % 32 == 0, "split_sums");
+constexpr int kMixedRows = 8;           // most rows per thread of a mixed form's solver tile (k_mx_q's shared buffer)
 constexpr int kMaxMerge = 4;            // most tiles a block takes (a shared buffer holds their values)
 
 // One work list per entity type, with each case's tile range for reductions.
@@ -194,6 +195,7 @@ struct WorkList {
     Merge merge{1, 1 << 30};            // merged lists: see merged_sums (cfdl_device.cuh)
     Tile *d_tiles = nullptr;
     int *d_case_first = nullptr, *d_case_ntiles = nullptr;
+    int rows = 0;                       // most entities per thread of a tile
     std::vector<Tile> h_tiles;
     std::vector<int> case_first, case_ntiles;
 };
@@ -232,6 +234,8 @@ struct cfdl_ctx {
     int next_id = 0;                     // id given to the next added case
     cfdl::CaseDev *d_cases = nullptr;
     int d_cases_cap = 0;
+    bool lists_stale = false;            // the tile lists or the case table do not match the cases (rebuilding them
+                                         // failed): check_ctx rebuilds them before anything is launched
     cfdl::WorkList cells, faces, halos;
     cfdl::WorkList cellsv;               // wide tiles (kTile*vec cells) for the solver kernels; at the default vec
                                          // more on large FP64 flow cases (rows_one_wave)
@@ -299,8 +303,10 @@ struct cfdl_ctx {
 
 namespace cfdl {
 int cuda_status(cudaError_t e);
+int dev_alloc(void **p, size_t bytes);            // cudaMalloc, its status as a CFDL_* code
 int case_alloc(HostCase *hc, void **p, size_t bytes);
 int rebuild_worklists(cfdl_ctx *ctx);
+int check_ctx(cfdl_ctx *ctx);                     // a context with cases and lists that match them
 int upload_case_table(cfdl_ctx *ctx);
 int create_case(cfdl_ctx *ctx, const cfdl_mesh *mesh, const cfdl_config *cfg, HostCase **out);
 // create_case in two halves: host tables (any thread), then device upload

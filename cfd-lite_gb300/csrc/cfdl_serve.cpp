@@ -320,14 +320,11 @@ void device_loop(cfdl_server *S) {
             changed = true;
         }
         if (res.empty()) continue;
-        if (changed && rebuild_worklists(ctx) != CFDL_OK) {
-            std::lock_guard<std::mutex> lk(S->mu);
-            S->device_status = CFDL_ERR_CUDA;
-        }
+        int st = changed || ctx->lists_stale ? rebuild_worklists(ctx) : CFDL_OK;
         // ---- run ----
         const auto t_run = Clock::now();
         int running = 0;
-        int st = run_outer(ctx, S->cfg.chunk, &running);
+        if (!st) st = run_outer(ctx, S->cfg.chunk, &running);    // never over lists of other cases
         const double dt_run = std::chrono::duration<double>(Clock::now() - t_run).count();
         std::lock_guard<std::mutex> lk(S->mu);
         S->resident = (int)res.size();

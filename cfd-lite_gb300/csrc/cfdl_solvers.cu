@@ -941,7 +941,8 @@ int solve_pressure(cfdl_ctx *ctx) {
 
 int solve_pressure_prepared(cfdl_ctx *ctx) {
     if (ctx->cells.ntiles == 0) return CFDL_OK;
-    if (ctx->cases[0]->cfg.precision >= 1) return solve_pressure_mixed(ctx);
+    if (ctx->cases[0]->cfg.precision >= 1)
+        return ctx->cellsv.rows <= kMixedRows ? solve_pressure_mixed(ctx) : CFDL_ERR_INVALID;
     if (ctx->cases[0]->cfg.precond == 1) return solve_pressure_amg(ctx);
     pcj_init(ctx);
     const int cap = max_cap(ctx);

@@ -87,7 +87,7 @@ extern "C" {
 
 int cfdl_set_tile(cfdl_ctx *ctx, int vec) {
     if (!ctx || ctx->cases.empty() || !valid_shape(vec)) return CFDL_ERR_INVALID;
-    if (vec == ctx->vec) return CFDL_OK;
+    if (vec == ctx->vec && !ctx->lists_stale) return CFDL_OK;
     int st = cuda_status(cudaStreamSynchronize(ctx->stream));
     if (st) return st;
     ctx->vec = vec;
@@ -98,7 +98,7 @@ int cfdl_get_tile(const cfdl_ctx *ctx) { return ctx ? ctx->vec : -1; }
 
 int cfdl_set_energy_tile(cfdl_ctx *ctx, int vec) {
     if (!ctx || ctx->cases.empty() || !valid_shape(vec)) return CFDL_ERR_INVALID;
-    if (vec == ctx->en_vec) return CFDL_OK;
+    if (vec == ctx->en_vec && !ctx->lists_stale) return CFDL_OK;
     int st = cuda_status(cudaStreamSynchronize(ctx->stream));
     if (st) return st;
     ctx->en_vec = vec;
@@ -154,10 +154,11 @@ static int time_energy(cfdl_ctx *ctx, Snapshot &snap, int outer, cudaEvent_t e0,
 }
 
 int cfdl_autotune(cfdl_ctx *ctx, int outer, int *best, double *ms) {
-    if (!ctx || ctx->cases.empty() || outer <= 0) return CFDL_ERR_INVALID;
-    Snapshot snap;
-    int st = snap.take(ctx);
+    int st = check_ctx(ctx);
     if (st) return st;
+    if (outer <= 0) return CFDL_ERR_INVALID;
+    Snapshot snap;
+    if ((st = snap.take(ctx))) return st;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if ((st = cuda_status(cudaEventCreate(&e0)))) return st;
     if ((st = cuda_status(cudaEventCreate(&e1)))) { cudaEventDestroy(e0); return st; }
