@@ -1310,16 +1310,14 @@ namespace {
 
 template <class T, class A> int dupload(HostCase *hc, T **d, const std::vector<T, A> &h) {
     size_t bytes = std::max<size_t>(1, h.size()) * sizeof(T);
-    cudaError_t e = cudaMalloc((void **)d, bytes);
-    if (e != cudaSuccess) { cudaGetLastError(); return cuda_status(e); }
+    if (int st = dev_alloc((void **)d, bytes)) return st;
     hc->amg_allocs.push_back(*d);
     hc->bytes += bytes;
     if (h.empty()) return CFDL_OK;
     return cuda_status(cudaMemcpy(*d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
 }
 template <class T> int dzeros(HostCase *hc, T **d, size_t n) {
-    cudaError_t e = cudaMalloc((void **)d, std::max<size_t>(1, n) * sizeof(T));
-    if (e != cudaSuccess) { cudaGetLastError(); return cuda_status(e); }
+    if (int st = dev_alloc((void **)d, std::max<size_t>(1, n) * sizeof(T))) return st;
     hc->amg_allocs.push_back(*d);
     hc->bytes += std::max<size_t>(1, n) * sizeof(T);
     return cuda_status(cudaMemset(*d, 0, std::max<size_t>(1, n) * sizeof(T)));
@@ -1440,12 +1438,10 @@ template <class T> static int build_tail_plan(HostCase *hc, const AmgLevelDev *l
     return CFDL_OK;
 }
 
-// Upload a host-built hierarchy into the case, which takes ownership of it.
-int upload_case_amg(HostCase *hc, AmgHierarchy *H) {
+static int upload_hierarchy(HostCase *hc, const AmgHierarchy *H) {
     CaseDev &d = hc->dev;
     const int ne = hc->ne;
     int st;
-    hc->amg = H;
     const int nlev = (int)H->levels.size();
     std::vector<AmgLevelDev> devl(nlev);
     for (int l = 0; l < nlev; l++) {
@@ -1506,6 +1502,25 @@ int upload_case_amg(HostCase *hc, AmgHierarchy *H) {
     return CFDL_OK;
 }
 
+// Upload a host-built hierarchy into the case, which takes ownership of it.
+// After a failure the case has none and the next solve builds it again.
+int upload_case_amg(HostCase *hc, AmgHierarchy *H) {
+    const size_t before = hc->bytes;
+    hc->amg = H;
+    const int st = upload_hierarchy(hc, H);
+    if (!st) return CFDL_OK;
+    for (void *p : hc->amg_allocs) cudaFree(p);
+    hc->amg_allocs.clear();
+    hc->bytes = before;
+    delete hc->amg;
+    hc->amg = nullptr;
+    CaseDev &d = hc->dev;
+    d.nlev = d.ncoarse = d.amg_tail = 0;
+    d.lev = nullptr; d.cinv = nullptr; d.cinv32 = nullptr; d.nb16 = nullptr;
+    d.tail64 = d.tail32 = nullptr;
+    return st;
+}
+
 
 int ensure_amg(cfdl_ctx *ctx) {
     bool changed = false;
@@ -1520,6 +1535,7 @@ int ensure_amg(cfdl_ctx *ctx) {
     for (HostCase *hc : ctx->cases) all16 = all16 && hc->dev.nb16 != nullptr;
     if (all16 != ctx->amg_nb16) { ctx->amg_nb16 = all16; destroy_graph(ctx); }
     if (!changed && ctx->amg_lmax >= 0) return CFDL_OK;
+    ctx->amg_lmax = -1;                  // until the lists below are there
     int lmax = 0;
     for (HostCase *hc : ctx->cases) lmax = std::max(lmax, hc->dev.nlev);
     for (auto &wl : ctx->amg_cells) free_worklist(wl);

@@ -103,3 +103,19 @@ def test_case_add_out_of_memory(need_gpu):
     for g in (a, b):
         g.step(2, 0)
     _same(a, b)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_hierarchy_out_of_memory(need_gpu, precision):
+    """The multigrid hierarchy is built by the first solve: one that runs out of
+    memory there leaves none half built for the next."""
+    s = cfdl.Setup(cfdl.Zone(24, jitter=0.1, seed=2))
+    a, b = (cfdl.Solver(s, cfdl.steady(precision=precision)) for _ in range(2))
+    L = cfdl.lib()
+    failed = _until_it_succeeds(lambda: L.cfdl_step(b._h, 1, 0, None), lambda n: None)
+    assert failed > 30
+    a.step(1, 0)
+    for g in (a, b):
+        g.step(1, 0)
+    for f in FIELDS:
+        assert np.array_equal(a.get(f), b.get(f)), f
