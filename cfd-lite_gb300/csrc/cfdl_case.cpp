@@ -541,6 +541,8 @@ static int rebuild_lists(cfdl_ctx *ctx) {
     for (auto &wl : ctx->amg_grestr) free_worklist(wl);
     ctx->amg_cells.clear(); ctx->amg_smooth.clear(); ctx->amg_gcells.clear(); ctx->amg_gsmooth.clear();
     ctx->amg_restr.clear(); ctx->amg_grestr.clear(); ctx->amg_lmax = -1;
+    // a case added since may have no 16-bit offsets (without multigrid ensure_amg does not look again)
+    for (const HostCase *hc : ctx->cases) ctx->amg_nb16 = ctx->amg_nb16 && hc->dev.nb16;
     int need = std::max({ctx->cells.ntiles, ctx->faces.ntiles, ctx->halos.ntiles, ctx->cellss.ntiles,
                          ctx->cellsem.ntiles * ctx->cellsem.merge.M, 1});
     if (need > ctx->partials_cap) {

@@ -806,8 +806,7 @@ static void mom_init(cfdl_ctx *ctx) { CFDL_LAUNCH("k_mom_init", k_mom_init, cell
 
 void mom_iter(cfdl_ctx *ctx) {
     if (ctx->cases[0]->cfg.precision >= 2) {
-        bool n16 = ctx->amg_nb16;           // the 16-bit neighbour offsets, where every case has them
-        for (const HostCase *hc : ctx->cases) n16 = n16 && hc->dev.nb16;   // (one added since may not)
+        const bool n16 = ctx->amg_nb16;     // the 16-bit neighbour offsets, where every case has them
         if (ctx->cellss.ntiles) {
             CFDL_LAUNCH("k_mom_p", (k_mom_p<float, 3>), cells);
             if (n16) CFDL_LAUNCH("k_mom_v", (k_mom_v<float, 3, true, true>), cellss, REDS32);

@@ -119,3 +119,23 @@ def test_hierarchy_out_of_memory(need_gpu, precision):
         g.step(1, 0)
     for f in FIELDS:
         assert np.array_equal(a.get(f), b.get(f)), f
+
+
+@pytest.mark.parametrize("precision", [1, 2, 3])
+def test_case_added_without_multigrid(need_gpu, precision):
+    """The 16-bit offsets come with the multigrid set-up: a case added after the
+    preconditioner was changed has none, so its context goes without them."""
+    s, t = (cfdl.Setup(cfdl.Zone(n, jitter=0.1, seed=n)) for n in (12, 7))
+    jac = cfdl.steady(precision=precision, precond=0)
+    a = cfdl.Batch([s], [cfdl.steady(precision=precision)])
+    b = cfdl.Batch([s, t], [jac, jac])
+    start = {f: a.case_get(0, f) for f in STATE}
+    a.step(1, 0)
+    assert a.index_bytes() == 2
+    a.set_config(jac)
+    assert a.add(t, jac) == 1
+    for f, v in start.items():
+        a.case_set(0, f, v)
+    for g in (a, b):
+        g.step(2, 0)
+    _same(a, b)
