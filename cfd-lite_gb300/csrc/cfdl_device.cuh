@@ -437,17 +437,28 @@ __device__ __forceinline__ double widen_f64(float f) {
 }
 
 // b / a, correctly rounded, for a row's quotients.  The built-in FP64 division
-// is about 18 FP64 instructions, 4 us each per 2.1M rows on GB300; this is 7.
-// The reciprocal of a starts from the FP32 one (22 bits; FP32 and integer
-// instructions only) and takes two Newton steps, y += y (1 - a y), to within
-// a half ulp; the quotient q = b y is then corrected by its remainder,
-// q += y (b - a q), which rounds it correctly (Markstein, IBM J. Res. Dev. 34,
-// 1990).  Numbers near the ends of either format's range, zeros and
-// non-finite values take the division.
-__device__ __forceinline__ bool rcp_in_range(double a) {      // 2^-100 <= |a| < 2^101
-    const unsigned e = (unsigned)(__double2hiint(a) >> 20) & 0x7ffu;
-    return e - (1023u - 100u) <= 200u;
+// is about 18 FP64 instructions; this is 7.  The reciprocal of a starts from
+// the FP32 one (22 bits; FP32 and integer instructions only) and takes two
+// Newton steps, y += y (1 - a y); the quotient q = b y is then corrected by its
+// remainder, q += y (b - a q) (Markstein, IBM J. Res. Dev. 34, 1990).
+//
+// Why it rounds correctly, with significands 1 <= a, b < 2: the second step's y
+// is within half an ulp of 1/a times 1 + 2^-32 (its exact value within 2^-86),
+// so |a y - 1| <= 2^-54 a (1 + 2^-32), and b y is off b/a by less than one ulp.
+// Where b/a is next to the middle of two numbers, q is therefore one of these
+// two, half an ulp away; its remainder is exact, and the corrected value is off
+// by less than half an ulp times 2^-54 a (1 + 2^-32).  The middle itself is at
+// least 1/(2^54 A) from b/a with A = 2^52 a the integer significand (both over
+// A, two integers that differ): 2/a against a/2 in the same unit, so the
+// rounding falls on the right side for every a below 2 (1 - 2^-33).  A
+// significand nearer to 2 can fail (1 / (2 - 2^-52) would come out 0.5), so all
+// whose upper 20 bits are ones take the division, and so do numbers near the
+// ends of either format's range, zeros and non-finite values.
+__device__ __forceinline__ bool rcp_in_range(double a) {      // 2^-100 <= |a| < 2^101, significand below 2 - 2^-20
+    const unsigned h = (unsigned)__double2hiint(a), e = h >> 20 & 0x7ffu;
+    return e - (1023u - 100u) <= 200u && (h & 0xfffffu) != 0xfffffu;
 }
+// 1 / a within half an ulp times 1 + 2^-32, for a in range
 __device__ __forceinline__ double rcp_near(double a) {
     const double y0 = widen_f64(__fdividef(1.0f, narrow_f32(a)));
     const double y1 = __fma_rn(y0, __fma_rn(-a, y0, 1.0), y0);
