@@ -288,8 +288,8 @@ __global__ void __launch_bounds__(kTile) k_coef_uvw_cell(const CaseDev *__restri
 // instructions: rows without a boundary slot (the whole warp's) start their
 // sums from the first slot and skip the boundary terms, and sum b'^2 is formed
 // in tight mode only (otherwise it is only asked whether it is finite, see
-// kBigExp).  FORM 0 (flow_fp64) also takes its quotients by reciprocals
-// (rcp_near) and chains its sums.  FORM 1 (precision 1 and 2, and FP64 with the energy equation) and 3 (FP32
+// kBigExp).  FORM 0 (flow_fp64) also takes the Jacobi scaling from the
+// reciprocal behind d (rcp_near) and chains its sums.  FORM 1 (precision 1 and 2, and FP64 with the energy equation) and 3 (FP32
 // explicit face terms) keep every rounding of the two kernels, spelled out
 // where the compiler could contract either of two products (div_rn rounds as
 // the division does).  At four CTAs per SM it
@@ -377,7 +377,7 @@ __device__ __forceinline__ void coef_init_row(const CaseDev &C, int i, const int
     if (FORM == 0) {
         C.rap[i] = rcp_in_range(ap) ? rcp_near(ap) : 1.0 / ap;   // the Jacobi scaling of the solve
         C.d[i] = div_rn(vol, ap);
-        C.dc[i] = rcp_in_range(ec) ? vol * rcp_near(ec) : vol / ec;
+        C.dc[i] = div_rn(vol, ec);
     } else {
         const double dd = div_rn(vol, ap);
         C.d[i] = dd;
