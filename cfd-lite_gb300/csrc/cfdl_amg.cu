@@ -429,10 +429,17 @@ __global__ void __launch_bounds__(kInvThreads) k_amg_coarse_inv(const CaseDev *_
     constexpr int kPer = kAmgCoarsest * kAmgCoarsest / kInvThreads;
     for (int e = tid; e < n * n; e += kInvThreads) M[e] = cc + (e / n == e % n ? dg[e / n] : 0.0);
     __syncthreads();
-    for (int s = tid; s < P.W * n; s += kInvThreads) {     // a row has one slot per neighbour
-        const int e = s % n, j = P.nb[s];
-        const double a = P.a[s];
-        if (j >= 0 && j < n) M[e * n + j] -= a;
+    if (C.nlev > 0) {
+        for (int s = tid; s < P.W * n; s += kInvThreads) { // a coarse row has one slot per neighbour
+            const int e = s % n, j = P.nb[s];
+            const double a = P.a[s];
+            if (j >= 0 && j < n) M[e * n + j] -= a;
+        }
+    } else if (tid < n) {                                  // cells of a mesh may share several faces: a thread to a row
+        for (int k = 0; k < P.W; k++) {
+            const int j = P.nb[k * n + tid];
+            if (j >= 0 && j < n) M[tid * n + j] -= P.a[k * n + tid];
+        }
     }
     __syncthreads();
     double m[kPer];
