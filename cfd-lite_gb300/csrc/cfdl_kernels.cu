@@ -438,7 +438,10 @@ __device__ __forceinline__ void coef_init_row(const CaseDev &C, int i, const int
 template <int FORM, int W>
 __device__ __forceinline__ void coef_init_rows(const CaseDev &C, const Tile &t, double (&v)[6]) {
     const int ne = C.ne;
-    FOR_CELLS(t) {
+    // every lane goes through the tile's rows, so that the whole warp votes; a
+    // lane past the tile's end votes with its last row and takes neither branch
+    for (int r = 0, row = t.first + (int)threadIdx.x; r < t.pad; r++, row += kTile) {
+        const int i = min(row, t.last - 1);
         int nb[W], fc[W];
         bool inner = true;
 #pragma unroll
@@ -447,7 +450,9 @@ __device__ __forceinline__ void coef_init_rows(const CaseDev &C, const Tile &t, 
             fc[k] = k < C.W ? C.hf_fc[k * ne + i] : 0;
             inner = inner && (k >= C.W || (nb[k] >= 0 && nb[k] < ne));
         }
-        if (__all_sync(__activemask(), inner)) coef_init_row<FORM, W, true>(C, i, nb, fc, v);
+        const bool whole = __all_sync(0xffffffffu, inner);
+        if (row >= t.last) continue;
+        if (whole) coef_init_row<FORM, W, true>(C, i, nb, fc, v);
         else coef_init_row<FORM, W, false>(C, i, nb, fc, v);
     }
 }
