@@ -1384,13 +1384,12 @@ int prepare_case_amg(CasePrep *p) {
     return CFDL_OK;
 }
 
-// The plan of a case's tail for one precision, uploaded once (its hierarchy
-// does not change).
-template <class T> static int build_tail_plan(HostCase *hc, const AmgLevelDev *lev, const TailPlan **out, int *smem) {
+// The plan of a case's tail for one precision.
+template <class T> static int build_tail_plan(const HostCase *hc, const AmgLevelDev *lev, TailPlan &plan, int *smem) {
     const CaseDev &d = hc->dev;
     const int lt = d.amg_tail, nl = d.nlev - lt;
     constexpr int sz = (int)sizeof(T);
-    TailPlan plan{}, *P = &plan;
+    TailPlan *P = &plan;
     int at = 0;
     auto take = [&](long bytes) { const int o = at; at += (int)((bytes + 15) & ~15L); return o; };
     auto rows = [&](int l) { return l == 0 ? hc->ne : lev[l - 1].n; };
@@ -1436,11 +1435,6 @@ template <class T> static int build_tail_plan(HostCase *hc, const AmgLevelDev *l
     }
     P->total = at;
     if (at > kTailMaxSmem) return CFDL_ERR_MESH;           // cannot happen (see TailPlan)
-    TailPlan *dp = nullptr;
-    int st = dzeros(hc, &dp, 1);
-    if (st) return st;
-    if ((st = cuda_status(cudaMemcpy(dp, P, sizeof(TailPlan), cudaMemcpyHostToDevice)))) return st;
-    *out = dp;
     *smem = at;
     return CFDL_OK;
 }
@@ -1501,11 +1495,14 @@ static int upload_hierarchy(HostCase *hc, const AmgHierarchy *H) {
     d.amg_tail = 0;
     for (int l = 1; l <= nlev; l++)
         if (H->levels[l - 1].n <= kTailRows) { d.amg_tail = l; break; }
-    const TailPlan *tp = nullptr;
-    if ((st = build_tail_plan<double>(hc, devl.data(), &tp, &hc->tail_smem64))) return st;
-    d.tail64 = tp;
-    if ((st = build_tail_plan<float>(hc, devl.data(), &tp, &hc->tail_smem32))) return st;
-    d.tail32 = tp;
+    // both plans, uploaded once: the hierarchy does not change
+    std::vector<TailPlan> plans(2);
+    if ((st = build_tail_plan<double>(hc, devl.data(), plans[0], &hc->tail_smem64))) return st;
+    if ((st = build_tail_plan<float>(hc, devl.data(), plans[1], &hc->tail_smem32))) return st;
+    TailPlan *dp = nullptr;
+    if ((st = dupload(hc, &dp, plans))) return st;
+    d.tail64 = dp;
+    d.tail32 = dp + 1;
     return CFDL_OK;
 }
 
@@ -1545,12 +1542,6 @@ int ensure_amg(cfdl_ctx *ctx) {
     ctx->amg_lmax = -1;                  // until the lists below are there
     int lmax = 0;
     for (HostCase *hc : ctx->cases) lmax = std::max(lmax, hc->dev.nlev);
-    for (auto &wl : ctx->amg_cells) free_worklist(wl);
-    for (auto &wl : ctx->amg_smooth) free_worklist(wl);
-    for (auto &wl : ctx->amg_gcells) free_worklist(wl);
-    for (auto &wl : ctx->amg_gsmooth) free_worklist(wl);
-    for (auto &wl : ctx->amg_restr) free_worklist(wl);
-    for (auto &wl : ctx->amg_grestr) free_worklist(wl);
     ctx->amg_cells.assign(lmax + 1, WorkList());
     ctx->amg_smooth.assign(lmax + 1, WorkList());
     ctx->amg_gcells.assign(lmax + 1, WorkList());
@@ -1566,23 +1557,27 @@ int ensure_amg(cfdl_ctx *ctx) {
             smooth.push_back(l < hc->dev.amg_tail ? n : 0);
             restr.push_back(l >= 1 && l <= hc->dev.amg_tail ? n : 0);
         }
-        int st;
-        if ((st = build_worklist(ctx, ctx->amg_cells[l], cells))) return st;
-        if ((st = build_worklist(ctx, ctx->amg_smooth[l], smooth))) return st;
-        if ((st = build_worklist(ctx, ctx->amg_restr[l], restr))) return st;
+        plan_worklist(ctx->amg_cells[l], cells);
+        plan_worklist(ctx->amg_smooth[l], smooth);
+        plan_worklist(ctx->amg_restr[l], restr);
         // lanes per row: 8 when every case's level is small, else the tuned
         // cgroup (1 = one thread per row); the mesh level is always 1
         const int nmax = *std::max_element(cells.begin(), cells.end());
         const int G = l == 0 ? 1 : nmax < kGroupedRows ? kG : ctx->cgroup;
         ctx->amg_grouped[l] = G;
         if (G > 1) {
-            if ((st = build_worklist(ctx, ctx->amg_gcells[l], cells, kTile / G))) return st;
-            if ((st = build_worklist(ctx, ctx->amg_gsmooth[l], smooth, kTile / G))) return st;
-            if ((st = build_worklist(ctx, ctx->amg_grestr[l], restr, kTile / G))) return st;
+            plan_worklist(ctx->amg_gcells[l], cells, kTile / G);
+            plan_worklist(ctx->amg_gsmooth[l], smooth, kTile / G);
+            plan_worklist(ctx->amg_grestr[l], restr, kTile / G);
         }
     }
-    ctx->amg_lmax = lmax;
-    return upload_case_table(ctx);
+    std::vector<WorkList *> lists;
+    for (auto *v : {&ctx->amg_cells, &ctx->amg_smooth, &ctx->amg_restr, &ctx->amg_gcells, &ctx->amg_gsmooth, &ctx->amg_grestr})
+        for (WorkList &wl : *v) lists.push_back(&wl);
+    int st = upload_worklists(ctx, ctx->amg_list_buf, lists);
+    if (!st) st = upload_case_table(ctx);
+    if (!st) ctx->amg_lmax = lmax;
+    return st;
 }
 
 #define ALAUNCH(name, kern, WL, ...) ALAUNCH_N(name, kern, WL, kTile, ##__VA_ARGS__)

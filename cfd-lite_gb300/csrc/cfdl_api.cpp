@@ -233,12 +233,10 @@ int cfdl_set_config(cfdl_ctx *ctx, const cfdl_config *cfg) {
             if ((st = ensure_f32_assembly(hc, ctx->stream))) return st;
     std::vector<cfdl_config> old;
     std::vector<double> rho, mu;
-    bool reshape = false;                   // the solver tiles go by the precision
     try {
         size_t most = 0;
         for (const HostCase *hc : ctx->cases) {
             old.push_back(hc->cfg);
-            reshape |= hc->cfg.precision != cfg->precision;
             if (hc->cfg.rho != cfg->rho || hc->cfg.mu != cfg->mu) most = std::max(most, (size_t)hc->ne);
         }
         rho.assign(most, cfg->rho);
@@ -247,7 +245,8 @@ int cfdl_set_config(cfdl_ctx *ctx, const cfdl_config *cfg) {
         return CFDL_ERR_OOM;
     }
     for (HostCase *hc : ctx->cases) apply_config(hc, cfg);
-    st = reshape ? rebuild_worklists(ctx) : upload_case_table(ctx);
+    // the solver tiles go by the precision
+    st = solver_shape(ctx) == ctx->shape ? upload_case_table(ctx) : rebuild_worklists(ctx, false);
     if (st) {                               // the old parameters stand; the next call restores their lists
         for (size_t c = 0; c < old.size(); c++) apply_config(ctx->cases[c], &old[c]);
         ctx->lists_stale = true;
@@ -283,19 +282,8 @@ int cfdl_ctx_destroy(cfdl_ctx *ctx) {
     if (!ctx) return CFDL_ERR_INVALID;
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     for (HostCase *hc : ctx->cases) destroy_case(hc);
-    WorkList *wls[3] = {&ctx->cells, &ctx->faces, &ctx->halos};
-    for (WorkList *wl : wls) free_worklist(*wl);
-    free_worklist(ctx->cellsv);
-    free_worklist(ctx->cellse);
-    free_worklist(ctx->cellsr);
-    free_worklist(ctx->cellsem); free_worklist(ctx->cellss); free_worklist(ctx->cellsw); free_worklist(ctx->facesw);
-    free_worklist(ctx->facesv);
-    for (auto &wl : ctx->amg_cells) free_worklist(wl);
-    for (auto &wl : ctx->amg_smooth) free_worklist(wl);
-    for (auto &wl : ctx->amg_gcells) free_worklist(wl);
-    for (auto &wl : ctx->amg_gsmooth) free_worklist(wl);
-    for (auto &wl : ctx->amg_restr) free_worklist(wl);
-    for (auto &wl : ctx->amg_grestr) free_worklist(wl);
+    cudaFree(ctx->list_buf.d);
+    cudaFree(ctx->amg_list_buf.d);
     cudaFree(ctx->d_cases);
     cudaFree(ctx->d_partials);
     cudaFree(ctx->d_flags);
@@ -512,10 +500,10 @@ int cfdl_energy_init(cfdl_ctx *ctx, double cp, double tc, double t_init) {
     for (HostCase *hc : ctx->cases)
         if ((st = energy_init_case(ctx, hc, cp, tc, t_init))) break;
     // the device table follows the host records even after a failure part way
-    // (the solver tiles go by it too; graphs captured without, or with, the
-    // energy launches are dropped with the old lists)
-    int st2 = cuda_status(cudaStreamSynchronize(ctx->stream));
-    if (!st2) st2 = rebuild_worklists(ctx);
+    // (the solver tiles go by it too)
+    destroy_graph(ctx);   // graphs captured without (or with) the energy launches
+    int st2 = solver_shape(ctx) == ctx->shape ? upload_case_table(ctx) : rebuild_worklists(ctx, false);
+    if (st2) ctx->lists_stale = true;
     if (st) return st;
     if (st2) return st2;
     return cuda_status(cudaStreamSynchronize(ctx->stream));

@@ -39,9 +39,11 @@ int cuda_status(cudaError_t e) {
 // cfdl_fail_alloc: allocations of this thread until the one that fails (negative: none does)
 static thread_local int fail_alloc_in = -1;
 
+static bool alloc_fails() { return fail_alloc_in >= 0 && fail_alloc_in-- == 0; }
+
 int dev_alloc(void **p, size_t bytes) {
     *p = nullptr;
-    if (fail_alloc_in >= 0 && fail_alloc_in-- == 0) return CFDL_ERR_OOM;
+    if (alloc_fails()) return CFDL_ERR_OOM;
     cudaError_t e = cudaMalloc(p, bytes);
     if (e != cudaSuccess) { *p = nullptr; cudaGetLastError(); return cuda_status(e); }
     return CFDL_OK;
@@ -63,16 +65,9 @@ void destroy_case(HostCase *hc) {
     delete hc;
 }
 
-void free_worklist(WorkList &wl) {
-    cudaFree(wl.d_tiles); cudaFree(wl.d_case_first); cudaFree(wl.d_case_ntiles);
-    wl.d_tiles = nullptr; wl.d_case_first = nullptr; wl.d_case_ntiles = nullptr;
-    wl.ntiles = 0;
-    wl.rows = 0;
-}
-
 // Tile list over per-case entity counts (sizes[c] = 0 leaves case c out).
-int build_worklist(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &sizes, int tile) {
-    return build_worklist(ctx, wl, sizes, std::vector<int>(sizes.size(), tile));
+void plan_worklist(WorkList &wl, const std::vector<int> &sizes, int tile) {
+    plan_worklist(wl, sizes, std::vector<int>(sizes.size(), tile));
 }
 
 // Rows per thread of the fused momentum assembly, which has a reduction at its
@@ -100,8 +95,8 @@ static int rows_one_wave(int ne, int least) {
 // tiles: entities per tile of each case
 // per_thread: entities per thread and sub-tile of a merged list (0: the tile's)
 // split: blocks to a tile of a split list
-int build_worklist(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &sizes, const std::vector<int> &tiles, int per_thread, int split) {
-    free_worklist(wl);
+void plan_worklist(WorkList &wl, const std::vector<int> &sizes, const std::vector<int> &tiles, int per_thread, int split) {
+    wl.rows = 0;
     wl.h_tiles.clear(); wl.case_first.clear(); wl.case_ntiles.clear();
     for (size_t c = 0; c < sizes.size(); c++) {
         wl.case_first.push_back((int)wl.h_tiles.size());
@@ -114,18 +109,41 @@ int build_worklist(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &sizes, c
         wl.case_ntiles.push_back(cnt);
     }
     wl.ntiles = (int)wl.h_tiles.size();
-    size_t nt = std::max<size_t>(1, wl.h_tiles.size()), ncs = std::max<size_t>(1, sizes.size());
+}
+
+// The planned lists in one device buffer by one copy: a context has eleven of
+// them and up to six a multigrid level, and three allocations and copies for
+// each were most of what adding or removing a case took.  The buffer is
+// written over, so the stream is waited for first.
+int upload_worklists(cfdl_ctx *ctx, ListBuf &buf, const std::vector<WorkList *> &lists) {
+    auto up = [](size_t n) { return (n + 15) & ~(size_t)15; };
+    size_t total = 16;
+    for (const WorkList *wl : lists) total += up(wl->h_tiles.size() * sizeof(Tile)) + 2 * up(wl->case_first.size() * sizeof(int));
     int st;
-    if ((st = dev_alloc((void **)&wl.d_tiles, nt * sizeof(Tile)))) return st;
-    if ((st = dev_alloc((void **)&wl.d_case_first, ncs * sizeof(int)))) return st;
-    if ((st = dev_alloc((void **)&wl.d_case_ntiles, ncs * sizeof(int)))) return st;
-    if (!wl.h_tiles.empty()) {
-        if ((st = cuda_status(cudaMemcpy(wl.d_tiles, wl.h_tiles.data(), wl.h_tiles.size() * sizeof(Tile), cudaMemcpyHostToDevice)))) return st;
-        if ((st = cuda_status(cudaMemcpy(wl.d_case_first, wl.case_first.data(), wl.case_first.size() * sizeof(int), cudaMemcpyHostToDevice)))) return st;
-        if ((st = cuda_status(cudaMemcpy(wl.d_case_ntiles, wl.case_ntiles.data(), wl.case_ntiles.size() * sizeof(int), cudaMemcpyHostToDevice)))) return st;
+    if ((st = cuda_status(cudaStreamSynchronize(ctx->stream)))) return st;
+    if (total > buf.cap) {
+        char *d = nullptr;
+        const size_t cap = total + total / 2;
+        if ((st = dev_alloc((void **)&d, cap))) return st;
+        cudaFree(buf.d);
+        buf = {d, cap};
     }
-    (void)ctx;
-    return CFDL_OK;
+    if (alloc_fails()) return CFDL_ERR_OOM;     // the staging copy
+    std::vector<char> host(total, 0);
+    size_t at = 0;
+    auto put = [&](const void *p, size_t n) {
+        char *d = buf.d + at;
+        if (n) std::memcpy(host.data() + at, p, n);
+        at += up(n);
+        return d;
+    };
+    for (WorkList *wl : lists) {
+        wl->d_tiles = (Tile *)put(wl->h_tiles.data(), wl->h_tiles.size() * sizeof(Tile));
+        wl->d_case_first = (int *)put(wl->case_first.data(), wl->case_first.size() * sizeof(int));
+        wl->d_case_ntiles = (int *)put(wl->case_ntiles.data(), wl->case_ntiles.size() * sizeof(int));
+    }
+    if ((st = cuda_status(cudaMemcpyAsync(buf.d, host.data(), total, cudaMemcpyHostToDevice, ctx->stream)))) return st;
+    return cuda_status(cudaStreamSynchronize(ctx->stream));
 }
 
 void apply_config(HostCase *hc, const cfdl_config *cfg) {
@@ -481,13 +499,13 @@ int create_case(cfdl_ctx *ctx, const cfdl_mesh *m, const cfdl_config *cfg, HostC
 
 // A list of tiles of kTile * vec entities, M to a block: as many as bring the
 // context's blocks down to one wave (152 SMs, four CTAs each), at most kMaxMerge.
-static int build_merged(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &sizes, int vec) {
+static void plan_merged(WorkList &wl, const std::vector<int> &sizes, int vec) {
     const int rows = kTile * vec;
     long n = 0;
     for (int s : sizes) n += (s + rows - 1) / rows;
     const int M = (int)std::min<long>(kMaxMerge, std::max<long>(1, (n + 152 * 4 - 1) / (152 * 4)));
     wl.merge = {M, rows};
-    return build_worklist(ctx, wl, sizes, std::vector<int>(sizes.size(), rows * M), vec);
+    plan_worklist(wl, sizes, std::vector<int>(sizes.size(), rows * M), vec);
 }
 
 // The solver tiles of a small context, kSplit blocks to a tile (Tile::pad: the
@@ -496,51 +514,51 @@ static int build_merged(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &siz
 // iterations, split against whole tiles: FP64 at 32^3 cells 452 against 517 us,
 // 45^3 640 / 717, 53^3 (584 blocks) 759 / 766; FP32 assembly and solves at 24^3
 // 334 / 368, 45^3 (356 blocks) 526 / 529, 53^3 645 / 638.
-static int build_split(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &sizes) {
+static bool split_shape(const cfdl_ctx *ctx) {
     long n = 0;
-    for (int s : sizes) n += (s + kTile * kVec - 1) / (kTile * kVec);
+    for (const HostCase *hc : ctx->cases) n += (hc->ne + kTile * kVec - 1) / (kTile * kVec);
     const bool fp64 = !ctx->cases.empty() && ctx->cases[0]->cfg.precision == 0;
-    const bool on = ctx->vec == kVec && n * kSplit <= 152 * (fp64 ? 4 : 3);
-    return build_worklist(ctx, wl, on ? sizes : std::vector<int>(sizes.size(), 0), std::vector<int>(sizes.size(), kTile * kVec), 0, kSplit);
+    return ctx->vec == kVec && n * kSplit <= 152 * (fp64 ? 4 : 3);
+}
+
+SolverShape solver_shape(const cfdl_ctx *ctx) {
+    SolverShape s;
+    for (const HostCase *hc : ctx->cases)
+        s.tiles.push_back(kTile * (ctx->vec == kVec && flow_fp64(hc->dev) ? rows_one_wave(hc->ne, kVec) : ctx->vec));
+    s.split = split_shape(ctx);
+    return s;
 }
 
 // Tile work lists over every case of the context.
-static int rebuild_lists(cfdl_ctx *ctx) {
+static int rebuild_lists(cfdl_ctx *ctx, bool cases) {
     destroy_graph(ctx);   // captured launch arguments refer to the old lists
+    if (cases) ctx->amg_lmax = -1;       // ensure_amg plans the levels' lists again
     std::vector<int> nc, nfc, nh;
     for (const HostCase *hc : ctx->cases) { nc.push_back(hc->ne); nfc.push_back(hc->nf); nh.push_back(hc->nbf); }
-    int st;
-    if ((st = build_worklist(ctx, ctx->cells, nc))) return st;
-    if ((st = build_worklist(ctx, ctx->faces, nfc))) return st;
+    plan_worklist(ctx->cells, nc);
+    plan_worklist(ctx->faces, nfc);
     // four faces per thread where that still fills the chip (8 CTAs per SM): a
     // face pass of one face per thread spends a fifth of its time starting CTAs
     // (128^3: 24 000 of them; an outer iteration of precision 3 2888 us, with two
     // or four faces per thread 2867, with eight 2879; FP64 4424 and 4412).  A face
     // is computed by itself, so the bits do not depend on it.
-    if ((st = build_worklist(ctx, ctx->facesw, nfc, kTile * (ctx->faces.ntiles >= 4 * 8 * 152 ? 4 : 1)))) return st;
-    if ((st = build_worklist(ctx, ctx->facesv, nfc, kTile * kFaceVec))) return st;
-    if ((st = build_worklist(ctx, ctx->halos, nh))) return st;
+    plan_worklist(ctx->facesw, nfc, kTile * (ctx->faces.ntiles >= 4 * 8 * 152 ? 4 : 1));
+    plan_worklist(ctx->facesv, nfc, kTile * kFaceVec);
+    plan_worklist(ctx->halos, nh);
+    ctx->shape = solver_shape(ctx);
+    plan_worklist(ctx->cellsv, nc, ctx->shape.tiles);
+    plan_worklist(ctx->cellse, nc, kTile * ctx->en_vec);
+    plan_merged(ctx->cellsem, nc, ctx->en_vec);
+    plan_worklist(ctx->cellss, ctx->shape.split ? nc : std::vector<int>(nc.size(), 0), std::vector<int>(nc.size(), kTile * kVec), 0, kSplit);
     std::vector<int> tiles;
-    for (const HostCase *hc : ctx->cases)
-        tiles.push_back(kTile * (ctx->vec == kVec && flow_fp64(hc->dev) ? rows_one_wave(hc->ne, kVec) : ctx->vec));
-    if ((st = build_worklist(ctx, ctx->cellsv, nc, tiles))) return st;
-    if ((st = build_worklist(ctx, ctx->cellse, nc, kTile * ctx->en_vec))) return st;
-    if ((st = build_merged(ctx, ctx->cellsem, nc, ctx->en_vec))) return st;
-    if ((st = build_split(ctx, ctx->cellss, nc))) return st;
-    tiles.clear();
     for (int ne : nc) tiles.push_back(kTile * (ctx->vec == kVec ? rows_one_wave(ne, kVec) : ctx->vec));
-    if ((st = build_worklist(ctx, ctx->cellsw, nc, tiles))) return st;
+    plan_worklist(ctx->cellsw, nc, tiles);
     tiles.clear();
     for (int ne : nc) tiles.push_back(kTile * rows_per_thread(ne));
-    if ((st = build_worklist(ctx, ctx->cellsr, nc, tiles))) return st;
-    for (auto &wl : ctx->amg_cells) free_worklist(wl);
-    for (auto &wl : ctx->amg_smooth) free_worklist(wl);
-    for (auto &wl : ctx->amg_gcells) free_worklist(wl);
-    for (auto &wl : ctx->amg_gsmooth) free_worklist(wl);
-    for (auto &wl : ctx->amg_restr) free_worklist(wl);
-    for (auto &wl : ctx->amg_grestr) free_worklist(wl);
-    ctx->amg_cells.clear(); ctx->amg_smooth.clear(); ctx->amg_gcells.clear(); ctx->amg_gsmooth.clear();
-    ctx->amg_restr.clear(); ctx->amg_grestr.clear(); ctx->amg_lmax = -1;
+    plan_worklist(ctx->cellsr, nc, tiles);
+    int st = upload_worklists(ctx, ctx->list_buf, {&ctx->cells, &ctx->faces, &ctx->facesw, &ctx->facesv, &ctx->halos, &ctx->cellsv,
+                                                   &ctx->cellse, &ctx->cellsem, &ctx->cellss, &ctx->cellsw, &ctx->cellsr});
+    if (st) return st;
     // a case added since may have no 16-bit offsets (without multigrid ensure_amg does not look again)
     for (const HostCase *hc : ctx->cases) ctx->amg_nb16 = ctx->amg_nb16 && hc->dev.nb16;
     int need = std::max({ctx->cells.ntiles, ctx->faces.ntiles, ctx->halos.ntiles, ctx->cellss.ntiles,
@@ -568,11 +586,11 @@ static int rebuild_lists(cfdl_ctx *ctx) {
 // The lists and the case table from the cases as they are.  Until all of it is
 // done the context is stale: nothing is launched over lists that belong to
 // other cases or another precision.
-int rebuild_worklists(cfdl_ctx *ctx) {
+int rebuild_worklists(cfdl_ctx *ctx, bool cases) {
     ctx->lists_stale = true;
     int st;
     try {
-        st = rebuild_lists(ctx);
+        st = rebuild_lists(ctx, cases);
     } catch (const std::bad_alloc &) {
         st = CFDL_ERR_OOM;
     }
@@ -583,9 +601,7 @@ int rebuild_worklists(cfdl_ctx *ctx) {
 
 int check_ctx(cfdl_ctx *ctx) {
     if (!ctx || ctx->cases.empty()) return CFDL_ERR_INVALID;
-    if (!ctx->lists_stale) return CFDL_OK;
-    if (int st = cuda_status(cudaStreamSynchronize(ctx->stream))) return st;
-    return rebuild_worklists(ctx);
+    return ctx->lists_stale ? rebuild_worklists(ctx) : CFDL_OK;
 }
 
 int upload_case_table(cfdl_ctx *ctx) {

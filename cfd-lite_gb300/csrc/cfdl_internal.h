@@ -190,6 +190,7 @@ constexpr int kMixedRows = 8;           // most rows per thread of a mixed form'
 constexpr int kMaxMerge = 4;            // most tiles a block takes (a shared buffer holds their values)
 
 // One work list per entity type, with each case's tile range for reductions.
+// The device arrays lie in the ListBuf that the list was uploaded to.
 struct WorkList {
     int ntiles = 0;
     Merge merge{1, 1 << 30};            // merged lists: see merged_sums (cfdl_device.cuh)
@@ -198,6 +199,17 @@ struct WorkList {
     int rows = 0;                       // most entities per thread of a tile
     std::vector<Tile> h_tiles;
     std::vector<int> case_first, case_ntiles;
+};
+// Device memory of a set of work lists, kept while it is large enough
+struct ListBuf {
+    char *d = nullptr;
+    size_t cap = 0;
+};
+// What the solver lists' shape goes by beside the cases: cells per tile of cellsv, whether cellss is there
+struct SolverShape {
+    std::vector<int> tiles;
+    bool split = false;
+    bool operator==(const SolverShape &o) const { return tiles == o.tiles && split == o.split; }
 };
 
 // Host-side record of one case.
@@ -247,6 +259,8 @@ struct cfdl_ctx {
     cfdl::WorkList cellss;               // cellsv's tiles, split (empty where they are not: see split_sums)
     cfdl::WorkList facesw;               // face tiles of the passes bound by their CTAs' start: wider on large contexts
     cfdl::WorkList facesv;               // wide face tiles (kTile*kFaceVec faces) for face reductions
+    cfdl::ListBuf list_buf, amg_list_buf; // the lists above, and the multigrid levels'
+    cfdl::SolverShape shape;             // what cellsv and cellss were built for
     int en_vec = 1;                      // cells per thread in those tiles (autotuned with the energy equation)
     int last_iters_m = 0, last_iters_p = 0, last_iters_e = 0;   // previous inner iteration counts (poll scheduling)
     double *d_partials = nullptr;        // [max tiles][kNPart]
@@ -305,7 +319,8 @@ namespace cfdl {
 int cuda_status(cudaError_t e);
 int dev_alloc(void **p, size_t bytes);            // cudaMalloc, its status as a CFDL_* code
 int case_alloc(HostCase *hc, void **p, size_t bytes);
-int rebuild_worklists(cfdl_ctx *ctx);
+int rebuild_worklists(cfdl_ctx *ctx, bool cases = true);   // cases: they changed, and the multigrid lists with them
+SolverShape solver_shape(const cfdl_ctx *ctx);             // of the cases as they are now
 int check_ctx(cfdl_ctx *ctx);                     // a context with cases and lists that match them
 int upload_case_table(cfdl_ctx *ctx);
 int create_case(cfdl_ctx *ctx, const cfdl_mesh *mesh, const cfdl_config *cfg, HostCase **out);
@@ -429,9 +444,9 @@ void pressure_operators(cfdl_ctx *ctx, bool prepped);   // what the pressure sol
 int ensure_amg(cfdl_ctx *ctx);
 int solve_pressure_amg(cfdl_ctx *ctx);
 int solve_pressure_mixed(cfdl_ctx *ctx);
-void free_worklist(WorkList &wl);
-int build_worklist(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &sizes, int tile = kTile);
-int build_worklist(cfdl_ctx *ctx, WorkList &wl, const std::vector<int> &sizes, const std::vector<int> &tiles, int per_thread = 0, int split = 1);
+void plan_worklist(WorkList &wl, const std::vector<int> &sizes, int tile = kTile);
+void plan_worklist(WorkList &wl, const std::vector<int> &sizes, const std::vector<int> &tiles, int per_thread = 0, int split = 1);
+int upload_worklists(cfdl_ctx *ctx, ListBuf &buf, const std::vector<WorkList *> &lists);
 int read_stats(cfdl_ctx *ctx, int c, cfdl_stats *st);
 int poll_kind(cfdl_ctx *ctx, int kind, int *maxit);
 int poll_chunk(int done, int expected);

@@ -91,7 +91,7 @@ int cfdl_set_tile(cfdl_ctx *ctx, int vec) {
     int st = cuda_status(cudaStreamSynchronize(ctx->stream));
     if (st) return st;
     ctx->vec = vec;
-    return rebuild_worklists(ctx);
+    return rebuild_worklists(ctx, ctx->lists_stale);
 }
 
 int cfdl_get_tile(const cfdl_ctx *ctx) { return ctx ? ctx->vec : -1; }
@@ -102,7 +102,7 @@ int cfdl_set_energy_tile(cfdl_ctx *ctx, int vec) {
     int st = cuda_status(cudaStreamSynchronize(ctx->stream));
     if (st) return st;
     ctx->en_vec = vec;
-    return rebuild_worklists(ctx);
+    return rebuild_worklists(ctx, ctx->lists_stale);
 }
 
 int cfdl_get_energy_tile(const cfdl_ctx *ctx) { return ctx ? ctx->en_vec : -1; }

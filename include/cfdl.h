@@ -333,8 +333,8 @@ int cfdl_solve_pc_noalloc(int ne, int nh, const int *ef2nb1, const int *ef2nb_id
                           int *iters, double *rnorm);
 
 /* For tests of the out-of-memory paths: of the calling thread's device
- * allocations from now on, the n-th (counted from 0) is not made and its call
- * returns CFDL_ERR_OOM; negative (the state a thread starts in): none fails. */
+ * allocations (and staging buffers of work lists) from now on, the n-th
+ * (counted from 0) is not made and its call returns CFDL_ERR_OOM; negative (the state a thread starts in): none fails. */
 int cfdl_fail_alloc(int n);
 
 /* solve_uvwp runs as one CUDA graph (inner solve loops as device-side while

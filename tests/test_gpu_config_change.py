@@ -46,17 +46,18 @@ def _same(a, b):
             assert np.array_equal(a.case_get(c, f), b.case_get(c, f)), (c, f)
 
 
-def _until_it_succeeds(call, after):
-    """call() with its n-th allocation failing, n = 0, 1, ...; after() follows each failure."""
+def _until_it_succeeds(call, after, order=range(400)):
+    """call() with its n-th allocation failing, n in `order`; after(tries so far)
+    follows each failure.  Returns the failures."""
     L = cfdl.lib()
-    for n in range(400):
+    for failed, n in enumerate(order):
         L.cfdl_fail_alloc(C.c_int(n))
         status = call()
         L.cfdl_fail_alloc(C.c_int(-1))
         if status == 0:
-            return n
+            return failed
         assert status == OOM, (n, status)
-        after(n)
+        after(failed)
     raise AssertionError("never succeeded")
 
 
@@ -69,14 +70,16 @@ def test_set_config_out_of_memory(need_gpu):
     cfg = cfdl.steady(mu=0.02, precision=3)
 
     def after(n):
-        if n % 5 == 0:
+        if n in (0, 3, 7):
             for g in (a, b):
                 g.step(1, 0)
             _same(a, b)
 
     L = cfdl.lib()
-    failed = _until_it_succeeds(lambda: L.cfdl_set_config(b._h, C.byref(cfg)), after)
-    assert failed >= 6                       # three arrays of each case, at least
+    # a case keeps its three arrays once it has them: each of the first case's
+    # fails, then the second's first and each of them, then the lists
+    failed = _until_it_succeeds(lambda: L.cfdl_set_config(b._h, C.byref(cfg)), after, [0, 1, 2, 3] * 2 + [50])
+    assert failed == 8
     a.set_config(cfg)
     for g in (a, b):
         g.step(2, 0)
