@@ -1575,6 +1575,9 @@ int ensure_amg(cfdl_ctx *ctx) {
     for (auto *v : {&ctx->amg_cells, &ctx->amg_smooth, &ctx->amg_restr, &ctx->amg_gcells, &ctx->amg_gsmooth, &ctx->amg_grestr})
         for (WorkList &wl : *v) lists.push_back(&wl);
     int st = upload_worklists(ctx, ctx->amg_list_buf, lists);
+    // the tail's shared memory, once for the launches over these lists
+    if (!st) st = cuda_status(cudaFuncSetAttribute(k_v_tail<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailMaxSmem));
+    if (!st) st = cuda_status(cudaFuncSetAttribute(k_v_tail<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailMaxSmem));
     if (!st) st = upload_case_table(ctx);
     if (!st) ctx->amg_lmax = lmax;
     return st;
@@ -1611,7 +1614,6 @@ template <class T> static void launch_tail(cfdl_ctx *ctx) {
     for (const HostCase *hc : ctx->cases) smem = std::max(smem, sizeof(T) == 8 ? hc->tail_smem64 : hc->tail_smem32);
     const bool p_ = ctx->prof && prof_wants(ctx, "k_v_tail");
     if (p_) prof_begin(ctx, "k_v_tail");
-    cudaFuncSetAttribute(k_v_tail<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailMaxSmem);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(nc * kTailCtas));
     cfg.blockDim = dim3((unsigned)kTailBlock);
