@@ -258,10 +258,11 @@ int cfdl_set_config(cfdl_ctx *ctx, const cfdl_config *cfg) {
         if (cfg->precision == 3 && old[c].precision != 3) hc->g32_stale = hc->props_dirty = true;
         if (old[c].rho == cfg->rho && old[c].mu == cfg->mu) continue;
         hc->props_dirty = true;
-        if ((st = cuda_status(cudaMemcpy(hc->dev.rho, rho.data(), hc->ne * sizeof(double), cudaMemcpyHostToDevice)))) return st;
-        if ((st = cuda_status(cudaMemcpy(hc->dev.mu, mu.data(), hc->ne * sizeof(double), cudaMemcpyHostToDevice)))) return st;
+        const size_t n = hc->ne * sizeof(double);
+        if ((st = cuda_status(cudaMemcpyAsync(hc->dev.rho, rho.data(), n, cudaMemcpyHostToDevice, ctx->stream)))) return st;
+        if ((st = cuda_status(cudaMemcpyAsync(hc->dev.mu, mu.data(), n, cudaMemcpyHostToDevice, ctx->stream)))) return st;
     }
-    return CFDL_OK;
+    return cuda_status(cudaStreamSynchronize(ctx->stream));
 }
 
 int cfdl_upload_fields(cfdl_ctx *ctx, const cfdl_fields *f) {
@@ -694,7 +695,8 @@ int cfdl_case_set_run(cfdl_ctx *ctx, int id, int n_outer, int ncoef, double conv
         if ((st = cuda_status(cudaMemcpy(&S, hc->dev.sc, sizeof(S), cudaMemcpyDeviceToHost)))) return st;
         S.run_left = n_outer; S.outer_done = 0; S.ncoef = ncoef; S.halted = 0; S.time_due = 0; S.converged = 0;
         S.conv_tol = conv_tol; S.mip_abs = 0.0; S.mass_ratio = 0.0;
-        if ((st = cuda_status(cudaMemcpy(hc->dev.sc, &S, sizeof(S), cudaMemcpyHostToDevice)))) return st;
+        if ((st = cuda_status(cudaMemcpyAsync(hc->dev.sc, &S, sizeof(S), cudaMemcpyHostToDevice, ctx->stream)))) return st;
+        if ((st = cuda_status(cudaStreamSynchronize(ctx->stream)))) return st;
     }
     return CFDL_OK;
 }

@@ -114,13 +114,16 @@ void plan_worklist(WorkList &wl, const std::vector<int> &sizes, const std::vecto
 // The planned lists in one device buffer by one copy: a context has eleven of
 // them and up to six a multigrid level, and three allocations and copies for
 // each were most of what adding or removing a case took.  The buffer is
-// written over, so the stream is waited for first.
+// written over, so the stream is waited for first; and the default stream, on
+// which the cases' own arrays were filled: the context's stream does not wait
+// for it by itself.
 int upload_worklists(cfdl_ctx *ctx, ListBuf &buf, const std::vector<WorkList *> &lists) {
     auto up = [](size_t n) { return (n + 15) & ~(size_t)15; };
     size_t total = 16;
     for (const WorkList *wl : lists) total += up(wl->h_tiles.size() * sizeof(Tile)) + 2 * up(wl->case_first.size() * sizeof(int));
     int st;
     if ((st = cuda_status(cudaStreamSynchronize(ctx->stream)))) return st;
+    if ((st = cuda_status(cudaStreamSynchronize(cudaStreamLegacy)))) return st;
     if (total > buf.cap) {
         char *d = nullptr;
         const size_t cap = total + total / 2;

@@ -169,7 +169,7 @@ static int ensure_graph_state(cfdl_ctx *ctx) {
     if (!ctx->d_loop_passes) {
         const size_t bytes = kLoopSlots * sizeof(unsigned long long);
         if ((st = cuda_status(cudaMalloc(&ctx->d_loop_passes, bytes)))) return st;
-        if ((st = cuda_status(cudaMemset(ctx->d_loop_passes, 0, bytes)))) return st;
+        if ((st = cuda_status(cudaMemsetAsync(ctx->d_loop_passes, 0, bytes, ctx->stream)))) return st;
     }
     return CFDL_OK;
 }
