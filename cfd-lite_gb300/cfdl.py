@@ -166,6 +166,9 @@ def lib():
     L.cfdl_profile_get.argtypes = [vp, C.c_int, C.c_char_p, C.POINTER(C.c_int64), dp]
     L.cfdl_solve_pc_noalloc.argtypes = [C.c_int, C.c_int, vp, vp, vp, vp, vp, vp, C.c_double, C.c_int,
                                         ip, dp]
+    L.cfdl_solve_pc_noalloc_sms.argtypes = [C.c_int, C.c_int, vp, vp, vp, vp, vp, vp, C.c_double, C.c_int,
+                                            C.c_int, ip, dp]
+    L.cfdl_fail_alloc.argtypes = [C.c_int]
     L.cfdl_amg_info.argtypes = [vp, C.c_int, ip, vp, vp]
     L.cfdl_amg_index_bytes.argtypes = [vp]
     L.cfdl_set_graph_mode.argtypes = [vp, C.c_int]

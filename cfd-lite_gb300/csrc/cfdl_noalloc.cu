@@ -26,6 +26,8 @@
 // failure and leaves, and so do the others after it.
 #include "cfdl_internal.h"
 #include "cfdl_device.cuh"
+#include <algorithm>
+#include <climits>
 #include <cstddef>
 
 namespace cfdl {
@@ -36,7 +38,9 @@ constexpr int kNaMaxCtas = 512;                     // CTAs of a solve (their pa
 constexpr int kNaMinBlock = 128, kNaMaxBlock = 1024;
 constexpr int kNaW = 6;                             // couplings of a row kept in registers
 constexpr int kNaVals = 3;                          // values of the widest all-reduce
-constexpr int kNaPolls = 1 << 22;                   // about a second
+constexpr int kNaPolls = 1 << 22;                   // polls of a wait, about a second; and four for every half-face,
+                                                    // all of which may lie in the row that the others wait for
+constexpr int kNaRows = 8;                          // rows per thread where the SMs are too few for one
 
 struct NoAllocScratch {
     double z[kNaMaxCells], p[kNaMaxCells];          // what neighbouring rows read
@@ -77,7 +81,7 @@ template <int NT> struct NaShared {
 // CTA after.
 template <int K, int NT, class F>
 __device__ __forceinline__ bool na_all_sum(NoAllocScratch *S, NaShared<NT> &B, const double (&v)[K], unsigned step,
-                                           bool exchange, F fin) {
+                                           int polls, bool exchange, F fin) {
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nt = blockDim.x, n = gridDim.x;
     ulonglong2(*slot)[kNaMaxCtas] = S->slot[step & 1];
 #pragma unroll
@@ -115,8 +119,8 @@ __device__ __forceinline__ bool na_all_sum(NoAllocScratch *S, NaShared<NT> &B, c
             do {
                 asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(x) : "l"(&w->x) : "memory");
                 asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(y) : "l"(&w->y) : "memory");
-            } while (((x >> 32) != step || (y >> 32) != step) && ++it < kNaPolls);
-            ok = ok && it < kNaPolls;
+            } while (((x >> 32) != step || (y >> 32) != step) && ++it < polls);
+            ok = ok && it < polls;
             if (cta < NT) B.sm[k][cta] = __longlong_as_double((long long)(x << 32 | (y & 0xffffffffull)));
         }
     if (exchange) __threadfence();
@@ -146,7 +150,7 @@ __device__ __forceinline__ bool na_all_sum(NoAllocScratch *S, NaShared<NT> &B, c
 template <int R, int NT>
 __global__ void __launch_bounds__(NT) k_na_solve(NoAllocScratch *S, int ne, int nh, const int *ef1, const int *idx,
                                                  const double *ap, const double *anb, const double *b, double *phic,
-                                                 double rtol, int maxit) {
+                                                 double rtol, int maxit, int polls) {
     const int T = (int)(gridDim.x * blockDim.x), t0 = (int)(blockIdx.x * blockDim.x + threadIdx.x);
     __shared__ NaShared<NT> B;
     NaScalars &c = B.c;
@@ -183,7 +187,7 @@ __global__ void __launch_bounds__(NT) k_na_solve(NoAllocScratch *S, int ne, int 
         }
     }
     auto give_up = [&]() { S->fail = 3; };
-    if (!na_all_sum<1>(S, B, s1, ++step, false, [&](const double *s) { c.mean = s[0] / ne; })) { give_up(); return; }
+    if (!na_all_sum<1>(S, B, s1, ++step, polls, false, [&](const double *s) { c.mean = s[0] / ne; })) { give_up(); return; }
 #pragma unroll
     for (int u = 0; u < R; u++) {
         const int i = t0 + u * T;
@@ -194,7 +198,7 @@ __global__ void __launch_bounds__(NT) k_na_solve(NoAllocScratch *S, int ne, int 
         s3[0] += r[u] * r[u];
         s3[1] += r[u] * z[u];
     }
-    if (!na_all_sum<3>(S, B, s3, ++step, true, [&](const double *s) {
+    if (!na_all_sum<3>(S, B, s3, ++step, polls, true, [&](const double *s) {
             c.rz = s[1];
             c.rr = s[0];
             c.tol2 = rtol * rtol * s[0];
@@ -239,7 +243,7 @@ __global__ void __launch_bounds__(NT) k_na_solve(NoAllocScratch *S, int ne, int 
             s1[0] += p[u] * s;
         }
         first = false;
-        if (!na_all_sum<1>(S, B, s1, ++step, false, [&](const double *s) {
+        if (!na_all_sum<1>(S, B, s1, ++step, polls, false, [&](const double *s) {
                 // only runs while ||r|| is above the tolerance, where an SPD system has p.Ap > 0
                 if (!isfinite(s[0])) { c.fail = 1; c.active = 0; }
                 else if (!(s[0] > 0.0)) { c.fail = 2; c.active = 0; }
@@ -260,7 +264,7 @@ __global__ void __launch_bounds__(NT) k_na_solve(NoAllocScratch *S, int ne, int 
             s2[0] += r[u] * r[u];
             s2[1] += r[u] * z[u];
         }
-        if (!na_all_sum<2>(S, B, s2, ++step, true, [&](const double *s) {
+        if (!na_all_sum<2>(S, B, s2, ++step, polls, true, [&](const double *s) {
                 c.rr = s[0];
                 c.iters += 1;
                 c.beta = c.rz != 0.0 ? s[1] / c.rz : 0.0;
@@ -302,9 +306,9 @@ int na_scratch(NoAllocScratch **out) {
 
 using namespace cfdl;
 
-extern "C" int cfdl_solve_pc_noalloc(int ne, int nh, const int *ef2nb1, const int *ef2nb_idx, const double *ap,
-                                     const double *anb, const double *b, double *phic, double rtol, int maxit,
-                                     int *iters, double *rnorm) {
+// On at most max_sms SMs (0: all of the device's)
+static int na_solve(int ne, int nh, const int *ef2nb1, const int *ef2nb_idx, const double *ap, const double *anb,
+                    const double *b, double *phic, double rtol, int maxit, int max_sms, int *iters, double *rnorm) {
     if (ne <= 0 || nh <= 0 || !ef2nb1 || !ef2nb_idx || !ap || !anb || !b || !phic || !(rtol > 0) || maxit < 0)
         return CFDL_ERR_INVALID;
     if (ne > kNaMaxCells) return CFDL_ERR_TOO_LARGE;
@@ -314,19 +318,22 @@ extern "C" int cfdl_solve_pc_noalloc(int ne, int nh, const int *ef2nb1, const in
     int st = na_scratch(&S);
     if (st) return st;
     const cudaStream_t s0 = 0;
-    // about one CTA per SM; a device of fewer SMs than the rows need at one row
-    // a thread takes eight
+    // about one CTA per SM; where the SMs are fewer than the rows need at one row
+    // a thread, a thread takes eight (its rows spill: an iteration on 10 SMs has
+    // eight rows' loads in a chain anyway)
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return cuda_status(e);
+    if (max_sms > 0 && sms > max_sms) sms = max_sms;
     if (sms > kNaMaxCtas) sms = kNaMaxCtas;
-    const int rows = (long long)sms * kNaMaxBlock >= ne ? 1 : 8;
+    const int rows = (long long)sms * kNaMaxBlock >= ne ? 1 : kNaRows;
     const int threads = (ne + rows - 1) / rows;
     int block = ((threads + sms - 1) / sms + 31) & ~31;
     if (block < kNaMinBlock) block = kNaMinBlock;
-    if (block > kNaMaxBlock) return CFDL_ERR_CUDA;
+    if (block > kNaMaxBlock) return CFDL_ERR_TOO_LARGE;
     const int grid = (threads + block - 1) / block;
+    const int polls = (int)std::min<long long>(kNaPolls + 4LL * nh, INT_MAX);
     // step numbers start over with every call: no slot may hold one
     e = cudaMemsetAsync(S->slot, 0, sizeof(NoAllocScratch) - offsetof(NoAllocScratch, slot), s0);
     if (e != cudaSuccess) return cuda_status(e);
@@ -339,8 +346,8 @@ extern "C" int cfdl_solve_pc_noalloc(int ne, int nh, const int *ef2nb1, const in
     at[0].val.cooperative = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, rows > 1 ? k_na_solve<8, 1024> : block > 512 ? k_na_solve<1, 1024> : k_na_solve<1, 512>, S, ne, nh, ef2nb1, ef2nb_idx, ap, anb, b, phic,
-                           rtol, maxit);
+    e = cudaLaunchKernelEx(&cfg, rows > 1 ? k_na_solve<kNaRows, 1024> : block > 512 ? k_na_solve<1, 1024> : k_na_solve<1, 512>, S, ne, nh, ef2nb1,
+                           ef2nb_idx, ap, anb, b, phic, rtol, maxit, polls);
     struct { double rnorm, tol; int iters, bad, fail; } end = {};
     static_assert(offsetof(NoAllocScratch, fail) == offsetof(NoAllocScratch, rnorm) + 24, "the end record is copied whole");
     if (e == cudaSuccess)
@@ -355,4 +362,17 @@ extern "C" int cfdl_solve_pc_noalloc(int ne, int nh, const int *ef2nb1, const in
     if (end.fail == 2) return CFDL_ERR_BREAKDOWN;
     if (end.rnorm > end.tol) return CFDL_ERR_ITER_CAP;       // stopped at maxit above the tolerance
     return CFDL_OK;
+}
+
+extern "C" int cfdl_solve_pc_noalloc(int ne, int nh, const int *ef2nb1, const int *ef2nb_idx, const double *ap,
+                                     const double *anb, const double *b, double *phic, double rtol, int maxit,
+                                     int *iters, double *rnorm) {
+    return na_solve(ne, nh, ef2nb1, ef2nb_idx, ap, anb, b, phic, rtol, maxit, 0, iters, rnorm);
+}
+
+extern "C" int cfdl_solve_pc_noalloc_sms(int ne, int nh, const int *ef2nb1, const int *ef2nb_idx, const double *ap,
+                                         const double *anb, const double *b, double *phic, double rtol, int maxit,
+                                         int sms, int *iters, double *rnorm) {
+    if (sms < 1) return CFDL_ERR_INVALID;
+    return na_solve(ne, nh, ef2nb1, ef2nb_idx, ap, anb, b, phic, rtol, maxit, sms, iters, rnorm);
 }

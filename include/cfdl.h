@@ -325,12 +325,25 @@ int cfdl_probe_fp64(double *fma_per_s, double *ms);
  * CFDL_ERR_ITER_CAP when CG stopped at maxit above it (as cfdl_solve_pc in
  * tight mode); CFDL_ERR_BREAKDOWN when p.Ap <= 0 above it; CFDL_ERR_NONFINITE
  * for a non-finite value (a zero diagonal entry, say); CFDL_ERR_INVALID for an
- * index outside the arrays (that access is skipped on the device). */
+ * index outside the arrays (that access is skipped on the device).  phic is
+ * written in all of these cases.  The solve is one cooperative launch whose
+ * CTAs wait for one another, each wait bounded (about a second, longer with
+ * many half-faces).  CFDL_ERR_CUDA, with phic unwritten: a wait ran out, or the
+ * launch was refused (the CTAs do not fit the device together, say because
+ * another process's share of it is limited); CFDL_ERR_TOO_LARGE also for a
+ * device of fewer than ne / 8192 SMs.
+ *
+ * cfdl_solve_pc_noalloc_sms is the same on at most `sms` SMs, which leaves the
+ * others to other work; with fewer than ne / 1024 of them a thread takes eight
+ * rows, and with fewer than ne / 8192 the call returns CFDL_ERR_TOO_LARGE. */
 #define CFDL_ERR_TOO_LARGE      9
 #define CFDL_NOALLOC_MAX_CELLS  131072
 int cfdl_solve_pc_noalloc(int ne, int nh, const int *ef2nb1, const int *ef2nb_idx, const double *ap,
                           const double *anb, const double *b, double *phic, double rtol, int maxit,
                           int *iters, double *rnorm);
+int cfdl_solve_pc_noalloc_sms(int ne, int nh, const int *ef2nb1, const int *ef2nb_idx, const double *ap,
+                              const double *anb, const double *b, double *phic, double rtol, int maxit,
+                              int sms, int *iters, double *rnorm);
 
 /* For tests of the out-of-memory paths: of the calling thread's device
  * allocations (and staging buffers of work lists) from now on, the n-th
