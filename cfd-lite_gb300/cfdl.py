@@ -168,6 +168,7 @@ def lib():
                                         ip, dp]
     L.cfdl_solve_pc_noalloc_sms.argtypes = [C.c_int, C.c_int, vp, vp, vp, vp, vp, vp, C.c_double, C.c_int,
                                             C.c_int, ip, dp]
+    L.cfdl_set_tail_smem.argtypes = [vp, C.c_int]
     L.cfdl_fail_alloc.argtypes = [C.c_int]
     L.cfdl_amg_info.argtypes = [vp, C.c_int, ip, vp, vp]
     L.cfdl_amg_index_bytes.argtypes = [vp]

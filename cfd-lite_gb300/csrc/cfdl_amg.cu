@@ -1385,7 +1385,9 @@ int prepare_case_amg(CasePrep *p) {
 }
 
 // The plan of a case's tail for one precision.
-template <class T> static int build_tail_plan(const HostCase *hc, const AmgLevelDev *lev, TailPlan &plan, int *smem) {
+// limit: the shared memory it may take.
+template <class T> static int build_tail_plan(const HostCase *hc, const AmgLevelDev *lev, TailPlan &plan, int *smem,
+                                              int limit = kTailMaxSmem) {
     const CaseDev &d = hc->dev;
     const int lt = d.amg_tail, nl = d.nlev - lt;
     constexpr int sz = (int)sizeof(T);
@@ -1428,13 +1430,13 @@ template <class T> static int build_tail_plan(const HostCase *hc, const AmgLevel
     }
     for (int l = nl - 1; l >= 0; l--) {                    // the small levels first: the tail level takes what is left
         TailLevel &v = P->lv[l];
-        const int room = kTailMaxSmem - at - 32, per = v.R * (sz + 4);
+        const int room = limit - at - 32, per = v.R * (sz + 4);
         v.S = std::min(lev[lt + l - 1].W, room > 0 ? room / per : 0);
         v.sa = take((long)v.R * v.S * sz);
         v.snb = take(4L * v.R * v.S);
     }
     P->total = at;
-    if (at > kTailMaxSmem) return CFDL_ERR_MESH;           // cannot happen (see TailPlan)
+    if (at > limit) return CFDL_ERR_MESH;                  // cannot happen with kTailMaxSmem (see TailPlan)
     *smem = at;
     return CFDL_OK;
 }
@@ -2137,4 +2139,34 @@ extern "C" int cfdl_amg_info(cfdl_ctx *ctx, int maxlev, int *nlev, int *n, int *
         if (W) W[l] = l == 0 ? hc->W : hc->amg->levels[l - 1].W;
     }
     return CFDL_OK;
+}
+
+extern "C" int cfdl_set_tail_smem(cfdl_ctx *ctx, int bytes) {
+    using namespace cfdl;
+    int st = check_ctx(ctx);
+    if (st) return st;
+    if (bytes < 0 || ctx->cases[0]->cfg.precond != 1) return CFDL_ERR_INVALID;
+    if ((st = ensure_amg(ctx))) return st;
+    const int limit = bytes == 0 || bytes > kTailMaxSmem ? kTailMaxSmem : bytes;
+    std::vector<TailPlan> plans(2 * ctx->cases.size());
+    std::vector<int> smem(2 * ctx->cases.size());
+    for (size_t c = 0; c < ctx->cases.size(); c++) {
+        const HostCase *hc = ctx->cases[c];
+        std::vector<AmgLevelDev> lev(hc->dev.nlev);
+        if (!lev.empty() && (st = cuda_status(cudaMemcpy(lev.data(), hc->dev.lev, lev.size() * sizeof(AmgLevelDev), cudaMemcpyDeviceToHost))))
+            return st;
+        if (build_tail_plan<double>(hc, lev.data(), plans[2 * c], &smem[2 * c], limit) ||
+            build_tail_plan<float>(hc, lev.data(), plans[2 * c + 1], &smem[2 * c + 1], limit))
+            return CFDL_ERR_INVALID;                       // less than the plans need beside the slots
+    }
+    if ((st = cuda_status(cudaStreamSynchronize(ctx->stream)))) return st;
+    destroy_graph(ctx);                                    // captured launches carry the size
+    for (size_t c = 0; c < ctx->cases.size(); c++) {
+        HostCase *hc = ctx->cases[c];
+        if ((st = cuda_status(cudaMemcpyAsync((void *)hc->dev.tail64, &plans[2 * c], 2 * sizeof(TailPlan), cudaMemcpyHostToDevice, ctx->stream))))
+            return st;
+        hc->tail_smem64 = smem[2 * c];
+        hc->tail_smem32 = smem[2 * c + 1];
+    }
+    return cuda_status(cudaStreamSynchronize(ctx->stream));
 }

@@ -345,6 +345,13 @@ int cfdl_solve_pc_noalloc_sms(int ne, int nh, const int *ef2nb1, const int *ef2n
                               const double *anb, const double *b, double *phic, double rtol, int maxit,
                               int sms, int *iters, double *rnorm);
 
+/* Shared memory that the V-cycle's tail kernel may take per CTA (0: the default,
+ * 200 KB, which the slots of every hierarchy met so far fit): the last slots of
+ * the largest levels that do not fit are read from global memory at every
+ * step.  Builds the multigrid set-up if it is not there; cases added later
+ * have the default.  CFDL_ERR_INVALID, and nothing changed, when the rest of
+ * the plan alone needs more, or without multigrid. */
+int cfdl_set_tail_smem(cfdl_ctx *ctx, int bytes);
 /* For tests of the out-of-memory paths: of the calling thread's device
  * allocations (and staging buffers of work lists) from now on, the n-th
  * (counted from 0) is not made and its call returns CFDL_ERR_OOM; negative (the state a thread starts in): none fails. */
