@@ -4,6 +4,7 @@
 // the header for the citation of each.  All work is queued on the context's
 // stream; entry points that return results to the host synchronise it.
 #include "cfdl_internal.h"
+#include "cfdl_amg.h"
 #include <cmath>
 #include <cstring>
 #include <new>
@@ -680,6 +681,10 @@ size_t cfdl_case_bytes_estimate(int ne, int nf, int nbf, int W) {
     bytes += 160 * c + w * c * 2;                     // multigrid hierarchy (bound), 16-bit mesh offsets
     bytes += 9 * c * 4 + 3 * w * c * 4 + 7 * f * 4;   // precision 3 FP32 gradients, stencil, face planes
     bytes += w * c * 12 + c * 32;                     // the pressure matrix's own storage and FP32 copies
+    // what does not grow with the mesh: the coarsest inverse (FP64 and FP32), the
+    // tail's plans, scalars and counters, allocations of a few bytes
+    const size_t m = std::min<size_t>(ne, kAmgCoarsest);
+    bytes += 12 * m * m + 2 * sizeof(TailPlan) + 5120;
     return bytes;
 }
 
