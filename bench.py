@@ -403,7 +403,7 @@ def fp64_roofline(cfdl, prof, ne, nf, nbf, W, peaks):
         return {"unavailable": str(e)[:200]}
     rows = {}
     for k, (launches, ms) in sorted(prof.items(), key=lambda kv: -kv[1][1]):
-        inst = fp64_inst(k, ne, nf, nbf, W)
+        inst = fp64_inst(k, ne, nf, nbf, W, "flow")
         if not inst or not launches:
             continue
         t = ms / launches / 1e3
