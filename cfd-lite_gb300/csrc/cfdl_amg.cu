@@ -14,7 +14,7 @@
 //   level l+1 -> l   prolongation (injection, scaled by kOverCorrect) added
 //                    in place, then two damped-Jacobi sweeps;
 //   small levels     a case's levels of at most kTailRows rows and its
-//                    coarsest solve run in one CTA (k_v_tail).
+//                    coarsest solve run on one cluster of CTAs (k_v_tail).
 // Pre- and post-smoothing match, so the preconditioner is symmetric and
 // positive semi-definite, as CG requires.  The coarse operators are rebuilt
 // at every pressure solve from the current coefficients (A_c = P^T A P).
@@ -408,7 +408,6 @@ __global__ void __launch_bounds__(kTile) k_amg_prep0(const CaseDev *__restrict__
 // two barriers and a quotient; 256, 512 and 1024 threads measure the same.
 // With the matrix in shared memory the 37-row inverse of the 128^3 cavity
 // took 77 us and the 8-row one of the 24^3 cavity 17; this takes 55 and 11.7.
-// The same with a branch per kind of entry took 101.
 constexpr int kInvThreads = 256;
 __global__ void __launch_bounds__(kInvThreads) k_amg_coarse_inv(const CaseDev *__restrict__ cases, int ncases) {
     CFDL_PDL_WAIT();
@@ -514,14 +513,16 @@ __global__ void __launch_bounds__(kTile) k_v_jac(const CaseDev *__restrict__ cas
     // the row's own values first: measured faster on the coarse levels
     y[i] = jacobi_step<T, kToT ? 1 : 2>(x[i], P.r[i], P.rd[i], offsum<T>(P, x, i));
 }
-// The FP64 mesh-level sweeps are bound by their FP64 instructions: 4.5 us each
-// per 2.1M rows, whatever the launch shape or the index width.  Eight per row
-// of six slots: the sum starts from r, and the second sweep's w2/D is a plane
-// of its own (rap2_p) instead of w/D times w2/w (ten: 45.7 us at 128^3; eight: 43.1).
+// The FP64 mesh-level sweeps wait for two things at once: the FP64 pipe is 65%
+// busy (eight instructions a row of six slots take 26.7 of 40.3 us at 128^3) and
+// the algorithmic bytes move at 0.8 of the copy bandwidth.  Neither the launch
+// shape nor the index width changed their time; two instructions a row fewer
+// did (45.7 -> 43.1 us): the sum starts from r, and the second sweep's w2/D is a
+// plane of its own (rap2_p) instead of w/D times w2/w.
 // 32 registers, 8 CTAs per SM: the coarse levels' sweeps would spill 100+
 // bytes under that cap, so these are kernels of their own.
-// The roundings of both launch shapes, spelled out: a case has the same result
-// alone and in a batch, whichever shape its launch takes.
+// The roundings of both launch shapes are spelled out, so a case's result does
+// not depend on the shape its launch takes.
 __device__ __forceinline__ double sweep64(double om, double x, double w, double s) { return __fma_rn(w, s, __dmul_rn(om, x)); }
 __device__ __forceinline__ double resid64(double r, double d, double z) { return __fma_rn(-d, z, r); }
 template <bool kToT>
@@ -748,7 +749,7 @@ __global__ void __launch_bounds__(kTile) k_v_restrict(const CaseDev *__restrict_
 // indices and then kCh values loaded side by side (one by one, each entry was
 // two trips to L2: at 128^3 the large levels took 79 us on average and now
 // take 71 with kCh = 2, the small ones 35 and now 26 with 8; at 24^3 13.2 and
-// 9.8.  A warp per row on the small levels took 30 and 11.6).
+// 9.8).
 template <int kCh>
 __device__ __forceinline__ double gather_sum(const double *__restrict__ af, const int *__restrict__ src, int q0, int q1) {
     double v = 0.0;
@@ -1563,7 +1564,10 @@ int ensure_amg(cfdl_ctx *ctx) {
         plan_worklist(ctx->amg_smooth[l], smooth);
         plan_worklist(ctx->amg_restr[l], restr);
         // lanes per row: 8 when every case's level is small, else the tuned
-        // cgroup (1 = one thread per row); the mesh level is always 1
+        // cgroup (1 = one thread per row); the mesh level is always 1.  The
+        // lanes order a row's sum, and they go by the context's largest case: a
+        // small case beside one whose level has kGroupedRows rows or more does
+        // not have the bits it has alone
         const int nmax = *std::max_element(cells.begin(), cells.end());
         const int G = l == 0 ? 1 : nmax < kGroupedRows ? kG : ctx->cgroup;
         ctx->amg_grouped[l] = G;
@@ -1682,7 +1686,7 @@ template <class T> static void vcycle(cfdl_ctx *ctx) {
     const int L = ctx->amg_lmax;
     // the FP32 mesh-level kernels read 16-bit neighbour offsets when every
     // case has them: 52 B a row instead of 64, 19% faster at 128^3; the FP64
-    // sweeps are bound by their FP64 instructions and keep int32
+    // sweeps did not gain by them and keep int32
     const bool n16 = ctx->amg_nb16;
     for (int l = 0; l < L; l++) {
         int G = ctx->amg_grouped[l];

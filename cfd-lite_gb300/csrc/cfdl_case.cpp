@@ -76,7 +76,7 @@ void plan_worklist(WorkList &wl, const std::vector<int> &sizes, int tile) {
 // leaves idle; else two: the block's reduction against the last wave (128^3, an
 // outer iteration of precision 3: 2926 us with one, 2915 with two, 2924 with
 // four or seven; tets of 45^3, 1367, 1365, 1371).  It goes by the case alone, so
-// a case's sums are the same alone and in a batch.
+// these sums are the same alone and in a batch.
 static int rows_per_thread(int ne) { return ne <= 152 * 4 * kTile ? 1 : 2; }
 
 // Rows per thread of the FP64 solver passes: at least `least`, and on large

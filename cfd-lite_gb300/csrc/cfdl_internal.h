@@ -370,9 +370,10 @@ bool energy_on(const cfdl_ctx *ctx);          // some case of the context has it
 // fastest.  The energy solve stops after a set number of iterations, on fine
 // meshes far from its solution, and its iterates amplify a rounding difference
 // in the fluxes by up to 1e10 (84^3 cells, Re 100: 1e-14 in u became 1e-4 in T),
-// so a case with the energy equation keeps the one order of precision 1.  A
-// context may hold cases of both kinds: each kind has its launch, which passes
-// over the other's tiles.
+// so a case with the energy equation keeps the one order of precision 1 (but for
+// the coarse multigrid levels' lanes per row, which go by the context's largest
+// case: ensure_amg).  A context may hold cases of both kinds: each kind has its
+// launch, which passes over the other's tiles.
 __host__ __device__ inline bool flow_fp64(const CaseDev &C) { return C.precision == 0 && !C.ee; }
 bool any_flow_fp64(const cfdl_ctx *ctx);      // some case is of the first kind
 bool any_ordered(const cfdl_ctx *ctx);        // some case is not

@@ -60,10 +60,10 @@ __global__ void __launch_bounds__(kTile) k_bc(const CaseDev *__restrict__ cases,
 // the neighbour takes them with the opposite sign.  Boundary faces: the wall
 // diffusion mu*area/ds of the BC loop (mod_uvwp.f90:257).
 // ---------------------------------------------------------------------------
-// Bound by the FP64 pipe (4.5 us per instruction and 2.1M faces).  kFast
-// (flow_fp64): interpolation as go + wt (gn - go) and each component's six
-// products as one chain, 36 FP64 instructions a face instead of 40
-// (445 -> 392 us at 128^3); the others keep the one order on which the mixed
+// Bound by the FP64 pipe, 92% busy.  kFast (flow_fp64): interpolation as
+// go + wt (gn - go) and each component's six products as one chain, 36 FP64
+// instructions a face instead of 40 (445 -> 392 us at 128^3, of which the
+// instructions take 358 at the pipe's measured rate); the others keep the one order on which the mixed
 // forms' FP32 roundings and the energy solve depend.
 template <bool kFast>
 __global__ void __launch_bounds__(kTile) k_coef_uvw_face(const CaseDev *__restrict__ cases, const Tile *__restrict__ tiles) {
@@ -289,14 +289,14 @@ __global__ void __launch_bounds__(kTile) k_coef_uvw_cell(const CaseDev *__restri
 // sums from the first slot and skip the boundary terms, and sum b'^2 is formed
 // in tight mode only (otherwise it is only asked whether it is finite, see
 // kBigExp).  FORM 0 (flow_fp64) also takes the Jacobi scaling from the
-// reciprocal behind d (rcp_near) and chains its sums.  FORM 1 (precision 1 and 2, and FP64 with the energy equation) and 3 (FP32
-// explicit face terms) keep every rounding of the two kernels, spelled out
-// where the compiler could contract either of two products (div_rn rounds as
-// the division does).  At four CTAs per SM it
-// spills, and is still faster than at three or two without (128^3, an outer
-// iteration: FP64 4.635 ms against 4.643 and 4.679, precision 3 2.996 against
-// 3.015 and 3.031).  The two
-// kernels took 543 us FP64 and 483 in precision 3, this one 440 and 456.
+// reciprocal behind d (rcp_near) and chains its sums.  FORM 1 (precision 1 and
+// 2, and FP64 with the energy equation) and 3 (FP32 explicit face terms) keep
+// every rounding of the two kernels, spelled out where the compiler could
+// contract either of two products (div_rn rounds as the division does).  At four
+// CTAs per SM it spills, and is still faster than at three or two without (128^3,
+// an outer iteration: FP64 4.635 ms against 4.643 and 4.679, precision 3 2.996
+// against 3.015 and 3.031).  The two kernels took 543 us FP64 and 483 in
+// precision 3, this one 458 and 428, the FP64 pipe 85 and 83% busy.
 constexpr int kBigExp = 1023 + 400;     // |b'| below 2^400: no sum of squares of fewer than 2^31 rows overflows
 __device__ __forceinline__ bool is_big(double x) { return ((int)((unsigned long long)__double_as_longlong(x) >> 52) & 0x7ff) >= kBigExp; }
 

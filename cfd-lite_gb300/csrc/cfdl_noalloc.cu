@@ -16,7 +16,7 @@
 // took 24 us an iteration at 729 rows, 28 at 64000 and 33 at 125000.  Here a
 // thread owns a row: its coefficients, x, r, z and p stay in registers, and an
 // iteration is two all-reduces with one exchange of z and p through L2 between
-// them: 7.0, 13.5 and 15.8 us.  About one CTA per SM, so that every SM's FP64
+// them: 7.0 to 7.5, 12.9 to 14.2 and 15.5 us (by the board).  About one CTA per SM, so that every SM's FP64
 // pipe (2 instructions per clock) takes an equal share.
 //
 // An all-reduce is barrier and sum in one: each CTA publishes its partials as
@@ -60,9 +60,9 @@ struct NaScalars {
     int iters, bad, fail, active;
 };
 // r / d, correctly rounded, from rd = 1 / d as div_rn takes it; rd = 0: d is out
-// of its range, divide.  The product r rd took 0.3 to 0.4 us less an iteration (729
-// to 125000 rows), with one rounding more, and left a system with subnormal
-// diagonal entries unsolved.
+// of its range, divide.  The product r rd took up to 0.5 us less an iteration
+// (64000 rows; on another board nothing at 729 and 125000), with one rounding
+// more, and left a system with subnormal diagonal entries unsolved.
 __device__ __forceinline__ double na_quotient(double r, double d, double rd) {
     if (__double2hiint(rd) == 0) return r / d;          // an integer test: the FP64 pipe is what an iteration waits for
     const double q = r * rd;

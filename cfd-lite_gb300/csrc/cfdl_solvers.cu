@@ -8,9 +8,9 @@
 //   momentum  Jacobi-preconditioned BiCGStab on the three components at once
 //             (one matrix, three right-hand sides, independent scalars);
 //   pressure  Jacobi-preconditioned CG on the singular Neumann system with
-//             its right-hand side projected to zero mean (cfdl_precond.cu adds
-//             the aggregation-AMG preconditioner and cfdl_mixed.cu the mixed-
-//             precision form).
+//             its right-hand side projected to zero mean (cfdl_amg.cu adds
+//             the aggregation-AMG preconditioner and the mixed-precision
+//             form).
 // Stopping: solve_mode 0 stops a component when ||r||2 <= rtol*||r0||2 (the
 // reference's 10x drop with rtol = 0.1) or after nit iterations; solve_mode 1
 // (tight, parity) stops at ||r||2 <= tight_rtol*||b||2.
