@@ -13,7 +13,7 @@ form "flow": FP64 flow without the energy equation, the default benchmark
 
   k_coef_uvw_face  36 per interior face
   k_calc_mip       23 per interior face (9 without the Rhie-Chow term)
-  k_coef_uvw_init  99.8, and 164 per wall face: a warp with a wall cell among
+  k_coef_uvw_init  99.8, and 164 per wall face, fitted to both sizes: a warp with a wall cell among
                    its 32 goes through the boundary terms with all its lanes,
                    half of the warps at 128^3
   k_mom_*          BiCGStab with three active right-hand sides, with the
